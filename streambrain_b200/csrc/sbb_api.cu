@@ -611,6 +611,7 @@ int update_mask_t(uint8_t *wmask, const void *weights, const void *Ci, const voi
   SBB_TRY(dcj.upload(Cj, M * s));
   SBB_TRY(dcij.upload(Cij, N * M * s));
   SBB_TRY(score.alloc(sbb::mask_scratch_bytes(N, s)));
+  SBB_CUDA(sbb::mask_scratch_init(score.d, 0));
   SBB_CUDA(sbb::launch_mask_update<T>(dm.as<uint8_t>(), dw.as<T>(), dci.as<T>(), dcj.as<T>(), dcij.as<T>(), (T)cthr, N,
                                       M, H, Mc, h, iterations, score.d, 0));
   SBB_CUDA(cudaDeviceSynchronize());
@@ -751,6 +752,7 @@ int sbb_layer_create(const sbb_layer_desc *desc, sbb_layer **out) {
   if (rc == SBB_OK) rc = L->rc.reserve(sbb::tc_trace_scratch_bytes(L->N, L->M));
   if (rc == SBB_OK && desc->kind == SBB_LAYER_PLASTIC) {
     rc = L->score.reserve(sbb::mask_scratch_bytes(L->N, s));
+    if (rc == SBB_OK && (e = sbb::mask_scratch_init(L->score.d, 0)) != cudaSuccess) rc = cuda_fail(e, "layer_create");
     if (rc == SBB_OK) rc = L->col_hc.reserve((size_t)(L->M + 4) * sizeof(int));
     if (rc == SBB_OK) {
       std::vector<int> hc((size_t)L->M);
@@ -1274,7 +1276,7 @@ int shard_train(sbb_layer *L, long B, long h, cudaStream_t st) {
                                                   static_cast<T *>(L->state[SBB_STATE_KBI]), Cj, (T)cthr,
                                                   (T)L->desc.khalf, (T)L->desc.pmin, (T)L->desc.taubdt, M, st));
   if (h >= 0 && nr > 0)   // scores of the owned rows, into every rank's work arrays
-    SBB_CUDA(sbb::launch_mask_score_rows<T>(wmask, Ci, Cj, Cij, (T)cthr, N, M, L->H, L->Mc, h, rb, re,
+    SBB_CUDA(sbb::launch_mask_score_rows<T>(wmask, nullptr, Ci, Cj, Cij, (T)cthr, N, M, L->H, L->Mc, h, rb, re,
                                             shard_table(L, kShardMask, 0), st));
   return SBB_OK;
 }
@@ -1338,7 +1340,10 @@ int sbb_layer_shard_init(sbb_layer *L, long rank, long world_size, long max_loca
   // every rank allocates a full block's width, so that the buffers have one size everywhere
   const size_t xg_bytes = (size_t)world_size * max_local_batch * S.rows_per_rank * s;
   for (auto &b : S.xg) SBB_TRY(b.reserve(xg_bytes));
-  if (L->score.d == nullptr) SBB_TRY(L->score.reserve(sbb::mask_scratch_bytes(L->N, s)));
+  if (L->score.d == nullptr) {
+    SBB_TRY(L->score.reserve(sbb::mask_scratch_bytes(L->N, s)));
+    SBB_CUDA(sbb::mask_scratch_init(L->score.d, 0));
+  }
   for (int b = 0; b < SBB_SHARD_BUFFERS; ++b)
     for (int r = 0; r < 8; ++r) {
       S.peer[b][r] = nullptr;

@@ -1172,632 +1172,6 @@ cudaError_t launch_apply_mask(T *w, const uint8_t *wmask, long N, long M, long H
 template cudaError_t launch_apply_mask<float>(float *, const uint8_t *, long, long, long, long, cudaStream_t);
 template cudaError_t launch_apply_mask<double>(double *, const uint8_t *, long, long, long, long, cudaStream_t);
 
-// ----------------------------------------------------------------------------
-// Structural plasticity: score, swap, rewrite.
-// ----------------------------------------------------------------------------
-// One warp per input row: the mutual-information score numerator over the
-// minicolumns of hypercolumn h (terms in REAL, accumulated in double) and the
-// row's count of active connections.
-template <typename T>
-__global__ void __launch_bounds__(256)
-    mask_score_kernel(const uint8_t *__restrict__ wmask, const T *__restrict__ weights, const T *__restrict__ Ci,
-                      const T *__restrict__ Cj, const T *__restrict__ Cij, T cthr, T cthr4, long N, long M, long H,
-                      long Mc, long h, T *score, int *csum, uint8_t *old_col) {
-  const int lane = threadIdx.x & 31;
-  const long i = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= N) return;  // whole warp leaves together
-  // Every load of the row (its trace, the mask bytes, the trace block) is issued before the first use of any of
-  // them: the loads do not depend on the row's trace value, only the arithmetic does, so the warp pays one
-  // memory round trip instead of three.
-  const T pi = Ci[i];
-  int cnt = 0;
-  for (long k = lane; k < H; k += 32) cnt += wmask[i * H + k];
-  double s = 0.0;
-  // four strided elements per lane at a time, all loads issued before the arithmetic
-  for (long j0 = 0; j0 < Mc; j0 += 128) {
-    T pj[4], pij[4], wv[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const long jj = j0 + lane + 32 * u, col = h * Mc + jj;
-      const bool in = jj < Mc;
-      pj[u] = in ? Cj[col] : (T)0;
-      pij[u] = in ? Cij[i * M + col] : (T)0;
-      wv[u] = (in && weights) ? weights[i * M + col] : (T)0;
-    }
-    if (pi >= cthr) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (j0 + lane + 32 * u < Mc && pj[u] >= cthr) {
-          const T w = weights ? wv[u] : log_ratio(pij[u], pi, pj[u], cthr4);
-          const T x = ((T)1 - pi) * pj[u];
-          const T y = (pj[u] - pij[u]) / x;
-          s += (double)(pij[u] * w + (pj[u] - pij[u]) * sbb_log(y));
-        }
-      }
-    }
-  }
-  for (int off = 16; off > 0; off >>= 1) {
-    s += __shfl_xor_sync(0xffffffffu, s, off);
-    cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
-  }
-  if (lane == 0) {
-    score[i] = (T)s;
-    csum[i] = cnt;
-    old_col[i] = wmask[i * H + h];   // the mask column before the swaps, for the weight rewrite
-  }
-}
-
-template <typename T>
-struct Pick {
-  T v;
-  long i;  // -1 = empty
-};
-// Maximum with ties to the larger index / minimum with ties to the larger index:
-// the outcome of a front-to-back scan that replaces on >= (resp. <=).
-template <typename T>
-__device__ __forceinline__ Pick<T> pick_max(Pick<T> a, Pick<T> b) {
-  if (b.i < 0) return a;
-  if (a.i < 0) return b;
-  return (b.v > a.v || (b.v == a.v && b.i > a.i)) ? b : a;
-}
-template <typename T>
-__device__ __forceinline__ Pick<T> pick_min(Pick<T> a, Pick<T> b) {
-  if (b.i < 0) return a;
-  if (a.i < 0) return b;
-  return (b.v < a.v || (b.v == a.v && b.i > a.i)) ? b : a;
-}
-template <typename T>
-__device__ __forceinline__ Pick<T> shfl_pick(Pick<T> p, int off) {
-  Pick<T> o;
-  o.v = __shfl_xor_sync(0xffffffffu, p.v, off);
-  o.i = __shfl_xor_sync(0xffffffffu, p.i, off);
-  return o;
-}
-
-// Single CTA.  Every iteration scans all rows: among silent connections
-// (mask 0) the highest score, among active ones (mask 1) the lowest, both with
-// the reference's sequential-scan semantics: ties go to the last index, and a
-// NaN score can only be selected when it belongs to the first candidate of its
-// class (a scan never replaces its holder with a NaN, nor a NaN holder at all).
-template <typename T>
-__global__ void __launch_bounds__(1024)
-    mask_swap_kernel(uint8_t *wmask, const T *__restrict__ nom, int *csum, long N, long M, long H, long Mc, long h,
-                     long iterations, T *rewrite_w,
-                     const uint8_t *__restrict__ old_col, const T *__restrict__ Ci, const T *__restrict__ Cj,
-                     const T *__restrict__ Cij, T cthr, T cthr4) {
-  __shared__ Pick<T> s_max[32], s_min[32];
-  __shared__ long s_first0[32], s_first1[32];
-  __shared__ int s_done;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  if (threadIdx.x == 0) s_done = 0;
-  __syncthreads();
-  for (long it = 0; it < iterations; ++it) {
-    Pick<T> bmax{(T)0, -1}, bmin{(T)0, -1};
-    long first0 = N, first1 = N;
-    for (long j = threadIdx.x; j < N; j += blockDim.x) {
-      const uint8_t m = wmask[j * H + h];
-      const T sc = (T)((double)nom[j] / (1.0 + (double)csum[j]));
-      if (m == 0) {
-        first0 = j < first0 ? j : first0;
-        if (sc == sc) bmax = pick_max(bmax, Pick<T>{sc, j});
-      } else if (m == 1) {
-        first1 = j < first1 ? j : first1;
-        if (sc == sc) bmin = pick_min(bmin, Pick<T>{sc, j});
-      }
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-      bmax = pick_max(bmax, shfl_pick(bmax, off));
-      bmin = pick_min(bmin, shfl_pick(bmin, off));
-      const long f0 = __shfl_xor_sync(0xffffffffu, first0, off);
-      const long f1 = __shfl_xor_sync(0xffffffffu, first1, off);
-      first0 = f0 < first0 ? f0 : first0;
-      first1 = f1 < first1 ? f1 : first1;
-    }
-    if (lane == 0) {
-      s_max[wid] = bmax;
-      s_min[wid] = bmin;
-      s_first0[wid] = first0;
-      s_first1[wid] = first1;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int w = 1; w < nwarps; ++w) {
-        bmax = pick_max(bmax, s_max[w]);
-        bmin = pick_min(bmin, s_min[w]);
-        first0 = s_first0[w] < first0 ? s_first0[w] : first0;
-        first1 = s_first1[w] < first1 ? s_first1[w] : first1;
-      }
-      long imax0 = N, imin1 = N;
-      T vmax0 = (T)0, vmin1 = (T)0;
-      if (first0 < N) {
-        const T sf = (T)((double)nom[first0] / (1.0 + (double)csum[first0]));
-        if (sf != sf) { imax0 = first0; vmax0 = sf; }
-        else { imax0 = bmax.i; vmax0 = bmax.v; }
-      }
-      if (first1 < N) {
-        const T sf = (T)((double)nom[first1] / (1.0 + (double)csum[first1]));
-        if (sf != sf) { imin1 = first1; vmin1 = sf; }
-        else { imin1 = bmin.i; vmin1 = bmin.v; }
-      }
-      if (imax0 == N || imin1 == N || vmax0 < vmin1) {
-        s_done = 1;
-      } else {
-        wmask[imax0 * H + h] = 1;
-        wmask[imin1 * H + h] = 0;
-        csum[imax0] += 1;
-        csum[imin1] -= 1;
-      }
-    }
-    __syncthreads();
-    if (s_done) break;
-  }
-  if (rewrite_w == nullptr) return;
-  // rows whose mask bit changed get new weights in hypercolumn h (at most 2 * iterations rows)
-  for (long j = threadIdx.x; j < N; j += blockDim.x) {
-    const uint8_t now = wmask[j * H + h];
-    if (now == old_col[j]) continue;
-    const T ci = Ci[j];
-    for (long jj = 0; jj < Mc; ++jj) {
-      const long col = h * Mc + jj;
-      const T cj = Cj[col];
-      T v = (T)0;
-      if (now != 0 && !(ci < cthr) && !(cj < cthr)) v = log_ratio(Cij[j * M + col], ci, cj, cthr4);
-      rewrite_w[j * M + col] = v;
-    }
-  }
-}
-
-// ---- fast swap: per-chunk candidate lists, then a short exact simulation -------------------
-// Only the two rows of a swap change their score, so the row chosen in iteration t is always
-// among the t+1 best of its class in the initial ordering or a row moved by an earlier swap.
-// Phase A extracts, per chunk of rows, the `iterations` best silent rows (highest score, ties
-// to the larger index) and the `iterations` worst active rows (lowest score, ties to the
-// larger index); phase B reduces the chunk lists to one list per class and replays the swaps
-// exactly.  A NaN score makes the reference's scan order-dependent; phase B reproduces that too
-// (see mask_replay_kernel).  Layers too small or too large for the lists, and more than
-// kSwapMaxIter iterations, take the one-CTA full scan (mask_swap_kernel).
-//
-// Scores are mapped to unsigned keys whose integer order is the class order (silent rows: score
-// descending first = larger key; active rows: the complement), so that one selection round is a
-// register-local maximum, one warp-wide integer maximum (redux) for the key and one for the row
-// index among equal keys (the reference's scans keep the last of equal scores), and a clear of the
-// winner's register: no shuffle trees, no block barrier inside a round.
-constexpr int kSwapMaxIter = 32;
-constexpr int kSwapSlots = 1024;          // candidate slots per class handed from phase A to phase B
-constexpr int kSwapCacheRows = 4096;      // rows per chunk whose score and class fit the chunk's shared memory
-constexpr int kSwapThreads = 256;         // both phases: 8 warps = 2 classes x 4 slices
-
-template <typename T>
-__device__ __forceinline__ T swap_score(T nom, int csum) {
-  return (T)((double)nom / (1.0 + (double)csum));
-}
-
-// Order-preserving keys: a < b  <=>  key(a) < key(b) for non-NaN scores (-0 counts as +0).
-// Key 0 is never produced by a score and marks an empty slot, also after complementing.
-template <typename T>
-struct ScoreKey;
-template <>
-struct ScoreKey<float> {
-  typedef uint32_t type;
-  static __device__ __forceinline__ type make(float v) {
-    const uint32_t u = __float_as_uint(v == 0.f ? 0.f : v);
-    return (u >> 31) ? ~u : (u | 0x80000000u);
-  }
-  static __device__ __forceinline__ float value(type k) {
-    return __uint_as_float((k >> 31) ? (k ^ 0x80000000u) : ~k);
-  }
-  static __device__ __forceinline__ type warp_max(type k) { return __reduce_max_sync(0xffffffffu, k); }
-};
-template <>
-struct ScoreKey<double> {
-  typedef unsigned long long type;
-  static __device__ __forceinline__ type make(double v) {
-    const unsigned long long u = (unsigned long long)__double_as_longlong(v == 0.0 ? 0.0 : v);
-    return (u >> 63) ? ~u : (u | 0x8000000000000000ull);
-  }
-  static __device__ __forceinline__ double value(type k) {
-    return __longlong_as_double((long long)((k >> 63) ? (k ^ 0x8000000000000000ull) : ~k));
-  }
-  static __device__ __forceinline__ type warp_max(type k) {
-    const uint32_t hi = __reduce_max_sync(0xffffffffu, (uint32_t)(k >> 32));
-    const uint32_t lo = __reduce_max_sync(0xffffffffu, (uint32_t)(k >> 32) == hi ? (uint32_t)k : 0u);
-    return ((type)hi << 32) | lo;
-  }
-};
-// Class key: maximum = first in the class order.  cls 0 (silent): highest score; cls 1 (active): lowest.
-template <typename T>
-__device__ __forceinline__ typename ScoreKey<T>::type class_key(int cls, T v) {
-  const typename ScoreKey<T>::type k = ScoreKey<T>::make(v);
-  return cls == 0 ? k : ~k;
-}
-template <typename T>
-__device__ __forceinline__ T class_key_value(int cls, typename ScoreKey<T>::type k) {
-  return ScoreKey<T>::value(cls == 0 ? k : ~k);
-}
-
-// One warp: the first `rounds` of its R x 32 register-resident entries (key 0 = empty) in class
-// order; lane 0 writes round k's (score, row) to out_v[k], out_i[k] (row -1 pads an exhausted list).
-template <typename T, int R>
-__device__ __forceinline__ void warp_select_regs(int cls, typename ScoreKey<T>::type (&key)[R], uint32_t (&row)[R],
-                                                 int rounds, T *out_v, long *out_i) {
-  typedef typename ScoreKey<T>::type K;
-  const int lane = threadIdx.x & 31;
-  for (int k = 0; k < rounds; ++k) {
-    K mine = 0;
-#pragma unroll
-    for (int r = 0; r < R; ++r) mine = key[r] > mine ? key[r] : mine;
-    const K best = ScoreKey<T>::warp_max(mine);
-    if (best == 0) {   // exhausted (uniform)
-      for (int kk = k + lane; kk < rounds; kk += 32) out_i[kk] = -1;
-      break;
-    }
-    uint32_t my_row = 0;   // rows are stored + 1 so that 0 means "not holding the best key"
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (key[r] == best && row[r] + 1u > my_row) my_row = row[r] + 1u;
-    const uint32_t win = __reduce_max_sync(0xffffffffu, my_row);
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (key[r] == best && row[r] + 1u == win) key[r] = 0;
-    if (lane == 0) {
-      out_v[k] = class_key_value<T>(cls, best);
-      out_i[k] = (long)win - 1;
-    }
-  }
-}
-
-// Phase A.  lists: [class][chunk][iterations] of (value, row); row -1 = empty.
-// CACHED: the chunk's scores and classes are first gathered into shared memory (coalesced).
-template <typename T, int R>
-__global__ void __launch_bounds__(kSwapThreads)
-    mask_candidates_kernel(const uint8_t *__restrict__ wmask, const T *__restrict__ nom, const int *__restrict__ csum,
-                           long N, long H, long h, int iterations, long rows_per_chunk, T *cand_v, long *cand_i) {
-  typedef typename ScoreKey<T>::type K;
-  __shared__ T s_lv[2][4 * kSwapMaxIter];
-  __shared__ long s_li[2][4 * kSwapMaxIter];
-  extern __shared__ __align__(16) unsigned char cand_dyn[];
-  T *s_sc = reinterpret_cast<T *>(cand_dyn);
-  uint8_t *s_cl = cand_dyn + rows_per_chunk * sizeof(T);
-  const long r0 = (long)blockIdx.x * rows_per_chunk;
-  const long r1 = r0 + rows_per_chunk < N ? r0 + rows_per_chunk : N;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (long j = r0 + threadIdx.x; j < r1; j += blockDim.x) {
-    const uint8_t m = wmask[j * H + h];
-    const T sc = swap_score(nom[j], csum[j]);
-    uint8_t cl = m <= 1 ? m : 2;
-    if (sc != sc) cl = 2;   // a NaN score is in no best list (the replay handles the one place it can matter)
-    s_sc[j - r0] = sc;
-    s_cl[j - r0] = cl;
-  }
-  __syncthreads();
-  // level 1: warp (cls, slice) lists the first `iterations` rows of its class in its quarter of the chunk
-  const int cls = wid & 1, slice = wid >> 1;
-  {
-    const long len = r1 - r0, q = (len + 3) / 4;
-    const long b = slice * q, e = b + q < len ? b + q : len;   // chunk-relative
-    K key[R];
-    uint32_t row[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const long j = b + lane + 32 * r;
-      const bool mine = j < e && s_cl[j < e ? j : 0] == cls;
-      key[r] = mine ? class_key<T>(cls, s_sc[j]) : (K)0;
-      row[r] = (uint32_t)(r0 + j);
-    }
-    warp_select_regs<T, R>(cls, key, row, iterations, s_lv[cls] + slice * iterations, s_li[cls] + slice * iterations);
-  }
-  __syncthreads();
-  // level 2: one warp per class merges the four slice lists (4 * iterations <= 128 entries) into the chunk's list
-  if (wid < 2) {
-    K key[4];
-    uint32_t row[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int e = lane + 32 * r;
-      const long i = e < 4 * iterations ? s_li[wid][e] : -1;
-      key[r] = i >= 0 ? class_key<T>(wid, s_lv[wid][e]) : (K)0;
-      row[r] = i >= 0 ? (uint32_t)i : 0u;
-    }
-    const long slot = ((long)wid * gridDim.x + blockIdx.x) * iterations;
-    warp_select_regs<T, 4>(wid, key, row, iterations, cand_v + slot, cand_i + slot);
-  }
-}
-
-// Phase B, one CTA: reduce the chunk lists to the first `iterations` rows of each class, replay
-// the swaps on them (warp 0; every lane keeps one listed row and one moved row per class), then
-// rewrite the weights of hypercolumn h for the rows a swap touched (rewrite_w != null).
-//
-// NaN scores follow the reference's front-to-back scan: the scan's first row of a class holds the
-// pick until a row compares better, and nothing compares better than NaN, so a class whose
-// lowest-index row has a NaN score picks that row; a NaN score anywhere else is never picked.
-// Besides the best rows, the replay therefore tracks the `iterations + 1` lowest-index rows of
-// each class (one row leaves a class per swap) with their NaN flags; NaN rows are in no best list.
-constexpr int kLowSlots = 2 * 32;   // >= kSwapMaxIter + 1 lowest-index rows per class, two per lane
-template <typename T>
-__global__ void __launch_bounds__(kSwapThreads)
-    mask_replay_kernel(uint8_t *wmask, const T *__restrict__ nom, int *csum, long N, long M, long H, long Mc, long h,
-                       int iterations, int chunks, const T *__restrict__ cand_v, const long *__restrict__ cand_i,
-                       T *rewrite_w, const T *__restrict__ Ci, const T *__restrict__ Cj, const T *__restrict__ Cij,
-                       T cthr, T cthr4) {
-  typedef typename ScoreKey<T>::type K;
-  constexpr int R1 = kSwapSlots / 4 / 32;   // registers per lane for a quarter of one class's chunk lists
-  constexpr uint32_t kNone = 0xFFFFFFFFu;
-  __shared__ T l1_v[2][4 * kSwapMaxIter], top_v[2][kSwapMaxIter];
-  __shared__ long l1_i[2][4 * kSwapMaxIter], top_i[2][kSwapMaxIter];
-  __shared__ uint32_t low_row[2][kLowSlots];
-  __shared__ int low_cs[2][kLowSlots];
-  __shared__ uint8_t low_nan[2][kLowSlots];
-  __shared__ int low_cnt[2], win_cnt[kSwapThreads / 32][2];
-  __shared__ long touched[2 * kSwapMaxIter];
-  __shared__ int n_touched;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int total = chunks * iterations;   // entries per class, <= kSwapSlots
-  if (threadIdx.x == 0) {
-    n_touched = 0;
-    low_cnt[0] = low_cnt[1] = 0;
-  }
-  for (int e = threadIdx.x; e < 2 * kLowSlots; e += blockDim.x) low_row[e / kLowSlots][e % kLowSlots] = kNone;
-  __syncthreads();
-  // the lowest-index rows of each class: windows of blockDim rows from row 0 until both lists are full
-  const int want = iterations + 1;
-  for (long w0 = 0; w0 < N; w0 += blockDim.x) {
-    const long j = w0 + threadIdx.x;
-    const uint8_t m = j < N ? wmask[j * H + h] : (uint8_t)2;
-    unsigned bal[2];
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      bal[c] = __ballot_sync(0xffffffffu, m == c);
-      if (lane == 0) win_cnt[wid][c] = __popc(bal[c]);
-    }
-    __syncthreads();
-    if (m <= 1) {
-      int pos = low_cnt[m] + __popc(bal[m] & ((1u << lane) - 1u));
-      for (int w = 0; w < wid; ++w) pos += win_cnt[w][m];
-      if (pos < want) {
-        const T nm = nom[j];
-        low_row[m][pos] = (uint32_t)j;
-        low_nan[m][pos] = nm != nm ? 1 : 0;
-        low_cs[m][pos] = csum[j];
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-        low_cnt[0] += win_cnt[w][0];
-        low_cnt[1] += win_cnt[w][1];
-      }
-    __syncthreads();
-    if (low_cnt[0] >= want && low_cnt[1] >= want) break;   // uniform: read after the barrier
-  }
-  {
-    const int cls = wid & 1, slice = wid >> 1;
-    const int q = (total + 3) / 4, b = slice * q, e = b + q < total ? b + q : total;
-    K key[R1];
-    uint32_t row[R1];
-#pragma unroll
-    for (int r = 0; r < R1; ++r) {
-      const int t = b + lane + 32 * r;
-      const long i = t < e ? cand_i[(long)cls * total + t] : -1;
-      key[r] = i >= 0 ? class_key<T>(cls, cand_v[(long)cls * total + t]) : (K)0;
-      row[r] = i >= 0 ? (uint32_t)i : 0u;
-    }
-    warp_select_regs<T, R1>(cls, key, row, iterations, l1_v[cls] + slice * iterations, l1_i[cls] + slice * iterations);
-  }
-  __syncthreads();
-  if (wid < 2) {
-    K key[4];
-    uint32_t row[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int e = lane + 32 * r;
-      const long i = e < 4 * iterations ? l1_i[wid][e] : -1;
-      key[r] = i >= 0 ? class_key<T>(wid, l1_v[wid][e]) : (K)0;
-      row[r] = i >= 0 ? (uint32_t)i : 0u;
-    }
-    warp_select_regs<T, 4>(wid, key, row, iterations, top_v[wid], top_i[wid]);
-  }
-  __syncthreads();
-  if (wid == 0) {
-    // per class c: slot A = listed best row number `lane`; slot B = the row moved into the class by swap
-    // `lane` (it may carry a NaN score: key 0, but still a member); L0, L1 = listed lowest rows lane, lane + 32
-    K ka[2], kb[2] = {0, 0};
-    uint32_t ra[2], rb[2] = {kNone, kNone}, l0[2], l1[2];
-    T na[2], nb[2] = {(T)0, (T)0};
-    int ca[2], cb[2] = {0, 0}, c0[2], c1[2];
-    bool nanb[2] = {false, false}, n0[2], n1[2];
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const long i = lane < iterations ? top_i[c][lane] : -1;
-      ka[c] = i >= 0 ? class_key<T>(c, top_v[c][lane]) : (K)0;
-      ra[c] = i >= 0 ? (uint32_t)i : kNone;
-      na[c] = i >= 0 ? nom[i] : (T)0;
-      ca[c] = i >= 0 ? csum[i] : 0;
-      l0[c] = low_row[c][lane];      n0[c] = low_nan[c][lane] != 0;      c0[c] = low_cs[c][lane];
-      l1[c] = low_row[c][lane + 32]; n1[c] = low_nan[c][lane + 32] != 0; c1[c] = low_cs[c][lane + 32];
-    }
-    const T quiet_nan = (T)NAN;
-    for (int it = 0; it < iterations; ++it) {
-      K best[2];
-      uint32_t pick[2];
-      bool pick_nan[2];
-      bool stop = false;
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        // the class's first row in index order, and whether its score is NaN
-        uint32_t f = l0[c] < l1[c] ? l0[c] : l1[c];
-        f = rb[c] < f ? rb[c] : f;
-        const uint32_t first = __reduce_min_sync(0xffffffffu, f);
-        const bool first_is_nan = __any_sync(0xffffffffu, first != kNone && ((l0[c] == first && n0[c]) ||
-                                                                           (l1[c] == first && n1[c]) ||
-                                                                           (rb[c] == first && nanb[c])));
-        // the best row among those with a number for a score
-        best[c] = ScoreKey<T>::warp_max(ka[c] > kb[c] ? ka[c] : kb[c]);
-        uint32_t mine = 0;
-        if (best[c] != 0 && ka[c] == best[c]) mine = ra[c] + 1u;
-        if (best[c] != 0 && kb[c] == best[c] && rb[c] + 1u > mine) mine = rb[c] + 1u;
-        const uint32_t win = __reduce_max_sync(0xffffffffu, mine);
-        pick_nan[c] = first_is_nan;
-        pick[c] = first_is_nan ? first : win - 1u;
-        if (first == kNone || (!first_is_nan && best[c] == 0)) stop = true;   // the class is empty
-      }
-      // the best silent row scores below the worst active one (never true with a NaN on either side)
-      if (stop || (!pick_nan[0] && !pick_nan[1] &&
-                   class_key_value<T>(0, best[0]) < class_key_value<T>(1, best[1])))
-        break;   // uniform across the warp
-      T mv_nom[2];
-      int mv_cs[2];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const uint32_t p = pick[c];
-        const bool own_a = ka[c] != 0 && ra[c] == p;
-        const bool own_b = rb[c] == p;
-        const bool own_l0 = l0[c] == p, own_l1 = l1[c] == p;
-        // the slots of the best lists know the numerator; a row picked for its NaN is only in L or B
-        unsigned who = __ballot_sync(0xffffffffu, own_a || own_b);
-        if (who == 0) who = __ballot_sync(0xffffffffu, own_l0 || own_l1);
-        const int src = __ffs(who) - 1;
-        const T my_nom = own_a ? na[c] : (own_b ? nb[c] : quiet_nan);
-        const int my_cs = own_a ? ca[c] : (own_b ? cb[c] : (own_l0 ? c0[c] : c1[c]));
-        mv_nom[c] = __shfl_sync(0xffffffffu, my_nom, src);
-        mv_cs[c] = __shfl_sync(0xffffffffu, my_cs, src);
-        if (own_a) ka[c] = 0;
-        if (own_b) { kb[c] = 0; rb[c] = kNone; nanb[c] = false; }
-        if (own_l0) l0[c] = kNone;
-        if (own_l1) l1[c] = kNone;
-      }
-      if (lane == it) {
-        // the silent row becomes active with one more connection, the active row silent with one fewer
-        const long up = (long)pick[0], down = (long)pick[1];
-        rb[1] = pick[0]; nb[1] = mv_nom[0]; cb[1] = mv_cs[0] + 1; nanb[1] = pick_nan[0];
-        kb[1] = nanb[1] ? (K)0 : class_key<T>(1, swap_score(nb[1], cb[1]));
-        rb[0] = pick[1]; nb[0] = mv_nom[1]; cb[0] = mv_cs[1] - 1; nanb[0] = pick_nan[1];
-        kb[0] = nanb[0] ? (K)0 : class_key<T>(0, swap_score(nb[0], cb[0]));
-        wmask[up * H + h] = 1;
-        wmask[down * H + h] = 0;
-        csum[up] = cb[1];
-        csum[down] = cb[0];
-        touched[2 * it] = up;
-        touched[2 * it + 1] = down;
-        n_touched = 2 * it + 2;
-      }
-    }
-  }
-  __syncthreads();
-  if (rewrite_w == nullptr) return;
-  // a touched row's weights in hypercolumn h follow its final mask bit (idempotent when a row was touched
-  // twice).  Row data first (one thread per touched row), so that the element loop has independent loads only.
-  __shared__ T t_ci[2 * kSwapMaxIter];
-  __shared__ uint8_t t_on[2 * kSwapMaxIter];
-  const int nt = n_touched;
-  if ((int)threadIdx.x < nt) {
-    const long i = touched[threadIdx.x];
-    const T ci = Ci[i];
-    t_ci[threadIdx.x] = ci;
-    t_on[threadIdx.x] = wmask[i * H + h] != 0 && !(ci < cthr);
-  }
-  __syncthreads();
-  const long total_elems = (long)nt * Mc;
-#pragma unroll 4
-  for (long t = threadIdx.x; t < total_elems; t += blockDim.x) {
-    const int r = (int)(t / Mc);
-    const long i = touched[r], col = h * Mc + t % Mc;
-    const T cj = Cj[col];
-    const T cij = Cij[i * M + col];
-    T v = (T)0;
-    if (t_on[r] && !(cj < cthr)) v = log_ratio(cij, t_ci[r], cj, cthr4);
-    rewrite_w[i * M + col] = v;
-  }
-}
-
-__host__ __device__ static inline size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
-static constexpr size_t kSwapListBytes = 256 + (size_t)2 * kSwapSlots * (sizeof(double) + sizeof(long));
-
-size_t mask_scratch_bytes(long N, size_t elem) {
-  return align256((size_t)N * elem) + align256((size_t)N * sizeof(int)) + align256((size_t)N) + kSwapListBytes;
-}
-
-// Scratch layout: [score N x T][active count N x int][old mask column N bytes][nan flag, candidate lists].
-template <typename T>
-struct MaskScratch {
-  T *score;
-  int *csum;
-  uint8_t *old_col;
-  int *nan_flag;
-  long *cand_i;
-  T *cand_v;
-  __host__ __device__ MaskScratch(void *scratch, long N) {
-    unsigned char *p = static_cast<unsigned char *>(scratch);
-    score = reinterpret_cast<T *>(p);
-    p += align256((size_t)N * sizeof(T));
-    csum = reinterpret_cast<int *>(p);
-    p += align256((size_t)N * sizeof(int));
-    old_col = p;
-    p += align256((size_t)N);
-    nan_flag = reinterpret_cast<int *>(p);
-    cand_i = reinterpret_cast<long *>(p + 256);
-    cand_v = reinterpret_cast<T *>(p + 256 + (size_t)2 * kSwapSlots * sizeof(long));
-  }
-};
-
-template <typename T>
-cudaError_t launch_mask_update(uint8_t *wmask, const T *weights, const T *Ci, const T *Cj, const T *Cij, T cthr,
-                               long N, long M, long H, long Mc, long h, long iterations, void *scratch,
-                               cudaStream_t st, T *rewrite_w) {
-  if (N == 0) return cudaSuccess;
-  MaskScratch<T> ms(scratch, N);
-  const T cthr4 = cthr * cthr * cthr * cthr;
-  mask_score_kernel<T><<<(unsigned)((N + 7) / 8), 256, 0, st>>>(wmask, weights, Ci, Cj, Cij, cthr, cthr4, N, M, H, Mc,
-                                                                 h, ms.score, ms.csum, ms.old_col);
-  cudaError_t e = launched();
-  if (e != cudaSuccess) return e;
-  return launch_mask_select<T>(wmask, Ci, Cj, Cij, cthr, N, M, H, Mc, h, iterations, scratch, st, rewrite_w);
-}
-
-// The swaps alone, from per-row scores, active counts and the old mask column already in `scratch`.
-template <typename T>
-cudaError_t launch_mask_select(uint8_t *wmask, const T *Ci, const T *Cj, const T *Cij, T cthr, long N, long M, long H,
-                               long Mc, long h, long iterations, void *scratch, cudaStream_t st, T *rewrite_w) {
-  if (N == 0) return cudaSuccess;
-  MaskScratch<T> ms(scratch, N);
-  const T cthr4 = cthr * cthr * cthr * cthr;
-  cudaError_t e = cudaSuccess;
-  // candidate lists: rows fit 32-bit indices and a chunk (<= kSwapCacheRows rows) fits shared memory
-  const int max_chunks = iterations >= 1 && iterations <= kSwapMaxIter ? kSwapSlots / (int)iterations : 0;
-  if (max_chunks > 0 && N >= 1024 && N < (1l << 31) && (N + max_chunks - 1) / max_chunks <= kSwapCacheRows) {
-    int chunks = (int)((N + 767) / 768);
-    if (chunks > max_chunks) chunks = max_chunks;
-    const long rows_per_chunk = (N + chunks - 1) / chunks;
-    chunks = (int)((N + rows_per_chunk - 1) / rows_per_chunk);
-    const size_t dyn = (size_t)rows_per_chunk * (sizeof(T) + 1);
-    const long slice = (rows_per_chunk + 3) / 4;   // rows one warp keeps in registers, 32 per register
-#define SBB_CAND(R)                                                                                              \
-  mask_candidates_kernel<T, R><<<chunks, kSwapThreads, dyn, st>>>(wmask, ms.score, ms.csum, N, H, h, (int)iterations, \
-                                                                  rows_per_chunk, ms.cand_v, ms.cand_i)
-    if (slice <= 4 * 32) SBB_CAND(4);
-    else if (slice <= 8 * 32) SBB_CAND(8);
-    else if (slice <= 16 * 32) SBB_CAND(16);
-    else SBB_CAND(32);
-#undef SBB_CAND
-    e = launched();
-    if (e != cudaSuccess) return e;
-    mask_replay_kernel<T><<<1, kSwapThreads, 0, st>>>(wmask, ms.score, ms.csum, N, M, H, Mc, h, (int)iterations, chunks,
-                                                     ms.cand_v, ms.cand_i, rewrite_w, Ci, Cj, Cij, cthr, cthr4);
-    return launched();
-  }
-  mask_swap_kernel<T><<<1, 1024, 0, st>>>(wmask, ms.score, ms.csum, N, M, H, Mc, h, iterations, rewrite_w,
-                                          ms.old_col, Ci, Cj, Cij, cthr, cthr4);
-  return launched();
-}
-template cudaError_t launch_mask_select<float>(uint8_t *, const float *, const float *, const float *, float, long, long,
-                                               long, long, long, long, void *, cudaStream_t, float *);
-template cudaError_t launch_mask_select<double>(uint8_t *, const double *, const double *, const double *, double, long,
-                                                long, long, long, long, long, void *, cudaStream_t, double *);
-template cudaError_t launch_mask_update<float>(uint8_t *, const float *, const float *, const float *, const float *,
-                                               float, long, long, long, long, long, long, void *, cudaStream_t,
-                                               float *);
-template cudaError_t launch_mask_update<double>(uint8_t *, const double *, const double *, const double *,
-                                                const double *, double, long, long, long, long, long, long, void *,
-                                                cudaStream_t, double *);
 
 
 // ----------------------------------------------------------------------------
@@ -1959,103 +1333,6 @@ cudaError_t launch_sum_partials(const T *partial, int splits, long n, T *out, cu
 }
 template cudaError_t launch_sum_partials<float>(const float *, int, long, float *, cudaStream_t);
 template cudaError_t launch_sum_partials<double>(const double *, int, long, double *, cudaStream_t);
-
-// Mask scores of the rows [row_begin, row_end) this rank owns, written into every rank's work arrays
-// (scratch_tab: base of each rank's mask scratch, laid out for N rows).
-template <typename T>
-__global__ void __launch_bounds__(256)
-    mask_score_rows_kernel(const uint8_t *__restrict__ wmask, const T *__restrict__ Ci, const T *__restrict__ Cj,
-                           const T *__restrict__ Cij, T cthr, T cthr4, long N, long M, long H, long Mc, long h,
-                           long row_begin, long row_end, PeerTable scratch_tab) {
-  const int lane = threadIdx.x & 31;
-  const long i = row_begin + (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= row_end) return;
-  const T pi = Ci[i];
-  double s = 0.0;
-  if (pi >= cthr) {
-    for (long jj = lane; jj < Mc; jj += 32) {
-      const long col = h * Mc + jj;
-      const T pj = Cj[col];
-      if (pj >= cthr) {
-        const T pij = Cij[i * M + col];
-        const T w = log_ratio(pij, pi, pj, cthr4);
-        const T x = ((T)1 - pi) * pj;
-        const T y = (pj - pij) / x;
-        s += (double)(pij * w + (pj - pij) * sbb_log(y));
-      }
-    }
-  }
-  int cnt = 0;
-  for (long k = lane; k < H; k += 32) cnt += wmask[i * H + k];
-  for (int off = 16; off > 0; off >>= 1) {
-    s += __shfl_xor_sync(0xffffffffu, s, off);
-    cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
-  }
-  if (lane == 0) {
-    const uint8_t bit = wmask[i * H + h];
-    for (int d = 0; d < scratch_tab.n; ++d) {
-      MaskScratch<T> ms(scratch_tab.ptr[d], N);
-      ms.score[i] = (T)s;
-      ms.csum[i] = cnt;
-      ms.old_col[i] = bit;
-    }
-  }
-}
-template <typename T>
-cudaError_t launch_mask_score_rows(const uint8_t *wmask, const T *Ci, const T *Cj, const T *Cij, T cthr, long N, long M,
-                                   long H, long Mc, long h, long row_begin, long row_end, const PeerTable &scratch_tab,
-                                   cudaStream_t st) {
-  if (row_end <= row_begin) return cudaSuccess;
-  const T cthr4 = cthr * cthr * cthr * cthr;
-  mask_score_rows_kernel<T><<<(unsigned)((row_end - row_begin + 7) / 8), 256, 0, st>>>(
-      wmask, Ci, Cj, Cij, cthr, cthr4, N, M, H, Mc, h, row_begin, row_end, scratch_tab);
-  return launched();
-}
-template cudaError_t launch_mask_score_rows<float>(const uint8_t *, const float *, const float *, const float *, float,
-                                                   long, long, long, long, long, long, long, const PeerTable &,
-                                                   cudaStream_t);
-template cudaError_t launch_mask_score_rows<double>(const uint8_t *, const double *, const double *, const double *,
-                                                    double, long, long, long, long, long, long, long, const PeerTable &,
-                                                    cudaStream_t);
-
-// After the swaps: owned rows whose mask bit changed get hypercolumn h's weights recomputed from the owner's
-// traces, in every rank's weight matrix.  One warp per owned row.
-template <typename T>
-__global__ void __launch_bounds__(256)
-    mask_rewrite_rows_kernel(const uint8_t *__restrict__ wmask, const uint8_t *__restrict__ old_col,
-                             const T *__restrict__ Ci, const T *__restrict__ Cj, const T *__restrict__ Cij, T cthr,
-                             T cthr4, long M, long H, long Mc, long h, long row_begin, long row_end, PeerTable wtab) {
-  const int lane = threadIdx.x & 31;
-  const long i = row_begin + (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= row_end) return;
-  const uint8_t now = wmask[i * H + h];
-  if (now == old_col[i]) return;
-  const T ci = Ci[i];
-  for (long jj = lane; jj < Mc; jj += 32) {
-    const long col = h * Mc + jj;
-    const T cj = Cj[col];
-    T v = (T)0;
-    if (now != 0 && !(ci < cthr) && !(cj < cthr)) v = log_ratio(Cij[i * M + col], ci, cj, cthr4);
-    for (int d = 0; d < wtab.n; ++d) static_cast<T *>(wtab.ptr[d])[i * M + col] = v;
-  }
-}
-template <typename T>
-cudaError_t launch_mask_rewrite_rows(const uint8_t *wmask, const void *scratch, const T *Ci, const T *Cj, const T *Cij,
-                                     T cthr, long N, long M, long H, long Mc, long h, long row_begin, long row_end,
-                                     const PeerTable &wtab, cudaStream_t st) {
-  if (row_end <= row_begin) return cudaSuccess;
-  MaskScratch<T> ms(const_cast<void *>(scratch), N);
-  const T cthr4 = cthr * cthr * cthr * cthr;
-  mask_rewrite_rows_kernel<T><<<(unsigned)((row_end - row_begin + 7) / 8), 256, 0, st>>>(
-      wmask, ms.old_col, Ci, Cj, Cij, cthr, cthr4, M, H, Mc, h, row_begin, row_end, wtab);
-  return launched();
-}
-template cudaError_t launch_mask_rewrite_rows<float>(const uint8_t *, const void *, const float *, const float *,
-                                                     const float *, float, long, long, long, long, long, long, long,
-                                                     const PeerTable &, cudaStream_t);
-template cudaError_t launch_mask_rewrite_rows<double>(const uint8_t *, const void *, const double *, const double *,
-                                                      const double *, double, long, long, long, long, long, long, long,
-                                                      const PeerTable &, cudaStream_t);
 
 }  // namespace sbb
 

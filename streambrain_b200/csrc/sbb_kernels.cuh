@@ -88,10 +88,12 @@ cudaError_t launch_apply_mask(T *w, const uint8_t *wmask, long N, long M, long H
 
 // Mask update for hypercolumn h.  `weights` null => the un-masked weight is
 // recomputed from the traces.  `scratch` holds mask_scratch_bytes(N, sizeof(T))
-// bytes (256-byte aligned): per-row score, active count and previous mask bit, candidate lists.
+// bytes (256-byte aligned): per-row score, active count and previous mask bit, candidate lists.  mask_scratch_init
+// prepares it once; every launch leaves it ready for the next.
 // `rewrite_w` non-null => the weights of hypercolumn h are recomputed from the traces, under the
 // new mask, for every row whose mask bit a swap changed.
 size_t mask_scratch_bytes(long N, size_t elem);
+cudaError_t mask_scratch_init(void *scratch, cudaStream_t st);
 template <typename T>
 cudaError_t launch_mask_update(uint8_t *wmask, const T *weights, const T *Ci, const T *Cj, const T *Cij, T cthr,
                                long N, long M, long H, long Mc, long h, long iterations, void *scratch,
@@ -121,8 +123,8 @@ cudaError_t launch_scatter_columns(const T *x, long B, long N, long block, const
 template <typename T>
 cudaError_t launch_sum_partials(const T *partial, int splits, long n, T *out, cudaStream_t st);
 template <typename T>
-cudaError_t launch_mask_score_rows(const uint8_t *wmask, const T *Ci, const T *Cj, const T *Cij, T cthr, long N, long M,
-                                   long H, long Mc, long h, long row_begin, long row_end, const PeerTable &scratch_tab,
+cudaError_t launch_mask_score_rows(const uint8_t *wmask, const T *weights, const T *Ci, const T *Cj, const T *Cij,
+                                   T cthr, long N, long M, long H, long Mc, long h, long row_begin, long row_end, const PeerTable &scratch_tab,
                                    cudaStream_t st);
 template <typename T>
 cudaError_t launch_mask_rewrite_rows(const uint8_t *wmask, const void *scratch, const T *Ci, const T *Cj, const T *Cij,

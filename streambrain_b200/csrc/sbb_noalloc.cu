@@ -9,7 +9,7 @@
 // no cudaMalloc, no cudaFree, no library routine that allocates.
 //
 // Cost and limits
-//   * The array is SBB_NOALLOC_MAX_ROWS * 13 bytes plus 40 KiB (1.7 MiB) and is resident on
+//   * The array is SBB_NOALLOC_MAX_ROWS * 17.5 bytes plus 1 KiB (2.2 MiB) and is resident on
 //     every GPU that loads the library, from load until the process exits.
 //   * Layers with more than SBB_NOALLOC_MAX_ROWS input rows are refused with
 //     SBB_ERR_UNSUPPORTED; nothing is launched in that case.
@@ -36,12 +36,13 @@ constexpr long kMaxRows = SBB_NOALLOC_MAX_ROWS;
 constexpr size_t kScoreBytes = (size_t)kMaxRows * sizeof(double);  // REAL score per row, sized for double
 constexpr size_t kCountBytes = (size_t)kMaxRows * sizeof(int);     // active connections per row
 constexpr size_t kColBytes = (size_t)kMaxRows;                     // previous mask bit per row
-constexpr size_t kListBytes = 40 * 1024;                           // candidate lists of the swap search
+constexpr size_t kFilterBytes = (size_t)kMaxRows * sizeof(uint32_t);  // filter key per row
+constexpr size_t kHeaderBytes = 1024 + (size_t)kMaxRows / 2;        // what the blocks of a launch share
 
 // In host code this name is only a handle for the runtime; it is NOT a device
 // address and must never be passed to a kernel.  The address a kernel can use
 // comes from cudaGetSymbolAddress, once per device.
-static __device__ __align__(256) unsigned char g_mask_scratch[kScoreBytes + kCountBytes + kColBytes + kListBytes];
+static __device__ __align__(256) unsigned char g_mask_scratch[kScoreBytes + kCountBytes + kFilterBytes + kColBytes + kHeaderBytes];
 
 constexpr int kMaxDevices = 64;
 void *g_scratch_ptr[kMaxDevices] = {nullptr};
@@ -125,7 +126,7 @@ static int update_mask_noalloc_impl(int dtype, uint8_t *wmask_dev, const void *w
   void *scratch = nullptr;
   int rc = scratch_for_current_device(&scratch);
   if (rc != SBB_OK) return rc;
-  if (sbb::mask_scratch_bytes(N, dtype == SBB_F32 ? 4 : 8) > kScoreBytes + kCountBytes + kColBytes + kListBytes) {
+  if (sbb::mask_scratch_bytes(N, dtype == SBB_F32 ? 4 : 8) > kScoreBytes + kCountBytes + kFilterBytes + kColBytes + kHeaderBytes) {
     snprintf(g_noalloc_error, sizeof(g_noalloc_error), "update_mask_noalloc: built-in work area too small");
     return SBB_ERR_UNSUPPORTED;
   }

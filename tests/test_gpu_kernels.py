@@ -306,3 +306,25 @@ np.savez(sys.argv[1], **out)
             for name, v in zip(("Ci", "Cj", "Cij"), want):
                 assert rel_inf(r[tag + "_" + name], v) < tol, (tag, pair, name)
             assert weight_err(r[tag + "_W"], want[3]) < 10 * tol, (tag, pair)
+
+
+@pytest.mark.parametrize("n,mc", [(600, 6), (2048, 40), (2049, 40), (20000, 5)])
+@pytest.mark.parametrize("case", ["equal rows", "one group of rows"])
+def test_update_mask_with_crowded_lists(k, port_kernels, n, mc, case):
+    """The lists of the best rows are bounded by the best rows of 16 or 32 groups of rows.  Equal scores everywhere (ties
+    go to the last row) and best rows that all fall into one group, more than the lists' slots, must come out as in the
+    reference's scan."""
+    rs = np.random.RandomState(n + mc)
+    wmask, w, Ci, Cj, Cij = _mask_case(rs, n, 2, mc, np.float64, density=0.5)
+    if case == "equal rows":
+        Ci[:], Cij[:], w[:], wmask[:, 0] = 0.5, 0.1, 0.2, (np.arange(n) % 3 == 0)
+        wmask[:, 1] = 1 - wmask[:, 0]
+    else:
+        hot = ((np.arange(n, dtype=np.uint64) * 0x9E3779B1 % (1 << 32)) >> 16) & 15 == 5
+        Ci[:] = 0.5
+        Cij[:] = np.where(hot, 0.9, 0.4)[:, None] * 0.5 * Cj[None, :] * (1 + 1e-3 * rs.rand(n, 1))
+        w[:] = np.log(Cij / (Ci[:, None] * Cj[None, :]))
+    for it in (3, 16, 32):
+        got = k.update_mask(wmask.copy(), w, Ci, Cj, Cij, 0.01, 2, mc, 0, it)
+        want = port_kernels.update_mask(wmask.copy(), w, Ci, Cj, Cij, 0.01, 2, mc, 0, it)
+        assert np.array_equal(got, want), it
