@@ -1190,6 +1190,8 @@ int current_device() {
 }
 
 bool init_once() {
+  static std::atomic<bool> ready{false};   // the steady state takes no lock
+  if (ready.load(std::memory_order_acquire)) return true;
   std::lock_guard<std::mutex> lock(g_mutex);
   if (g_available < 0) {
     g_available = 0;
@@ -1203,11 +1205,14 @@ bool init_once() {
       (void)cudaGetLastError();
     }
   }
+  ready.store(g_available == 1, std::memory_order_release);
   return g_available == 1;
 }
 
 int *status_word() {
   const int dev = current_device();
+  static std::atomic<int *> known[64];
+  if (int *p = known[dev].load(std::memory_order_acquire)) return p;
   std::lock_guard<std::mutex> lock(g_mutex);
   if (g_status[dev] == nullptr) {
     int *p = nullptr;
@@ -1218,6 +1223,7 @@ int *status_word() {
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
     g_sm_count_tc[dev] = n > 0 ? n : 148;
   }
+  known[dev].store(g_status[dev], std::memory_order_release);
   return g_status[dev];
 }
 
@@ -1398,7 +1404,10 @@ bool tc_available() {
   if (!init_once()) return false;
   int dev = 0, major = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  static std::atomic<int> known[64];   // compute capability of the devices asked about
+  if (dev >= 0 && dev < 64 && (major = known[dev].load()) != 0) return major == 10;
   if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess) return false;
+  if (dev >= 0 && dev < 64) known[dev].store(major);
   return major == 10;
 }
 
@@ -1424,6 +1433,17 @@ constexpr int kLongBN = 128, kLongStages = 5;   // tiles of the row-block produc
 // one more partial result.  A unit count just above a multiple of the SM count would otherwise
 // run a nearly empty last wave (192 units on 148 SMs take as long as 296).
 void forward_split_plan(long B, long N, long M, int &splits, int &k_per_split) {
+  // (a step asks three times for the same shape, and trying every split count costs microseconds)
+  struct Plan {
+    long B, N, M;
+    int splits, k_per_split, dev;
+  };
+  static thread_local Plan last{-1, -1, -1, 0, 0, -1};
+  if (last.B == B && last.N == N && last.M == M && last.dev == current_device()) {
+    splits = last.splits;
+    k_per_split = last.k_per_split;
+    return;
+  }
   const long tiles = ((B + 127) / 128) * ((M + kFwdBN - 1) / kFwdBN);
   const long kblocks = (N + kFwdBK - 1) / kFwdBK;
   const int dev = current_device();
@@ -1447,6 +1467,7 @@ void forward_split_plan(long B, long N, long M, int &splits, int &k_per_split) {
   }
   splits = (int)((kblocks + best_per - 1) / best_per);
   k_per_split = (int)best_per * kFwdBK;
+  last = Plan{B, N, M, splits, k_per_split, dev};
 }
 }  // namespace
 
