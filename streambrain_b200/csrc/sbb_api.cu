@@ -165,6 +165,7 @@ struct sbb_layer {
   Scratch fwd_partial;   // k-split partial sums of the forward product
   Scratch score;         // mask-update scratch: per-row score, active count, candidate lists
   Scratch hx, hy, ht;    // staging for the host-buffer entry points
+  Scratch ticket;        // counts the blocks of a launch that have finished; zero between launches
   Scratch col_hc;        // M ints: hypercolumn of every output column (j / Mc)
   Scratch rc;            // threshold-gated reciprocals of Ci and Cj for the tensor-core trace update
   Scratch lo;            // low parts of x[B, N] and y[B, M] for the split TF32 products of the batch contractions
@@ -231,6 +232,12 @@ struct PhaseTimer {
 template <typename T>
 int layer_forward(sbb_layer *L, const T *x, long B, T *y, cudaStream_t st) {
   const T *W = static_cast<const T *>(L->state[SBB_STATE_WEIGHTS]);
+  if (sbb::narrow_forward(B, L->N, L->M, sizeof(T))) {
+    PhaseTimer timer(L, SBB_PHASE_FORWARD, st);
+    SBB_CUDA(sbb::launch_narrow_forward<T>(x, W, static_cast<const T *>(L->state[SBB_STATE_BIAS]), y, B, L->N, L->M, L->Mc, st));
+    timer.stop();
+    return SBB_OK;
+  }
   bool tc = tensor_path<T>(x, W, L->N, L->M);
   // an unsplit tensor-core product writes straight into y, which must then be 8-byte aligned
   if (tc && sbb::forward_splits_tc(B, L->N, L->M) == 1 && (reinterpret_cast<uintptr_t>(y) & 7u)) tc = false;
@@ -254,25 +261,32 @@ int layer_forward(sbb_layer *L, const T *x, long B, T *y, cudaStream_t st) {
 }
 
 template <typename T>
+sbb::BiasParams<T> layer_bias(const sbb_layer *L) {   // kbi is null for a dense layer: its bias waits for train_finalize
+  return sbb::make_bias<T>(static_cast<T *>(L->state[SBB_STATE_BIAS]), static_cast<T *>(L->state[SBB_STATE_KBI]),
+                           (T)L->desc.khalf, (T)L->desc.pmin, (T)L->desc.taubdt);
+}
+
+template <typename T>
+int layer_mask(sbb_layer *L, long h, cudaStream_t st) {
+  if (L->desc.kind != SBB_LAYER_PLASTIC || h < 0) return SBB_OK;
+  // The score uses the freshly recomputed, un-masked weight of every connection,
+  // which is a function of the traces alone; the masked weights already written
+  // for hypercolumn h are then rewritten under the updated mask.
+  SBB_CUDA(sbb::launch_mask_update<T>(static_cast<uint8_t *>(L->state[SBB_STATE_WMASK]), nullptr,
+                                      static_cast<const T *>(L->state[SBB_STATE_CI]), static_cast<const T *>(L->state[SBB_STATE_CJ]),
+                                      static_cast<const T *>(L->state[SBB_STATE_CIJ]), (T)(L->desc.taupdt / 2), L->N, L->M, L->H,
+                                      L->Mc, h, L->desc.mask_iterations, L->score.d, st, static_cast<T *>(L->state[SBB_STATE_WEIGHTS])));
+  return SBB_OK;
+}
+
+template <typename T>
 int layer_finish(sbb_layer *L, long h, cudaStream_t st) {
   if (L->desc.kind != SBB_LAYER_PLASTIC) return SBB_OK;
-  const double cthr = L->desc.taupdt / 2;
-  T *W = static_cast<T *>(L->state[SBB_STATE_WEIGHTS]);
-  T *Ci = static_cast<T *>(L->state[SBB_STATE_CI]);
-  T *Cj = static_cast<T *>(L->state[SBB_STATE_CJ]);
-  T *Cij = static_cast<T *>(L->state[SBB_STATE_CIJ]);
-  uint8_t *wmask = static_cast<uint8_t *>(L->state[SBB_STATE_WMASK]);
   SBB_CUDA(sbb::launch_update_bias_regularized<T>(static_cast<T *>(L->state[SBB_STATE_BIAS]),
-                                                  static_cast<T *>(L->state[SBB_STATE_KBI]), Cj, (T)cthr,
+                                                  static_cast<T *>(L->state[SBB_STATE_KBI]),
+                                                  static_cast<const T *>(L->state[SBB_STATE_CJ]), (T)(L->desc.taupdt / 2),
                                                   (T)L->desc.khalf, (T)L->desc.pmin, (T)L->desc.taubdt, L->M, st));
-  if (h >= 0) {
-    // The score uses the freshly recomputed, un-masked weight of every connection,
-    // which is a function of the traces alone; the masked weights already written
-    // for hypercolumn h are then rewritten under the updated mask.
-    SBB_CUDA(sbb::launch_mask_update<T>(wmask, nullptr, Ci, Cj, Cij, (T)cthr, L->N, L->M, L->H, L->Mc, h,
-                                        L->desc.mask_iterations, L->score.d, st, W));
-  }
-  return SBB_OK;
+  return layer_mask<T>(L, h, st);
 }
 
 template <typename T>
@@ -280,6 +294,15 @@ int layer_train_step(sbb_layer *L, const T *x, const T *y, long B, long h, cudaS
   const sbb::TraceParams<T> p = sbb::make_trace_params<T>(L->desc.taupdt, L->desc.taupdt / 2, B);
   T *Ci = static_cast<T *>(L->state[SBB_STATE_CI]);
   T *Cj = static_cast<T *>(L->state[SBB_STATE_CJ]);
+  if (sbb::narrow_layer(L->N, L->M)) {
+    PhaseTimer timer(L, SBB_PHASE_TRACE, st);
+    SBB_CUDA(sbb::launch_narrow_train<T>(x, y, B, L->N, L->M, L->H, L->Mc, Ci, Cj, static_cast<T *>(L->state[SBB_STATE_CIJ]),
+                                         static_cast<T *>(L->state[SBB_STATE_WEIGHTS]),
+                                         static_cast<const uint8_t *>(L->state[SBB_STATE_WMASK]), p, layer_bias<T>(L),
+                                         static_cast<int *>(L->ticket.d), st));
+    timer.stop();
+    return layer_mask<T>(L, h, st);
+  }
   const bool tc = tensor_path<T>(x, y, L->N, L->M);
   SBB_CUDA(sbb::launch_colsum<T>(x, B, L->N, nullptr, Ci, p, 1, st));
   SBB_CUDA(sbb::launch_colsum<T>(y, B, L->M, nullptr, Cj, p, 1, st));
@@ -749,6 +772,8 @@ int sbb_layer_create(const sbb_layer_desc *desc, sbb_layer **out) {
     }
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&L->own_stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) rc = cuda_fail(e, "layer_create");
+  if (rc == SBB_OK) rc = L->ticket.reserve(256);
+  if (rc == SBB_OK && (e = cudaMemsetAsync(L->ticket.d, 0, 256, 0)) != cudaSuccess) rc = cuda_fail(e, "layer_create");
   if (rc == SBB_OK) rc = L->rc.reserve(sbb::tc_trace_scratch_bytes(L->N, L->M));
   if (rc == SBB_OK && desc->kind == SBB_LAYER_PLASTIC) {
     rc = L->score.reserve(sbb::mask_scratch_bytes(L->N, s));
@@ -761,6 +786,8 @@ int sbb_layer_create(const sbb_layer_desc *desc, sbb_layer **out) {
       if (e != cudaSuccess) rc = cuda_fail(e, "layer_create");
     }
   }
+  // the caller may step the layer on a stream that does not wait for these initialisations
+  if (rc == SBB_OK && (e = cudaStreamSynchronize(0)) != cudaSuccess) rc = cuda_fail(e, "layer_create");
   if (rc != SBB_OK) {
     std::string keep = g_error;
     sbb_layer_destroy(L);
@@ -781,6 +808,7 @@ int sbb_layer_destroy(sbb_layer *L) {
   L->hy.release();
   L->ht.release();
   L->col_hc.release();
+  L->ticket.release();
   L->rc.release();
   L->lo.release();
   if (L->shard.on) {

@@ -1114,24 +1114,26 @@ template cudaError_t launch_update_bias<float>(float *, const float *, float, lo
 template cudaError_t launch_update_bias<double>(double *, const double *, double, long, cudaStream_t);
 
 template <typename T>
+BiasParams<T> make_bias(T *bias, T *kbi, T khalf, T pmin, T taubdt) {
+  const T pmin4 = pmin / (T)4;
+  return BiasParams<T>{bias, kbi, khalf, pmin4, (khalf - (T)1) * (pmin4 * pmin4), taubdt};
+}
+template BiasParams<float> make_bias<float>(float *, float *, float, float, float);
+template BiasParams<double> make_bias<double>(double *, double *, double, double, double);
+
+template <typename T>
 __global__ void update_bias_regularized_kernel(T *bias, T *kbi, const T *__restrict__ Cj, T cthr, T khalf, T pmin4,
                                                T k, T taubdt, long M) {
   const long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= M) return;
-  const T pj = Cj[j];
-  T kb = (T)1 + k / ((pj - pmin4) * (pj - pmin4));
-  if (pj < pmin4 || kb < khalf) kb = khalf;
-  const T g = ((T)1 - taubdt) * kbi[j] + taubdt * kb;
-  kbi[j] = g;
-  bias[j] = pj < cthr ? g * sbb_log((T)2 * cthr) : g * sbb_log(pj);
+  bias_regularized(bias[j], kbi[j], Cj[j], cthr, khalf, pmin4, k, taubdt);
 }
 template <typename T>
 cudaError_t launch_update_bias_regularized(T *bias, T *kbi, const T *Cj, T cthr, T khalf, T pmin, T taubdt, long M,
                                            cudaStream_t st) {
   if (M == 0) return cudaSuccess;
-  const T pmin4 = pmin / (T)4;
-  const T k = (khalf - (T)1) * (pmin4 * pmin4);
-  update_bias_regularized_kernel<T><<<(unsigned)((M + 255) / 256), 256, 0, st>>>(bias, kbi, Cj, cthr, khalf, pmin4, k,
+  const BiasParams<T> b = make_bias<T>(bias, kbi, khalf, pmin, taubdt);
+  update_bias_regularized_kernel<T><<<(unsigned)((M + 255) / 256), 256, 0, st>>>(bias, kbi, Cj, cthr, khalf, b.pmin4, b.k,
                                                                                   taubdt, M);
   return launched();
 }

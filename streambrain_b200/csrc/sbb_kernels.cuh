@@ -49,6 +49,24 @@ cudaError_t launch_colsum(const T *a, long B, long cols, T *sums, T *c, TracePar
 template <typename T>
 cudaError_t launch_vector_ema(T *c, const T *sums, long n, TraceParams<T> p, cudaStream_t st);
 
+// Layers of at most 32 units: the forward pass (contraction, bias, softmax) and the train step (Ci, Cj, Cij, weights
+// and, with kbi != null, the regularised bias) as one launch each.  `ticket`: one int, zero between launches.
+template <typename T>
+struct BiasParams {
+  T *bias, *kbi;
+  T khalf, pmin4, k, taubdt;
+};
+template <typename T>
+BiasParams<T> make_bias(T *bias, T *kbi, T khalf, T pmin, T taubdt);
+bool narrow_layer(long N, long M);
+bool narrow_forward(long B, long N, long M, size_t elem);
+template <typename T>
+cudaError_t launch_narrow_forward(const T *x, const T *W, const T *bias, T *out, long B, long N, long M, long Mc,
+                                  cudaStream_t st);
+template <typename T>
+cudaError_t launch_narrow_train(const T *x, const T *y, long B, long N, long M, long H, long Mc, T *Ci, T *Cj, T *Cij, T *W,
+                                const uint8_t *wmask, TraceParams<T> p, BiasParams<T> nb, int *ticket, cudaStream_t st);
+
 // Fused trace step for rows [row_begin,row_end) of Cij: acc = x^T y over the batch,
 // Cij = EMA(Cij, acc), w = log-ratio(Cij, Ci, Cj) with rows/columns below cthr and
 // masked connections (wmask may be null) set to zero.  Ci, Cj hold the NEW values.

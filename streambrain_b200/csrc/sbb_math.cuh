@@ -30,6 +30,16 @@ __device__ __forceinline__ T log_ratio(T cij, T ci, T cj, T cthr4) {
   return sbb_log(num / (ci * cj));
 }
 
+// One unit's gain and bias from its new trace (kernels_openmp_internal.cc:221-246); k = (khalf - 1) pmin4^2.
+template <typename T>
+__device__ __forceinline__ void bias_regularized(T &bias, T &kbi, T pj, T cthr, T khalf, T pmin4, T k, T taubdt) {
+  T kb = (T)1 + k / ((pj - pmin4) * (pj - pmin4));
+  if (pj < pmin4 || kb < khalf) kb = khalf;
+  const T g = ((T)1 - taubdt) * kbi + taubdt * kb;
+  kbi = g;
+  bias = pj < cthr ? g * sbb_log((T)2 * cthr) : g * sbb_log(pj);
+}
+
 // The arithmetic of the tensor-core path (fused epilogue, and the element-wise tail of the
 // data-parallel step when that path is selected): the batch mean and the moving-average weight
 // folded into one factor taupdt / batch, the ratio by IEEE reciprocals of Ci and Cj formed once per

@@ -1,0 +1,290 @@
+// Layers with few units (the 10-class output layer above all): both halves of a step as one launch each.
+//
+// Such a layer is nothing but latency: 3000 x 10 weights are 120 kB, the whole step some 2 MB of traffic and 15 MFLOP.
+// The tiled contraction kernels spend it on 128-column tiles that are nine tenths padding and on one dependent round
+// trip to memory per k-slab, and the column sums, the reduction with the softmax and the bias are launches of their
+// own: the 3000 -> 10 layer at batch 128 took 20.4 + 5.7 us for the forward pass and 31.0 + 2 x 2.6 us for the train
+// step.  Here every thread has all its loads of the inputs in flight at once.
+#include "sbb_kernels.cuh"
+#include "sbb_math.cuh"
+
+namespace sbb {
+
+void count_launches(int n);   // sbb_kernels.cu
+
+namespace {
+
+inline cudaError_t launched() {
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+// ----------------------------------------------------------------------------
+// out[b, :] = softmax per hypercolumn of (x[b, :] W + bias), M <= MP units.  WARPS warps share R samples: each thread
+// takes every (32 * WARPS)-th input, keeps R x MP sums, and shuffles and one pass through shared memory add them up.
+// ----------------------------------------------------------------------------
+template <typename T, int MP, int R, int WARPS>
+__global__ void __launch_bounds__(256)
+    narrow_forward_kernel(const T *__restrict__ x, const T *__restrict__ W, const T *__restrict__ bias, T *__restrict__ out,
+                          long B, int N, int M, int Mc) {
+  constexpr int SETS = 8 / WARPS;   // groups of R samples per block
+  __shared__ T part[8][R][MP];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int set = wid / WARPS;
+  const long b0 = ((long)blockIdx.x * SETS + set) * R;
+  T acc[R][MP];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int j = 0; j < MP; ++j) acc[r][j] = (T)0;
+  constexpr int STEP = 32 * WARPS;
+  constexpr int U = R > 2 || MP * (int)sizeof(T) > 64 ? 1 : (MP * (int)sizeof(T) > 32 ? 2 : 4);   // inputs in flight per thread, as registers allow
+  for (int k0 = (wid % WARPS) * 32 + lane; k0 < N; k0 += U * STEP) {
+    T xv[U][R], w[U][MP];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 + u * STEP;
+#pragma unroll
+      for (int r = 0; r < R; ++r) xv[u][r] = k < N && b0 + r < B ? x[(b0 + r) * N + k] : (T)0;
+#pragma unroll
+      for (int j = 0; j < MP; ++j) w[u][j] = k < N && j < M ? W[(long)k * M + j] : (T)0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int j = 0; j < MP; ++j) acc[r][j] = fma(xv[u][r], w[u][j], acc[r][j]);
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int j = 0; j < MP; ++j) {
+      T v = acc[r][j];
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+      if (lane == 0) part[wid][r][j] = v;
+    }
+  __syncthreads();
+  // the support of (sample, unit) in the first warp's slots, then the softmax of its hypercolumn
+  for (int t = threadIdx.x; t < SETS * R * M; t += 256) {
+    const int s = t / (R * M), r = t / M % R, j = t % M;
+    T v = part[s * WARPS][r][j];
+#pragma unroll
+    for (int w = 1; w < WARPS; ++w) v += part[s * WARPS + w][r][j];
+    part[s * WARPS][r][j] = v + bias[j];
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < SETS * R * M; t += 256) {
+    const int s = t / (R * M), r = t / M % R, j = t % M;
+    const long b = ((long)blockIdx.x * SETS + s) * R + r;
+    if (b >= B) continue;
+    const T *v = part[s * WARPS][r] + j / Mc * Mc;
+    T mx = v[0];
+    for (int q = 1; q < Mc; ++q) mx = v[q] > mx ? v[q] : mx;
+    T sum = (T)0;
+    for (int q = 0; q < Mc; ++q) sum += sbb_exp(v[q] - mx);
+    out[b * M + j] = sbb_exp(v[j % Mc] - mx) / sum;
+  }
+}
+
+// ----------------------------------------------------------------------------
+// The whole train step but the mask: Ci, Cj, Cij, weights, and (kbi != null) the regularised bias.  A block owns 32
+// inputs: lane = input, warp = every eighth sample; the targets pass through shared memory, where all lanes read the same
+// word.  Every block forms the new Cj for itself (it reads all targets anyway); the old one stays in place until the
+// last block writes the new one and the bias.
+// ----------------------------------------------------------------------------
+template <typename T, int MP>
+struct NarrowTrain {
+  static constexpr int STAGE = sizeof(T) * MP <= 128 ? 128 : 64;   // samples of the targets in shared memory at a time
+  static constexpr int CH = sizeof(T) == 4 && MP > 16 ? 16 : (sizeof(T) == 8 ? 8 : MP);   // units reduced at a time
+};
+
+template <typename T, int MP>
+__global__ void __launch_bounds__(256)
+    narrow_train_kernel(const T *__restrict__ x, const T *__restrict__ y, long B, int N, int M, int H, int Mc, T *Ci, T *Cj,
+                        T *Cij, T *W, const uint8_t *__restrict__ wmask, TraceParams<T> p, BiasParams<T> nb, int *ticket) {
+  constexpr int STAGE = NarrowTrain<T, MP>::STAGE, CH = NarrowTrain<T, MP>::CH;
+  constexpr int NCH = MP / CH, E = 32 * CH / 256;   // outputs per thread: NCH chunks of E
+  __shared__ __align__(16) T ys[STAGE][MP];
+  __shared__ T red[8][32][CH + 1], redx[8][32];
+  __shared__ T cj_new[MP], ci_new[32];
+  __shared__ int s_last;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const long i0 = (long)blockIdx.x * 32, i = i0 + lane;
+  const int rows = (int)(N - i0 < 32 ? N - i0 : 32);
+  constexpr int U = STAGE / 8;             // a warp's samples of a stage
+  constexpr int UY = STAGE * MP / 256;     // a thread's targets of a stage
+  T xv[U], yv[UY];
+  auto fetch = [&](long c0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) xv[u] = c0 + wid + 8 * u < B && i < N ? x[(c0 + wid + 8 * u) * N + i] : (T)0;
+#pragma unroll
+    for (int u = 0; u < UY; ++u) {
+      const int t = threadIdx.x + 256 * u, b = t / MP, j = t % MP;
+      yv[u] = c0 + b < B && j < M ? y[(c0 + b) * M + j] : (T)0;
+    }
+  };
+  fetch(0);
+  // the old state too is on its way before the sums are formed
+  T old[NCH][E], c_old = (T)0;
+  uint8_t bit[NCH][E];
+#pragma unroll
+  for (int c = 0; c < NCH; ++c)
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int t = threadIdx.x + 256 * e, r = t / CH, j = c * CH + t % CH;
+      const bool in = r < rows && j < M;
+      old[c][e] = in ? Cij[(i0 + r) * M + j] : (T)0;
+      bit[c][e] = in && wmask != nullptr ? wmask[(i0 + r) * H + j / Mc] : (uint8_t)1;
+    }
+  if (threadIdx.x < 32) {
+    if ((int)threadIdx.x < rows) c_old = Ci[i0 + threadIdx.x];
+  } else if ((int)threadIdx.x - 32 < M) {
+    c_old = Cj[threadIdx.x - 32];
+  }
+  T acc[MP], sx = (T)0, sy = (T)0;
+#pragma unroll
+  for (int j = 0; j < MP; ++j) acc[j] = (T)0;
+  for (long c0 = 0; c0 < B; c0 += STAGE) {
+    const int len = (int)(B - c0 < STAGE ? B - c0 : STAGE);
+    if (c0 > 0) __syncthreads();   // the previous stage has been read
+    T xs[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) xs[u] = xv[u];
+#pragma unroll
+    for (int u = 0; u < UY; ++u) (&ys[0][0])[threadIdx.x + 256 * u] = yv[u];
+    __syncthreads();
+    if (c0 + STAGE < B) fetch(c0 + STAGE);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      sx += xs[u];   // (samples past the end are zero)
+#pragma unroll
+      for (int j = 0; j < MP; ++j) acc[j] = fma(xs[u], ys[wid + 8 * u][j], acc[j]);
+    }
+    // column sums of the targets: 256 / MP threads per column
+    for (int b = threadIdx.x / MP; b < len; b += 256 / MP) sy += ys[b][threadIdx.x % MP];
+  }
+  redx[wid][lane] = sx;
+  __syncthreads();
+  T *ysum = &ys[0][0];   // [256 / MP][MP]
+  ysum[threadIdx.x] = sy;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    if ((int)threadIdx.x < rows) {
+      T s = redx[0][threadIdx.x];
+#pragma unroll
+      for (int w = 1; w < 8; ++w) s += redx[w][threadIdx.x];
+      const T c = trace_ema(c_old, s, p);
+      Ci[i0 + threadIdx.x] = c;
+      ci_new[threadIdx.x] = c;
+    }
+  } else if ((int)threadIdx.x - 32 < M) {
+    const int j = threadIdx.x - 32;
+    T s = ysum[j];
+#pragma unroll 4
+    for (int k = 1; k < 256 / MP; ++k) s += ysum[k * MP + j];
+    cj_new[j] = trace_ema(c_old, s, p);
+  }
+#pragma unroll
+  for (int c = 0; c < NCH; ++c) {
+    if (c > 0) __syncthreads();
+#pragma unroll
+    for (int j = 0; j < CH; ++j) red[wid][lane][j] = acc[c * CH + j];
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int t = threadIdx.x + 256 * e, r = t / CH, j = c * CH + t % CH;
+      if (r >= rows || j >= M) continue;
+      T s = red[0][r][t % CH];
+#pragma unroll
+      for (int w = 1; w < 8; ++w) s += red[w][r][t % CH];
+      const T v = trace_ema(old[c][e], s, p);
+      const T ci = ci_new[r], cj = cj_new[j];
+      const bool on = !(ci < p.cthr) && !(cj < p.cthr) && bit[c][e] != 0;
+      const long at = (i0 + r) * M + j;
+      Cij[at] = v;
+      W[at] = on ? log_ratio(v, ci, cj, p.cthr4) : (T)0;
+    }
+  }
+  // the block that finishes last: no other one needs the old Cj any more
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  if (threadIdx.x == 0) *ticket = 0;
+  if ((int)threadIdx.x < M) {
+    const T cj = cj_new[threadIdx.x];
+    Cj[threadIdx.x] = cj;
+    if (nb.kbi != nullptr) bias_regularized(nb.bias[threadIdx.x], nb.kbi[threadIdx.x], cj, p.cthr, nb.khalf, nb.pmin4, nb.k, nb.taubdt);
+  }
+}
+
+// Samples a thread can keep sums for: 64 registers of them.
+constexpr int narrow_samples(long M, size_t elem) { return (M <= 8 ? 8 : (M <= 16 ? 4 : 2)) / (elem == 8 ? 2 : 1); }
+
+template <typename T, int MP>
+cudaError_t forward_mp(const T *x, const T *W, const T *bias, T *out, long B, long N, long M, long Mc, cudaStream_t st) {
+  constexpr int RMAX = narrow_samples(MP, sizeof(T));
+  // few samples: one per block (or warp), so that all SMs take part; more of them share each read of the weights
+  const long per = (B + 295) / 296;
+#define SBB_NARROW_FWD(R)                                                                                              \
+  do {                                                                                                                 \
+    if (N <= 512) /* not enough inputs to share among the warps of a block */                                          \
+      narrow_forward_kernel<T, MP, R, 1><<<(unsigned)((B + 8 * R - 1) / (8 * R)), 256, 0, st>>>(x, W, bias, out, B, (int)N, (int)M, (int)Mc); \
+    else                                                                                                               \
+      narrow_forward_kernel<T, MP, R, 8><<<(unsigned)((B + R - 1) / R), 256, 0, st>>>(x, W, bias, out, B, (int)N, (int)M, (int)Mc); \
+  } while (0)
+  if (per <= 1 || RMAX == 1) SBB_NARROW_FWD(1);
+  else if (per <= 2 || RMAX == 2) SBB_NARROW_FWD((RMAX < 2 ? RMAX : 2));
+  else if (per <= 4 || RMAX == 4) SBB_NARROW_FWD((RMAX < 4 ? RMAX : 4));
+  else SBB_NARROW_FWD(RMAX);
+#undef SBB_NARROW_FWD
+  return launched();
+}
+
+}  // namespace
+
+// Up to 32 units; beyond that the tiles of the contraction kernels are full enough.  The forward pass reads all weights
+// once per block of samples: with very many samples that is more L2 traffic than the tiled kernels cause.
+bool narrow_layer(long N, long M) { return M <= 32 && N < (1l << 30); }
+bool narrow_forward(long B, long N, long M, size_t elem) {
+  const long r = narrow_samples(M, elem);
+  return narrow_layer(N, M) && ((B + r - 1) / r) * N * M <= (1l << 28);
+}
+
+template <typename T>
+cudaError_t launch_narrow_forward(const T *x, const T *W, const T *bias, T *out, long B, long N, long M, long Mc,
+                                  cudaStream_t st) {
+  if (M <= 8) return forward_mp<T, 8>(x, W, bias, out, B, N, M, Mc, st);
+  if (M <= 16) return forward_mp<T, 16>(x, W, bias, out, B, N, M, Mc, st);
+  return forward_mp<T, 32>(x, W, bias, out, B, N, M, Mc, st);
+}
+template cudaError_t launch_narrow_forward<float>(const float *, const float *, const float *, float *, long, long, long, long,
+                                                  cudaStream_t);
+template cudaError_t launch_narrow_forward<double>(const double *, const double *, const double *, double *, long, long, long,
+                                                   long, cudaStream_t);
+
+template <typename T>
+cudaError_t launch_narrow_train(const T *x, const T *y, long B, long N, long M, long H, long Mc, T *Ci, T *Cj, T *Cij, T *W,
+                                const uint8_t *wmask, TraceParams<T> p, BiasParams<T> nb, int *ticket, cudaStream_t st) {
+  const unsigned blocks = (unsigned)((N + 31) / 32);
+#define SBB_NARROW_TRAIN(MP)                                                                                            \
+  narrow_train_kernel<T, MP><<<blocks, 256, 0, st>>>(x, y, B, (int)N, (int)M, (int)H, (int)Mc, Ci, Cj, Cij, W, wmask, p, nb, ticket)
+  if (M <= 8) SBB_NARROW_TRAIN(8);
+  else if (M <= 16) SBB_NARROW_TRAIN(16);
+  else SBB_NARROW_TRAIN(32);
+#undef SBB_NARROW_TRAIN
+  return launched();
+}
+template cudaError_t launch_narrow_train<float>(const float *, const float *, long, long, long, long, long, float *, float *,
+                                                float *, float *, const uint8_t *, TraceParams<float>, BiasParams<float>, int *,
+                                                cudaStream_t);
+template cudaError_t launch_narrow_train<double>(const double *, const double *, long, long, long, long, long, double *,
+                                                 double *, double *, double *, const uint8_t *, TraceParams<double>,
+                                                 BiasParams<double>, int *, cudaStream_t);
+
+}  // namespace sbb

@@ -531,3 +531,43 @@ def test_errors_are_reported_not_fatal(B200):
     out = layer.compute_activation(np.random.rand(4, 8).astype(np.float32))
     assert np.allclose(out.reshape(4, 2, 2).sum(axis=2), 1.0, atol=1e-6)
     assert _lib.lib.sbb_kernel_launches() > 0
+
+
+@pytest.mark.parametrize("tag,dtype", [("f32", np.float32), ("f64", np.float64)])
+@pytest.mark.parametrize("kind", ["dense", "plastic"])
+@pytest.mark.parametrize("B,N,H,Mc", [(1, 1, 1, 2), (3, 31, 1, 8), (64, 33, 3, 3), (65, 512, 2, 8), (129, 513, 1, 10),
+                                      (300, 700, 5, 5), (700, 1040, 4, 8), (2500, 96, 1, 6), (130, 2050, 16, 2)])
+def test_layers_of_few_units_vs_oracle(port_kernels, tag, dtype, kind, B, N, H, Mc):
+    """At most 32 units: forward pass and train step run as one launch each.  Sizes around the blocks of 32 inputs, the
+    stages of 64 and 128 samples, one to eight samples per block, and 8, 16 and 32 units."""
+    import oracle
+    import streambrain_b200 as B200
+    hp = dict(taupdt=0.05, khalf=-100.0, pmin=0.05, taubdt=0.02, density=0.5)
+    rs = np.random.RandomState(B + N)
+    init = (0.5, 1 / Mc, 0.5 / Mc)
+    np.random.seed(0)
+    if kind == "dense":
+        dev = B200.DenseLayer(N, H, Mc, hp["taupdt"], init, dtype=dtype)
+    else:
+        dev = B200.StructuralPlasticityLayer(N, H, Mc, hp["taupdt"], hp["khalf"], hp["pmin"], hp["taubdt"], hp["density"],
+                                             16, init, dtype=dtype)
+    np.random.seed(0)
+    ref = oracle.OracleLayer(port_kernels, kind, N, H, Mc, hp["taupdt"], init, dtype,
+                             **({} if kind == "dense" else {k: hp[k] for k in ("khalf", "pmin", "taubdt", "density")}))
+    tol = TOL[np.dtype(dtype)]
+    for step in range(3):
+        x = rs.rand(B, N).astype(dtype)
+        a_ref, a_dev = ref.compute_activation(x), dev.compute_activation(x)
+        assert rel_inf(a_dev, a_ref) < tol, step
+        if kind == "dense":
+            t = np.eye(H * Mc, dtype=dtype)[rs.randint(0, H * Mc, B)]
+            ref.train_step(x, t)
+            dev.train_step(x, t)
+        else:
+            ref.train_step(x, a_ref, None)
+            dev.train_step(x, a_ref, None)
+        for name in ("Ci", "Cj", "Cij", "bias"):
+            assert rel_inf(getattr(dev, name), getattr(ref, name)) < tol, (name, step)
+        assert weight_err(dev.weights, ref.weights) < 10 * tol, step
+        for name in ("weights", "bias", "Ci", "Cj", "Cij"):
+            setattr(dev, name, getattr(ref, name))
