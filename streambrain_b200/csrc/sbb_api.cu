@@ -166,8 +166,7 @@ struct sbb_layer {
   Scratch score;         // mask-update scratch: per-row score, active count, candidate lists
   Scratch hx, hy, ht;    // staging for the host-buffer entry points
   Scratch ticket;        // counts the blocks of a launch that have finished; zero between launches
-  Scratch col_hc;        // M ints: hypercolumn of every output column (j / Mc)
-  Scratch rc;            // threshold-gated reciprocals of Ci and Cj for the tensor-core trace update
+  Scratch rc;            // reciprocals of Ci and Cj (0 below the threshold) for the tensor-core trace update
   Scratch lo;            // low parts of x[B, N] and y[B, M] for the split TF32 products of the batch contractions
   long lo_batch = 0;     // batch rows the planes in `lo` were written for (0 = none)
   cudaStream_t own_stream = nullptr;
@@ -215,7 +214,7 @@ struct PhaseTimer {
   cudaStream_t st;
   long slot = -1;
   PhaseTimer(sbb_layer *l, int ph, cudaStream_t s) : L(l), phase(ph), st(s) {
-    if (L->profiling) {
+    if (L != nullptr && L->profiling) {
       slot = L->phase_calls[phase] % SBB_PROFILE_SLOTS;
       cudaEventRecord(L->ev_begin[phase][slot], st);
     }
@@ -229,10 +228,18 @@ struct PhaseTimer {
   }
 };
 
+// Whether the kernels for layers of few units may take the layer: they sum in another order than the tiled ones.  In a
+// float32 layer that learns from its own activations a difference in the last digit of an activation reaches the weights
+// of all its inputs alike and adds up over tens of thousands of them in the next forward pass, so those keep their order.
+template <typename T>
+bool narrow(const sbb_layer *L) {
+  return std::is_same<T, double>::value || L->desc.kind == SBB_LAYER_DENSE;
+}
+
 template <typename T>
 int layer_forward(sbb_layer *L, const T *x, long B, T *y, cudaStream_t st) {
   const T *W = static_cast<const T *>(L->state[SBB_STATE_WEIGHTS]);
-  if (sbb::narrow_forward(B, L->N, L->M, sizeof(T))) {
+  if (narrow<T>(L) && sbb::narrow_forward(B, L->N, L->M, sizeof(T))) {
     PhaseTimer timer(L, SBB_PHASE_FORWARD, st);
     SBB_CUDA(sbb::launch_narrow_forward<T>(x, W, static_cast<const T *>(L->state[SBB_STATE_BIAS]), y, B, L->N, L->M, L->Mc, st));
     timer.stop();
@@ -289,12 +296,38 @@ int layer_finish(sbb_layer *L, long h, cudaStream_t st) {
   return layer_mask<T>(L, h, st);
 }
 
+// Traces, weights and (bias.kbi != null) the bias of `N` input rows.  `L` (may be null) times the contraction; `vectors`
+// holds the reciprocals of Ci and Cj on the tensor path.
+template <typename T>
+int train_rows(sbb_layer *L, const T *x, const T *y, long B, long N, long M, long H, T *Ci, T *Cj, T *Cij, T *W,
+               const uint8_t *wmask, const sbb::TraceParams<T> &p, const sbb::BiasParams<T> &bias, Scratch &vectors,
+               cudaStream_t st) {
+  const bool tc = N > 0 && tensor_path<T>(x, y, N, M);
+  T *rci = nullptr, *rcj = nullptr;
+  if (tc) {
+    SBB_TRY(vectors.reserve((size_t)((N + 3) / 4 * 4 + M) * sizeof(T)));
+    rci = static_cast<T *>(vectors.d);
+    rcj = rci + (N + 3) / 4 * 4;
+  }
+  SBB_CUDA(sbb::launch_column_vectors<T>(sbb::ColumnVectors<T>{x, N, Ci, rci}, sbb::ColumnVectors<T>{y, M, Cj, rcj}, B, p, bias, st));
+  if (N == 0) return SBB_OK;
+  PhaseTimer timer(L, SBB_PHASE_TRACE, st);
+  if (tc) {
+    if constexpr (std::is_same<T, float>::value)
+      SBB_CUDA(sbb::launch_trace_update_tc(x, y, B, N, M, wmask ? H : 0, rci, rcj, Cij, W, wmask, p, st));
+  } else {
+    SBB_CUDA(sbb::launch_trace_update_fused<T>(x, y, B, N, M, H, M / H, Ci, Cj, Cij, W, wmask, p, 0, N, st));
+  }
+  timer.stop();
+  return SBB_OK;
+}
+
 template <typename T>
 int layer_train_step(sbb_layer *L, const T *x, const T *y, long B, long h, cudaStream_t st) {
   const sbb::TraceParams<T> p = sbb::make_trace_params<T>(L->desc.taupdt, L->desc.taupdt / 2, B);
   T *Ci = static_cast<T *>(L->state[SBB_STATE_CI]);
   T *Cj = static_cast<T *>(L->state[SBB_STATE_CJ]);
-  if (sbb::narrow_layer(L->N, L->M)) {
+  if (narrow<T>(L) && sbb::narrow_layer(L->N, L->M)) {
     PhaseTimer timer(L, SBB_PHASE_TRACE, st);
     SBB_CUDA(sbb::launch_narrow_train<T>(x, y, B, L->N, L->M, L->H, L->Mc, Ci, Cj, static_cast<T *>(L->state[SBB_STATE_CIJ]),
                                          static_cast<T *>(L->state[SBB_STATE_WEIGHTS]),
@@ -303,31 +336,14 @@ int layer_train_step(sbb_layer *L, const T *x, const T *y, long B, long h, cudaS
     timer.stop();
     return layer_mask<T>(L, h, st);
   }
-  const bool tc = tensor_path<T>(x, y, L->N, L->M);
-  SBB_CUDA(sbb::launch_colsum<T>(x, B, L->N, nullptr, Ci, p, 1, st));
-  SBB_CUDA(sbb::launch_colsum<T>(y, B, L->M, nullptr, Cj, p, 1, st));
-  PhaseTimer timer(L, SBB_PHASE_TRACE, st);
-  if (tc) {
-    if constexpr (std::is_same<T, float>::value)
-      SBB_CUDA(sbb::launch_trace_update_tc(x, y, B, L->N, L->M, L->H, Ci, Cj, static_cast<T *>(L->state[SBB_STATE_CIJ]),
-                                           static_cast<T *>(L->state[SBB_STATE_WEIGHTS]),
-                                           static_cast<const uint8_t *>(L->state[SBB_STATE_WMASK]),
-                                           static_cast<const int *>(L->col_hc.d), static_cast<float *>(L->rc.d), p,
-                                           0, L->N, st));
-  } else {
-    SBB_CUDA(sbb::launch_trace_update_fused<T>(x, y, B, L->N, L->M, L->H, L->Mc, Ci, Cj,
-                                               static_cast<T *>(L->state[SBB_STATE_CIJ]),
-                                               static_cast<T *>(L->state[SBB_STATE_WEIGHTS]),
-                                               static_cast<const uint8_t *>(L->state[SBB_STATE_WMASK]), p, 0, L->N,
-                                               st));
-  }
-  timer.stop();
-  return layer_finish<T>(L, h, st);
+  SBB_TRY(train_rows<T>(L, x, y, B, L->N, L->M, L->H, Ci, Cj, static_cast<T *>(L->state[SBB_STATE_CIJ]),
+                        static_cast<T *>(L->state[SBB_STATE_WEIGHTS]), static_cast<const uint8_t *>(L->state[SBB_STATE_WMASK]), p,
+                        layer_bias<T>(L), L->rc, st));
+  return layer_mask<T>(L, h, st);
 }
 
 template <typename T>
 int layer_dp_local(sbb_layer *L, const T *x, const T *y, long B, T *delta, long rb, long re, cudaStream_t st) {
-  sbb::TraceParams<T> p = sbb::make_trace_params<T>(L->desc.taupdt, L->desc.taupdt / 2, B);
   T *xty = delta + L->N + L->M;
   // remembered for sbb_layer_dp_apply_rows: the element-wise tail uses the arithmetic of the path that formed the sums
   L->dp_fast = tensor_path<T>(x, y, L->N, L->M) && (reinterpret_cast<uintptr_t>(xty) & 7u) == 0;
@@ -336,8 +352,8 @@ int layer_dp_local(sbb_layer *L, const T *x, const T *y, long B, T *delta, long 
     // the first row block of a step also forms the column sums and, for the tensor path, the operands' low parts,
     // which the later row blocks of the same step (same x, y, B) re-use
     SBB_TRY(reserve_lo<T>(L->lo, B, L->N, L->M, L->dp_fast, &lo));
-    SBB_CUDA(sbb::launch_colsum<T>(x, B, L->N, delta, nullptr, p, 0, st, lo_as<T>(lo.x)));
-    SBB_CUDA(sbb::launch_colsum<T>(y, B, L->M, delta + L->N, nullptr, p, 0, st, lo_as<T>(lo.y)));
+    SBB_CUDA(sbb::launch_colsum<T>(x, B, L->N, delta, st, lo_as<T>(lo.x)));
+    SBB_CUDA(sbb::launch_colsum<T>(y, B, L->M, delta + L->N, st, lo_as<T>(lo.y)));
     L->lo_batch = lo.x ? B : 0;
   } else if (L->dp_fast && L->lo_batch == B) {
     lo.x = static_cast<float *>(L->lo.d);
@@ -548,7 +564,6 @@ int update_counters_t(void *Ci, void *Cj, void *Cij, const void *a_i, const void
   SBB_TRY(dx.upload(a_i, B * N * s));
   SBB_TRY(dy.upload(a_o, B * M * s));
   SBB_TRY(sums.alloc((size_t)(N + M + N * M + 4) * s));
-  const sbb::TraceParams<T> p = sbb::make_trace_params<T>(taupdt, taupdt / 2, B);
   T *sx = sums.as<T>();
   T *sy = sx + N;
   // keep the [N, M] block 16-byte aligned whatever N + M is
@@ -559,8 +574,8 @@ int update_counters_t(void *Ci, void *Cj, void *Cij, const void *a_i, const void
   int lo_rc = reserve_lo<T>(lo_buf, B, N, M, tc, &lo);
   struct Release { Scratch &s; ~Release() { s.release(); } } release_lo{lo_buf};
   SBB_TRY(lo_rc);
-  SBB_CUDA(sbb::launch_colsum<T>(dx.as<T>(), B, N, sx, nullptr, p, 0, 0, lo_as<T>(lo.x)));
-  SBB_CUDA(sbb::launch_colsum<T>(dy.as<T>(), B, M, sy, nullptr, p, 0, 0, lo_as<T>(lo.y)));
+  SBB_CUDA(sbb::launch_colsum<T>(dx.as<T>(), B, N, sx, 0, lo_as<T>(lo.x)));
+  SBB_CUDA(sbb::launch_colsum<T>(dy.as<T>(), B, M, sy, 0, lo_as<T>(lo.y)));
   if (tc) {
     if constexpr (std::is_same<T, float>::value)
       SBB_CUDA(sbb::launch_outer_product_tc(dx.as<T>(), dy.as<T>(), B, N, M, sxy, 0, N, 0, lo.x, lo.y));
@@ -587,20 +602,11 @@ int update_weights_t(void *Ci, void *Cj, void *Cij, const void *a_i, const void 
   SBB_TRY(dx.upload(a_i, B * N * s));
   SBB_TRY(dy.upload(a_o, B * M * s));
   SBB_TRY(dw.alloc(N * M * s));
-  Staged drc;
-  SBB_TRY(drc.alloc(sbb::tc_trace_scratch_bytes(N, M)));
-  const sbb::TraceParams<T> p = sbb::make_trace_params<T>(taupdt, cthr, B);
-  const bool tc = tensor_path<T>(dx.d, dy.d, N, M);
-  SBB_CUDA(sbb::launch_colsum<T>(dx.as<T>(), B, N, nullptr, dci.as<T>(), p, 1, 0));
-  SBB_CUDA(sbb::launch_colsum<T>(dy.as<T>(), B, M, nullptr, dcj.as<T>(), p, 1, 0));
-  if (tc) {
-    if constexpr (std::is_same<T, float>::value)
-      SBB_CUDA(sbb::launch_trace_update_tc(dx.as<T>(), dy.as<T>(), B, N, M, 1, dci.as<T>(), dcj.as<T>(), dcij.as<T>(),
-                                           dw.as<T>(), nullptr, nullptr, drc.as<float>(), p, 0, N, 0));
-  } else {
-    SBB_CUDA(sbb::launch_trace_update_fused<T>(dx.as<T>(), dy.as<T>(), B, N, M, 1, M, dci.as<T>(), dcj.as<T>(),
-                                               dcij.as<T>(), dw.as<T>(), nullptr, p, 0, N, 0));
-  }
+  struct Vectors : Scratch {
+    ~Vectors() { release(); }
+  } vectors;
+  SBB_TRY(train_rows<T>(nullptr, dx.as<T>(), dy.as<T>(), B, N, M, 1, dci.as<T>(), dcj.as<T>(), dcij.as<T>(), dw.as<T>(), nullptr,
+                        sbb::make_trace_params<T>(taupdt, cthr, B), sbb::BiasParams<T>{}, vectors, 0));
   SBB_CUDA(cudaDeviceSynchronize());
   SBB_TRY(dci.download(Ci));
   SBB_TRY(dcj.download(Cj));
@@ -774,17 +780,10 @@ int sbb_layer_create(const sbb_layer_desc *desc, sbb_layer **out) {
   if (e != cudaSuccess) rc = cuda_fail(e, "layer_create");
   if (rc == SBB_OK) rc = L->ticket.reserve(256);
   if (rc == SBB_OK && (e = cudaMemsetAsync(L->ticket.d, 0, 256, 0)) != cudaSuccess) rc = cuda_fail(e, "layer_create");
-  if (rc == SBB_OK) rc = L->rc.reserve(sbb::tc_trace_scratch_bytes(L->N, L->M));
+  if (rc == SBB_OK) rc = L->rc.reserve((size_t)((L->N + 3) / 4 * 4 + L->M) * s);
   if (rc == SBB_OK && desc->kind == SBB_LAYER_PLASTIC) {
     rc = L->score.reserve(sbb::mask_scratch_bytes(L->N, s));
     if (rc == SBB_OK && (e = sbb::mask_scratch_init(L->score.d, 0)) != cudaSuccess) rc = cuda_fail(e, "layer_create");
-    if (rc == SBB_OK) rc = L->col_hc.reserve((size_t)(L->M + 4) * sizeof(int));
-    if (rc == SBB_OK) {
-      std::vector<int> hc((size_t)L->M);
-      for (long j = 0; j < L->M; ++j) hc[(size_t)j] = (int)(j / L->Mc);
-      e = cudaMemcpy(L->col_hc.d, hc.data(), hc.size() * sizeof(int), cudaMemcpyHostToDevice);
-      if (e != cudaSuccess) rc = cuda_fail(e, "layer_create");
-    }
   }
   // the caller may step the layer on a stream that does not wait for these initialisations
   if (rc == SBB_OK && (e = cudaStreamSynchronize(0)) != cudaSuccess) rc = cuda_fail(e, "layer_create");
@@ -807,7 +806,6 @@ int sbb_layer_destroy(sbb_layer *L) {
   L->hx.release();
   L->hy.release();
   L->ht.release();
-  L->col_hc.release();
   L->ticket.release();
   L->rc.release();
   L->lo.release();
@@ -1283,26 +1281,10 @@ int shard_train(sbb_layer *L, long B, long h, cudaStream_t st) {
   const uint8_t *wmask = static_cast<const uint8_t *>(L->state[SBB_STATE_WMASK]);
   // Cj from the whole batch on every rank (identical inputs, identical results); Ci, Cij and the weights for the
   // own rows only, addressed as a layer of `nr` inputs that starts at row rb
-  SBB_CUDA(sbb::launch_colsum<T>(yg, Bg, M, nullptr, Cj, p, 1, st));
-  if (nr > 0) {
-    SBB_CUDA(sbb::launch_colsum<T>(xg, Bg, nr, nullptr, Ci + rb, p, 1, st));
-    PhaseTimer timer(L, SBB_PHASE_TRACE, st);
-    if (tensor_path<T>(xg, yg, nr, M)) {
-      if constexpr (std::is_same<T, float>::value)
-        SBB_CUDA(sbb::launch_trace_update_tc(xg, yg, Bg, nr, M, L->H, Ci + rb, Cj, Cij + rb * M, W + rb * M,
-                                             wmask ? wmask + rb * L->H : nullptr, static_cast<const int *>(L->col_hc.d),
-                                             static_cast<float *>(L->rc.d), p, 0, nr, st));
-    } else {
-      SBB_CUDA(sbb::launch_trace_update_fused<T>(xg, yg, Bg, nr, M, L->H, L->Mc, Ci + rb, Cj, Cij + rb * M, W + rb * M,
-                                                 wmask ? wmask + rb * L->H : nullptr, p, 0, nr, st));
-    }
-    timer.stop();
-  }
+  SBB_TRY(train_rows<T>(L, xg, yg, Bg, nr, M, L->H, Ci + rb, Cj, Cij + rb * M, W + rb * M, wmask ? wmask + rb * L->H : nullptr, p,
+                        layer_bias<T>(L), L->rc, st));
   if (L->desc.kind != SBB_LAYER_PLASTIC) return SBB_OK;
   const double cthr = L->desc.taupdt / 2;
-  SBB_CUDA(sbb::launch_update_bias_regularized<T>(static_cast<T *>(L->state[SBB_STATE_BIAS]),
-                                                  static_cast<T *>(L->state[SBB_STATE_KBI]), Cj, (T)cthr,
-                                                  (T)L->desc.khalf, (T)L->desc.pmin, (T)L->desc.taubdt, M, st));
   if (h >= 0 && nr > 0)   // scores of the owned rows, into every rank's work arrays
     SBB_CUDA(sbb::launch_mask_score_rows<T>(wmask, nullptr, Ci, Cj, Cij, (T)cthr, N, M, L->H, L->Mc, h, rb, re,
                                             shard_table(L, kShardMask, 0), st));

@@ -876,12 +876,12 @@ template cudaError_t launch_reduce_bias_softmax<double>(const double *, int, con
                                                         long, int, cudaStream_t);
 
 // ----------------------------------------------------------------------------
-// Column sums over the batch (and, fused, the Ci / Cj moving averages).
+// Column sums over the batch.
 // Block = 32 columns x 8 row lanes; rows are summed in a fixed order.
 // ----------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256)
-    colsum_kernel(const T *__restrict__ a, long B, long cols, T *sums, T *c, TraceParams<T> p, int ema, T *lo) {
+    colsum_kernel(const T *__restrict__ a, long B, long cols, T *sums, T *lo) {
   __shared__ T part[8][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const long col = (long)blockIdx.x * 32 + tx;
@@ -911,22 +911,76 @@ __global__ void __launch_bounds__(256)
     T t = part[0][tx];
 #pragma unroll
     for (int r = 1; r < 8; ++r) t += part[r][tx];
-    if (ema) c[col] = trace_ema(c[col], t, p);
-    else sums[col] = t;
+    sums[col] = t;
   }
 }
 
 template <typename T>
-cudaError_t launch_colsum(const T *a, long B, long cols, T *sums, T *c, TraceParams<T> p, int ema, cudaStream_t st,
-                          T *lo) {
+cudaError_t launch_colsum(const T *a, long B, long cols, T *sums, cudaStream_t st, T *lo) {
   if (cols == 0) return cudaSuccess;
-  colsum_kernel<T><<<(unsigned)((cols + 31) / 32), 256, 0, st>>>(a, B, cols, sums, c, p, ema, lo);
+  colsum_kernel<T><<<(unsigned)((cols + 31) / 32), 256, 0, st>>>(a, B, cols, sums, lo);
   return launched();
 }
-template cudaError_t launch_colsum<float>(const float *, long, long, float *, float *, TraceParams<float>, int,
-                                          cudaStream_t, float *);
-template cudaError_t launch_colsum<double>(const double *, long, long, double *, double *, TraceParams<double>, int,
-                                           cudaStream_t, double *);
+template cudaError_t launch_colsum<float>(const float *, long, long, float *, cudaStream_t, float *);
+template cudaError_t launch_colsum<double>(const double *, long, long, double *, cudaStream_t, double *);
+
+// What a train step derives from the column sums of its batch, for both operands in one launch: Ci and Cj, their
+// reciprocals (rc != null; 0 below the threshold) and, from Cj, gain and bias (kbi != null).  The sums are formed in the
+// order of colsum_kernel.  Bound by latency for small layers, by HBM otherwise: sixteen loads per thread in flight.  (The two
+// column sums, the reciprocals and the bias were four launches, 2 x 3.3 + 1.9 + 1.9 us at 1568 + 3000 columns, batch 128;
+// 3.7 us now.  1568 + 30000 columns, batch 1024: 67 -> 28 us.)
+template <typename T>
+__global__ void __launch_bounds__(256)
+    column_vectors_kernel(ColumnVectors<T> x, ColumnVectors<T> y, long B, TraceParams<T> p, BiasParams<T> nb, unsigned x_blocks) {
+  __shared__ T part[8][33];
+  const bool is_x = blockIdx.x < x_blocks;
+  const ColumnVectors<T> &o = is_x ? x : y;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const long col = (long)(is_x ? blockIdx.x : blockIdx.x - x_blocks) * 32 + tx;
+  T s = (T)0;
+  if (col < o.cols) {
+    constexpr int U = 16;
+    const T *src = o.a + col;
+    long b = ty;
+    for (; b + 8 * (U - 1) < B; b += 8 * U) {
+      T v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = __ldg(src + (b + 8 * u) * o.cols);
+#pragma unroll
+      for (int u = 0; u < U; ++u) s += v[u];
+    }
+    T v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = b + 8 * u < B ? __ldg(src + (b + 8 * u) * o.cols) : (T)0;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (b + 8 * u < B) s += v[u];
+  }
+  part[ty][tx] = s;
+  __syncthreads();
+  if (ty == 0 && col < o.cols) {
+    T t = part[0][tx];
+#pragma unroll
+    for (int r = 1; r < 8; ++r) t += part[r][tx];
+    const T c = trace_ema(o.c[col], t, p);
+    o.c[col] = c;
+    if (o.rc != nullptr) o.rc[col] = c < p.cthr ? (T)0 : (T)1 / c;
+    if (!is_x && nb.kbi != nullptr)
+      bias_regularized(nb.bias[col], nb.kbi[col], c, p.cthr, nb.khalf, nb.pmin4, nb.k, nb.taubdt);
+  }
+}
+template <typename T>
+cudaError_t launch_column_vectors(const ColumnVectors<T> &x, const ColumnVectors<T> &y, long B, TraceParams<T> p,
+                                  BiasParams<T> bias, cudaStream_t st) {
+  const unsigned xb = (unsigned)((x.cols + 31) / 32), yb = (unsigned)((y.cols + 31) / 32);
+  if (xb + yb == 0) return cudaSuccess;
+  column_vectors_kernel<T><<<xb + yb, 256, 0, st>>>(x, y, B, p, bias, xb);
+  return launched();
+}
+template cudaError_t launch_column_vectors<float>(const ColumnVectors<float> &, const ColumnVectors<float> &, long,
+                                                  TraceParams<float>, BiasParams<float>, cudaStream_t);
+template cudaError_t launch_column_vectors<double>(const ColumnVectors<double> &, const ColumnVectors<double> &, long,
+                                                   TraceParams<double>, BiasParams<double>, cudaStream_t);
 
 template <typename T>
 __global__ void vector_ema_kernel(T *c, const T *__restrict__ sums, long n, TraceParams<T> p) {

@@ -38,12 +38,10 @@ template <typename T>
 cudaError_t launch_reduce_bias_softmax(const T *partial, int splits, const T *bias, T *out, long rows, long H,
                                        long Mc, int softmax, cudaStream_t st);
 
-// sums[j] = sum_b a[b, j]                       (ema == 0)
-// c[j]    = EMA(c[j], sum_b a[b, j])            (ema != 0; sums unused)
+// sums[j] = sum_b a[b, j]
 // lo != nullptr (float32): also writes lo[b, j] = the low part of a[b, j] for a split TF32 product (sbb_math.cuh).
 template <typename T>
-cudaError_t launch_colsum(const T *a, long B, long cols, T *sums, T *c, TraceParams<T> p, int ema, cudaStream_t st,
-                          T *lo = nullptr);
+cudaError_t launch_colsum(const T *a, long B, long cols, T *sums, cudaStream_t st, T *lo = nullptr);
 
 // c[j] = EMA(c[j], sums[j])
 template <typename T>
@@ -58,6 +56,16 @@ struct BiasParams {
 };
 template <typename T>
 BiasParams<T> make_bias(T *bias, T *kbi, T khalf, T pmin, T taubdt);
+// One operand of a train step, a[B, cols], and what its column sums give: c = moving average, rc = 1 / c (may be null).
+template <typename T>
+struct ColumnVectors {
+  const T *a;
+  long cols;
+  T *c, *rc;
+};
+template <typename T>
+cudaError_t launch_column_vectors(const ColumnVectors<T> &x, const ColumnVectors<T> &y, long B, TraceParams<T> p,
+                                  BiasParams<T> bias, cudaStream_t st);
 bool narrow_layer(long N, long M);
 bool narrow_forward(long B, long N, long M, size_t elem);
 template <typename T>

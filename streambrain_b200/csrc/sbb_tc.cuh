@@ -26,14 +26,11 @@ int forward_splits_tc(long B, long N, long M);
 cudaError_t launch_forward_product_tc(const float *x, const float *w, float *partial, long B, long N, long M,
                                       int splits, cudaStream_t st);
 
-// Fused trace step (same contract as launch_trace_update_fused); col_hc[j] = j / Mc.
-// `scratch` holds tc_trace_scratch_bytes(N, M) bytes, 16-byte aligned (threshold-gated
-// reciprocals of Ci and Cj, written by a small kernel ahead of the contraction).
-size_t tc_trace_scratch_bytes(long N, long M);
-cudaError_t launch_trace_update_tc(const float *x, const float *y, long B, long N, long M, long H,
-                                   const float *Ci, const float *Cj, float *Cij, float *w, const uint8_t *wmask,
-                                   const int *col_hc, float *scratch, TraceParams<float> p, long row_begin,
-                                   long row_end, cudaStream_t st);
+// Fused trace step: Cij = moving average of x^T y / B, w = log(Cij / (Ci Cj)) under the mask (null: none), from the
+// reciprocals of the new Ci and Cj (0 where the trace is below the threshold).
+cudaError_t launch_trace_update_tc(const float *x, const float *y, long B, long N, long M, long H, const float *rci,
+                                   const float *rcj, float *Cij, float *w, const uint8_t *wmask, TraceParams<float> p,
+                                   cudaStream_t st);
 
 // delta[i, j] = sum_b x[b, i] y[b, j] for rows [row_begin,row_end)
 // x_lo / y_lo (both or neither): planes of the operands' low parts as launch_colsum writes them; with them the
@@ -52,6 +49,17 @@ long long tc_get_wait_limit();
 // Test hook: each of the next `launches` tensor-core launches that convert operands inside the kernel loses one
 // barrier arrival in its first CTA, so that a wait there runs into its time limit.
 void tc_debug_lose_arrive(int launches);
+
+// What the launches of both tensor-core files share (sbb_tc_kernels.cu): per-device facts, settings, and tensor maps
+// cached per host thread (maps are CUtensorMap).
+struct TcHost {
+  int *status;   // status word of the bounded waits on the current device
+  int sms, lose_arrive;
+  long long wait_limit;
+};
+bool tc_host(TcHost *out);
+bool tc_map_2d(void *map, const float *base, long inner, long outer, int box_inner, int box_outer, bool mn_major);
+bool tc_map_chunks(void *map, const float *base, long cols, long rows, int box_rows, int box_chunks);
 
 // Status word of the bounded device-side waits on the current device: 0 = all
 // waits completed, otherwise the code of the first wait that gave up.

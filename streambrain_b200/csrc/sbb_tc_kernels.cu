@@ -1,9 +1,9 @@
 // tcgen05 / TMEM / TMA contraction kernels for sm_100a.
 //
-// One persistent, warp-specialised kernel template serves both contractions of
-// the layer step:
+// One persistent, warp-specialised kernel template serves the forward product and the raw batch product of the
+// data-parallel step (the fused trace step of one device: sbb_tc_trace.cu):
 //
-//   trace update   D[i, j] = sum_b x[b, i] * y[b, j]   A = x  (MN-major), B = y (MN-major), K = batch
+//   raw product    D[i, j] = sum_b x[b, i] * y[b, j]   A = x  (MN-major), B = y (MN-major), K = batch
 //   forward        D[b, j] = sum_k x[b, k] * w[k, j]   A = x  (K-major),  B = w (MN-major), K = in_features
 //
 // float32 accuracy on TF32 tensor cores: every operand value v is used as
@@ -17,15 +17,13 @@
 // Roles inside a CTA (512 threads, one CTA per SM, tiles walked persistently):
 //   warps 0-3   A converters: wait for a TMA stage, write A's hi / lo parts to tensor
 //               memory (one tile row per thread)
-//               and (multi-chain trace update, raw products) B's lo parts to shared memory
-//   warps 14-15 B converters (forward product, single-chain trace update): B's lo parts to shared memory
+//               and (raw products) B's lo parts to shared memory
+//   warps 14-15 B converters (forward product): B's lo parts to shared memory
 //   warps 4-11  epilogue: tcgen05.ld the accumulator (16x256b shape, so that four
-//               lanes cover 32 contiguous bytes of a row) and either store it or run
-//               the trace / weight arithmetic against 32 x 32 blocks of Cij that TMA
-//               stages in shared memory two blocks ahead
+//               lanes cover 32 contiguous bytes of a row), add up the chains and store
 //   warp 12     TMA producer (one lane): cp.async.bulk.tensor loads, no multicast
 //   warp 13     MMA issuer (one lane) and owner of the TMEM allocation
-// CTA pairs (PAIR; the forward product and the fused trace update): the kernel is launched in clusters of
+// CTA pairs (PAIR; the forward product): the kernel is launched in clusters of
 // two CTAs that work on two vertically adjacent row tiles with one 256-row tcgen05.mma.cta_group::2 per k-step,
 // issued by the leader CTA.  Each CTA stages and converts its own 128 rows of A into its own tensor memory and
 // half of the tile's columns of B into its own shared memory; the converters and the epilogue warps of both
@@ -36,8 +34,7 @@
 // abort flag, and every role falls through to the common tear-down (drain the
 // tensor pipe, free TMEM) instead of spinning.
 #include "sbb_tc.cuh"
-
-#include <cuda.h>
+#include "sbb_tc_ptx.cuh"
 
 #include <atomic>
 #include <cstdlib>
@@ -54,10 +51,6 @@ constexpr int kTmaWarp = kConvWarps + kEpiWarps;
 constexpr int kMmaWarp = kTmaWarp + 1;
 constexpr int kBConvWarps = 2;                 // warps kMmaWarp + 1 ..: the low parts of B
 constexpr int kThreads = (kMmaWarp + 1 + kBConvWarps) * 32;  // 512: with 128 registers each, the whole register file
-constexpr long long kWaitLimitCycles = 4000000000ll;  // default limit of one wait: about 2 s of SM clock
-
-enum WaitCode { kWaitEmpty = 1, kWaitFull = 2, kWaitConv = 3, kWaitAccEmpty = 4, kWaitAccFull = 5, kWaitDrain = 6, kWaitSlab = 7 };
-
 struct TcWork {
   int m_tiles, n_tiles, splits;
   int k_total;      // extent of the reduction dimension
@@ -69,276 +62,17 @@ struct TcWork {
   int b_prefetch;   // B k-blocks requested into L2 ahead of the load into shared memory (0 = none)
   long long wait_limit;  // SM clock cycles after which a wait on an mbarrier gives up
   int lose_arrive;  // test hook: converter thread 0 of CTA 0 skips its arrival for the first stage
-  int chain_kb;     // kernels without register-resident sums (CHAIN == 0): k-blocks per tensor-memory
-                    // accumulation chain (0 = the whole k-range); later chains are added to the result of
-                    // the earlier ones by the epilogue, through the output itself
 };
 
 struct TcEpilogue {
   // raw store: out[(split*rows + m)*ld + n]
   float *out;
   long rows, cols, ld;
-  // fused trace step (rows = row_end - row_begin, global row = row0 + m)
-  const float *rci;    // per global row: 1 / Ci, or 0 when Ci < cthr
-  const float *rcj;    // per column: 1 / Cj, or 0 when Cj < cthr
-  float *Cij;
-  float *W;
-  const uint8_t *wmask;
-  const int *col_hc;
-  uint32_t hc_magic;   // ceil(2^32 / Mc) when floor(n * magic / 2^32) == n / Mc for every column, else 0
-  long H, Mc, row0;
-  int fast_ok;         // select-word epilogue usable: Mc >= 32 (or no mask) and cthr^4 a normal float
-  TraceParams<float> p;
-  float ema_scale;  // taupdt / batch: weight of the batch sum in the moving average
   // raw store of an MN-major product: the tile leaves through shared memory and TMA stores of 32 x 32 blocks
   // (tmC = the output, row 0 = first row of this launch) instead of register stores: whole 128-byte rows per
   // request, which is what a destination in another GPU's memory needs to be written at link speed
   int tma_store;
 };
-
-// ------------------------------------------------------------------ PTX wrappers
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-constexpr float kLn2 = 0.693147180559945309f;
-// log2 by the special-function unit alone (subnormal arguments read as zero).
-__device__ __forceinline__ float lg2_ftz(float v) {
-  float r;
-  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
-  return r;
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait.  Returns false when the CTA is aborting or the time limit passed
-// (in which case it raises the abort flag and records `code`).  The limit is
-// counted on the SM's own cycle counter: %globaltimer is read through the memory
-// system and costs microseconds per read on a busy GPU, which a wait taken
-// thousands of times per launch cannot afford.
-// The limit (cycles) sits in shared memory right behind the abort flag (written once at start-up).
-__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status,
-                                            int code, bool heed_abort = true) {
-  const long long t0 = clock64();
-  const long long limit = *reinterpret_cast<volatile long long *>(abort_flag + 1);
-  unsigned spins = 0;
-  while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((++spins & 1023u) == 0) {
-      if (heed_abort && *abort_flag) return false;
-      if (clock64() - t0 > limit) {
-        *abort_flag = 1;
-        atomicCAS(status, 0, code);
-        return false;
-      }
-    }
-  }
-}
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status,
-                                          int code) {
-  if (mbar_try_wait(bar, parity)) return true;
-  return mbar_wait_slow(bar, parity, abort_flag, status, code);
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-      : "memory");
-}
-
-// One box over the 3-D view [chunk][row][32] of an MN-major matrix: a whole stage of an operand
-// (every 32-element group along MN, all k-rows) in a single instruction.
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar)
-      : "memory");
-}
-// The same boxes requested into L2 only: takes DRAM latency out of the shared-memory pipeline.
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap *map, int x, int y) {
-  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];"
-               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y)
-               : "memory");
-}
-__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap *map, int x, int y, int z) {
-  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
-               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z)
-               : "memory");
-}
-// One box from shared memory to global memory (bulk async group of the issuing thread).
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, uint32_t src, int x, int y) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
-               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(src)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// at most one store group of this thread may still be reading its shared-memory source
-__device__ __forceinline__ void bulk_wait_read_1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// ---- CTA pairs (cluster of two CTAs driving one 256-row tcgen05.mma.cta_group::2)
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Arrival on the mbarrier at the same shared-memory offset in CTA `rank` of the cluster (own rank: local).
-__device__ __forceinline__ void mbar_arrive_rank(uint32_t bar, uint32_t rank) {
-  asm volatile(
-      "{\n\t.reg .b32 ra;\n\t"
-      "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
-      "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}"
-      ::"r"(bar), "r"(rank)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish_pair() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// D[256 x N] (+)= A[256 x 8] * B[8 x N] over the pair: each CTA holds its 128 rows of A and D in its own tensor
-// memory and N / 2 columns of B in its own shared memory, all at the same addresses; issued by the leader alone.
-__device__ __forceinline__ void mma_tf32_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                                 uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Completion of the pair's MMAs issued so far, signalled on the mbarrier at this offset in both CTAs.
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-      ::"r"(bar), "h"((uint16_t)3)
-      : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
-
-// D[128 x N] (+)= A[128 x 8] * B[8 x N]: A read from tensor memory (128 lanes x 8 columns of 32-bit
-// values at a_tmem), B through a shared-memory descriptor, TF32 inputs, float32 accumulation.
-__device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The same with A through a shared-memory descriptor as well.
-__device__ __forceinline__ void mma_tf32_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Each lane writes NCOL (16 or 32) consecutive 32-bit columns of its own tensor-memory lane.
-template <int NCOL>
-__device__ __forceinline__ void tmem_st_32x32b(uint32_t taddr, const uint32_t (&r)[NCOL]) {
-  static_assert(NCOL == 16 || NCOL == 32, "column count");
-  if constexpr (NCOL == 32) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
-          "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
-          "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-        : "memory");
-  } else {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-  }
-}
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-// 16 TMEM lanes x 32 columns: thread t gets, for rep = 0..3, registers
-//   r[4*rep+0..1] = lane t/4,     columns 8*rep + 2*(t%4) + {0,1}
-//   r[4*rep+2..3] = lane t/4 + 8, same columns.
-__device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, float (&r)[16]) {
-  uint32_t u[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
-      "[%16];"
-      : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]),
-        "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int k = 0; k < 16; ++k) r[k] = __uint_as_float(u[k]);
-}
-
-// Shared-memory matrix descriptor (sm_100 version field set).
-//   K-major operand:  rows of 128 bytes along k, 128-byte swizzle with 16-byte base (layout type 2);
-//                     SBO = 1024 (eight rows), LBO unused.
-//   MN-major 32-bit operand: the only layout the tensor core accepts is the 128-byte swizzle with
-//                     32-byte base (layout type 1): atoms of 4 k-rows x 128 bytes (32 elements along
-//                     MN); SBO = distance between consecutive 4-row atoms along k, LBO = distance
-//                     between 32-element groups along MN.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes,
-                                              uint32_t layout_type) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16;
-  d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32;
-  d |= 1ull << 46;  // descriptor version
-  d |= (uint64_t)layout_type << 61;
-  return d;
-}
-__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t saddr, uint32_t lbo_bytes) {
-  return smem_desc(saddr, lbo_bytes, 512u, 1u);       // MN-major, SWIZZLE_128B_BASE32B
-}
 
 // Optional timeline (compile with -DSBB_TC_TRACE): CTA 0 stamps clock64() at the hand-offs of its first
 // 64 tiles -- event numbers: 0 / 8 first / last TMA issue, 5 / 9 first / last conversion, 7 accumulator
@@ -352,7 +86,7 @@ __device__ unsigned long long g_tc_trace[64 * 16];
 #endif
 
 // ------------------------------------------------------------------ the kernel
-constexpr int kSlabBytes = 32 * 32 * 4;  // one epilogue warp's 32-row x 32-column block of the trace matrix
+constexpr int kSlabBytes = 32 * 32 * 4;  // one epilogue warp's 32-row x 32-column block of the output
 
 // The A operand's hi / lo parts live in tensor memory (written by the converters), so only B
 // has a "lo" copy in shared memory and the tensor core fetches only B from there.
@@ -373,8 +107,7 @@ struct TcSmem {
   static_assert(2 * BN + (PRESPLIT ? 0 : STAGES * 2 * BK) <= TMEM_COLS, "tensor memory budget");
   static_assert(STAGE_BYTES % 1024 == 0, "stages keep the 1024-byte swizzle alignment");
   static constexpr int SLAB_OFFSET = STAGES * STAGE_BYTES;
-  // two 32 x 32 block buffers per epilogue warp: landing zones for blocks of the trace matrix (fused
-  // epilogue) or staging for the TMA stores of the raw product
+  // two 32 x 32 block buffers per epilogue warp: staging for the TMA stores of the raw product
   static constexpr int SLAB_TOTAL = SLABS ? kEpiWarps * 2 * kSlabBytes : 0;
   static constexpr int BAR_OFFSET = SLAB_OFFSET + SLAB_TOTAL;
   // full, conv, empty per stage; acc_full[2], acc_empty[2], drain; slab[warp][2]
@@ -383,42 +116,13 @@ struct TcSmem {
   static_assert(TOTAL <= 232448, "shared memory budget");
 };
 
-// Two 16-lane halves of a warp's TMEM lane quarter, 32 columns each, one wait.
-__device__ __forceinline__ void tmem_ld_pair(uint32_t taddr_lo, uint32_t taddr_hi, float (&a)[16], float (&b)[16]) {
-  uint32_t u[16], v[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
-      "[%16];"
-      : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]),
-        "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
-      : "r"(taddr_lo)
-      : "memory");
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
-      "[%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr_hi)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    a[k] = __uint_as_float(u[k]);
-    b[k] = __uint_as_float(v[k]);
-  }
-}
-
 // CHAIN = number of k-blocks accumulated in tensor memory before the running sum
 // is taken over by float32 registers (0 = the whole k-range in tensor memory).
 // The tensor core adds each MMA into its accumulator with less than IEEE
 // rounding, so the error of a chain grows with its length; long reductions
 // (the forward pass sums over in_features) are cut into short chains whose
 // results the epilogue warps add in full float32.
-// MULTI (kernels without register-resident sums, CHAIN == 0): the k-range of a tile is cut into chains of
-// wk.chain_kb k-blocks and the epilogue carries the running sum through its output in memory; without it a
-// tile is one chain and the epilogue is the plain one.
-template <bool A_KMAJOR, int BN, int BK, int STAGES, bool FUSED, int CHAIN, bool MULTI = false, bool PRESPLIT = false,
-          bool PAIR = false>
+template <bool A_KMAJOR, int BN, int BK, int STAGES, int CHAIN, bool PRESPLIT = false, bool PAIR = false>
 // 14 warps are allocated registers as 16: 128 registers per thread is the most that fits one CTA per SM.
 __global__ void __launch_bounds__(kThreads, 1)
     tc_contraction_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -426,19 +130,17 @@ __global__ void __launch_bounds__(kThreads, 1)
                           const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmAlo,
                           const __grid_constant__ CUtensorMap tmBlo, const __grid_constant__ CUtensorMap tmA3lo,
                           const __grid_constant__ CUtensorMap tmB3lo, TcWork wk, TcEpilogue ep, int *status) {
-  using SM = TcSmem<BN, BK, STAGES, FUSED || !A_KMAJOR, PRESPLIT, PAIR>;
+  using SM = TcSmem<BN, BK, STAGES, !A_KMAJOR, PRESPLIT, PAIR>;
   static_assert(!(PRESPLIT && A_KMAJOR), "pre-split operands are the two MN-major ones of the batch contractions");
   static_assert(!PAIR || (!PRESPLIT && BN % 64 == 0), "CTA pairs convert their operands themselves");
   // In a pair, CTA `rank` of the cluster works on row tile 2 * (pair's tile) + rank; the leader (rank 0) issues the MMAs.
-  // B's low parts by the two extra warps (see their role below): forward product and single-chain trace update
-  constexpr bool BWARPS = !PRESPLIT && !MULTI && (A_KMAJOR || FUSED);
+  // B's low parts by the two extra warps (see their role below): forward product
+  constexpr bool BWARPS = A_KMAJOR;
   const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
   constexpr int BNH = PAIR ? BN / 2 : BN;   // columns of B this CTA stages
   static_assert(!A_KMAJOR || BK == 32, "a K-major operand is loaded as one 128-byte-wide box");
   static_assert(BN % 64 == 0 && BN <= 256 && BK % 8 == 0 && BK <= 32, "tile shape");
-  static_assert(!(FUSED && CHAIN > 0), "the fused epilogue consumes a whole-range accumulator");
   static_assert(CHAIN == 0 || BN <= 128, "register-resident running sums are sized for 128 columns");
-  static_assert(!(MULTI && CHAIN > 0), "chains are carried either in registers or through memory");
   extern __shared__ uint8_t smem_dyn[];
   const uint32_t dyn_base = smem_u32(smem_dyn);
   const uint32_t base = (dyn_base + 1023u) & ~1023u;  // swizzle atoms need 1024-byte alignment
@@ -606,7 +308,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           TC_TRACE(chain, 7);
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + buf * BN;
-          const int kb_end = CHAIN > 0 ? min(nkb, kb + CHAIN) : (MULTI ? min(nkb, kb + wk.chain_kb) : nkb);
+          const int kb_end = CHAIN > 0 ? min(nkb, kb + CHAIN) : nkb;
           for (bool first = true; kb < kb_end; ++kb, ++it) {
             const int s = it % STAGES;
             const uint32_t ph = (it / STAGES) & 1u;
@@ -728,9 +430,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     // ------------------------------------------------------------ B's lo parts (BWARPS kernels)
     // Two warps of their own: on the A converters' path this work lengthens the chain (wait for the stage, load,
     // split, store, fence, arrive) that every k-block of the MMA stream waits for.  Measured: forward product
-    // 0.437 -> 0.396 ms, single-chain trace update 0.561 -> 0.557 ms; the multi-chain trace update, whose eight
-    // epilogue warps keep the SM's issue slots and shared memory busier, lost 5 %, so there the A converters
-    // keep this work and these two warps go straight to the tear-down.
+    // 0.437 -> 0.396 ms.
     uint32_t it = 0;
     bool ok = true;
     const int t = threadIdx.x - (kMmaWarp + 1) * 32;   // 0 .. 63
@@ -773,24 +473,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint32_t swz[4];                             // byte offset of column pair `rep` inside a swizzled 128-byte row
 #pragma unroll
     for (int rep = 0; rep < 4; ++rep) swz[rep] = ((uint32_t)((2 * rep + (lc >> 2)) ^ lr) << 4) + (uint32_t)(lc & 3) * 4u;
-    uint32_t slab = 0;                           // blocks of the trace matrix consumed so far (fused epilogue)
-    // Hypercolumn of a column: exact multiply-shift division when the host verified it, else the table.
-    auto hc_of = [&](long n) -> int {
-      return ep.hc_magic ? (int)__umulhi((uint32_t)n, ep.hc_magic) : __ldg(ep.col_hc + n);
-    };
-    // Block number s of this warp (buffer s % 2): column group g of tile (mt, nt).
-    auto issue_slab_at = [&](uint32_t s, int mt, int nt, int g) {
-      const uint32_t b = s & 1u;
-      mbar_arrive_expect_tx(bar_slab(ew, b), kSlabBytes);
-      tma_load_2d(base + SM::SLAB_OFFSET + (ew * 2 + b) * kSlabBytes, &tmC, nt * BN + ch * (BN / 2) + g * 32,
-                  (int)ep.row0 + mt * 128 + 32 * q, bar_slab(ew, b));
-    };
-    if (FUSED && lane == 0 && w_first < total) {
-      int mt, nt, sp, kbeg, nkb;
-      decode(w_first, mt, nt, sp, kbeg, nkb);
-      issue_slab_at(0, mt, nt, 0);
-      issue_slab_at(1, mt, nt, 1);
-    }
     // Raw product leaving by TMA: this warp's 32 x 32 block of column group g (lo: tile rows lr, lr + 8; hi:
     // 16 + lr, 24 + lr; four column pairs each) goes to a staging buffer in the swizzled layout of the
     // tensor map and one lane sends it.  Blocks past the edge of the output are clipped by the TMA unit.
@@ -820,11 +502,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (long w = w_first; w < total && ok; w += w_step) {
       int mt, nt, sp, kbeg, nkb;
       decode(w, mt, nt, sp, kbeg, nkb);
-      int mt_next = 0, nt_next = 0;
-      if (FUSED && w + w_step < total) {
-        int sp2, kb2, nk2;
-        decode(w + w_step, mt_next, nt_next, sp2, kb2, nk2);
-      }
       const long m_base = (long)mt * 128 + 32 * q;   // first tile row of this warp's lane quarter
       const long n_base = (long)nt * BN + ch * (BN / 2);
       bool rv[4];
@@ -885,271 +562,48 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
         }
       } else {
-        // The k-range of a tile may be cut into several tensor-memory accumulation chains (the tensor core
-        // truncates every accumulate, so the error of a chain grows with its length): chain 0 forms the
-        // result as if it were the whole sum, every later chain adds its part to what the earlier ones
-        // stored (read back through L2), and only the last chain clamps the trace and writes the weight.
-        const int nchains = MULTI ? (nkb + wk.chain_kb - 1) / wk.chain_kb : 1;
-       for (int cc = 0; cc < nchains && ok; ++cc) {
-        const bool first_chain = !MULTI || cc == 0, last_chain = !MULTI || cc == nchains - 1;
         const uint32_t buf = chain & 1u, aph = (chain >> 1) & 1u;
-        // Everything the fused epilogue needs besides the accumulator is fetched before waiting for
-        // the accumulator, so these global-memory latencies overlap the wait.
-        const bool has_mask = FUSED && ep.wmask != nullptr;
-        int hc_first = 0, hc_last = 0;
-        bool bits_ok = true, tile_fast = false;
-        float rci[4] = {0.f, 0.f, 0.f, 0.f};
-        uint32_t mbits[4] = {0xFFu, 0xFFu, 0xFFu, 0xFFu};
-        float *crow[4] = {nullptr, nullptr, nullptr, nullptr};
-        float2 rcj_next[4];
-        float lane_rcj_next = 0.f;
-        long w_minus_c = 0;
-        if constexpr (FUSED) {
-          // per tile: reciprocal of Ci (0 = row below threshold), trace row pointers and the row's mask
-          // bytes for every hypercolumn this half tile touches (bit k: hypercolumn hc_first + k)
-          if (has_mask) {
-            hc_first = hc_of(n_base < ep.cols ? n_base : ep.cols - 1);
-            hc_last = hc_of(n_base + BN / 2 - 1 < ep.cols ? n_base + BN / 2 - 1 : ep.cols - 1);
-          }
-          bits_ok = hc_last - hc_first <= 7;
-          const int nhc = hc_last - hc_first + 1;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const long i = ep.row0 + grow[j];
-            rci[j] = rv[j] ? __ldg(ep.rci + i) : 0.f;
-            crow[j] = ep.Cij + i * ep.cols + n_base + lc;
-            if (has_mask && rv[j] && bits_ok) {
-              // every byte is loaded (index clamped into the row's range) so that the loads go out together
-              const uint8_t *mr = ep.wmask + i * ep.H + hc_first;
-              uint32_t byte[8];
-#pragma unroll
-              for (int k = 0; k < 8; ++k) byte[k] = __ldg(mr + (k < nhc ? k : 0));
-              uint32_t bits = 0;
-#pragma unroll
-              for (int k = 0; k < 8; ++k)
-                if (k < nhc && byte[k] != 0) bits |= 1u << k;
-              mbits[j] = bits;
-            }
-          }
-          // reciprocals of Cj for the first column group: this thread's pairs and, one per lane, the whole group
-#pragma unroll
-          for (int rep = 0; rep < 4; ++rep) {
-            const long n = n_base + lc + rep * 8;
-            rcj_next[rep] = n < ep.cols ? __ldg(reinterpret_cast<const float2 *>(ep.rcj + n)) : make_float2(0.f, 0.f);
-          }
-          lane_rcj_next = n_base + lane < ep.cols ? __ldg(ep.rcj + n_base + lane) : 0.f;
-          tile_fast = ep.fast_ok && bits_ok && (long)mt * 128 + 128 <= ep.rows;
-          w_minus_c = ep.W - ep.Cij;   // the weight of an element sits this far from its trace
-        }
         if (!mbar_wait(bar_acc_full(buf), aph, abort_flag, status, kWaitAccFull)) { ok = false; break; }
         if (threadIdx.x == kConvWarps * 32) TC_TRACE(chain, 3);
         __syncwarp();
         tc_fence_after();
         // this warp's accumulator block: TMEM lanes 32q.., columns of its half tile
         const uint32_t tacc = tmem_base + buf * BN + ch * (BN / 2) + ((uint32_t)(32 * q) << 16);
-        if constexpr (FUSED) {
-          if (threadIdx.x == kConvWarps * 32) TC_TRACE(chain, 10);
 #pragma unroll 1
-          for (int g = 0; g < NG; ++g) {
-            // This warp's 32 x 32 block of the trace matrix was fetched by TMA two blocks ago
-            // (128-byte swizzle: 16-byte chunk c of row r sits at chunk c ^ (r % 8); every row
-            // of this thread has r % 8 == lane / 4).
-            const uint32_t sb = slab & 1u;
-            if (!mbar_wait(bar_slab(ew, sb), (slab >> 1) & 1u, abort_flag, status, kWaitSlab)) { ok = false; break; }
-            const uint8_t *sl = smem + SM::SLAB_OFFSET + (ew * 2 + sb) * kSlabBytes + lr * 128;
-            const long gs = n_base + g * 32;   // first column of the group
-            float2 rcj[4];
-#pragma unroll
-            for (int rep = 0; rep < 4; ++rep) rcj[rep] = rcj_next[rep];
-            const float lane_rcj = lane_rcj_next;
-            if (g + 1 < NG) {   // the next group's values, in flight while this group is processed
-#pragma unroll
-              for (int rep = 0; rep < 4; ++rep) {
-                const long nn = gs + 32 + lc + rep * 8;
-                rcj_next[rep] = nn < ep.cols ? __ldg(reinterpret_cast<const float2 *>(ep.rcj + nn)) : make_float2(0.f, 0.f);
-              }
-              lane_rcj_next = gs + 32 + lane < ep.cols ? __ldg(ep.rcj + gs + 32 + lane) : 0.f;
-            }
-            // Fast groups (whole block inside the matrix, at most two hypercolumns per group): one
-            // select word per row, bit 8*rep + e = "element e of column pair rep keeps its weight".
-            const bool g_fast = tile_fast && gs + 32 <= ep.cols;
-            uint32_t sel[4] = {0u, 0u, 0u, 0u};
-            if (g_fast) {
-              const uint32_t live32 = __ballot_sync(0xFFFFFFFFu, lane_rcj != 0.f);   // columns at or above the threshold
-              uint32_t first32 = 0xFFFFFFFFu;   // columns of the group's first hypercolumn
-              int k0 = 0;
-              if (has_mask) {
-                const int hc0 = hc_of(gs);
-                const long bnd = (long)(hc0 + 1) * ep.Mc - gs;
-                if (bnd < 32) first32 = (1u << bnd) - 1u;
-                k0 = hc0 - hc_first;
-              }
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const uint32_t m0 = 0u - ((mbits[j] >> k0) & 1u), m1 = 0u - ((mbits[j] >> (k0 + 1)) & 1u);
-                const uint32_t word = ((m0 & first32) | (m1 & ~first32)) & live32;
-                sel[j] = rci[j] != 0.f ? (word >> lc) & 0x03030303u : 0u;
-              }
-            }
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-              // 16 of the warp's 32 TMEM lanes at a time keeps the live registers within budget
-              float a[16];
-              __syncwarp();  // tcgen05.ld is warp-collective
-              tmem_ld_16x256b_x4(tacc + g * 32 + ((uint32_t)(16 * hh) << 16), a);
-              float2 c[2][4];
-#pragma unroll
-              for (int rr = 0; rr < 2; ++rr)
-#pragma unroll
-                for (int rep = 0; rep < 4; ++rep)
-                  c[rr][rep] = *reinterpret_cast<const float2 *>(sl + (16 * hh + 8 * rr) * 128 + swz[rep]);
-              if (hh == 1) {
-                // The buffer is about to be overwritten by the async proxy (TMA): every lane's
-                // reads above must have been performed first, not merely issued.  With several chains the
-                // block about to be fetched may be one this warp stored a moment ago: those global writes
-                // are ordered before the fetch as well.
-                fence_async_smem();
-                __syncwarp();
-                if (lane == 0) {
-                  // block slab+2: two column groups ahead in this tile, or the next tile's first groups.  With
-                  // several chains the blocks of the next pass are fetched at the end of this one (below).
-                  if (g + 2 < NG) issue_slab_at(slab + 2, mt, nt, g + 2);
-                  else if (!MULTI && w + w_step < total) issue_slab_at(slab + 2, mt_next, nt_next, g + 2 - NG);
-                }
-              }
-              if (g_fast) {
-#pragma unroll
-                for (int rr = 0; rr < 2; ++rr) {
-                  const int j = 2 * hh + rr;
-                  float *cp = crow[j] + g * 32;
-                  const float r = rci[j];
-                  const uint32_t sj = sel[j];
-#pragma unroll
-                  for (int rep = 0; rep < 4; ++rep) {
-                    float2 c2 = c[rr][rep];
-                    // the old trace decays once, in chain 0
-                    c2.x = fmaf(c2.x, first_chain ? ep.p.one_minus : 1.f, a[rep * 4 + rr * 2 + 0] * ep.ema_scale);
-                    c2.y = fmaf(c2.y, first_chain ? ep.p.one_minus : 1.f, a[rep * 4 + rr * 2 + 1] * ep.ema_scale);
-                    if (!last_chain) {   // a partial sum: parked in the trace matrix (it stays in L2)
-                      __stcg(reinterpret_cast<float2 *>(cp + rep * 8), c2);
-                      continue;
-                    }
-                    c2.x = fmaxf(c2.x, 0.f);
-                    c2.y = fmaxf(c2.y, 0.f);
-                    const float wx = lg2_ftz(fmaxf(c2.x, ep.p.cthr4) * (r * rcj[rep].x)) * kLn2;
-                    const float wy = lg2_ftz(fmaxf(c2.y, ep.p.cthr4) * (r * rcj[rep].y)) * kLn2;
-                    __stcs(reinterpret_cast<float2 *>(cp + rep * 8), c2);
-                    __stcs(reinterpret_cast<float2 *>(cp + w_minus_c + rep * 8),
-                           make_float2((sj & (1u << (8 * rep))) ? wx : 0.f, (sj & (2u << (8 * rep))) ? wy : 0.f));
-                  }
-                }
-              } else {
-                // edge blocks and layouts the select words do not cover: every element checked
-#pragma unroll
-                for (int rr = 0; rr < 2; ++rr) {
-                  const int j = 2 * hh + rr;
-                  if (!rv[j]) continue;
-                  float *cp = crow[j] + g * 32;
-                  const uint8_t *mr = has_mask ? ep.wmask + (ep.row0 + grow[j]) * ep.H : nullptr;
-#pragma unroll
-                  for (int rep = 0; rep < 4; ++rep) {
-                    const long n = gs + lc + rep * 8;
-                    if (!(n < ep.cols)) continue;   // cols is even: n + 1 is in range too
-                    float2 c2 = c[rr][rep];
-                    // the old trace decays once, in chain 0
-                    c2.x = fmaf(c2.x, first_chain ? ep.p.one_minus : 1.f, a[rep * 4 + rr * 2 + 0] * ep.ema_scale);
-                    c2.y = fmaf(c2.y, first_chain ? ep.p.one_minus : 1.f, a[rep * 4 + rr * 2 + 1] * ep.ema_scale);
-                    if (!last_chain) {
-                      __stcg(reinterpret_cast<float2 *>(cp + rep * 8), c2);
-                      continue;
-                    }
-                    c2.x = fmaxf(c2.x, 0.f);
-                    c2.y = fmaxf(c2.y, 0.f);
-                    bool on0 = rci[j] != 0.f && rcj[rep].x != 0.f, on1 = rci[j] != 0.f && rcj[rep].y != 0.f;
-                    if (has_mask) {
-                      const int h0 = hc_of(n), h1 = hc_of(n + 1);
-                      if (bits_ok) {
-                        on0 = on0 && ((mbits[j] >> (h0 - hc_first)) & 1u);
-                        on1 = on1 && ((mbits[j] >> (h1 - hc_first)) & 1u);
-                      } else {
-                        on0 = on0 && __ldg(mr + h0) != 0;
-                        on1 = on1 && __ldg(mr + h1) != 0;
-                      }
-                    }
-                    const float wx = __logf(fmaxf(c2.x, ep.p.cthr4) * (rci[j] * rcj[rep].x));
-                    const float wy = __logf(fmaxf(c2.y, ep.p.cthr4) * (rci[j] * rcj[rep].y));
-                    __stcs(reinterpret_cast<float2 *>(cp + rep * 8), c2);
-                    __stcs(reinterpret_cast<float2 *>(cp + w_minus_c + rep * 8), make_float2(on0 ? wx : 0.f, on1 ? wy : 0.f));
-                  }
-                }
-              }
-            }
-            ++slab;
-            if (threadIdx.x == kConvWarps * 32 && g < 3) TC_TRACE(chain, 13 + g);
+        for (int g = 0; g < NG; ++g) {
+          float a0[16], a1[16];
+          const uint32_t t0 = tacc + g * 32;
+          __syncwarp();  // tcgen05.ld is warp-collective
+          tmem_ld_pair(t0, t0 + (16u << 16), a0, a1);
+          if (!A_KMAJOR && ep.tma_store) {
+            store_block(a0, a1, mt, nt, g);
+            continue;
           }
-          if (MULTI && ok) {
-            // The next pass re-reads blocks this warp has just stored (the running sums): one fence per pass
-            // orders those global writes, and the shared-memory reads of both landing buffers, before the
-            // async-proxy fetches of the next pass's first two blocks (or the next tile's).
-            static_assert(!MULTI || NG >= 2, "two landing buffers are refilled at the end of a pass");
-            fence_async_all();
-            __syncwarp();
-            if (lane == 0) {
-              if (!last_chain) {
-                issue_slab_at(slab, mt, nt, 0);
-                issue_slab_at(slab + 1, mt, nt, 1);
-              } else if (w + w_step < total) {
-                issue_slab_at(slab, mt_next, nt_next, 0);
-                issue_slab_at(slab + 1, mt_next, nt_next, 1);
-              }
-            }
-          }
-        } else {
-#pragma unroll 1
-          for (int g = 0; g < NG; ++g) {
-            float a0[16], a1[16];
-            const uint32_t t0 = tacc + g * 32;
-            __syncwarp();  // tcgen05.ld is warp-collective
-            tmem_ld_pair(t0, t0 + (16u << 16), a0, a1);
-            if (!A_KMAJOR && !MULTI && ep.tma_store) {
-              store_block(a0, a1, mt, nt, g);
-              continue;
-            }
-            const long n0 = n_base + g * 32 + lc;
+          const long n0 = n_base + g * 32 + lc;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              if (!rv[j]) continue;
-              const float *acc = (j >> 1) ? a1 : a0;
-              float *orow = ep.out + ((long)sp * ep.rows + grow[j]) * ep.ld;
+          for (int j = 0; j < 4; ++j) {
+            if (!rv[j]) continue;
+            const float *acc = (j >> 1) ? a1 : a0;
+            float *orow = ep.out + ((long)sp * ep.rows + grow[j]) * ep.ld;
 #pragma unroll
-              for (int rep = 0; rep < 4; ++rep)
-                if (n0 + rep * 8 < ep.cols) {   // cols is even: n+1 is in range too
-                  float2 v = make_float2(acc[rep * 4 + (j & 1) * 2], acc[rep * 4 + (j & 1) * 2 + 1]);
-                  float2 *dst = reinterpret_cast<float2 *>(orow + n0 + rep * 8);
-                  if (!first_chain) {   // this thread stored the sum of the earlier chains at the same place
-                    const float2 prev = __ldcg(dst);
-                    v.x += prev.x;
-                    v.y += prev.y;
-                  }
-                  if (last_chain) __stcs(dst, v); else __stcg(dst, v);
-                }
-            }
+            for (int rep = 0; rep < 4; ++rep)
+              if (n0 + rep * 8 < ep.cols)   // cols is even: n+1 is in range too
+                __stcs(reinterpret_cast<float2 *>(orow + n0 + rep * 8),
+                       make_float2(acc[rep * 4 + (j & 1) * 2], acc[rep * 4 + (j & 1) * 2 + 1]));
           }
         }
-        if (!ok) break;
         if (threadIdx.x == kConvWarps * 32) TC_TRACE(chain, 4);
         tc_fence_before();
         // the accumulator buffer may be overwritten (PAIR: the leader's MMA warp waits for both CTAs' epilogues)
         if constexpr (PAIR) mbar_arrive_rank(bar_acc_empty(buf), 0);
         else mbar_arrive(bar_acc_empty(buf));
         ++chain;
-       }   // chains of this tile
       }
     }
   }
 
   // stores this thread sent by TMA must have left shared memory (and landed) before the CTA retires
-  if (!FUSED && !A_KMAJOR && warp >= kConvWarps && warp < kTmaWarp && lane == 0) bulk_wait_all();
+  if (!A_KMAJOR && warp >= kConvWarps && warp < kTmaWarp && lane == 0) bulk_wait_all();
   // ------------------------------------------------------------ tear-down
   __syncwarp();
   tc_fence_before();
@@ -1320,13 +774,13 @@ struct TcMaps {
   CUtensorMap alo, blo, a3lo, b3lo;   // the operands' low-part planes (pre-split kernels)
 };
 
-template <bool A_KMAJOR, int BN, int BK, int STAGES, bool FUSED, int CHAIN, bool MULTI = false, bool PRESPLIT = false>
+template <bool A_KMAJOR, int BN, int BK, int STAGES, int CHAIN, bool PRESPLIT = false>
 cudaError_t launch_tc(const TcMaps &tm, const TcWork &wk, const TcEpilogue &ep, cudaStream_t st,
                       bool leave_reserved_sms = false) {
-  using SM = TcSmem<BN, BK, STAGES, FUSED || !A_KMAJOR, PRESPLIT>;
+  using SM = TcSmem<BN, BK, STAGES, !A_KMAJOR, PRESPLIT>;
   int *status = status_word();
   if (status == nullptr) return cudaErrorMemoryAllocation;
-  auto kernel = tc_contraction_kernel<A_KMAJOR, BN, BK, STAGES, FUSED, CHAIN, MULTI, PRESPLIT>;
+  auto kernel = tc_contraction_kernel<A_KMAJOR, BN, BK, STAGES, CHAIN, PRESPLIT>;
   static std::atomic<bool> configured[64];   // per device; setting the attribute twice is harmless
   const int dev = current_device();
   if (!configured[dev].load()) {
@@ -1354,12 +808,12 @@ bool pairs_enabled() {
 }
 
 // The CTA-pair form of a kernel: clusters of two CTAs, one 256 x BN tile per pair.
-template <bool A_KMAJOR, int BN, int BK, int STAGES, bool FUSED, int CHAIN, bool MULTI = false>
+template <bool A_KMAJOR, int BN, int BK, int STAGES, int CHAIN>
 cudaError_t launch_tc_pair(const TcMaps &tm, const TcWork &wk, const TcEpilogue &ep, cudaStream_t st) {
-  using SM = TcSmem<BN, BK, STAGES, FUSED || !A_KMAJOR, false, true>;
+  using SM = TcSmem<BN, BK, STAGES, !A_KMAJOR, false, true>;
   int *status = status_word();
   if (status == nullptr) return cudaErrorMemoryAllocation;
-  auto kernel = tc_contraction_kernel<A_KMAJOR, BN, BK, STAGES, FUSED, CHAIN, MULTI, false, true>;
+  auto kernel = tc_contraction_kernel<A_KMAJOR, BN, BK, STAGES, CHAIN, false, true>;
   static std::atomic<bool> configured[64];
   const int dev = current_device();
   if (!configured[dev].load()) {
@@ -1397,6 +851,20 @@ cudaError_t launch_tc_pair(const TcMaps &tm, const TcWork &wk, const TcEpilogue 
 
 }  // namespace
 
+bool tc_host(TcHost *out) {
+  out->status = status_word();
+  out->sms = g_sm_count_tc[current_device()];
+  out->wait_limit = wait_limit_now();
+  out->lose_arrive = out->status != nullptr ? take_lose_arrive() : 0;
+  return out->status != nullptr && init_once();
+}
+bool tc_map_2d(void *map, const float *base, long inner, long outer, int box_inner, int box_outer, bool mn_major) {
+  return make_map(static_cast<CUtensorMap *>(map), base, inner, outer, box_inner, box_outer, mn_major);
+}
+bool tc_map_chunks(void *map, const float *base, long cols, long rows, int box_rows, int box_chunks) {
+  return make_map_chunks(static_cast<CUtensorMap *>(map), base, cols, rows, box_rows, box_chunks);
+}
+
 // Launch counter shared with the general-shape kernels (defined in sbb_kernels.cu).
 void count_launches(int n);
 
@@ -1425,7 +893,6 @@ constexpr int kTrBN = 192, kTrBK = 16, kTrStages = 4;
 // epilogue takes the partial sum over in float32.  Measured on B200: the tensor-memory accumulate truncates,
 // so a chain's sum is low by about 1e-8 x (samples in the chain) relative; 256 keeps that below 4e-6.
 constexpr int kTrChainKb = 16;
-constexpr int kPairStages = 4;   // (tensor memory holds the A parts of four stages beside the two accumulators)
 constexpr int kLongBN = 128, kLongStages = 5;   // tiles of the row-block product when the batch spans several chains
 
 // k-blocks per split and the number of (non-empty) splits for the forward product: the split count
@@ -1495,7 +962,7 @@ cudaError_t launch_forward_product_tc(const float *x, const float *w, float *par
   if (!b3) tm.b3 = tm.b;
   tm.alo = tm.blo = tm.a3lo = tm.b3lo = tm.a;
   TcWork wk{(int)((B + 127) / 128), (int)((M + kFwdBN - 1) / kFwdBN), splits, (int)N, k_per_split, 1, 0, 0,
-            b3 ? full_chunk_tiles(M, kFwdBN) : 0, kFwdPrefetch, wait_limit_now(), take_lose_arrive(), 0};
+            b3 ? full_chunk_tiles(M, kFwdBN) : 0, kFwdPrefetch, wait_limit_now(), take_lose_arrive()};
 #ifdef SBB_TC_TRACE
   if (const char *e = getenv("SBB_FWD_PREFETCH")) wk.b_prefetch = atoi(e);   // timeline builds may vary the distance
 #endif
@@ -1504,40 +971,11 @@ cudaError_t launch_forward_product_tc(const float *x, const float *w, float *par
   ep.rows = B;
   ep.cols = M;
   ep.ld = M;
-  cudaError_t e = pair ? launch_tc_pair<true, kFwdBN, kFwdBK, kFwdStages, false, kFwdChain>(tm, wk, ep, st)
-                       : launch_tc<true, kFwdBN, kFwdBK, kFwdStages, false, kFwdChain>(tm, wk, ep, st);
+  cudaError_t e = pair ? launch_tc_pair<true, kFwdBN, kFwdBK, kFwdStages, kFwdChain>(tm, wk, ep, st)
+                       : launch_tc<true, kFwdBN, kFwdBK, kFwdStages, kFwdChain>(tm, wk, ep, st);
   if (e == cudaSuccess) count_launches(1);
   return e;
 }
-
-// Multiplier for n / d by multiply-high, or 0 if it is not exact for every n < limit.
-static uint32_t exact_division_magic(long d, long limit) {
-  if (d <= 1 || d >= (1L << 31) || limit >= (1L << 31)) return 0;
-  const uint64_t magic = ((1ull << 32) + (uint64_t)d - 1) / (uint64_t)d;
-  if (magic >> 32) return 0;
-  for (long n = 0; n < limit; ++n)
-    if ((long)(((uint64_t)n * magic) >> 32) != n / d) return 0;
-  return (uint32_t)magic;
-}
-
-namespace {
-// out = C < cthr ? 0 : 1 / C  for rows [row_begin, row_end) of Ci and every column of Cj: the
-// epilogue multiplies by these and reads "below the threshold" off the zero.
-__global__ void trace_reciprocals_kernel(const float *__restrict__ Ci, long row_begin, long row_end,
-                                         const float *__restrict__ Cj, long M, float cthr, float *__restrict__ rci,
-                                         float *__restrict__ rcj) {
-  const long rows = row_end - row_begin;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < rows + M; t += (long)gridDim.x * blockDim.x) {
-    if (t < rows) {
-      const float c = Ci[row_begin + t];
-      rci[row_begin + t] = c < cthr ? 0.f : 1.f / c;
-    } else {
-      const float c = Cj[t - rows];
-      rcj[t - rows] = c < cthr ? 0.f : 1.f / c;
-    }
-  }
-}
-}  // namespace
 
 namespace {
 // Tensor maps of the two MN-major operands x[B, N] and y[B, M] of a batch contraction with `bn`-column tiles, and
@@ -1566,86 +1004,6 @@ bool lo_planes_usable(const float *x_lo, const float *y_lo) {
 }
 }  // namespace
 
-size_t tc_trace_scratch_bytes(long N, long M) { return (size_t)(((N + 3) / 4) * 4 + M + 4) * sizeof(float); }
-
-cudaError_t launch_trace_update_tc(const float *x, const float *y, long B, long N, long M, long H, const float *Ci,
-                                   const float *Cj, float *Cij, float *w, const uint8_t *wmask, const int *col_hc,
-                                   float *scratch, TraceParams<float> p, long row_begin, long row_end,
-                                   cudaStream_t st) {
-  // verified once per layer shape and host thread
-  static thread_local long magic_for_mc = -1, magic_for_m = -1;
-  static thread_local uint32_t magic_value = 0;
-  uint32_t hc_magic = 0;
-  if (wmask != nullptr && H > 0) {
-    const long Mc = M / H;
-    if (magic_for_mc != Mc || magic_for_m != M) {
-      magic_value = exact_division_magic(Mc, M + 2);
-      magic_for_mc = Mc;
-      magic_for_m = M;
-    }
-    hc_magic = magic_value;
-  }
-  if (!tc_available() || !tc_shape_ok(x, y, N, M) || row_begin % 128 != 0) return cudaErrorNotSupported;
-  if ((reinterpret_cast<uintptr_t>(Cij) & 7u) || (reinterpret_cast<uintptr_t>(w) & 7u) ||
-      scratch == nullptr || (reinterpret_cast<uintptr_t>(scratch) & 15u) ||
-      (wmask && (col_hc == nullptr || (reinterpret_cast<uintptr_t>(col_hc) & 7u))))
-    return cudaErrorNotSupported;
-  if (row_end <= row_begin) return cudaSuccess;
-  TcMaps tm;
-  bool a3 = false, b3 = false;
-  // The fused kernel splits its operands itself (A's parts go to tensor memory): with pre-split planes both
-  // operands would come from shared memory, whose bandwidth the Cij blocks of the epilogue also need; measured
-  // on the 55296 x 3000 layer the launch takes 0.608 ms that way against 0.587 ms.
-  // a batch of more than one chain carries its running sum through the trace matrix (see the kernel)
-  const bool multi = B > (long)kTrChainKb * kTrBK;
-  // CTA pairs (one 256-row MMA over two SMs, each staging half of the tile's columns of y): single-chain batches
-  const bool pair = pairs_enabled();
-  // (pairs: y's one-box 3-D map covers half a tile's column chunks)
-  if (!batch_operand_maps(tm, x, y, nullptr, nullptr, false, B, N, M, pair ? kTrBN / 2 : kTrBN, a3, b3))
-    return cudaErrorInvalidValue;
-  if (!make_map(&tm.c, Cij, M, N, 32, 32, false)) return cudaErrorInvalidValue;   // 32 x 32 blocks, 128-byte swizzle
-  const long rows = row_end - row_begin;
-  const int kper = (int)((B + kTrBK - 1) / kTrBK) * kTrBK;
-  // tiles are walked so that the larger operand is the one re-used by consecutive tiles: column tiles
-  // fastest when x (B x N) is the larger, row tiles fastest when y (B x M) is
-  TcWork wk{(int)((rows + 127) / 128), (int)((M + kTrBN - 1) / kTrBN), 1, (int)B, kper, M > N ? 1 : 0, (int)row_begin,
-            a3 ? 1 : 0, b3 ? full_chunk_tiles(M, kTrBN) : 0, 0, wait_limit_now(), take_lose_arrive(), kTrChainKb};
-  TcEpilogue ep{};
-  ep.rows = rows;
-  ep.cols = M;
-  float *rci = scratch, *rcj = scratch + ((N + 3) / 4) * 4;
-  {
-    const long n = rows + M;
-    const unsigned blocks = (unsigned)((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184);
-    trace_reciprocals_kernel<<<blocks, 256, 0, st>>>(Ci, row_begin, row_end, Cj, M, p.cthr, rci, rcj);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    count_launches(1);
-  }
-  ep.rci = rci;
-  ep.rcj = rcj;
-  ep.Cij = Cij;
-  ep.W = w;
-  ep.wmask = wmask;
-  ep.col_hc = col_hc;
-  ep.hc_magic = hc_magic;
-  ep.H = H;
-  ep.Mc = H > 0 ? M / H : M;
-  ep.fast_ok = (wmask == nullptr || ep.Mc >= 32) && p.cthr4 >= 1e-30f;
-  ep.row0 = row_begin;
-  ep.p = p;
-  ep.ema_scale = p.taupdt / p.batch;
-  cudaError_t e;
-  if (pair)
-    e = multi ? launch_tc_pair<false, kTrBN, kTrBK, kPairStages, true, 0, true>(tm, wk, ep, st)
-              : launch_tc_pair<false, kTrBN, kTrBK, kPairStages, true, 0>(tm, wk, ep, st);
-  else
-    e = multi ? launch_tc<false, kTrBN, kTrBK, kTrStages, true, 0, true>(tm, wk, ep, st)
-              : launch_tc<false, kTrBN, kTrBK, kTrStages, true, 0>(tm, wk, ep, st);
-  if (e == cudaSuccess) count_launches(1);
-  return e;
-}
-
 cudaError_t launch_outer_product_tc(const float *x, const float *y, long B, long N, long M, float *delta,
                                     long row_begin, long row_end, cudaStream_t st, const float *x_lo,
                                     const float *y_lo) {
@@ -1666,7 +1024,7 @@ cudaError_t launch_outer_product_tc(const float *x, const float *y, long B, long
     // registers (as in the forward product), so no partial sum travels through memory.
     const bool b3n = b3;
     TcWork wk{(int)((rows + 127) / 128), (int)((M + kLongBN - 1) / kLongBN), 1, (int)B, kper, M > N ? 1 : 0,
-              (int)row_begin, a3 ? 1 : 0, b3n ? full_chunk_tiles(M, kLongBN) : 0, 0, wait_limit_now(), 0, 0};
+              (int)row_begin, a3 ? 1 : 0, b3n ? full_chunk_tiles(M, kLongBN) : 0, 0, wait_limit_now(), 0};
     TcEpilogue ep{};
     ep.out = delta + row_begin * M;
     ep.rows = rows;
@@ -1674,15 +1032,15 @@ cudaError_t launch_outer_product_tc(const float *x, const float *y, long B, long
     ep.ld = M;
     ep.tma_store = (reinterpret_cast<uintptr_t>(ep.out) & 15u) == 0 && make_map(&tm.c, ep.out, M, rows, 32, 32, false);
     if (!ep.tma_store) tm.c = tm.a;
-    cudaError_t e = pre ? launch_tc<false, kLongBN, kTrBK, kLongStages, false, kTrChainKb, false, true>(tm, wk, ep, st, true)
-                        : launch_tc<false, kLongBN, kTrBK, kLongStages, false, kTrChainKb>(tm, wk, ep, st, true);
+    cudaError_t e = pre ? launch_tc<false, kLongBN, kTrBK, kLongStages, kTrChainKb, true>(tm, wk, ep, st, true)
+                        : launch_tc<false, kLongBN, kTrBK, kLongStages, kTrChainKb>(tm, wk, ep, st, true);
     if (e == cudaSuccess) count_launches(1);
     return e;
   }
   // tiles are walked so that the larger operand is the one re-used by consecutive tiles: column tiles
   // fastest when x (B x N) is the larger, row tiles fastest when y (B x M) is
   TcWork wk{(int)((rows + 127) / 128), (int)((M + kTrBN - 1) / kTrBN), 1, (int)B, kper, M > N ? 1 : 0, (int)row_begin,
-            a3 ? 1 : 0, b3 ? full_chunk_tiles(M, kTrBN) : 0, 0, wait_limit_now(), take_lose_arrive(), kTrChainKb};
+            a3 ? 1 : 0, b3 ? full_chunk_tiles(M, kTrBN) : 0, 0, wait_limit_now(), take_lose_arrive()};
   TcEpilogue ep{};
   ep.out = delta + row_begin * M;
   ep.rows = rows;
@@ -1691,8 +1049,8 @@ cudaError_t launch_outer_product_tc(const float *x, const float *y, long B, long
   ep.tma_store = (reinterpret_cast<uintptr_t>(ep.out) & 15u) == 0 && make_map(&tm.c, ep.out, M, rows, 32, 32, false);
   if (!ep.tma_store) tm.c = tm.a;
   // the one contraction that runs beside a collective (the reduction of the previous row block)
-  cudaError_t e = pre ? launch_tc<false, kTrBN, kTrBK, kTrStages, false, 0, false, true>(tm, wk, ep, st, true)
-                      : launch_tc<false, kTrBN, kTrBK, kTrStages, false, 0>(tm, wk, ep, st, true);
+  cudaError_t e = pre ? launch_tc<false, kTrBN, kTrBK, kTrStages, 0, true>(tm, wk, ep, st, true)
+                      : launch_tc<false, kTrBN, kTrBK, kTrStages, 0>(tm, wk, ep, st, true);
   if (e == cudaSuccess) count_launches(1);
   return e;
 }

@@ -571,3 +571,35 @@ def test_layers_of_few_units_vs_oracle(port_kernels, tag, dtype, kind, B, N, H, 
         assert weight_err(dev.weights, ref.weights) < 10 * tol, step
         for name in ("weights", "bias", "Ci", "Cj", "Cij"):
             setattr(dev, name, getattr(ref, name))
+
+
+@pytest.mark.parametrize("B,N,H,Mc,scale", [(1, 128, 3, 12, 1.0), (16, 256, 2, 128, 1.0), (255, 260, 4, 65, 1.0),
+                                            (256, 516, 33, 8, 1.0), (257, 252, 7, 36, 1e-5), (300, 600, 1, 260, 300.0),
+                                            (2049, 132, 3, 88, 1.0), (40, 140, 80, 4, 1.0), (530, 257, 3, 40, 1.0)])
+def test_tensor_core_train_step_vs_oracle(port_kernels, B, N, H, Mc, scale):
+    """The float32 train step: one and several accumulation chains, ragged row and column tiles, operands with and without
+    one-box loads, hypercolumns wider and narrower than a 32-column group and more of them than a mask word holds, inputs
+    far from one, and a shape that takes the general kernels."""
+    import streambrain_b200 as B200
+    hp = dict(taupdt=0.1, khalf=-100.0, pmin=0.05, taubdt=0.02, density=0.5)
+    rs = np.random.RandomState(B + N)
+    init = (0.5 * scale, 1 / Mc, 0.5 * scale / Mc)
+    np.random.seed(0)
+    dev = B200.StructuralPlasticityLayer(N, H, Mc, hp["taupdt"], hp["khalf"], hp["pmin"], hp["taubdt"], hp["density"], 16, init,
+                                         dtype=np.float32)
+    np.random.seed(0)
+    ref = oracle.OracleLayer(port_kernels, "plastic", N, H, Mc, hp["taupdt"], init, np.float32, **{
+        k: hp[k] for k in ("khalf", "pmin", "taubdt", "density")})
+    tol = TOL[np.dtype(np.float32)]
+    for step in range(2):
+        x = (scale * rs.rand(B, N) * (rs.rand(B, N) > 0.3)).astype(np.float32)
+        y = rs.dirichlet(np.ones(Mc), size=(B, H)).reshape(B, H * Mc).astype(np.float32)
+        ref.train_step(x, y, None)
+        dev.train_step(x, y, None)
+        for name in ("Ci", "Cj", "Cij", "bias", "kbi"):
+            assert rel_inf(getattr(dev, name), getattr(ref, name)) < tol, (name, step)
+        assert weight_err(dev.weights, ref.weights) < 10 * tol, step
+        off = np.repeat(ref.wmask == 0, Mc, axis=1)
+        assert not dev.weights[off].any()
+        for name in ("weights", "bias", "Ci", "Cj", "Cij", "kbi"):
+            setattr(dev, name, getattr(ref, name))
