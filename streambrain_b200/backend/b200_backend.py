@@ -626,8 +626,8 @@ class Network:
                 if self.world_rank == 0 and self.verbose:
                     print('Layer - %d/%d' % (layer + 1, len(self._layers)), flush=True)
                 # the two draws of an epoch, in the reference's order
-                order = np.ascontiguousarray(np.random.permutation(range(n)), dtype=np.int64)
-                hc_order = np.ascontiguousarray(np.random.permutation(range(hypercolumns)), dtype=np.int64)
+                order = np.ascontiguousarray(np.random.permutation(n), dtype=np.int64)
+                hc_order = np.ascontiguousarray(np.random.permutation(hypercolumns), dtype=np.int64)
                 check(lib.sbb_network_set_epoch_order(self._handle, host_ptr(order)))
                 with self._progress(batches, 'Epoch %d/%d' % (epoch + 1, epochs)) as bar:
                     for first in range(0, batches, self.CHUNK):

@@ -3,6 +3,7 @@
 // include/sbb200.h for the contract of every entry point.
 #include "../../include/sbb200.h"
 #include "sbb_kernels.cuh"
+#include "sbb_host.cuh"
 #include "sbb_tc.cuh"
 
 #include <cstdarg>
@@ -78,26 +79,26 @@ int check_dtype(int dtype) {
   return SBB_OK;
 }
 
-// Device buffer that lives for one host-buffer call.
+// Device buffer that lives for one host-buffer call, on that call's stream.
 struct Staged {
+  sbb::HostCall &call;
   void *d = nullptr;
   size_t bytes = 0;
-  ~Staged() {
-    if (d) cudaFree(d);
-  }
+  explicit Staged(sbb::HostCall &c) : call(c) {}
+  ~Staged() { sbb::HostCall::free(d, call.stream()); }
   int alloc(size_t n) {
     bytes = n;
     if (n == 0) return SBB_OK;
-    SBB_CUDA(cudaMalloc(&d, n));
+    SBB_CUDA(sbb::HostCall::allocate(&d, n, call.stream()));
     return SBB_OK;
   }
   int upload(const void *h, size_t n) {
     SBB_TRY(alloc(n));
-    if (n) SBB_CUDA(cudaMemcpy(d, h, n, cudaMemcpyHostToDevice));
+    SBB_CUDA(call.upload(d, h, n, call.stream()));
     return SBB_OK;
   }
-  int download(void *h) const {
-    if (bytes) SBB_CUDA(cudaMemcpy(h, d, bytes, cudaMemcpyDeviceToHost));
+  int download(void *h) const {   // waits for everything queued so far
+    SBB_CUDA(call.download(h, d, bytes, call.stream()));
     return SBB_OK;
   }
   template <typename T>
@@ -105,6 +106,10 @@ struct Staged {
     return static_cast<T *>(d);
   }
 };
+#define HOST_CALL(name)                                            \
+  sbb::HostCall name;                                              \
+  if (name.error() != cudaSuccess) return cuda_fail(name.error(), "host call"); \
+  const cudaStream_t st = name.stream()
 
 // Scratch that grows on demand and is kept (no allocation in steady state).
 struct Scratch {
@@ -170,6 +175,7 @@ struct sbb_layer {
   Scratch lo;            // low parts of x[B, N] and y[B, M] for the split TF32 products of the batch contractions
   long lo_batch = 0;     // batch rows the planes in `lo` were written for (0 = none)
   cudaStream_t own_stream = nullptr;
+  cudaEvent_t ev_forward = nullptr;   // sbb_layer_step_host: the activation is there
   // sbb_layer_step_host_async: two staging slots, copies on their own streams
   Scratch ax[2], ay[2], at[2];
   cudaStream_t h2d_stream = nullptr, d2h_stream = nullptr;
@@ -491,7 +497,8 @@ int sbb_update_state(int dtype, void *activation, const void *inputs, const void
   ARG(B > 0 && N > 0 && M > 0, "update_state: non-positive shape B=%ld N=%ld M=%ld", B, N, M);
   SBB_TRY(need_device());
   const size_t s = esize(dtype);
-  Staged x, w, b, out, part;
+  HOST_CALL(call);
+  Staged x(call), w(call), b(call), out(call), part(call);
   SBB_TRY(x.upload(inputs, B * N * s));
   SBB_TRY(w.upload(weights, N * M * s));
   SBB_TRY(b.upload(bias, M * s));
@@ -506,17 +513,16 @@ int sbb_update_state(int dtype, void *activation, const void *inputs, const void
   }
   if (dtype == SBB_F32) {
     if (tc)
-      SBB_CUDA(sbb::launch_forward_product_tc(x.as<float>(), w.as<float>(), (float *)partial, B, N, M, splits, 0));
+      SBB_CUDA(sbb::launch_forward_product_tc(x.as<float>(), w.as<float>(), (float *)partial, B, N, M, splits, st));
     else
-      SBB_CUDA(sbb::launch_forward_product<float>(x.as<float>(), w.as<float>(), (float *)partial, B, N, M, splits, 0));
+      SBB_CUDA(sbb::launch_forward_product<float>(x.as<float>(), w.as<float>(), (float *)partial, B, N, M, splits, st));
     SBB_CUDA(sbb::launch_reduce_bias_softmax<float>((float *)partial, splits, b.as<float>(), out.as<float>(), B, 1, M,
-                                                    0, 0));
+                                                    0, st));
   } else {
-    SBB_CUDA(sbb::launch_forward_product<double>(x.as<double>(), w.as<double>(), (double *)partial, B, N, M, splits, 0));
+    SBB_CUDA(sbb::launch_forward_product<double>(x.as<double>(), w.as<double>(), (double *)partial, B, N, M, splits, st));
     SBB_CUDA(sbb::launch_reduce_bias_softmax<double>((double *)partial, splits, b.as<double>(), out.as<double>(), B, 1,
-                                                     M, 0, 0));
+                                                     M, 0, st));
   }
-  SBB_CUDA(cudaDeviceSynchronize());
   return out.download(activation);
 }
 
@@ -526,12 +532,12 @@ int sbb_add_bias(int dtype, void *a, const void *bias, long rows, long M) {
   ARG(rows > 0 && M > 0, "add_bias: non-positive shape");
   SBB_TRY(need_device());
   const size_t s = esize(dtype);
-  Staged da, db;
+  HOST_CALL(call);
+  Staged da(call), db(call);
   SBB_TRY(da.upload(a, rows * M * s));
   SBB_TRY(db.upload(bias, M * s));
-  if (dtype == SBB_F32) SBB_CUDA(sbb::launch_add_bias<float>(da.as<float>(), db.as<float>(), rows, M, 0));
-  else SBB_CUDA(sbb::launch_add_bias<double>(da.as<double>(), db.as<double>(), rows, M, 0));
-  SBB_CUDA(cudaDeviceSynchronize());
+  if (dtype == SBB_F32) SBB_CUDA(sbb::launch_add_bias<float>(da.as<float>(), db.as<float>(), rows, M, st));
+  else SBB_CUDA(sbb::launch_add_bias<double>(da.as<double>(), db.as<double>(), rows, M, st));
   return da.download(a);
 }
 
@@ -540,13 +546,13 @@ int sbb_softmax_minicolumns(int dtype, void *a, long rows, long H, long Mc) {
   ARG(a, "softmax_minicolumns: null pointer");
   ARG(rows > 0 && H > 0 && Mc > 0, "softmax_minicolumns: non-positive shape");
   SBB_TRY(need_device());
-  Staged da;
+  HOST_CALL(call);
+  Staged da(call);
   SBB_TRY(da.upload(a, rows * H * Mc * esize(dtype)));
   if (dtype == SBB_F32)
-    SBB_CUDA(sbb::launch_reduce_bias_softmax<float>(da.as<float>(), 1, nullptr, da.as<float>(), rows, H, Mc, 1, 0));
+    SBB_CUDA(sbb::launch_reduce_bias_softmax<float>(da.as<float>(), 1, nullptr, da.as<float>(), rows, H, Mc, 1, st));
   else
-    SBB_CUDA(sbb::launch_reduce_bias_softmax<double>(da.as<double>(), 1, nullptr, da.as<double>(), rows, H, Mc, 1, 0));
-  SBB_CUDA(cudaDeviceSynchronize());
+    SBB_CUDA(sbb::launch_reduce_bias_softmax<double>(da.as<double>(), 1, nullptr, da.as<double>(), rows, H, Mc, 1, st));
   return da.download(a);
 }
 
@@ -557,7 +563,8 @@ template <typename T>
 int update_counters_t(void *Ci, void *Cj, void *Cij, const void *a_i, const void *a_o, double taupdt, long B, long N,
                       long M) {
   const size_t s = sizeof(T);
-  Staged dci, dcj, dcij, dx, dy, sums;
+  HOST_CALL(call);
+  Staged dci(call), dcj(call), dcij(call), dx(call), dy(call), sums(call);
   SBB_TRY(dci.upload(Ci, N * s));
   SBB_TRY(dcj.upload(Cj, M * s));
   SBB_TRY(dcij.upload(Cij, N * M * s));
@@ -569,23 +576,24 @@ int update_counters_t(void *Ci, void *Cj, void *Cij, const void *a_i, const void
   // keep the [N, M] block 16-byte aligned whatever N + M is
   T *sxy = sx + ((N + M + 3) / 4) * 4;
   const bool tc = tensor_path<T>(dx.d, dy.d, N, M);
-  Scratch lo_buf;
+  Staged planes(call);
   LoPlanes lo;
-  int lo_rc = reserve_lo<T>(lo_buf, B, N, M, tc, &lo);
-  struct Release { Scratch &s; ~Release() { s.release(); } } release_lo{lo_buf};
-  SBB_TRY(lo_rc);
-  SBB_CUDA(sbb::launch_colsum<T>(dx.as<T>(), B, N, sx, 0, lo_as<T>(lo.x)));
-  SBB_CUDA(sbb::launch_colsum<T>(dy.as<T>(), B, M, sy, 0, lo_as<T>(lo.y)));
+  if (tc) {
+    SBB_TRY(planes.alloc((size_t)B * (size_t)(N + M) * sizeof(float)));
+    lo.x = planes.as<float>();
+    lo.y = lo.x + (size_t)B * N;
+  }
+  SBB_CUDA(sbb::launch_colsum<T>(dx.as<T>(), B, N, sx, st, lo_as<T>(lo.x)));
+  SBB_CUDA(sbb::launch_colsum<T>(dy.as<T>(), B, M, sy, st, lo_as<T>(lo.y)));
   if (tc) {
     if constexpr (std::is_same<T, float>::value)
-      SBB_CUDA(sbb::launch_outer_product_tc(dx.as<T>(), dy.as<T>(), B, N, M, sxy, 0, N, 0, lo.x, lo.y));
+      SBB_CUDA(sbb::launch_outer_product_tc(dx.as<T>(), dy.as<T>(), B, N, M, sxy, 0, N, st, lo.x, lo.y));
   } else {
-    SBB_CUDA(sbb::launch_outer_product<T>(dx.as<T>(), dy.as<T>(), B, N, M, sxy, 0, N, 0));
+    SBB_CUDA(sbb::launch_outer_product<T>(dx.as<T>(), dy.as<T>(), B, N, M, sxy, 0, N, st));
   }
-  SBB_CUDA(sbb::launch_counters_apply<T>(dci.as<T>(), sx, N, (T)taupdt, (T)B, 0));
-  SBB_CUDA(sbb::launch_counters_apply<T>(dcj.as<T>(), sy, M, (T)taupdt, (T)B, 0));
-  SBB_CUDA(sbb::launch_counters_apply<T>(dcij.as<T>(), sxy, N * M, (T)taupdt, (T)B, 0));
-  SBB_CUDA(cudaDeviceSynchronize());
+  SBB_CUDA(sbb::launch_counters_apply<T>(dci.as<T>(), sx, N, (T)taupdt, (T)B, st));
+  SBB_CUDA(sbb::launch_counters_apply<T>(dcj.as<T>(), sy, M, (T)taupdt, (T)B, st));
+  SBB_CUDA(sbb::launch_counters_apply<T>(dcij.as<T>(), sxy, N * M, (T)taupdt, (T)B, st));
   SBB_TRY(dci.download(Ci));
   SBB_TRY(dcj.download(Cj));
   return dcij.download(Cij);
@@ -595,19 +603,21 @@ template <typename T>
 int update_weights_t(void *Ci, void *Cj, void *Cij, const void *a_i, const void *a_o, double taupdt, long B, long N,
                      long M, void *weights, double cthr) {
   const size_t s = sizeof(T);
-  Staged dci, dcj, dcij, dx, dy, dw;
+  HOST_CALL(call);
+  Staged dci(call), dcj(call), dcij(call), dx(call), dy(call), dw(call);
   SBB_TRY(dci.upload(Ci, N * s));
   SBB_TRY(dcj.upload(Cj, M * s));
   SBB_TRY(dcij.upload(Cij, N * M * s));
   SBB_TRY(dx.upload(a_i, B * N * s));
   SBB_TRY(dy.upload(a_o, B * M * s));
   SBB_TRY(dw.alloc(N * M * s));
-  struct Vectors : Scratch {
-    ~Vectors() { release(); }
-  } vectors;
+  Staged space(call);
+  SBB_TRY(space.alloc((size_t)((N + 3) / 4 * 4 + M) * s));
+  Scratch vectors;   // (borrows)
+  vectors.d = space.d;
+  vectors.cap = space.bytes;
   SBB_TRY(train_rows<T>(nullptr, dx.as<T>(), dy.as<T>(), B, N, M, 1, dci.as<T>(), dcj.as<T>(), dcij.as<T>(), dw.as<T>(), nullptr,
-                        sbb::make_trace_params<T>(taupdt, cthr, B), sbb::BiasParams<T>{}, vectors, 0));
-  SBB_CUDA(cudaDeviceSynchronize());
+                        sbb::make_trace_params<T>(taupdt, cthr, B), sbb::BiasParams<T>{}, vectors, st));
   SBB_TRY(dci.download(Ci));
   SBB_TRY(dcj.download(Cj));
   SBB_TRY(dcij.download(Cij));
@@ -617,15 +627,15 @@ int update_weights_t(void *Ci, void *Cj, void *Cij, const void *a_i, const void 
 template <typename T>
 int recompute_weights_t(void *weights, const void *Ci, const void *Cj, const void *Cij, double cthr, long N, long M) {
   const size_t s = sizeof(T);
-  Staged dci, dcj, dcij, dw;
+  HOST_CALL(call);
+  Staged dci(call), dcj(call), dcij(call), dw(call);
   SBB_TRY(dci.upload(Ci, N * s));
   SBB_TRY(dcj.upload(Cj, M * s));
   SBB_TRY(dcij.upload(Cij, N * M * s));
   SBB_TRY(dw.alloc(N * M * s));
   sbb::TraceParams<T> p = sbb::make_trace_params<T>(2 * cthr, cthr, 1);
   SBB_CUDA(sbb::launch_trace_apply<T>(nullptr, N, M, 1, M, dci.as<T>(), dcj.as<T>(), dcij.as<T>(), dw.as<T>(), nullptr,
-                                      p, 0, 0, N, 0));
-  SBB_CUDA(cudaDeviceSynchronize());
+                                      p, 0, 0, N, st));
   return dw.download(weights);
 }
 
@@ -633,17 +643,17 @@ template <typename T>
 int update_mask_t(uint8_t *wmask, const void *weights, const void *Ci, const void *Cj, const void *Cij, double cthr,
                   long N, long M, long H, long Mc, long h, long iterations) {
   const size_t s = sizeof(T);
-  Staged dm, dw, dci, dcj, dcij, score;
+  HOST_CALL(call);
+  Staged dm(call), dw(call), dci(call), dcj(call), dcij(call), score(call);
   SBB_TRY(dm.upload(wmask, N * H));
   SBB_TRY(dw.upload(weights, N * M * s));
   SBB_TRY(dci.upload(Ci, N * s));
   SBB_TRY(dcj.upload(Cj, M * s));
   SBB_TRY(dcij.upload(Cij, N * M * s));
   SBB_TRY(score.alloc(sbb::mask_scratch_bytes(N, s)));
-  SBB_CUDA(sbb::mask_scratch_init(score.d, 0));
+  SBB_CUDA(sbb::mask_scratch_init(score.d, st));
   SBB_CUDA(sbb::launch_mask_update<T>(dm.as<uint8_t>(), dw.as<T>(), dci.as<T>(), dcj.as<T>(), dcij.as<T>(), (T)cthr, N,
-                                      M, H, Mc, h, iterations, score.d, 0));
-  SBB_CUDA(cudaDeviceSynchronize());
+                                      M, H, Mc, h, iterations, score.d, st));
   return dm.download(wmask);
 }
 }  // namespace
@@ -686,12 +696,12 @@ int sbb_update_bias(int dtype, void *bias, const void *Cj, double cthr, long M) 
   ARG(M > 0, "update_bias: non-positive size");
   SBB_TRY(need_device());
   const size_t s = esize(dtype);
-  Staged db, dc;
+  HOST_CALL(call);
+  Staged db(call), dc(call);
   SBB_TRY(db.alloc(M * s));
   SBB_TRY(dc.upload(Cj, M * s));
-  if (dtype == SBB_F32) SBB_CUDA(sbb::launch_update_bias<float>(db.as<float>(), dc.as<float>(), (float)cthr, M, 0));
-  else SBB_CUDA(sbb::launch_update_bias<double>(db.as<double>(), dc.as<double>(), cthr, M, 0));
-  SBB_CUDA(cudaDeviceSynchronize());
+  if (dtype == SBB_F32) SBB_CUDA(sbb::launch_update_bias<float>(db.as<float>(), dc.as<float>(), (float)cthr, M, st));
+  else SBB_CUDA(sbb::launch_update_bias<double>(db.as<double>(), dc.as<double>(), cthr, M, st));
   return db.download(bias);
 }
 
@@ -702,17 +712,17 @@ int sbb_update_bias_regularized(int dtype, void *bias, void *kbi, const void *Cj
   ARG(M > 0, "update_bias_regularized: non-positive size");
   SBB_TRY(need_device());
   const size_t s = esize(dtype);
-  Staged db, dk, dc;
+  HOST_CALL(call);
+  Staged db(call), dk(call), dc(call);
   SBB_TRY(db.alloc(M * s));
   SBB_TRY(dk.upload(kbi, M * s));
   SBB_TRY(dc.upload(Cj, M * s));
   if (dtype == SBB_F32)
     SBB_CUDA(sbb::launch_update_bias_regularized<float>(db.as<float>(), dk.as<float>(), dc.as<float>(), (float)cthr,
-                                                        (float)khalf, (float)pmin, (float)taubdt, M, 0));
+                                                        (float)khalf, (float)pmin, (float)taubdt, M, st));
   else
     SBB_CUDA(sbb::launch_update_bias_regularized<double>(db.as<double>(), dk.as<double>(), dc.as<double>(), cthr, khalf,
-                                                         pmin, taubdt, M, 0));
-  SBB_CUDA(cudaDeviceSynchronize());
+                                                         pmin, taubdt, M, st));
   SBB_TRY(db.download(bias));
   return dk.download(kbi);
 }
@@ -734,12 +744,12 @@ int sbb_apply_mask(int dtype, void *weights, const uint8_t *wmask, long N, long 
   ARG(weights && wmask, "apply_mask: null pointer");
   ARG(N > 0 && H > 0 && Mc > 0 && M == H * Mc, "apply_mask: shape mismatch N=%ld M=%ld H=%ld Mc=%ld", N, M, H, Mc);
   SBB_TRY(need_device());
-  Staged dw, dm;
+  HOST_CALL(call);
+  Staged dw(call), dm(call);
   SBB_TRY(dw.upload(weights, N * M * esize(dtype)));
   SBB_TRY(dm.upload(wmask, N * H));
-  if (dtype == SBB_F32) SBB_CUDA(sbb::launch_apply_mask<float>(dw.as<float>(), dm.as<uint8_t>(), N, M, H, Mc, 0));
-  else SBB_CUDA(sbb::launch_apply_mask<double>(dw.as<double>(), dm.as<uint8_t>(), N, M, H, Mc, 0));
-  SBB_CUDA(cudaDeviceSynchronize());
+  if (dtype == SBB_F32) SBB_CUDA(sbb::launch_apply_mask<float>(dw.as<float>(), dm.as<uint8_t>(), N, M, H, Mc, st));
+  else SBB_CUDA(sbb::launch_apply_mask<double>(dw.as<double>(), dm.as<uint8_t>(), N, M, H, Mc, st));
   return dw.download(weights);
 }
 
@@ -777,6 +787,7 @@ int sbb_layer_create(const sbb_layer_desc *desc, sbb_layer **out) {
       if (e == cudaSuccess) e = cudaMemset(L->state[k], 0, L->state_bytes[k]);
     }
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&L->own_stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&L->ev_forward, cudaEventDisableTiming);
   if (e != cudaSuccess) rc = cuda_fail(e, "layer_create");
   if (rc == SBB_OK) rc = L->ticket.reserve(256);
   if (rc == SBB_OK && (e = cudaMemsetAsync(L->ticket.d, 0, 256, 0)) != cudaSuccess) rc = cuda_fail(e, "layer_create");
@@ -817,6 +828,7 @@ int sbb_layer_destroy(sbb_layer *L) {
     L->shard.yg.release();
   }
   if (L->own_stream) cudaStreamDestroy(L->own_stream);
+  if (L->ev_forward) cudaEventDestroy(L->ev_forward);
   if (L->h2d_stream) cudaStreamDestroy(L->h2d_stream);
   if (L->d2h_stream) cudaStreamDestroy(L->d2h_stream);
   for (int k = 0; k < 2; ++k) {
@@ -852,7 +864,9 @@ int sbb_layer_set_state(sbb_layer *L, int which, const void *host, size_t bytes)
   ARG(host, "set_state: null pointer");
   SBB_TRY(check_layer(L));
   SBB_CUDA(cudaDeviceSynchronize());
-  SBB_CUDA(cudaMemcpy(L->state[which], host, bytes, cudaMemcpyHostToDevice));
+  HOST_CALL(call);
+  SBB_CUDA(call.upload(L->state[which], host, bytes, st));
+  SBB_CUDA(cudaStreamSynchronize(st));
   return SBB_OK;
 }
 
@@ -861,7 +875,8 @@ int sbb_layer_get_state(sbb_layer *L, int which, void *host, size_t bytes) {
   ARG(host, "get_state: null pointer");
   SBB_TRY(check_layer(L));
   SBB_CUDA(cudaDeviceSynchronize());
-  SBB_CUDA(cudaMemcpy(host, L->state[which], bytes, cudaMemcpyDeviceToHost));
+  HOST_CALL(call);
+  SBB_CUDA(call.download(host, L->state[which], bytes, st));
   return check_wait_status();
 }
 
@@ -956,15 +971,16 @@ int sbb_layer_forward_host(sbb_layer *L, const void *x_host, long B, void *y_hos
   const size_t s = esize(L->desc.dtype);
   SBB_TRY(L->hx.reserve((size_t)B * L->N * s));
   SBB_TRY(L->hy.reserve((size_t)B * L->M * s));
+  sbb::HostCall call;
+  if (call.error() != cudaSuccess) return cuda_fail(call.error(), "host call");
   cudaStream_t st = L->own_stream;
   // Work queued earlier on other streams (a device-buffer call) must have landed
   // before this call reads or rewrites the layer state on its own stream.
   SBB_CUDA(cudaDeviceSynchronize());
-  SBB_CUDA(cudaMemcpyAsync(L->hx.d, x_host, (size_t)B * L->N * s, cudaMemcpyHostToDevice, st));
+  SBB_CUDA(call.upload(L->hx.d, x_host, (size_t)B * L->N * s, st));
   SBB_TRY(DISPATCH(L->desc.dtype, layer_forward<float>(L, (const float *)L->hx.d, B, (float *)L->hy.d, st),
                    layer_forward<double>(L, (const double *)L->hx.d, B, (double *)L->hy.d, st)));
-  SBB_CUDA(cudaMemcpyAsync(y_host, L->hy.d, (size_t)B * L->M * s, cudaMemcpyDeviceToHost, st));
-  SBB_CUDA(cudaStreamSynchronize(st));
+  SBB_CUDA(call.download(y_host, L->hy.d, (size_t)B * L->M * s, st));
   return check_wait_status();
 }
 
@@ -977,12 +993,14 @@ int sbb_layer_train_step_host(sbb_layer *L, const void *x_host, const void *y_ho
   const size_t s = esize(L->desc.dtype);
   SBB_TRY(L->hx.reserve((size_t)B * L->N * s));
   SBB_TRY(L->ht.reserve((size_t)B * L->M * s));
+  sbb::HostCall call;
+  if (call.error() != cudaSuccess) return cuda_fail(call.error(), "host call");
   cudaStream_t st = L->own_stream;
   // Work queued earlier on other streams (a device-buffer call) must have landed
   // before this call reads or rewrites the layer state on its own stream.
   SBB_CUDA(cudaDeviceSynchronize());
-  SBB_CUDA(cudaMemcpyAsync(L->hx.d, x_host, (size_t)B * L->N * s, cudaMemcpyHostToDevice, st));
-  SBB_CUDA(cudaMemcpyAsync(L->ht.d, y_host, (size_t)B * L->M * s, cudaMemcpyHostToDevice, st));
+  SBB_CUDA(call.upload(L->hx.d, x_host, (size_t)B * L->N * s, st));
+  SBB_CUDA(call.upload(L->ht.d, y_host, (size_t)B * L->M * s, st));
   SBB_TRY(DISPATCH(L->desc.dtype,
                    layer_train_step<float>(L, (const float *)L->hx.d, (const float *)L->ht.d, B, hypercolumn, st),
                    layer_train_step<double>(L, (const double *)L->hx.d, (const double *)L->ht.d, B, hypercolumn, st)));
@@ -1001,22 +1019,26 @@ int sbb_layer_step_host(sbb_layer *L, const void *x_host, const void *target_hos
   SBB_TRY(L->hx.reserve((size_t)B * L->N * s));
   SBB_TRY(L->hy.reserve((size_t)B * L->M * s));
   if (target_host) SBB_TRY(L->ht.reserve((size_t)B * L->M * s));
+  sbb::HostCall call;
+  if (call.error() != cudaSuccess) return cuda_fail(call.error(), "host call");
   cudaStream_t st = L->own_stream;
   // Work queued earlier on other streams (a device-buffer call) must have landed
   // before this call reads or rewrites the layer state on its own stream.
   SBB_CUDA(cudaDeviceSynchronize());
-  SBB_CUDA(cudaMemcpyAsync(L->hx.d, x_host, (size_t)B * L->N * s, cudaMemcpyHostToDevice, st));
+  SBB_CUDA(call.upload(L->hx.d, x_host, (size_t)B * L->N * s, st));
   if (target_host)
-    SBB_CUDA(cudaMemcpyAsync(L->ht.d, target_host, (size_t)B * L->M * s, cudaMemcpyHostToDevice, st));
+    SBB_CUDA(call.upload(L->ht.d, target_host, (size_t)B * L->M * s, st));
   const void *train_on = target_host ? L->ht.d : L->hy.d;
-  if (L->desc.dtype == SBB_F32) {
-    SBB_TRY(layer_forward<float>(L, (const float *)L->hx.d, B, (float *)L->hy.d, st));
-    SBB_TRY(layer_train_step<float>(L, (const float *)L->hx.d, (const float *)train_on, B, hypercolumn, st));
-  } else {
-    SBB_TRY(layer_forward<double>(L, (const double *)L->hx.d, B, (double *)L->hy.d, st));
-    SBB_TRY(layer_train_step<double>(L, (const double *)L->hx.d, (const double *)train_on, B, hypercolumn, st));
+  SBB_TRY(DISPATCH(L->desc.dtype, layer_forward<float>(L, (const float *)L->hx.d, B, (float *)L->hy.d, st),
+                   layer_forward<double>(L, (const double *)L->hx.d, B, (double *)L->hy.d, st)));
+  if (y_host) SBB_CUDA(cudaEventRecord(L->ev_forward, st));
+  SBB_TRY(DISPATCH(L->desc.dtype,
+                   layer_train_step<float>(L, (const float *)L->hx.d, (const float *)train_on, B, hypercolumn, st),
+                   layer_train_step<double>(L, (const double *)L->hx.d, (const double *)train_on, B, hypercolumn, st)));
+  if (y_host) {   // the activation leaves beside the train step
+    SBB_CUDA(cudaStreamWaitEvent(call.stream(), L->ev_forward, 0));
+    SBB_CUDA(call.download(y_host, L->hy.d, (size_t)B * L->M * s, call.stream()));
   }
-  if (y_host) SBB_CUDA(cudaMemcpyAsync(y_host, L->hy.d, (size_t)B * L->M * s, cudaMemcpyDeviceToHost, st));
   SBB_CUDA(cudaStreamSynchronize(st));
   return check_wait_status();
 }
@@ -1492,15 +1514,20 @@ int sbb_count_correct(int dtype, const void *pred_dev, const void *labels_dev, l
   ARG(rows >= 0 && classes > 0, "count_correct: bad shape");
   SBB_TRY(need_device());
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  Staged cnt;
-  SBB_TRY(cnt.alloc(sizeof(unsigned long long)));
+  struct Counter {   // on the caller's stream
+    void *d = nullptr;
+    cudaStream_t st;
+    ~Counter() { sbb::HostCall::free(d, st); }
+  } cnt;
+  cnt.st = st;
+  SBB_CUDA(sbb::HostCall::allocate(&cnt.d, sizeof(unsigned long long), st));
   SBB_CUDA(cudaMemsetAsync(cnt.d, 0, sizeof(unsigned long long), st));
   if (dtype == SBB_F32)
     SBB_CUDA(sbb::launch_count_correct<float>((const float *)pred_dev, (const float *)labels_dev, rows, classes,
-                                              cnt.as<unsigned long long>(), st));
+                                              static_cast<unsigned long long *>(cnt.d), st));
   else
     SBB_CUDA(sbb::launch_count_correct<double>((const double *)pred_dev, (const double *)labels_dev, rows, classes,
-                                               cnt.as<unsigned long long>(), st));
+                                               static_cast<unsigned long long *>(cnt.d), st));
   unsigned long long h = 0;
   SBB_CUDA(cudaMemcpyAsync(&h, cnt.d, sizeof(h), cudaMemcpyDeviceToHost, st));
   SBB_CUDA(cudaStreamSynchronize(st));

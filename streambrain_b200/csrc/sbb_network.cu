@@ -11,6 +11,7 @@
 // no host synchronisation in between, and evaluation hits are counted on the device and read once.
 // The file uses the layer objects only through the public C ABI.
 #include "../../include/sbb200.h"
+#include "sbb_host.cuh"
 #include "sbb_kernels.cuh"
 
 #include <cstdarg>
@@ -359,8 +360,11 @@ int sbb_network_set_dataset(sbb_network *net, const void *images_host, const voi
   NET_CUDA(cudaStreamSynchronize(net->stream));
   NET_TRY(net->images.reserve((size_t)samples * features * s));
   NET_TRY(net->labels.reserve((size_t)samples * classes * s));
-  NET_CUDA(cudaMemcpy(net->images.d, images_host, (size_t)samples * features * s, cudaMemcpyHostToDevice));
-  NET_CUDA(cudaMemcpy(net->labels.d, labels_host, (size_t)samples * classes * s, cudaMemcpyHostToDevice));
+  sbb::HostCall call;
+  NET_CUDA(call.error());
+  NET_CUDA(call.upload(net->images.d, images_host, (size_t)samples * features * s, net->stream));
+  NET_CUDA(call.upload(net->labels.d, labels_host, (size_t)samples * classes * s, net->stream));
+  NET_CUDA(cudaStreamSynchronize(net->stream));
   net->samples = samples;
   net->features = features;
   net->classes = classes;

@@ -624,7 +624,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
 std::mutex g_mutex;
 EncodeTiledFn g_encode = nullptr;
 int g_available = -1;           // -1 unknown, 0 no, 1 yes
-int *g_status[64] = {nullptr};  // per-device status word
+int *g_status[64] = {nullptr};  // per-device status word, in mapped host memory: read without a copy
 int g_sm_count_tc[64] = {0};
 std::atomic<int> g_reserved_sms{-1};   // -1: not set yet (the environment decides on first use)
 std::atomic<long long> g_wait_limit{kWaitLimitCycles};
@@ -670,8 +670,8 @@ int *status_word() {
   std::lock_guard<std::mutex> lock(g_mutex);
   if (g_status[dev] == nullptr) {
     int *p = nullptr;
-    if (cudaMalloc(&p, sizeof(int)) != cudaSuccess) return nullptr;
-    cudaMemset(p, 0, sizeof(int));
+    if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+    *p = 0;
     g_status[dev] = p;
     int n = 0;
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
@@ -1079,44 +1079,30 @@ int tc_get_reserved_sms() {
   return v;
 }
 
+static volatile int *status_if_any() {
+  const int dev = current_device();
+  std::lock_guard<std::mutex> lock(g_mutex);
+  return g_status[dev];
+}
+
 // The status word without synchronising the device: meaningful for work the caller has already waited for.
 cudaError_t tc_peek_status(int *status) {
-  *status = 0;
-  const int dev = current_device();
-  int *p = nullptr;
-  {
-    std::lock_guard<std::mutex> lock(g_mutex);
-    p = g_status[dev];
-  }
-  if (p == nullptr) return cudaSuccess;
-  return cudaMemcpy(status, p, sizeof(int), cudaMemcpyDeviceToHost);
+  volatile int *p = status_if_any();
+  *status = p ? *p : 0;
+  return cudaSuccess;
 }
 
 cudaError_t tc_clear_status() {
-  const int dev = current_device();
-  int *p = nullptr;
-  {
-    std::lock_guard<std::mutex> lock(g_mutex);
-    p = g_status[dev];
-  }
-  if (p == nullptr) return cudaSuccess;
-  cudaError_t e = cudaDeviceSynchronize();
+  const cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return e;
-  return cudaMemset(p, 0, sizeof(int));
+  if (volatile int *p = status_if_any()) *p = 0;
+  return cudaSuccess;
 }
 
 cudaError_t tc_read_status(int *status) {
   *status = 0;
-  const int dev = current_device();
-  int *p = nullptr;
-  {
-    std::lock_guard<std::mutex> lock(g_mutex);
-    p = g_status[dev];
-  }
-  if (p == nullptr) return cudaSuccess;
-  cudaError_t e = cudaDeviceSynchronize();
-  if (e != cudaSuccess) return e;
-  return cudaMemcpy(status, p, sizeof(int), cudaMemcpyDeviceToHost);
+  const cudaError_t e = cudaDeviceSynchronize();
+  return e != cudaSuccess ? e : tc_peek_status(status);
 }
 
 }  // namespace sbb

@@ -603,3 +603,26 @@ def test_tensor_core_train_step_vs_oracle(port_kernels, B, N, H, Mc, scale):
         assert not dev.weights[off].any()
         for name in ("weights", "bias", "Ci", "Cj", "Cij", "kbi"):
             setattr(dev, name, getattr(ref, name))
+
+
+@pytest.mark.parametrize("n,m", [(64, 256), (5461, 3), (8193, 8), (65537, 4), (2048, 1024), (1399, 1499)])
+def test_state_round_trip_through_the_copy_slots(n, m):
+    """Host arrays of 64 kB up to several pinned slots, whole and ragged, from two threads at once."""
+    import threading
+    import streambrain_b200 as B200
+    np.random.seed(1)
+    layers = [B200.DenseLayer(n, 1, m, 0.1, (1, 1, 1), dtype=np.float32) for _ in range(2)]
+    values = [np.random.rand(n, m).astype(np.float32) for _ in range(2)]
+    bad = []
+
+    def turn(layer, value):
+        for _ in range(3):
+            layer.weights = value
+            if not np.array_equal(layer.weights, value):
+                bad.append(value.shape)
+    threads = [threading.Thread(target=turn, args=a) for a in zip(layers, values)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
