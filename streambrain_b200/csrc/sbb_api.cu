@@ -170,7 +170,7 @@ struct sbb_layer {
   Scratch fwd_partial;   // k-split partial sums of the forward product
   Scratch score;         // mask-update scratch: per-row score, active count, candidate lists
   Scratch hx, hy, ht;    // staging for the host-buffer entry points
-  Scratch ticket;        // counts the blocks of a launch that have finished; zero between launches
+  Scratch ticket;        // finished blocks of a launch: [whole launch][per hypercolumn]; zero between launches
   Scratch rc;            // reciprocals of Ci and Cj (0 below the threshold) for the tensor-core trace update
   Scratch lo;            // low parts of x[B, N] and y[B, M] for the split TF32 products of the batch contractions
   long lo_batch = 0;     // batch rows the planes in `lo` were written for (0 = none)
@@ -248,6 +248,15 @@ int layer_forward(sbb_layer *L, const T *x, long B, T *y, cudaStream_t st) {
   if (narrow<T>(L) && sbb::narrow_forward(B, L->N, L->M, sizeof(T))) {
     PhaseTimer timer(L, SBB_PHASE_FORWARD, st);
     SBB_CUDA(sbb::launch_narrow_forward<T>(x, W, static_cast<const T *>(L->state[SBB_STATE_BIAS]), y, B, L->N, L->M, L->Mc, st));
+    timer.stop();
+    return SBB_OK;
+  }
+  size_t few = 0;
+  if (sbb::few_samples<T>(W, B, L->N, L->H, L->Mc, &few)) {
+    SBB_TRY(L->fwd_partial.reserve(few * sizeof(T)));
+    PhaseTimer timer(L, SBB_PHASE_FORWARD, st);
+    SBB_CUDA(sbb::launch_few_forward<T>(x, W, static_cast<const T *>(L->state[SBB_STATE_BIAS]), y, B, L->N, L->H, L->Mc,
+                                        static_cast<T *>(L->fwd_partial.d), static_cast<int *>(L->ticket.d) + 1, st));
     timer.stop();
     return SBB_OK;
   }
@@ -789,8 +798,8 @@ int sbb_layer_create(const sbb_layer_desc *desc, sbb_layer **out) {
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&L->own_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&L->ev_forward, cudaEventDisableTiming);
   if (e != cudaSuccess) rc = cuda_fail(e, "layer_create");
-  if (rc == SBB_OK) rc = L->ticket.reserve(256);
-  if (rc == SBB_OK && (e = cudaMemsetAsync(L->ticket.d, 0, 256, 0)) != cudaSuccess) rc = cuda_fail(e, "layer_create");
+  if (rc == SBB_OK) rc = L->ticket.reserve((size_t)(L->H + 1) * sizeof(int));
+  if (rc == SBB_OK && (e = cudaMemsetAsync(L->ticket.d, 0, L->ticket.cap, 0)) != cudaSuccess) rc = cuda_fail(e, "layer_create");
   if (rc == SBB_OK) rc = L->rc.reserve((size_t)((L->N + 3) / 4 * 4 + L->M) * s);
   if (rc == SBB_OK && desc->kind == SBB_LAYER_PLASTIC) {
     rc = L->score.reserve(sbb::mask_scratch_bytes(L->N, s));

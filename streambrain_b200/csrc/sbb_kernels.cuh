@@ -75,6 +75,14 @@ template <typename T>
 cudaError_t launch_narrow_train(const T *x, const T *y, long B, long N, long M, long H, long Mc, T *Ci, T *Cj, T *Cij, T *W,
                                 const uint8_t *wmask, TraceParams<T> p, BiasParams<T> nb, int *ticket, cudaStream_t st);
 
+// Forward pass of up to kFewSamples samples as one launch.  `tickets`: one int per hypercolumn, zero between launches.
+constexpr long kFewSamples = 4;
+template <typename T>
+bool few_samples(const T *W, long B, long N, long H, long Mc, size_t *scratch_elems);
+template <typename T>
+cudaError_t launch_few_forward(const T *x, const T *W, const T *bias, T *out, long B, long N, long H, long Mc, T *partial,
+                               int *tickets, cudaStream_t st);
+
 // Fused trace step for rows [row_begin,row_end) of Cij: acc = x^T y over the batch,
 // Cij = EMA(Cij, acc), w = log-ratio(Cij, Ci, Cj) with rows/columns below cthr and
 // masked connections (wmask may be null) set to zero.  Ci, Cj hold the NEW values.

@@ -626,3 +626,24 @@ def test_state_round_trip_through_the_copy_slots(n, m):
     for t in threads:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("tag,dtype", DTYPES)
+@pytest.mark.parametrize("B", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("N,H,Mc", [(1, 1, 33), (17, 3, 37), (1568, 30, 100), (4096, 2, 256), (4097, 5, 64), (700, 13, 4), (333, 2, 300),
+                                    (260, 1, 1024)])
+def test_forward_of_few_samples_vs_oracle(port_kernels, tag, dtype, B, N, H, Mc):
+    """One to four samples take a kernel of their own: vector and scalar columns, one and many hypercolumns per block, wide
+    hypercolumns, inputs that do and do not divide into ranges, and the first sizes that do not take it."""
+    import streambrain_b200 as B200
+    np.random.seed(2)
+    args = (N, H, Mc, 0.01, -100.0, 0.05, 0.02, 0.5, 16, (0.5, 1 / Mc, 0.5 / Mc))
+    dev = B200.StructuralPlasticityLayer(*args, dtype=dtype)
+    ref = oracle.OracleLayer(port_kernels, "plastic", N, H, Mc, 0.01, (0.5, 1 / Mc, 0.5 / Mc), dtype, khalf=-100.0, pmin=0.05,
+                             taubdt=0.02, density=0.5)
+    for name in ("weights", "bias"):
+        setattr(ref, name, getattr(dev, name))
+    x = np.random.rand(B, N).astype(dtype)
+    want = ref.compute_activation(x)
+    for _ in range(2):   # the tickets are zero again after a launch
+        assert rel_inf(dev.compute_activation(x), want) < TOL[np.dtype(dtype)]
