@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(kFewThreads)
   for (int t = threadIdx.x; t < R * width; t += kFewThreads) {
     const T *p = partial + (long)(t / width) * M + c0 + t % width;
     T s = (T)0;
-#pragma unroll 8
+#pragma unroll 16
     for (int q = 0; q < (int)gridDim.y; ++q) s += __ldcg(p + (long)q * R * M);
     s_support[t] = s + bias[c0 + t % width];
   }
@@ -125,14 +125,15 @@ bool few_plan(const void *W, long B, long N, long H, long Mc, FewPlan &p) {
   if (sizeof(T) == 4 && N > 4096) return false;
   p.vec = 16 / (int)sizeof(T);
   if (M % p.vec != 0 || (reinterpret_cast<uintptr_t>(W) & 15u) != 0) p.vec = 1;
-  // whole hypercolumns per block, their start on a vector boundary: up to half a block of threads across them
+  // whole hypercolumns per block, their start on a vector boundary: a quarter of the threads across them (wider blocks need
+  // more ranges to fill the chip, and the last block reads a partial sum per range)
   const long most = (long)kFewThreads * p.vec;
-  long hcs = most / 2 / Mc > 0 ? most / 2 / Mc : 1;
+  long hcs = most / 4 / Mc > 0 ? most / 4 / Mc : 1;
   if (hcs > H) hcs = H;
   while (hcs > 1 && (hcs * Mc) % p.vec != 0) --hcs;
   if ((hcs * Mc) % p.vec != 0) {
     if (hcs * Mc != M) p.vec = 1;
-    hcs = kFewThreads / Mc / 2 > 0 ? kFewThreads / Mc / 2 : 1;
+    hcs = kFewThreads / Mc / 4 > 0 ? kFewThreads / Mc / 4 : 1;
     if (hcs > H) hcs = H;
   }
   const long cols = hcs * Mc;

@@ -787,8 +787,12 @@ __global__ void __launch_bounds__(256)
   // (entries inside, partial sums outside: all entries' loads are in flight at once.  With the loops the other way round
   // each partial sum was a round trip to memory of its own: 11.2 us for 128 x 15 groups of 200 doubles in six partial
   // sums)
+  T bias_v[NC];
 #pragma unroll
-  for (int e = 0; e < NC; ++e) v[e] = e * 32 < left ? src[e * 32] : -INFINITY;
+  for (int e = 0; e < NC; ++e) {
+    v[e] = e * 32 < left ? src[e * 32] : -INFINITY;
+    bias_v[e] = bs && e * 32 < left ? bs[e * 32] : (T)0;
+  }
   if (SPLIT) {
 #pragma unroll 2
     for (int z = 1; z < splits; ++z) {
@@ -802,20 +806,34 @@ __global__ void __launch_bounds__(256)
   }
 #pragma unroll
   for (int e = 0; e < NC; ++e) {
-    if (bs && e * 32 < left) v[e] += bs[e * 32];
+    if (bs) v[e] += bias_v[e];
     mx = v[e] > mx ? v[e] : mx;
   }
   mx = subwarp_max(mx, 32);
   T sum = (T)0;
+  if constexpr (sizeof(T) == 8) {
+    // one copy of the float64 exponential (the entries rotate through slot 0) and one division: unrolled, a kernel of a
+    // few microseconds spends most of them fetching instructions
+#pragma unroll 1
+    for (int e = 0; e < NC; ++e) {
+      const T x = e * 32 < left ? sbb_exp(v[0] - mx) : (T)0;
+      sum += x;
 #pragma unroll
-  for (int e = 0; e < NC; ++e) {
-    v[e] = e * 32 < left ? sbb_exp(v[e] - mx) : (T)0;
-    sum += v[e];
+      for (int q = 0; q + 1 < NC; ++q) v[q] = v[q + 1];
+      v[NC - 1] = x;
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < NC; ++e) {
+      v[e] = e * 32 < left ? sbb_exp(v[e] - mx) : (T)0;
+      sum += v[e];
+    }
   }
   sum = subwarp_sum(sum, 32);
+  const T scale = sizeof(T) == 8 ? (T)1 / sum : (T)0;
 #pragma unroll
   for (int e = 0; e < NC; ++e)
-    if (e * 32 < left) dst[e * 32] = v[e] / sum;
+    if (e * 32 < left) dst[e * 32] = sizeof(T) == 8 ? v[e] * scale : v[e] / sum;
 }
 
 // out[r, j] = sum_s partial[s, r, j] + bias[j]   (no softmax)
