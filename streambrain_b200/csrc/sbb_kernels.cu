@@ -787,11 +787,10 @@ __global__ void __launch_bounds__(256)
   // (entries inside, partial sums outside: all entries' loads are in flight at once.  With the loops the other way round
   // each partial sum was a round trip to memory of its own: 11.2 us for 128 x 15 groups of 200 doubles in six partial
   // sums)
-  T bias_v[NC];
 #pragma unroll
   for (int e = 0; e < NC; ++e) {
     v[e] = e * 32 < left ? src[e * 32] : -INFINITY;
-    bias_v[e] = bs && e * 32 < left ? bs[e * 32] : (T)0;
+    if (!SPLIT && bs && e * 32 < left) v[e] += bs[e * 32];
   }
   if (SPLIT) {
 #pragma unroll 2
@@ -806,7 +805,7 @@ __global__ void __launch_bounds__(256)
   }
 #pragma unroll
   for (int e = 0; e < NC; ++e) {
-    if (bs) v[e] += bias_v[e];
+    if (SPLIT && bs && e * 32 < left) v[e] += bs[e * 32];
     mx = v[e] > mx ? v[e] : mx;
   }
   mx = subwarp_max(mx, 32);
@@ -830,10 +829,17 @@ __global__ void __launch_bounds__(256)
     }
   }
   sum = subwarp_sum(sum, 32);
-  const T scale = sizeof(T) == 8 ? (T)1 / sum : (T)0;
+  if constexpr (sizeof(T) == 8) {
+    const T scale = (T)1 / sum;
 #pragma unroll
-  for (int e = 0; e < NC; ++e)
-    if (e * 32 < left) dst[e * 32] = sizeof(T) == 8 ? v[e] * scale : v[e] / sum;
+    for (int e = 0; e < NC; ++e)
+      if (e * 32 < left) dst[e * 32] = v[e] * scale;
+  } else {   // (a NaN sum: the method's NaN is the division's)
+    const DivideBy by(sum);
+#pragma unroll
+    for (int e = 0; e < NC; ++e)
+      if (e * 32 < left) dst[e * 32] = by(v[e]);
+  }
 }
 
 // out[r, j] = sum_s partial[s, r, j] + bias[j]   (no softmax)
