@@ -312,14 +312,14 @@ int layer_finish(sbb_layer *L, long h, cudaStream_t st) {
 }
 
 // Traces, weights and (bias.kbi != null) the bias of `N` input rows.  `L` (may be null) times the contraction; `vectors`
-// holds the reciprocals of Ci and Cj on the tensor path.
+// holds the reciprocals of Ci and Cj where the kernels take them.
 template <typename T>
 int train_rows(sbb_layer *L, const T *x, const T *y, long B, long N, long M, long H, T *Ci, T *Cj, T *Cij, T *W,
                const uint8_t *wmask, const sbb::TraceParams<T> &p, const sbb::BiasParams<T> &bias, Scratch &vectors,
                cudaStream_t st) {
   const bool tc = N > 0 && tensor_path<T>(x, y, N, M);
   T *rci = nullptr, *rcj = nullptr;
-  if (tc) {
+  if (tc || std::is_same<T, double>::value) {
     SBB_TRY(vectors.reserve((size_t)((N + 3) / 4 * 4 + M) * sizeof(T)));
     rci = static_cast<T *>(vectors.d);
     rcj = rci + (N + 3) / 4 * 4;
@@ -331,7 +331,7 @@ int train_rows(sbb_layer *L, const T *x, const T *y, long B, long N, long M, lon
     if constexpr (std::is_same<T, float>::value)
       SBB_CUDA(sbb::launch_trace_update_tc(x, y, B, N, M, wmask ? H : 0, rci, rcj, Cij, W, wmask, p, st));
   } else {
-    SBB_CUDA(sbb::launch_trace_update_fused<T>(x, y, B, N, M, H, M / H, Ci, Cj, Cij, W, wmask, p, 0, N, st));
+    SBB_CUDA(sbb::launch_trace_update_fused<T>(x, y, B, N, M, H, M / H, Ci, Cj, rci, rcj, Cij, W, wmask, p, 0, N, st));
   }
   timer.stop();
   return SBB_OK;

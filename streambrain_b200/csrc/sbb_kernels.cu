@@ -360,6 +360,7 @@ struct TraceEpilogue {
   long M, H, Mc;
   TraceParams<T> p;
   bool vec;
+  const T *rci, *rcj;    // reciprocals of Ci and Cj (float64 tensor-core kernel)
   __device__ __forceinline__ void operator()(T (&acc)[8][8], long m0, long n0, int ty, int tx, int) const {
     T cj[8];
     int hc[8];
@@ -436,13 +437,15 @@ struct StorePairs {
   }
 };
 
-// The fused trace epilogue on accumulator pairs.  Its memory accesses are what it waits for, so they are
-// arranged in two phases: first every load the thread needs (its 16 pairs of the old trace, the mask bytes,
-// Ci and Cj; the trace block was requested into L2 before the main loop), folded into the accumulators as
-// they arrive; then the arithmetic and the stores.  With a load, a logarithm and two stores per pair in turn,
-// the sixteen dependent memory round trips per thread left the tensor pipe idle half of the time.
+// The fused trace epilogue on accumulator pairs.  Its memory accesses are what it waits for, so they are arranged in two
+// phases: first every load the thread needs (its 16 pairs of the old trace, the mask bytes, the reciprocals of Ci and Cj;
+// the trace block was requested into L2 before the main loop), folded into the accumulators as they arrive; then the
+// arithmetic and the stores.  With a load, a logarithm and two stores per pair in turn, the sixteen dependent memory round
+// trips per thread left the tensor pipe idle half of the time.  The second phase is one row of the thread's block at a time
+// from one copy of the code (the accumulators rotate): unrolled it was 32 logarithms long and ran from a cold instruction
+// cache.  1568 x 3000, batch 128: 96 us with that, a 64-bit division per column and a float64 division per row and column.
 struct TracePairs {
-  const double *Ci, *Cj;
+  const double *rci, *rcj;   // reciprocals of Ci and Cj, 0 below the threshold
   double *Cij, *W;
   const uint8_t *wmask;
   long row0, row_end, M, H, Mc;
@@ -460,31 +463,37 @@ struct TracePairs {
   }
   __device__ __forceinline__ void tile(double (&acc)[4][4][2], long m_first, long n_first, int) const {
     // ---- phase 1: loads
-    double rci[4];
+    double rj[4][2], ri[4];
     unsigned on = 0;   // bit 8*mi + 2*ni + e: the element keeps a weight (row, column and mask allow it)
-    double rcj[4][2];
-    int hc[4][2];
-    bool col_on[4][2];
+    unsigned col_on = 0, second = 0;   // bit 2*ni + e: column at or above the threshold; in the second hypercolumn
+    const unsigned mc = (unsigned)Mc, last = (unsigned)(M - 1);
+    const unsigned h0 = min((unsigned)n_first, last) / mc, next = (h0 + 1) * mc;
+    bool two = true;   // the thread's columns (25 apart at most) lie in two hypercolumns
 #pragma unroll
-    for (int ni = 0; ni < 4; ++ni)
+    for (int ni = 0; ni < 4; ++ni) {
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const long j = n_first + ni * 8 + e;
-        const bool in = j < M;
-        const double cj = in ? Cj[j] : 1.0;
-        col_on[ni][e] = in && !(cj < p.cthr);
-        rcj[ni][e] = col_on[ni][e] ? 1.0 / cj : 0.0;
-        hc[ni][e] = in ? (int)(j / Mc) : 0;
+        rj[ni][e] = j < M ? __ldg(rcj + j) : 0.0;
+        if ((unsigned)j >= next) second |= 1u << (2 * ni + e);
+        if (j < M && (unsigned)j >= next + mc) two = false;
       }
+    }
+    const unsigned h1 = h0 + 1 < (unsigned)H ? h0 + 1 : h0;
+    uint8_t m0[4], m1[4];
+#pragma unroll
+    for (int mi = 0; mi < 4; ++mi) {
+      const long i = row0 + m_first + mi * 8;
+      const bool in = i < row_end;
+      ri[mi] = in ? __ldg(rci + i) : 0.0;
+      m0[mi] = wmask == nullptr ? 1 : (in ? wmask[i * H + h0] : 0);
+      m1[mi] = wmask == nullptr ? 1 : (in ? wmask[i * H + h1] : 0);
+    }
     const double scale = inv_batch * p.taupdt;
 #pragma unroll
     for (int mi = 0; mi < 4; ++mi) {
       const long i = row0 + m_first + mi * 8;
       const bool row_in = i < row_end;
-      const double ci = row_in ? Ci[i] : 1.0;
-      const bool row_on = row_in && !(ci < p.cthr);
-      rci[mi] = row_on ? 1.0 / ci : 0.0;
-      const uint8_t *mrow = wmask ? wmask + i * H : nullptr;
       double2 old[4];
 #pragma unroll
       for (int ni = 0; ni < 4; ++ni) {
@@ -495,9 +504,6 @@ struct TracePairs {
           if (vec) old[ni] = *reinterpret_cast<const double2 *>(cp);
           else old[ni] = make_double2(cp[0], n + 1 < M ? cp[1] : 0.0);
         }
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-          if (row_on && col_on[ni][e] && (mrow == nullptr || mrow[hc[ni][e]] != 0)) on |= 1u << (8 * mi + 2 * ni + e);
       }
       // the moving average, with the batch mean and the averaging weight folded into one factor (the reciprocal
       // of the batch size is exact for powers of two, one rounding more otherwise); a NaN clamps to zero
@@ -509,31 +515,65 @@ struct TracePairs {
         acc[mi][ni][1] = a1 > 0.0 ? a1 : 0.0;
       }
     }
-    // ---- phase 2: weights and stores.  Cij / (Ci * Cj) by the reciprocals taken above: three roundings more
-    // than the division, a few 1e-16 on the weight.
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (rj[ni][e] != 0.0) col_on |= 1u << (2 * ni + e);
 #pragma unroll
     for (int mi = 0; mi < 4; ++mi) {
-      const long i = row0 + m_first + mi * 8;
-      if (i >= row_end) continue;
+      unsigned row = (m0[mi] != 0 ? ~second : 0u) | (m1[mi] != 0 ? second : 0u);
+      if (!two) {   // hypercolumns narrower than the thread's columns: every byte
+        row = 0;
+        const long i = row0 + m_first + mi * 8;
+        if (i < row_end) {
 #pragma unroll
-      for (int ni = 0; ni < 4; ++ni) {
-        const long n = n_first + ni * 8;
-        if (n >= M) continue;
-        const double n0 = acc[mi][ni][0], n1 = acc[mi][ni][1];
-        double w0 = 0.0, w1 = 0.0;
-        if (on & (1u << (8 * mi + 2 * ni))) w0 = f64mma::log_positive((n0 < p.cthr4 ? p.cthr4 : n0) * (rci[mi] * rcj[ni][0]));
-        if (on & (2u << (8 * mi + 2 * ni))) w1 = f64mma::log_positive((n1 < p.cthr4 ? p.cthr4 : n1) * (rci[mi] * rcj[ni][1]));
-        double *cp = Cij + i * M + n, *wp = W + i * M + n;
-        if (vec) {
-          *reinterpret_cast<double2 *>(cp) = make_double2(n0, n1);
-          *reinterpret_cast<double2 *>(wp) = make_double2(w0, w1);
-        } else {
-          cp[0] = n0;
-          wp[0] = w0;
-          if (n + 1 < M) {
-            cp[1] = n1;
-            wp[1] = w1;
+          for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const unsigned j = (unsigned)(n_first + ni * 8 + e);
+              if (j <= last && (wmask == nullptr || wmask[i * H + j / mc] != 0)) row |= 1u << (2 * ni + e);
+            }
+        }
+      }
+      if (ri[mi] != 0.0) on |= (row & col_on & 0xFFu) << (8 * mi);
+    }
+    // ---- phase 2: weights and stores, a row of the block at a time.  Cij / (Ci * Cj) by the reciprocals: three roundings
+    // more than the division, a few 1e-16 on the weight.
+#pragma unroll 1
+    for (int mi = 0; mi < 4; ++mi) {
+      const long i = row0 + m_first + mi * 8;
+      if (i < row_end) {
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) {
+          const long n = n_first + ni * 8;
+          if (n >= M) continue;
+          const double n0 = acc[0][ni][0], n1 = acc[0][ni][1];
+          double w0 = 0.0, w1 = 0.0;
+          if (on & (1u << (2 * ni))) w0 = f64mma::log_positive((n0 < p.cthr4 ? p.cthr4 : n0) * (ri[0] * rj[ni][0]));
+          if (on & (2u << (2 * ni))) w1 = f64mma::log_positive((n1 < p.cthr4 ? p.cthr4 : n1) * (ri[0] * rj[ni][1]));
+          double *cp = Cij + i * M + n, *wp = W + i * M + n;
+          if (vec) {
+            *reinterpret_cast<double2 *>(cp) = make_double2(n0, n1);
+            *reinterpret_cast<double2 *>(wp) = make_double2(w0, w1);
+          } else {
+            cp[0] = n0;
+            wp[0] = w0;
+            if (n + 1 < M) {
+              cp[1] = n1;
+              wp[1] = w1;
+            }
           }
+        }
+      }
+      on >>= 8;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        ri[q] = ri[q + 1];
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) {
+          acc[q][ni][0] = acc[q + 1][ni][0];
+          acc[q][ni][1] = acc[q + 1][ni][1];
         }
       }
     }
@@ -543,8 +583,8 @@ struct TracePairs {
 static StorePairs to_pairs(const StoreEpilogue<double> &e) { return StorePairs{e.out, e.rows, e.cols, e.ld, e.zstride, e.vec}; }
 static TracePairs to_pairs(const TraceEpilogue<double> &e) {
   TracePairs t{};
-  t.Ci = e.Ci;
-  t.Cj = e.Cj;
+  t.rci = e.rci;
+  t.rcj = e.rcj;
   t.Cij = e.Cij;
   t.W = e.W;
   t.wmask = e.wmask;
@@ -1035,22 +1075,23 @@ template cudaError_t launch_vector_ema<double>(double *, const double *, long, T
 // ----------------------------------------------------------------------------
 template <typename T>
 cudaError_t launch_trace_update_fused(const T *x, const T *y, long B, long N, long M, long H, long Mc, const T *Ci,
-                                      const T *Cj, T *Cij, T *w, const uint8_t *wmask, TraceParams<T> p,
-                                      long row_begin, long row_end, cudaStream_t st) {
+                                      const T *Cj, const T *rci, const T *rcj, T *Cij, T *w, const uint8_t *wmask,
+                                      TraceParams<T> p, long row_begin, long row_end, cudaStream_t st) {
   constexpr int V = Vec16<T>::N;
   if (row_end <= row_begin) return cudaSuccess;
   const bool vec = (N % V == 0) && (M % V == 0) && (row_begin % V == 0) && ((row_end - row_begin) % V == 0) &&
                    aligned16(x) && aligned16(y);
   TraceEpilogue<T> ep{Ci, Cj, Cij, w, wmask, row_begin, row_end, M, H, Mc, p,
-                      (M % V == 0) && aligned16(Cij) && aligned16(w)};
+                      (M % V == 0) && aligned16(Cij) && aligned16(w), rci, rcj};
   const int kper = (int)((B + Tile<T>::BK - 1) / Tile<T>::BK) * Tile<T>::BK;
   return launch_contraction<T, false>(x + row_begin, N, y, M, row_end - row_begin, M, (int)B, 1, kper, vec, true, ep, st);
 }
 template cudaError_t launch_trace_update_fused<float>(const float *, const float *, long, long, long, long, long,
-                                                      const float *, const float *, float *, float *,
+                                                      const float *, const float *, const float *, const float *, float *, float *,
                                                       const uint8_t *, TraceParams<float>, long, long, cudaStream_t);
 template cudaError_t launch_trace_update_fused<double>(const double *, const double *, long, long, long, long, long,
-                                                       const double *, const double *, double *, double *,
+                                                       const double *, const double *, const double *, const double *, double *,
+                                                       double *,
                                                        const uint8_t *, TraceParams<double>, long, long,
                                                        cudaStream_t);
 

@@ -85,11 +85,12 @@ cudaError_t launch_few_forward(const T *x, const T *W, const T *bias, T *out, lo
 
 // Fused trace step for rows [row_begin,row_end) of Cij: acc = x^T y over the batch,
 // Cij = EMA(Cij, acc), w = log-ratio(Cij, Ci, Cj) with rows/columns below cthr and
-// masked connections (wmask may be null) set to zero.  Ci, Cj hold the NEW values.
+// masked connections (wmask may be null) set to zero.  Ci, Cj hold the NEW values; rci, rcj (float64 only) their
+// reciprocals, 0 below the threshold.
 template <typename T>
 cudaError_t launch_trace_update_fused(const T *x, const T *y, long B, long N, long M, long H, long Mc, const T *Ci,
-                                      const T *Cj, T *Cij, T *w, const uint8_t *wmask, TraceParams<T> p,
-                                      long row_begin, long row_end, cudaStream_t st);
+                                      const T *Cj, const T *rci, const T *rcj, T *Cij, T *w, const uint8_t *wmask,
+                                      TraceParams<T> p, long row_begin, long row_end, cudaStream_t st);
 
 // delta[i, j] = sum_b x[b, i] y[b, j] for rows [row_begin,row_end)  (delta is [N, M])
 template <typename T>
