@@ -320,6 +320,110 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1)
   ep(acc, m0, n0, ty, tx, (int)blockIdx.z);
 }
 
+// The same contraction for float32 outputs of few 128 x 128 tiles: a 32 x 64 tile per CTA of four warps, each 8 rows x 64
+// columns (a lane owns columns lane and lane + 32, so every global access of a warp is 32 neighbouring elements whatever the
+// row length, and its reads of A are broadcasts).  Such launches are bound by latency and by the SMs they leave idle, not by
+// arithmetic: the slabs arrive by 4-byte cp.async (any alignment) with three of four stages in flight, and what the epilogue
+// reads is requested before the main loop.  Each output is the same chain of FMAs over ascending k as in the kernel above.
+struct SmallTile {
+  static constexpr int BM = 32, BN = 64, BK = 32, STAGES = 4, THREADS = 128;
+  static constexpr int LDA = 32 + 4;   // K-major A as [m][k], MN-major as [k][m]: 16-byte rows
+  static constexpr int A_STAGE = 32 * LDA, B_STAGE = BK * BN;
+  static constexpr size_t SMEM_BYTES = (size_t)STAGES * (A_STAGE + B_STAGE) * sizeof(float);
+};
+__device__ __forceinline__ void cp_async4(float *dst, const float *src, bool valid) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(valid ? 4 : 0) : "memory");
+}
+
+template <bool A_KMAJOR>
+__device__ __forceinline__ void load_small_slab(float *As, float *Bs, const float *__restrict__ A, long lda,
+                                                const float *__restrict__ Bm, long ldb, long m0, long Mdim, long n0,
+                                                long Ndim, int k0, int kend) {
+  const int w8 = (threadIdx.x >> 5) * 8, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {
+    const long m = m0 + (A_KMAJOR ? w8 + t : lane);
+    const int k = k0 + (A_KMAJOR ? lane : w8 + t);
+    const bool ok = m < Mdim && k < kend;
+    cp_async4(As + (w8 + t) * SmallTile::LDA + lane, ok ? A + (A_KMAJOR ? m * lda + k : (long)k * lda + m) : A, ok);
+  }
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {
+    const int k = k0 + w8 + t;
+    const float *row = Bm + (long)k * ldb + n0 + lane;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const bool ok = k < kend && n0 + lane + 32 * c < Ndim;
+      cp_async4(Bs + (w8 + t) * SmallTile::BN + lane + 32 * c, ok ? row + 32 * c : Bm, ok);
+    }
+  }
+}
+
+// grid.x = column tiles, grid.y = row tiles, grid.z = k-splits
+template <bool A_KMAJOR, class Epilogue>
+__global__ void __launch_bounds__(SmallTile::THREADS)
+    small_contraction_kernel(const float *__restrict__ A, long lda, const float *__restrict__ Bm, long ldb, long Mdim,
+                             long Ndim, int K, int kper, Epilogue ep) {
+  using S = SmallTile;
+  extern __shared__ __align__(16) float small_smem[];
+  float *As = small_smem, *Bs = small_smem + S::STAGES * S::A_STAGE;
+  const int w8 = (threadIdx.x >> 5) * 8, lane = threadIdx.x & 31;
+  const long m0 = (long)blockIdx.y * S::BM, n0 = (long)blockIdx.x * S::BN;
+  const int kbeg = blockIdx.z * kper;
+  const int kend = min(K, kbeg + kper);
+  const int nk = kend > kbeg ? (kend - kbeg + S::BK - 1) / S::BK : 0;
+#pragma unroll
+  for (int s = 0; s < S::STAGES - 1; ++s) {
+    if (s < nk)
+      load_small_slab<A_KMAJOR>(As + s * S::A_STAGE, Bs + s * S::B_STAGE, A, lda, Bm, ldb, m0, Mdim, n0, Ndim,
+                                kbeg + s * S::BK, kend);
+    f64mma::cp_async_commit();
+  }
+  typename Epilogue::Strip strip(ep, m0 + w8, n0 + lane, lane);
+  float acc[8][2];
+#pragma unroll
+  for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = 0.f;
+  for (int kt = 0; kt < nk; ++kt) {
+    f64mma::cp_async_wait<S::STAGES - 2>();   // slab kt has landed
+    __syncthreads();                          // ... for every thread, and the stage refilled below is free
+    const int nx = kt + S::STAGES - 1;
+    if (nx < nk)
+      load_small_slab<A_KMAJOR>(As + nx % S::STAGES * S::A_STAGE, Bs + nx % S::STAGES * S::B_STAGE, A, lda, Bm, ldb, m0,
+                                Mdim, n0, Ndim, kbeg + nx * S::BK, kend);
+    f64mma::cp_async_commit();
+    const float *as = As + kt % S::STAGES * S::A_STAGE, *bs = Bs + kt % S::STAGES * S::B_STAGE + lane;
+#pragma unroll
+    for (int k4 = 0; k4 < S::BK; k4 += 4) {
+      float a[8][4];   // [row][k]
+      if constexpr (A_KMAJOR) {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) lds4(as + (w8 + r) * S::LDA + k4, a[r]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          float v[8];
+          lds4(as + (k4 + k) * S::LDA + w8, v);
+          lds4(as + (k4 + k) * S::LDA + w8 + 4, v + 4);
+#pragma unroll
+          for (int r = 0; r < 8; ++r) a[r][k] = v[r];
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float b0 = bs[(k4 + k) * S::BN], b1 = bs[(k4 + k) * S::BN + 32];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          acc[r][0] = fmaf(a[r][k], b0, acc[r][0]);
+          acc[r][1] = fmaf(a[r][k], b1, acc[r][1]);
+        }
+      }
+    }
+  }
+  f64mma::cp_async_wait<0>();
+  strip.finish(ep, acc, m0 + w8, n0 + lane, (int)blockIdx.z);
+}
+
 // Epilogue: partial[z, m, n] = acc  (forward product) or delta[m, n] = acc.
 template <typename T>
 struct StoreEpilogue {
@@ -344,6 +448,18 @@ struct StoreEpilogue {
       }
     }
   }
+  // Rows m .. m + 7, columns n and n + 32 of the small-tile kernel.
+  struct Strip {
+    __device__ __forceinline__ Strip(const StoreEpilogue &, long, long, int) {}
+    __device__ __forceinline__ void finish(const StoreEpilogue &e, T (&acc)[8][2], long m, long n, int z) const {
+      T *p = e.out + (long)z * e.zstride + m * e.ld + n;
+#pragma unroll
+      for (int r = 0; r < 8; ++r, p += e.ld) {
+        if (m + r < e.rows && n < e.cols) p[0] = acc[r][0];
+        if (m + r < e.rows && n + 32 < e.cols) p[32] = acc[r][1];
+      }
+    }
+  };
 };
 
 // Epilogue of the fused trace step: moving average of Cij, log-ratio weight,
@@ -405,6 +521,57 @@ struct TraceEpilogue {
       }
     }
   }
+  // Rows m .. m + 7, columns n and n + 32 of the small-tile kernel: everything the epilogue reads is requested before the
+  // main loop, and its arithmetic (the same as above) is one row at a time from one copy of the code, the rows rotating
+  // through slot 0: unrolled, sixteen logarithms and divisions come from a cold instruction cache.
+  struct Strip {
+    T old[8][2], ci, cj[2];   // ci: lane r holds row r's
+    unsigned on = 0;          // bit 2 * r + c: the mask keeps the element's weight
+    __device__ __forceinline__ Strip(const TraceEpilogue &e, long m, long n, int lane) {
+      const long i0 = e.row0 + m, i = i0 + (lane & 7);
+      ci = i < e.row_end ? e.Ci[i] : (T)0;
+      const T *src = e.Cij + i0 * e.M + n;
+      const uint8_t *mrow[2];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const long j = n + 32 * c < e.M ? n + 32 * c : 0;
+        cj[c] = e.Cj[j];
+        mrow[c] = e.wmask ? e.wmask + i0 * e.H + (unsigned)j / (unsigned)e.Mc : nullptr;
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r, src += e.M)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const bool in = i0 + r < e.row_end && n + 32 * c < e.M;
+          old[r][c] = in ? src[32 * c] : (T)0;
+          if (in && (mrow[c] == nullptr || mrow[c][r * e.H] != 0)) on |= 1u << (2 * r + c);
+        }
+    }
+    __device__ __forceinline__ void finish(const TraceEpilogue &e, T (&acc)[8][2], long m, long n, int) {
+      const long i0 = e.row0 + m;
+      const int rows = (int)min(8L, e.row_end - i0);
+      T *pc = e.Cij + i0 * e.M + n, *pw = e.W + i0 * e.M + n;
+#pragma unroll 1
+      for (int r = 0; r < rows; ++r, pc += e.M, pw += e.M) {
+        const T row = __shfl_sync(0xffffffffu, ci, r);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          if (n + 32 * c < e.M) {
+            const T cij = trace_ema(old[0][c], acc[0][c], e.p);
+            T w = (T)0;
+            if (!(row < e.p.cthr) && !(cj[c] < e.p.cthr) && (on >> (2 * r + c) & 1u)) w = log_ratio(cij, row, cj[c], e.p.cthr4);
+            pc[32 * c] = cij;
+            pw[32 * c] = w;
+          }
+#pragma unroll
+          for (int k = 0; k < 7; ++k) {
+            acc[k][c] = acc[k + 1][c];
+            old[k][c] = old[k + 1][c];
+          }
+        }
+      }
+    }
+  };
 };
 
 // ----------------------------------------------------------------------------
@@ -653,6 +820,30 @@ static cudaError_t launch_f64_mma(const double *A, long lda, const double *Bm, l
   return launch_f64_mma_tiles<A_KMAJOR, 128>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, ep, st);
 }
 
+static bool small_tiles(long tiles) {
+  static const long limit = [] { const char *e = getenv("SBB_SMALL_TILES"); return e ? atol(e) : 2 * 148; }();
+  return tiles < limit;
+}
+
+template <bool A_KMAJOR, class Ep>
+static cudaError_t launch_small_contraction(const float *A, long lda, const float *Bm, long ldb, long Mdim, long Ndim,
+                                            int K, int splits, int kper, Ep ep, cudaStream_t st) {
+  using S = SmallTile;
+  auto kernel = small_contraction_kernel<A_KMAJOR, Ep>;
+  static bool configured[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !configured[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM_BYTES);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) configured[dev] = true;
+  }
+  const dim3 grid((unsigned)((Ndim + S::BN - 1) / S::BN), (unsigned)((Mdim + S::BM - 1) / S::BM), (unsigned)splits);
+  if (grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
+  kernel<<<grid, S::THREADS, S::SMEM_BYTES, st>>>(A, lda, Bm, ldb, Mdim, Ndim, K, kper, ep);
+  return launched();
+}
+
 template <typename T, bool A_KMAJOR, class Ep>
 static cudaError_t launch_contraction(const T *A, long lda, const T *Bm, long ldb, long Mdim, long Ndim, int K,
                                       int splits, int kper, bool vec, bool cols_fastest, Ep ep, cudaStream_t st) {
@@ -662,6 +853,10 @@ static cudaError_t launch_contraction(const T *A, long lda, const T *Bm, long ld
     // `vec`: every operand row starts on a 16-byte boundary and holds an even number of elements
     if (vec && lda % 2 == 0 && ldb % 2 == 0 && f64_mma_enabled())
       return launch_f64_mma<A_KMAJOR>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, to_pairs(ep), st);
+  }
+  if constexpr (std::is_same<T, float>::value) {
+    if (small_tiles((long)mt * nt * splits))
+      return launch_small_contraction<A_KMAJOR>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, ep, st);
   }
   if (cols_fastest && mt > 65535u) cols_fastest = false;
   dim3 grid(cols_fastest ? nt : mt, cols_fastest ? mt : nt, (unsigned)splits);
