@@ -1,12 +1,13 @@
-// float64 contraction on the FP64 tensor-core instruction (mma.sync.m8n8k4.f64), for shapes whose
-// rows start on 16-byte boundaries.  tcgen05 has no float64 kind; mma.sync peaks no higher than DFMA
+// float64 contraction on the FP64 tensor-core instruction (mma.sync.m8n8k4.f64).  tcgen05 has no float64 kind; mma.sync peaks no higher than DFMA
 // on this part, but one instruction carries 256 FMAs, so the issue slots, the shared-memory pipe and
 // the register file (32 accumulators per thread instead of 64) are left with room to hide latencies:
 // two CTAs of eight warps per SM instead of one.
 //
 // CTA tile 128 x 64 (eight warps, two CTAs per SM) or 64 x 64 (four warps, three CTAs per SM: for
 // launches whose 128-row tiles would leave most of a last wave of CTAs empty), k-slabs of 16 in a
-// three-stage cp.async pipeline, warp tile 32 x 32 (4 x 4 instruction tiles).  Shared-memory rows
+// three-stage cp.async pipeline, warp tile 32 x 32 (4 x 4 instruction tiles).  A launch of no more
+// 128-row tiles than SMs has one CTA per SM and takes six stages instead.  The copies are 16 bytes
+// wide where rows start on 16-byte boundaries and one element otherwise.  Shared-memory rows
 // are padded so that a half-warp's fragment loads (four rows of four consecutive doubles) fall into
 // 16 different bank pairs.
 #pragma once
@@ -16,15 +17,16 @@
 namespace sbb {
 namespace f64mma {
 
-constexpr int BN = 64, BK = 16, STAGES = 3;
+constexpr int BN = 64, BK = 16;
 constexpr int LDA_K = BK + 4;   // K-major A in shared memory: [m][k]
 constexpr int LDB = BN + 4;     // B: [k][n]
 constexpr int B_STAGE = BK * LDB;
-template <int BM>
+template <int BM, bool DEEP = false>
 struct Cfg {
   static_assert(BM == 128 || BM == 64, "row tiles of 128 or 64");
   static constexpr int THREADS = BM * 2;        // (BM / 32) x 2 warps
-  static constexpr int CTAS_PER_SM = BM == 128 ? 2 : 3;
+  static constexpr int CTAS_PER_SM = DEEP ? 1 : BM == 128 ? 2 : 3;
+  static constexpr int STAGES = DEEP ? 6 : 3;
   static constexpr int LDA_M = BM + 4;          // MN-major A: [k][m]
   static constexpr int A_STAGE = BM * LDA_K > BK * LDA_M ? BM * LDA_K : BK * LDA_M;   // doubles
   static constexpr size_t SMEM_BYTES = (size_t)STAGES * (A_STAGE + B_STAGE) * sizeof(double);
@@ -34,6 +36,16 @@ __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc, boo
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
   const int bytes = valid ? 16 : 0;   // 0: nothing is read, the destination is filled with zeros
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(gsrc), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async8(void *smem_dst, const void *gsrc, bool valid) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
+  const int bytes = valid ? 8 : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(gsrc), "r"(bytes) : "memory");
+}
+template <int V>
+__device__ __forceinline__ void cp_async(void *smem_dst, const void *gsrc, bool valid) {
+  if constexpr (V == 2) cp_async16(smem_dst, gsrc, valid);
+  else cp_async8(smem_dst, gsrc, valid);
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -139,10 +151,10 @@ __device__ __forceinline__ double log_positive(double x) {
   return fma((double)e, 0.693147180559945309417232, t.y + q);
 }
 
-// One k-slab of both operands into stage buffers As / Bs (zero-filled outside the operands).
+// One k-slab of both operands into stage buffers As / Bs (zero-filled outside the operands), V elements per copy.
 // A is [K x Mdim] MN-major (element (k, m) at A[k*lda + m]) or, A_KMAJOR, [Mdim x K] (at A[m*lda + k]);
-// B is [K x Ndim] MN-major.  All row starts and the 2-element chunks are 16-byte aligned (checked by the host).
-template <bool A_KMAJOR, int BM>
+// B is [K x Ndim] MN-major.  V = 2: all row starts and the 2-element chunks are 16-byte aligned (checked by the host).
+template <bool A_KMAJOR, int BM, int V>
 __device__ __forceinline__ void load_slab(double *As, double *Bs, const double *__restrict__ A, long lda,
                                           const double *__restrict__ Bm, long ldb, long m0, long Mdim, long n0,
                                           long Ndim, int k0, int kend) {
@@ -150,33 +162,33 @@ __device__ __forceinline__ void load_slab(double *As, double *Bs, const double *
   const int tid = threadIdx.x;
   if constexpr (A_KMAJOR) {
 #pragma unroll
-    for (int t = 0; t < BM * (BK / 2) / THREADS; ++t) {
+    for (int t = 0; t < BM * (BK / V) / THREADS; ++t) {
       const int v = tid + t * THREADS;
-      const int r = v / (BK / 2), c = (v % (BK / 2)) * 2;
+      const int r = v / (BK / V), c = (v % (BK / V)) * V;
       const long m = m0 + r;
       const int k = k0 + c;
       const bool ok = m < Mdim && k < kend;
-      cp_async16(As + r * LDA_K + c, ok ? A + m * lda + k : A, ok);
+      cp_async<V>(As + r * LDA_K + c, ok ? A + m * lda + k : A, ok);
     }
   } else {
 #pragma unroll
-    for (int t = 0; t < BK * (BM / 2) / THREADS; ++t) {
+    for (int t = 0; t < BK * (BM / V) / THREADS; ++t) {
       const int v = tid + t * THREADS;
-      const int r = v / (BM / 2), c = (v % (BM / 2)) * 2;
+      const int r = v / (BM / V), c = (v % (BM / V)) * V;
       const int k = k0 + r;
       const long m = m0 + c;
       const bool ok = k < kend && m < Mdim;
-      cp_async16(As + r * LDA_M + c, ok ? A + (long)k * lda + m : A, ok);
+      cp_async<V>(As + r * LDA_M + c, ok ? A + (long)k * lda + m : A, ok);
     }
   }
 #pragma unroll
-  for (int t = 0; t < BK * (BN / 2) / THREADS; ++t) {
+  for (int t = 0; t < BK * (BN / V) / THREADS; ++t) {
     const int v = tid + t * THREADS;
-    const int r = v / (BN / 2), c = (v % (BN / 2)) * 2;
+    const int r = v / (BN / V), c = (v % (BN / V)) * V;
     const int k = k0 + r;
     const long n = n0 + c;
     const bool ok = k < kend && n < Ndim;
-    cp_async16(Bs + r * LDB + c, ok ? Bm + (long)k * ldb + n : Bm, ok);
+    cp_async<V>(Bs + r * LDB + c, ok ? Bm + (long)k * ldb + n : Bm, ok);
   }
 }
 
@@ -184,11 +196,11 @@ __device__ __forceinline__ void load_slab(double *As, double *Bs, const double *
 // k-split z covers [z*kper, min(K, (z+1)*kper)), kper a multiple of BK.  The epilogue receives the thread's
 // accumulators: ep.tile(acc, m, n, z) with acc[mi][ni][e] = output element (m + 8*mi, n + 8*ni + e), n even;
 // ep.prefetch(m, n, lane) is called before the main loop with the first element of the warp's 32 x 32 block.
-template <bool A_KMAJOR, int BM, class Epilogue>
-__global__ void __launch_bounds__(Cfg<BM>::THREADS, Cfg<BM>::CTAS_PER_SM)
+template <bool A_KMAJOR, int BM, bool DEEP, int V, class Epilogue>
+__global__ void __launch_bounds__(Cfg<BM>::THREADS, Cfg<BM, DEEP>::CTAS_PER_SM)
     contraction_kernel(const double *__restrict__ A, long lda, const double *__restrict__ Bm, long ldb, long Mdim,
                        long Ndim, int K, int kper, bool cols_fastest, Epilogue ep) {
-  constexpr int A_STAGE = Cfg<BM>::A_STAGE, LDA_M = Cfg<BM>::LDA_M;
+  constexpr int A_STAGE = Cfg<BM>::A_STAGE, LDA_M = Cfg<BM>::LDA_M, STAGES = Cfg<BM, DEEP>::STAGES;
   extern __shared__ __align__(16) double smem[];
   double *As = smem, *Bs = smem + STAGES * A_STAGE;
   const long m0 = (long)(cols_fastest ? blockIdx.y : blockIdx.x) * BM;
@@ -209,7 +221,7 @@ __global__ void __launch_bounds__(Cfg<BM>::THREADS, Cfg<BM>::CTAS_PER_SM)
   ep.prefetch(m0 + wm, n0 + wn, lane);
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
-    if (s < nk) load_slab<A_KMAJOR, BM>(As + s * A_STAGE, Bs + s * B_STAGE, A, lda, Bm, ldb, m0, Mdim, n0, Ndim, kbeg + s * BK, kend);
+    if (s < nk) load_slab<A_KMAJOR, BM, V>(As + s * A_STAGE, Bs + s * B_STAGE, A, lda, Bm, ldb, m0, Mdim, n0, Ndim, kbeg + s * BK, kend);
     cp_async_commit();
   }
   for (int kt = 0; kt < nk; ++kt) {
@@ -219,7 +231,7 @@ __global__ void __launch_bounds__(Cfg<BM>::THREADS, Cfg<BM>::CTAS_PER_SM)
       const int nx = kt + STAGES - 1;
       if (nx < nk) {
         const int s = nx % STAGES;
-        load_slab<A_KMAJOR, BM>(As + s * A_STAGE, Bs + s * B_STAGE, A, lda, Bm, ldb, m0, Mdim, n0, Ndim, kbeg + nx * BK, kend);
+        load_slab<A_KMAJOR, BM, V>(As + s * A_STAGE, Bs + s * B_STAGE, A, lda, Bm, ldb, m0, Mdim, n0, Ndim, kbeg + nx * BK, kend);
       }
       cp_async_commit();
     }

@@ -765,33 +765,22 @@ static TracePairs to_pairs(const TraceEpilogue<double> &e) {
   t.vec = e.vec;
   return t;
 }
-template <typename T>
-static int to_pairs(const T &) { return 0; }   // float32 epilogues never take this path
-
-// SBB_F64_CONTRACTION=dfma keeps float64 on the DFMA tile kernel (read once).
-static bool f64_mma_enabled() {
-  static const bool on = [] {
-    const char *e = getenv("SBB_F64_CONTRACTION");
-    return !(e != nullptr && strcmp(e, "dfma") == 0);
-  }();
-  return on;
-}
 
 static int sm_count();
 
-template <bool A_KMAJOR, int BM, class Pairs>
+template <bool A_KMAJOR, int BM, bool DEEP, int V, class Pairs>
 static cudaError_t launch_f64_mma_tiles(const double *A, long lda, const double *Bm, long ldb, long Mdim, long Ndim,
                                         int K, int splits, bool cols_fastest, Pairs ep, cudaStream_t st) {
   namespace F = f64mma;
-  using C = F::Cfg<BM>;
-  auto kernel = F::contraction_kernel<A_KMAJOR, BM, Pairs>;
+  using C = F::Cfg<BM, DEEP>;
+  auto kernel = F::contraction_kernel<A_KMAJOR, BM, DEEP, V, Pairs>;
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && !configured[dev]) {
+  if (dev < 0 || dev >= 64 || !configured[dev]) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_BYTES);
     if (e != cudaSuccess) return e;
-    configured[dev] = true;
+    if (dev >= 0 && dev < 64) configured[dev] = true;
   }
   const unsigned mt = (unsigned)((Mdim + BM - 1) / BM), nt = (unsigned)((Ndim + F::BN - 1) / F::BN);
   if (cols_fastest && mt > 65535u) cols_fastest = false;
@@ -803,26 +792,31 @@ static cudaError_t launch_f64_mma_tiles(const double *A, long lda, const double 
   return launched();
 }
 
-// Row tiles of 128 unless 64 finishes in fewer waves of resident CTAs: time ~ waves x (rows of a tile) x (CTAs
-// that share an SM).  1568 x 3000 outputs: 611 tiles of 128 rows are two full waves of 296 CTAs and a third with
-// 19, 1175 tiles of 64 rows three waves of 444 half-sized CTAs.
-template <bool A_KMAJOR, class Pairs>
+// Row tiles of 128 unless the fullest SM has fewer rows to do in tiles of 64: 1568 x 3000 outputs are 611 tiles of 128
+// rows, five on some SMs, or 1175 tiles of 64 rows, at most eight.  The forward product's 128-row tiles on as many SMs
+// take the deep pipeline (the trace step's few-tile launches have one short chain of slabs, which it does not help).
+template <bool A_KMAJOR, int V, class Pairs>
 static cudaError_t launch_f64_mma(const double *A, long lda, const double *Bm, long ldb, long Mdim, long Ndim, int K,
                                   int splits, bool cols_fastest, Pairs ep, cudaStream_t st) {
   namespace F = f64mma;
   const long nt = (Ndim + F::BN - 1) / F::BN, sms = sm_count();
-  auto cost = [&](long bm, long ctas_per_sm) {
-    const long tiles = ((Mdim + bm - 1) / bm) * nt * splits, slots = sms * ctas_per_sm;
-    return ((tiles + slots - 1) / slots) * bm * ctas_per_sm;
-  };
-  if (cost(64, F::Cfg<64>::CTAS_PER_SM) < cost(128, F::Cfg<128>::CTAS_PER_SM))
-    return launch_f64_mma_tiles<A_KMAJOR, 64>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, ep, st);
-  return launch_f64_mma_tiles<A_KMAJOR, 128>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, ep, st);
+  auto ctas = [&](long bm) { return ((Mdim + bm - 1) / bm) * nt * splits; };
+  auto rows = [&](long bm) { return (ctas(bm) + sms - 1) / sms * bm; };
+  if (rows(64) < rows(128))
+    return launch_f64_mma_tiles<A_KMAJOR, 64, false, V>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, ep, st);
+  if constexpr (A_KMAJOR) {
+    if (ctas(128) <= sms)
+      return launch_f64_mma_tiles<A_KMAJOR, 128, true, V>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, ep, st);
+  }
+  return launch_f64_mma_tiles<A_KMAJOR, 128, false, V>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, ep, st);
 }
 
-static bool small_tiles(long tiles) {
-  static const long limit = [] { const char *e = getenv("SBB_SMALL_TILES"); return e ? atol(e) : 2 * 148; }();
-  return tiles < limit;
+// When the 32 x 64 tiles take over.  Forward products (no epilogue to speak of): below two thirds of an SM's worth of 128 x
+// 128 tiles; 28 tiles 21.6 -> 10.0 us, 92 tiles 22.0 -> 20.8, but 112 tiles 23.3 -> 27.7.  Trace steps, whose epilogue is a
+// logarithm and a division per output: below one wave of the large kernel's CTAs (two per SM); 32 tiles 40.5 -> 13.1 us,
+// 96 tiles 41.4 -> 28.9, 216 tiles 59.6 -> 57.0, but 800 tiles 144 -> 156.
+static bool small_tiles(long tiles, bool forward) {
+  return forward ? 3 * tiles < 2L * sm_count() : tiles < 2L * sm_count();
 }
 
 template <bool A_KMAJOR, class Ep>
@@ -851,13 +845,12 @@ static cudaError_t launch_contraction(const T *A, long lda, const T *Bm, long ld
   if (mt == 0 || nt == 0 || K <= 0) return cudaSuccess;
   if constexpr (std::is_same<T, double>::value) {
     // `vec`: every operand row starts on a 16-byte boundary and holds an even number of elements
-    if (vec && lda % 2 == 0 && ldb % 2 == 0 && f64_mma_enabled())
-      return launch_f64_mma<A_KMAJOR>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, to_pairs(ep), st);
-  }
-  if constexpr (std::is_same<T, float>::value) {
-    if (small_tiles((long)mt * nt * splits))
-      return launch_small_contraction<A_KMAJOR>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, ep, st);
-  }
+    if (vec && lda % 2 == 0 && ldb % 2 == 0)
+      return launch_f64_mma<A_KMAJOR, 2>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, to_pairs(ep), st);
+    return launch_f64_mma<A_KMAJOR, 1>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, to_pairs(ep), st);
+  } else {
+  if (small_tiles((long)mt * nt * splits, A_KMAJOR))
+    return launch_small_contraction<A_KMAJOR>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, ep, st);
   if (cols_fastest && mt > 65535u) cols_fastest = false;
   dim3 grid(cols_fastest ? nt : mt, cols_fastest ? mt : nt, (unsigned)splits);
   if (grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
@@ -867,6 +860,7 @@ static cudaError_t launch_contraction(const T *A, long lda, const T *Bm, long ld
   else
     contraction_kernel<T, A_KMAJOR, 1, Ep><<<grid, 256, 0, st>>>(A, lda, Bm, ldb, Mdim, Ndim, K, kper, cols_fastest, ep);
   return launched();
+  }
 }
 
 // ----------------------------------------------------------------------------
@@ -885,14 +879,29 @@ static int sm_count() {
   return g_sm_count;
 }
 
+// k-splits of the forward product.  float32: output tiles of 128 x 128 until two CTAs per SM are busy, at least eight slabs
+// each.  float64 (128 x 64 tiles, slabs of 16): the split whose fullest SM has the least to do, in slabs, counting each
+// partial sum's way to memory and back (16 bytes per output at about 4 TB/s against about 1.05 us per slab of a tile); 47
+// tiles of 98 slabs: three splits on 141 SMs, 33 slabs each, half of the partial sums that two CTAs per SM need for 34.
 template <typename T>
 int forward_splits(long B, long N, long M) {
-  // output tiles: 128 x 128 (float32 FFMA kernel), 128 x 64 (float64 tensor-core kernel)
-  const long tiles = ((B + 127) / 128) * (sizeof(T) == 8 ? (M + 63) / 64 : (M + 127) / 128);
-  const long want = 2L * sm_count();           // two resident CTAs per SM
+  const long sms = sm_count();
+  if (sizeof(T) == 8) {
+    const long tiles = ((B + 127) / 128) * ((M + f64mma::BN - 1) / f64mma::BN), slabs = (N + f64mma::BK - 1) / f64mma::BK;
+    const double per_split = (double)B * M / 262144.0;
+    int best = 1;
+    double least = 0;
+    for (long s = 1; s <= 16 && (s == 1 || slabs / s >= 4); ++s) {
+      const double cost = (double)((tiles * s + sms - 1) / sms) * ((slabs + s - 1) / s) + per_split * s;
+      if (s == 1 || cost < least) least = cost, best = (int)s;
+    }
+    return best;
+  }
+  const long tiles = ((B + 127) / 128) * ((M + 127) / 128);
+  const long want = 2 * sms;
   long s = tiles >= want ? 1 : want / (tiles > 0 ? tiles : 1);
   const long slabs = (N + Tile<T>::BK - 1) / Tile<T>::BK;
-  const long max_s = slabs / 8 > 0 ? slabs / 8 : 1;  // at least 8 slabs per split
+  const long max_s = slabs / 8 > 0 ? slabs / 8 : 1;
   if (s > max_s) s = max_s;
   if (s > 64) s = 64;
   if (s < 1) s = 1;
