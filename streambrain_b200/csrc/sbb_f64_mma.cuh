@@ -32,20 +32,14 @@ struct Cfg {
   static constexpr size_t SMEM_BYTES = (size_t)STAGES * (A_STAGE + B_STAGE) * sizeof(double);
 };
 
-__device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc, bool valid) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
-  const int bytes = valid ? 16 : 0;   // 0: nothing is read, the destination is filled with zeros
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(gsrc), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void *smem_dst, const void *gsrc, bool valid) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
-  const int bytes = valid ? 8 : 0;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(gsrc), "r"(bytes) : "memory");
-}
+// One copy of V doubles into shared memory; not valid: nothing is read, the destination is filled with zeros.
 template <int V>
-__device__ __forceinline__ void cp_async(void *smem_dst, const void *gsrc, bool valid) {
-  if constexpr (V == 2) cp_async16(smem_dst, gsrc, valid);
-  else cp_async8(smem_dst, gsrc, valid);
+__device__ __forceinline__ void cp_async(uint32_t dst, const double *src, bool valid) {
+  const int bytes = valid ? 8 * V : 0;
+  if constexpr (V == 2)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -151,46 +145,53 @@ __device__ __forceinline__ double log_positive(double x) {
   return fma((double)e, 0.693147180559945309417232, t.y + q);
 }
 
-// One k-slab of both operands into stage buffers As / Bs (zero-filled outside the operands), V elements per copy.
-// A is [K x Mdim] MN-major (element (k, m) at A[k*lda + m]) or, A_KMAJOR, [Mdim x K] (at A[m*lda + k]);
-// B is [K x Ndim] MN-major.  V = 2: all row starts and the 2-element chunks are 16-byte aligned (checked by the host).
+// A thread's share of the k-slabs of both operands: N copies of V elements per slab into the stage buffers, zero-filled
+// outside the operands.  A is [K x Mdim] MN-major (element (k, m) at A[k*lda + m]) or, A_KMAJOR, [Mdim x K] (at
+// A[m*lda + k]); B is [K x Ndim] MN-major.  V = 2: all row starts and the 2-element chunks are 16-byte aligned (checked by
+// the host).  A thread's copies of one operand lie RA (RB) rows of its memory layout apart in the same column, so one
+// pointer and one count of what is left per operand are all it keeps.
 template <bool A_KMAJOR, int BM, int V>
-__device__ __forceinline__ void load_slab(double *As, double *Bs, const double *__restrict__ A, long lda,
-                                          const double *__restrict__ Bm, long ldb, long m0, long Mdim, long n0,
-                                          long Ndim, int k0, int kend) {
-  constexpr int THREADS = Cfg<BM>::THREADS, LDA_M = Cfg<BM>::LDA_M;
-  const int tid = threadIdx.x;
-  if constexpr (A_KMAJOR) {
-#pragma unroll
-    for (int t = 0; t < BM * (BK / V) / THREADS; ++t) {
-      const int v = tid + t * THREADS;
-      const int r = v / (BK / V), c = (v % (BK / V)) * V;
-      const long m = m0 + r;
-      const int k = k0 + c;
-      const bool ok = m < Mdim && k < kend;
-      cp_async<V>(As + r * LDA_K + c, ok ? A + m * lda + k : A, ok);
-    }
-  } else {
-#pragma unroll
-    for (int t = 0; t < BK * (BM / V) / THREADS; ++t) {
-      const int v = tid + t * THREADS;
-      const int r = v / (BM / V), c = (v % (BM / V)) * V;
-      const int k = k0 + r;
-      const long m = m0 + c;
-      const bool ok = k < kend && m < Mdim;
-      cp_async<V>(As + r * LDA_M + c, ok ? A + (long)k * lda + m : A, ok);
+struct Slab {
+  static constexpr int THREADS = Cfg<BM>::THREADS;
+  static constexpr int CA = (A_KMAJOR ? BK : BM) / V, CB = BN / V;   // copies per row
+  static constexpr int RA = THREADS / CA, RB = THREADS / CB;         // rows per pass of the block
+  static constexpr int NA = BM * BK / V / THREADS, N = NA + BK * BN / V / THREADS;
+  static constexpr int LDA = A_KMAJOR ? LDA_K : Cfg<BM>::LDA_M;
+  const double *pa, *pb;     // the first copy of the next slab
+  long lda, ldb;
+  uint32_t da, db;           // its place in stage 0
+  int rows_a, left_a, left_b;   // rows of A at and below the first copy's (K-major); k left from the first copies on
+  __device__ __forceinline__ Slab(const double *A, long lda_, const double *Bm, long ldb_, long m0, long Mdim, long n0,
+                                  long Ndim, int kbeg, int kend, const double *As, const double *Bs)
+      : lda(lda_), ldb(ldb_) {
+    const int ra = threadIdx.x / CA, ca = threadIdx.x % CA * V, rb = threadIdx.x / CB, cb = threadIdx.x % CB * V;
+    const long m = m0 + (A_KMAJOR ? ra : ca);
+    pa = A + (A_KMAJOR ? m * lda + kbeg + ca : (long)(kbeg + ra) * lda + m);
+    pb = Bm + (long)(kbeg + rb) * ldb + n0 + cb;
+    rows_a = (int)min(Mdim - m, (long)BM);
+    left_a = kend - kbeg - (A_KMAJOR ? ca : ra);
+    if (!A_KMAJOR && m >= Mdim) left_a = 0;
+    left_b = n0 + cb < Ndim ? kend - kbeg - rb : 0;
+    da = (uint32_t)__cvta_generic_to_shared(As + ra * LDA + ca);
+    db = (uint32_t)__cvta_generic_to_shared(Bs + rb * LDB + cb);
+  }
+  // Copy t of the next slab, into the stage that starts at element a (b) of the buffers.
+  __device__ __forceinline__ void copy(int t, int a, int b, const double *A, const double *Bm) const {
+    if (t < NA) {
+      const bool ok = A_KMAJOR ? t * RA < rows_a && left_a > 0 : t * RA < left_a;
+      cp_async<V>(da + (uint32_t)(a + t * RA * LDA) * 8u, ok ? pa + t * RA * lda : A, ok);
+    } else if (t < N) {
+      const bool ok = (t - NA) * RB < left_b;
+      cp_async<V>(db + (uint32_t)(b + (t - NA) * RB * LDB) * 8u, ok ? pb + (t - NA) * RB * ldb : Bm, ok);
     }
   }
-#pragma unroll
-  for (int t = 0; t < BK * (BN / V) / THREADS; ++t) {
-    const int v = tid + t * THREADS;
-    const int r = v / (BN / V), c = (v % (BN / V)) * V;
-    const int k = k0 + r;
-    const long n = n0 + c;
-    const bool ok = k < kend && n < Ndim;
-    cp_async<V>(Bs + r * LDB + c, ok ? Bm + (long)k * ldb + n : Bm, ok);
+  __device__ __forceinline__ void advance() {
+    pa += A_KMAJOR ? (long)BK : BK * lda;
+    pb += BK * ldb;
+    left_a -= BK;
+    left_b -= BK;
   }
-}
+};
 
 // grid.x = row tiles of the output, grid.y = column tiles (swapped when cols_fastest), grid.z = k-splits.
 // k-split z covers [z*kper, min(K, (z+1)*kper)), kper a multiple of BK.  The epilogue receives the thread's
@@ -219,37 +220,58 @@ __global__ void __launch_bounds__(Cfg<BM>::THREADS, Cfg<BM, DEEP>::CTAS_PER_SM)
     for (int ni = 0; ni < 4; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
 
   ep.prefetch(m0 + wm, n0 + wn, lane);
+  using L = Slab<A_KMAJOR, BM, V>;
+  L slab(A, lda, Bm, ldb, m0, Mdim, n0, Ndim, kbeg, kend, As, Bs);
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
-    if (s < nk) load_slab<A_KMAJOR, BM, V>(As + s * A_STAGE, Bs + s * B_STAGE, A, lda, Bm, ldb, m0, Mdim, n0, Ndim, kbeg + s * BK, kend);
+#pragma unroll
+    for (int c = 0; c < L::N; ++c) slab.copy(c, s * A_STAGE, s * B_STAGE, A, Bm);
+    slab.advance();
     cp_async_commit();
   }
+  double a[2][4], b[2][4];
+  auto fragments = [&](int buf, int stage, int kk) {
+    const double *as = As + stage * A_STAGE, *bs = Bs + stage * B_STAGE;
+#pragma unroll
+    for (int mi = 0; mi < 4; ++mi)
+      a[buf][mi] = A_KMAJOR ? as[(wm + mi * 8 + g) * LDA_K + kk * 4 + t] : as[(kk * 4 + t) * LDA_M + wm + mi * 8 + g];
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni) b[buf][ni] = bs[(kk * 4 + t) * LDB + wn + ni * 8 + g];
+  };
+  cp_async_wait<STAGES - 2>();
+  __syncthreads();
+  fragments(0, 0, 0);
+  // A slab is four steps of 16 instructions.  The next step's operands are read before a step's instructions, across the
+  // slab boundary too, and the copies of a later slab are issued between them a few at a time: with one or two CTAs per SM
+  // the tensor pipe otherwise drains at every barrier and idles through the copies' address arithmetic (128 x 3000 outputs
+  // of 1568: 47 us).
+  constexpr int STEPS = (BK / 4 - 1) * 4, PER_STEP = (L::N + STEPS - 1) / STEPS;
+  int cur = 0, fill = STAGES - 1;
+#pragma unroll 1
   for (int kt = 0; kt < nk; ++kt) {
-    cp_async_wait<STAGES - 2>();   // slab kt has landed (for this thread's copies; the barrier covers the others')
-    __syncthreads();               // ... and everyone has finished with the stage refilled below
-    {
-      const int nx = kt + STAGES - 1;
-      if (nx < nk) {
-        const int s = nx % STAGES;
-        load_slab<A_KMAJOR, BM, V>(As + s * A_STAGE, Bs + s * B_STAGE, A, lda, Bm, ldb, m0, Mdim, n0, Ndim, kbeg + nx * BK, kend);
-      }
-      cp_async_commit();
-    }
-    const double *as = As + (kt % STAGES) * A_STAGE;
-    const double *bs = Bs + (kt % STAGES) * B_STAGE;
+    const int next = cur + 1 < STAGES ? cur + 1 : 0;
 #pragma unroll
     for (int kk = 0; kk < BK / 4; ++kk) {
-      double a[4], b[4];
+      if (kk == BK / 4 - 1) {
+        slab.advance();
+        cp_async_commit();
+        cp_async_wait<STAGES - 2>();   // slab kt + 1 has landed (for this thread's copies; the barrier covers the others')
+        __syncthreads();               // ... and everyone has read slab kt, whose stage the next turn refills
+      }
+      fragments((kk + 1) & 1, kk == BK / 4 - 1 ? next : cur, kk == BK / 4 - 1 ? 0 : kk + 1);
 #pragma unroll
-      for (int mi = 0; mi < 4; ++mi)
-        a[mi] = A_KMAJOR ? as[(wm + mi * 8 + g) * LDA_K + kk * 4 + t] : as[(kk * 4 + t) * LDA_M + wm + mi * 8 + g];
+      for (int mi = 0; mi < 4; ++mi) {
 #pragma unroll
-      for (int ni = 0; ni < 4; ++ni) b[ni] = bs[(kk * 4 + t) * LDB + wn + ni * 8 + g];
+        for (int ni = 0; ni < 4; ++ni) dmma(acc[mi][ni][0], acc[mi][ni][1], a[kk & 1][mi], b[kk & 1][ni]);
+        if (kk < BK / 4 - 1) {
 #pragma unroll
-      for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) dmma(acc[mi][ni][0], acc[mi][ni][1], a[mi], b[ni]);
+          for (int c = 0; c < PER_STEP; ++c)
+            slab.copy((kk * 4 + mi) * PER_STEP + c, fill * A_STAGE, fill * B_STAGE, A, Bm);
+        }
+      }
     }
+    fill = cur;
+    cur = next;
   }
   cp_async_wait<0>();
   ep.tile(acc, m0 + wm + g, n0 + wn + 2 * t, (int)blockIdx.z);
