@@ -11,8 +11,7 @@
 // are padded so that a half-warp's fragment loads (four rows of four consecutive doubles) fall into
 // 16 different bank pairs.
 #pragma once
-#include <cuda_runtime.h>
-#include <stdint.h>
+#include "sbb_slab.cuh"
 
 namespace sbb {
 namespace f64mma {
@@ -31,21 +30,13 @@ struct Cfg {
   static constexpr int A_STAGE = BM * LDA_K > BK * LDA_M ? BM * LDA_K : BK * LDA_M;   // doubles
   static constexpr size_t SMEM_BYTES = (size_t)STAGES * (A_STAGE + B_STAGE) * sizeof(double);
 };
+template <bool A_KMAJOR, int BM_>
+struct Shape {
+  static constexpr bool KMAJOR = A_KMAJOR;
+  static constexpr int BM = BM_, BN = f64mma::BN, BK = f64mma::BK, THREADS = Cfg<BM>::THREADS;
+  static constexpr int LDA = A_KMAJOR ? LDA_K : Cfg<BM>::LDA_M, LDB = f64mma::LDB;
+};
 
-// One copy of V doubles into shared memory; not valid: nothing is read, the destination is filled with zeros.
-template <int V>
-__device__ __forceinline__ void cp_async(uint32_t dst, const double *src, bool valid) {
-  const int bytes = valid ? 8 * V : 0;
-  if constexpr (V == 2)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 __device__ __forceinline__ void dmma(double &c0, double &c1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
                : "+d"(c0), "+d"(c1)
@@ -145,54 +136,6 @@ __device__ __forceinline__ double log_positive(double x) {
   return fma((double)e, 0.693147180559945309417232, t.y + q);
 }
 
-// A thread's share of the k-slabs of both operands: N copies of V elements per slab into the stage buffers, zero-filled
-// outside the operands.  A is [K x Mdim] MN-major (element (k, m) at A[k*lda + m]) or, A_KMAJOR, [Mdim x K] (at
-// A[m*lda + k]); B is [K x Ndim] MN-major.  V = 2: all row starts and the 2-element chunks are 16-byte aligned (checked by
-// the host).  A thread's copies of one operand lie RA (RB) rows of its memory layout apart in the same column, so one
-// pointer and one count of what is left per operand are all it keeps.
-template <bool A_KMAJOR, int BM, int V>
-struct Slab {
-  static constexpr int THREADS = Cfg<BM>::THREADS;
-  static constexpr int CA = (A_KMAJOR ? BK : BM) / V, CB = BN / V;   // copies per row
-  static constexpr int RA = THREADS / CA, RB = THREADS / CB;         // rows per pass of the block
-  static constexpr int NA = BM * BK / V / THREADS, N = NA + BK * BN / V / THREADS;
-  static constexpr int LDA = A_KMAJOR ? LDA_K : Cfg<BM>::LDA_M;
-  const double *pa, *pb;     // the first copy of the next slab
-  long lda, ldb;
-  uint32_t da, db;           // its place in stage 0
-  int rows_a, left_a, left_b;   // rows of A at and below the first copy's (K-major); k left from the first copies on
-  __device__ __forceinline__ Slab(const double *A, long lda_, const double *Bm, long ldb_, long m0, long Mdim, long n0,
-                                  long Ndim, int kbeg, int kend, const double *As, const double *Bs)
-      : lda(lda_), ldb(ldb_) {
-    const int ra = threadIdx.x / CA, ca = threadIdx.x % CA * V, rb = threadIdx.x / CB, cb = threadIdx.x % CB * V;
-    const long m = m0 + (A_KMAJOR ? ra : ca);
-    pa = A + (A_KMAJOR ? m * lda + kbeg + ca : (long)(kbeg + ra) * lda + m);
-    pb = Bm + (long)(kbeg + rb) * ldb + n0 + cb;
-    rows_a = (int)min(Mdim - m, (long)BM);
-    left_a = kend - kbeg - (A_KMAJOR ? ca : ra);
-    if (!A_KMAJOR && m >= Mdim) left_a = 0;
-    left_b = n0 + cb < Ndim ? kend - kbeg - rb : 0;
-    da = (uint32_t)__cvta_generic_to_shared(As + ra * LDA + ca);
-    db = (uint32_t)__cvta_generic_to_shared(Bs + rb * LDB + cb);
-  }
-  // Copy t of the next slab, into the stage that starts at element a (b) of the buffers.
-  __device__ __forceinline__ void copy(int t, int a, int b, const double *A, const double *Bm) const {
-    if (t < NA) {
-      const bool ok = A_KMAJOR ? t * RA < rows_a && left_a > 0 : t * RA < left_a;
-      cp_async<V>(da + (uint32_t)(a + t * RA * LDA) * 8u, ok ? pa + t * RA * lda : A, ok);
-    } else if (t < N) {
-      const bool ok = (t - NA) * RB < left_b;
-      cp_async<V>(db + (uint32_t)(b + (t - NA) * RB * LDB) * 8u, ok ? pb + (t - NA) * RB * ldb : Bm, ok);
-    }
-  }
-  __device__ __forceinline__ void advance() {
-    pa += A_KMAJOR ? (long)BK : BK * lda;
-    pb += BK * ldb;
-    left_a -= BK;
-    left_b -= BK;
-  }
-};
-
 // grid.x = row tiles of the output, grid.y = column tiles (swapped when cols_fastest), grid.z = k-splits.
 // k-split z covers [z*kper, min(K, (z+1)*kper)), kper a multiple of BK.  The epilogue receives the thread's
 // accumulators: ep.tile(acc, m, n, z) with acc[mi][ni][e] = output element (m + 8*mi, n + 8*ni + e), n even;
@@ -220,7 +163,7 @@ __global__ void __launch_bounds__(Cfg<BM>::THREADS, Cfg<BM, DEEP>::CTAS_PER_SM)
     for (int ni = 0; ni < 4; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
 
   ep.prefetch(m0 + wm, n0 + wn, lane);
-  using L = Slab<A_KMAJOR, BM, V>;
+  using L = Slab<double, Shape<A_KMAJOR, BM>, V>;
   L slab(A, lda, Bm, ldb, m0, Mdim, n0, Ndim, kbeg, kend, As, Bs);
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
@@ -244,7 +187,7 @@ __global__ void __launch_bounds__(Cfg<BM>::THREADS, Cfg<BM, DEEP>::CTAS_PER_SM)
   // A slab is four steps of 16 instructions.  The next step's operands are read before a step's instructions, across the
   // slab boundary too, and the copies of a later slab are issued between them a few at a time: with one or two CTAs per SM
   // the tensor pipe otherwise drains at every barrier and idles through the copies' address arithmetic (128 x 3000 outputs
-  // of 1568: 47 us).
+  // of 1568: 47 us then, 39 now; the instruction's own time is 33).
   constexpr int STEPS = (BK / 4 - 1) * 4, PER_STEP = (L::N + STEPS - 1) / STEPS;
   int cur = 0, fill = STAGES - 1;
 #pragma unroll 1

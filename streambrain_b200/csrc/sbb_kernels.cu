@@ -106,218 +106,124 @@ __device__ __forceinline__ void store4(double *p, const double *r, bool vec, int
   }
 }
 
-// One group of a micro-tile row (four floats / two doubles) from / to memory, same contract as load4 / store4.
-__device__ __forceinline__ void loadg(const float *p, float *r, bool vec, int valid) { load4(p, r, vec, valid); }
-__device__ __forceinline__ void storeg(float *p, const float *r, bool vec, int valid) { store4(p, r, vec, valid); }
-__device__ __forceinline__ void loadg(const double *p, double *r, bool vec, int valid) {
-  if (vec && valid == 2) {
-    unpack(*reinterpret_cast<const double2 *>(p), r);
-  } else {
-#pragma unroll
-    for (int c = 0; c < 2; ++c) r[c] = c < valid ? p[c] : 0.0;
-  }
-}
-__device__ __forceinline__ void storeg(double *p, const double *r, bool vec, int valid) {
-  if (vec && valid == 2) {
-    *reinterpret_cast<double2 *>(p) = pack(r);
-  } else {
-#pragma unroll
-    for (int c = 0; c < 2; ++c)
-      if (c < valid) p[c] = r[c];
-  }
-}
-
 static inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // ----------------------------------------------------------------------------
-// Tiled contraction core: C[Mdim, Ndim] (+)= A^T-or-A * B over k in [k0, k1).
-// 128x128 output tile per 256-thread CTA, 8x8 micro-tile per thread split into
-// two 4-wide halves in each dimension (rows ty*4+r and 64+ty*4+r; columns
-// tx*4+c and 64+tx*4+c) so shared-memory reads are conflict-free 16-byte loads
-// and global stores are 16 bytes per thread, 256 contiguous bytes per half-warp.
-// The next k-slab is fetched into registers while the current one is multiplied.
+// Tiled float32 contraction: C[Mdim, Ndim] = A^T-or-A * B over k in [k0, k1), on the FMA pipe; it serves rows that the
+// tensor-core kernels' copies cannot address.  128 x 128 output tile per 256-thread CTA, 8 x 8 micro-tile per thread split
+// into two 4-wide halves in each dimension (rows ty*4+r and 64+ty*4+r; columns tx*4+c and 64+tx*4+c) so shared-memory reads
+// are conflict-free 16-byte loads and global stores are 16 bytes per thread, 256 contiguous bytes per half-warp.  The slabs
+// arrive by cp.async, three of four stages in flight, and the multiplications are the two-wide FMA (two columns; each half
+// rounds like a single FMA): one issue slot for two leaves the others to the operand reads and copies.
 // ----------------------------------------------------------------------------
-template <typename T>
 struct Tile {
-  static constexpr int BM = 128, BN = 128, THREADS = 256;
-  static constexpr int BK = sizeof(T) == 4 ? 16 : 8;
-  static constexpr int LD = 128 + 4;                // shared row stride, elements
-  static constexpr int EPT = BK * 128 / THREADS;    // elements per thread per operand slab
+  static constexpr int BM = 128, BN = 128, BK = 16, THREADS = 256, STAGES = 4;
+  static constexpr int LDA_K = BK + 4, LDA_M = BM + 4, LDB = BN + 4;
+  static constexpr int A_STAGE = BM * LDA_K > BK * LDA_M ? BM * LDA_K : BK * LDA_M, B_STAGE = BK * LDB;
+  static constexpr size_t SMEM_BYTES = (size_t)STAGES * (A_STAGE + B_STAGE) * sizeof(float);
 };
-
-// Operand stored "MN-major": element (k, m) at p[k*ld + m].
-template <typename T, int VEC>
-__device__ __forceinline__ void load_mn(T (&r)[Tile<T>::EPT], const T *__restrict__ p, long ld, int k0, int k1,
-                                        long m0, long mn) {
-  constexpr int VPR = 128 / VEC;
-#pragma unroll
-  for (int t = 0; t < Tile<T>::EPT / VEC; ++t) {
-    const int v = threadIdx.x + t * Tile<T>::THREADS;
-    const int k = k0 + v / VPR;
-    const long m = m0 + (long)(v % VPR) * VEC;
-    const bool ok = k < k1 && m < mn;
-    if constexpr (VEC == 1) {
-      r[t] = ok ? __ldg(p + (long)k * ld + m) : (T)0;
-    } else {
-      using V = typename Vec16<T>::type;
-      if (ok) {
-        unpack(__ldg(reinterpret_cast<const V *>(p + (long)k * ld + m)), &r[t * VEC]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) r[t * VEC + e] = (T)0;
-      }
-    }
-  }
-}
-template <typename T, int VEC>
-__device__ __forceinline__ void store_mn(T *s, const T (&r)[Tile<T>::EPT]) {
-  constexpr int VPR = 128 / VEC;
-#pragma unroll
-  for (int t = 0; t < Tile<T>::EPT / VEC; ++t) {
-    const int v = threadIdx.x + t * Tile<T>::THREADS;
-    const int k = v / VPR;
-    const int m = (v % VPR) * VEC;
-    if constexpr (VEC == 1) {
-      s[k * Tile<T>::LD + m] = r[t];
-    } else {
-      using V = typename Vec16<T>::type;
-      *reinterpret_cast<V *>(s + k * Tile<T>::LD + m) = pack(&r[t * VEC]);
-    }
-  }
-}
-
-// Operand stored "K-major": element (k, m) at p[m*ld + k]; transposed into shared.
-template <typename T, int VEC>
-__device__ __forceinline__ void load_km(T (&r)[Tile<T>::EPT], const T *__restrict__ p, long ld, int k0, int k1,
-                                        long m0, long mn) {
-  constexpr int VPR = Tile<T>::BK / VEC;
-#pragma unroll
-  for (int t = 0; t < Tile<T>::EPT / VEC; ++t) {
-    const int v = threadIdx.x + t * Tile<T>::THREADS;
-    const long m = m0 + v / VPR;
-    const int k = k0 + (v % VPR) * VEC;
-    const bool ok = m < mn && k < k1;
-    if constexpr (VEC == 1) {
-      r[t] = ok ? __ldg(p + m * ld + k) : (T)0;
-    } else {
-      using V = typename Vec16<T>::type;
-      if (ok) {
-        unpack(__ldg(reinterpret_cast<const V *>(p + m * ld + k)), &r[t * VEC]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) r[t * VEC + e] = (T)0;
-      }
-    }
-  }
-}
-template <typename T, int VEC>
-__device__ __forceinline__ void store_km(T *s, const T (&r)[Tile<T>::EPT]) {
-  constexpr int VPR = Tile<T>::BK / VEC;
-#pragma unroll
-  for (int t = 0; t < Tile<T>::EPT / VEC; ++t) {
-    const int v = threadIdx.x + t * Tile<T>::THREADS;
-    const int m = v / VPR;
-    const int k = (v % VPR) * VEC;
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) s[(k + e) * Tile<T>::LD + m] = r[t * VEC + e];
-  }
-}
+template <bool A_KMAJOR>
+struct TileShape : Tile {
+  static constexpr bool KMAJOR = A_KMAJOR;
+  static constexpr int LDA = A_KMAJOR ? LDA_K : LDA_M;
+};
 
 __device__ __forceinline__ void lds4(const float *p, float *r) { unpack(*reinterpret_cast<const float4 *>(p), r); }
-__device__ __forceinline__ void lds4(const double *p, double *r) {
-  unpack(*reinterpret_cast<const double2 *>(p), r);
-  unpack(*reinterpret_cast<const double2 *>(p + 2), r + 2);
-}
-
-// Columns of a thread's micro-tile.  A thread owns 8 columns as groups of one 16-byte vector each: float32
-// two groups of four (columns g*64 + tx*4 ..), float64 four groups of two (columns g*32 + tx*2 ..), so that
-// the 16 threads of a half-warp read (and later store) contiguous 16-byte pieces: 256 bytes per request, no
-// shared-memory bank conflicts.  (With four doubles per thread and group the 16-byte reads of a half-warp sat
-// 32 bytes apart: two-way conflicts on 40 % of the wavefronts of the float64 kernels.)
-template <typename T>
-struct MicroCols {
-  static constexpr int GW = 16 / (int)sizeof(T);   // columns per group
-  static constexpr int NG = 8 / GW;                // groups per thread
-  static constexpr int STRIDE = 128 / NG;          // columns between the starts of a thread's groups
-  __device__ static __forceinline__ int group_start(int tx, int g) { return g * STRIDE + tx * GW; }
-  __device__ static __forceinline__ int col(int tx, int e) { return group_start(tx, e / GW) + e % GW; }
-};
-__device__ __forceinline__ void ldsv(const float *p, float *r) { unpack(*reinterpret_cast<const float4 *>(p), r); }
-__device__ __forceinline__ void ldsv(const double *p, double *r) { unpack(*reinterpret_cast<const double2 *>(p), r); }
-
-template <typename T>
-__device__ __forceinline__ void multiply_slab(const T *As, const T *Bs, T (&acc)[8][8], int ty, int tx) {
-  using MC = MicroCols<T>;
-#pragma unroll
-  for (int k = 0; k < Tile<T>::BK; ++k) {
-    T a[8], b[8];
-    lds4(As + k * Tile<T>::LD + ty * 4, a);
-    lds4(As + k * Tile<T>::LD + 64 + ty * 4, a + 4);
-#pragma unroll
-    for (int g = 0; g < MC::NG; ++g) ldsv(Bs + k * Tile<T>::LD + MC::group_start(tx, g), b + g * MC::GW);
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-#pragma unroll
-      for (int c = 0; c < 8; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
-  }
-}
 
 // Row / column of micro-tile entry e (0..7) inside the 128-wide tile.
 __device__ __forceinline__ int micro_index(int t, int e) { return (e < 4 ? 0 : 64) + t * 4 + (e & 3); }
 
-// grid.x = row tiles of the output, grid.y = column tiles (swapped when cols_fastest), grid.z = k-splits.
-// A is [K x Mdim] MN-major (A_KMAJOR=false) or [Mdim x K] K-major (true); B is
-// [K x Ndim] MN-major.  k-split z covers [z*kper, min(K,(z+1)*kper)), kper a
-// multiple of the slab depth.
-template <typename T, bool A_KMAJOR, int VEC, class Epilogue>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1)
-    contraction_kernel(const T *__restrict__ A, long lda, const T *__restrict__ Bm, long ldb, long Mdim, long Ndim,
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  return (uint64_t)__float_as_uint(hi) << 32 | __float_as_uint(lo);
+}
+__device__ __forceinline__ void fma2(uint64_t &acc, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+// grid.x = row tiles of the output, grid.y = column tiles (swapped when cols_fastest: the fastest dimension walks the tiles
+// that share the larger re-used operand), grid.z = k-splits.  k-split z covers [z*kper, min(K,(z+1)*kper)), kper a multiple
+// of the slab depth.
+template <bool A_KMAJOR, int V, class Epilogue>
+__global__ void __launch_bounds__(Tile::THREADS, 2)
+    contraction_kernel(const float *__restrict__ A, long lda, const float *__restrict__ Bm, long ldb, long Mdim, long Ndim,
                        int K, int kper, bool cols_fastest, Epilogue ep) {
-  using TL = Tile<T>;
-  __shared__ __align__(16) T As[2][TL::BK * TL::LD];
-  __shared__ __align__(16) T Bs[2][TL::BK * TL::LD];
+  using S = TileShape<A_KMAJOR>;
+  using L = Slab<float, S, V>;
+  extern __shared__ __align__(16) float tile_smem[];
+  float *As = tile_smem, *Bs = tile_smem + S::STAGES * S::A_STAGE;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  // Rasterisation: the fastest grid dimension walks the tiles that share the larger re-used operand.
-  const long m0 = (long)(cols_fastest ? blockIdx.y : blockIdx.x) * TL::BM;
-  const long n0 = (long)(cols_fastest ? blockIdx.x : blockIdx.y) * TL::BN;
+  const long m0 = (long)(cols_fastest ? blockIdx.y : blockIdx.x) * S::BM;
+  const long n0 = (long)(cols_fastest ? blockIdx.x : blockIdx.y) * S::BN;
   const int kbeg = blockIdx.z * kper;
   const int kend = min(K, kbeg + kper);
-
-  T acc[8][8];
+  const int nk = kend > kbeg ? (kend - kbeg + S::BK - 1) / S::BK : 0;
+  L slab(A, lda, Bm, ldb, m0, Mdim, n0, Ndim, kbeg, kend, As, Bs);
+#pragma unroll
+  for (int s = 0; s < S::STAGES - 1; ++s) {
+#pragma unroll
+    for (int c = 0; c < L::N; ++c) slab.copy(c, s * S::A_STAGE, s * S::B_STAGE, A, Bm);
+    slab.advance();
+    cp_async_commit();
+  }
+  uint64_t acc[8][4];   // pairs of neighbouring columns
 #pragma unroll
   for (int r = 0; r < 8; ++r)
 #pragma unroll
-    for (int c = 0; c < 8; ++c) acc[r][c] = (T)0;
-
-  T ra[TL::EPT], rb[TL::EPT];
-  if (kbeg < kend) {
-    if constexpr (A_KMAJOR) load_km<T, VEC>(ra, A, lda, kbeg, kend, m0, Mdim);
-    else load_mn<T, VEC>(ra, A, lda, kbeg, kend, m0, Mdim);
-    load_mn<T, VEC>(rb, Bm, ldb, kbeg, kend, n0, Ndim);
-    if constexpr (A_KMAJOR) store_km<T, VEC>(As[0], ra);
-    else store_mn<T, VEC>(As[0], ra);
-    store_mn<T, VEC>(Bs[0], rb);
-  }
-  __syncthreads();
-  int buf = 0;
-  for (int k0 = kbeg; k0 < kend; k0 += TL::BK) {
-    const int kn = k0 + TL::BK;
-    const bool more = kn < kend;
-    if (more) {
-      if constexpr (A_KMAJOR) load_km<T, VEC>(ra, A, lda, kn, kend, m0, Mdim);
-      else load_mn<T, VEC>(ra, A, lda, kn, kend, m0, Mdim);
-      load_mn<T, VEC>(rb, Bm, ldb, kn, kend, n0, Ndim);
+    for (int c = 0; c < 4; ++c) acc[r][c] = 0;
+  int cur = 0, fill = S::STAGES - 1;
+#pragma unroll 1
+  for (int kt = 0; kt < nk; ++kt) {
+    cp_async_wait<S::STAGES - 2>();   // slab kt has landed (for this thread's copies; the barrier covers the others')
+    __syncthreads();                  // ... and everyone has finished with the stage refilled below
+    const float *as = As + cur * S::A_STAGE, *bs = Bs + cur * S::B_STAGE;
+    constexpr int PER_STEP = (L::N + S::BK / 2 - 1) / (S::BK / 2);
+#pragma unroll
+    for (int k2 = 0; k2 < S::BK; k2 += 2) {
+      float a[2][8];
+      if constexpr (A_KMAJOR) {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const float2 v = *reinterpret_cast<const float2 *>(as + micro_index(ty, r) * S::LDA + k2);
+          a[0][r] = v.x;
+          a[1][r] = v.y;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        if constexpr (!A_KMAJOR) {
+          lds4(as + (k2 + k) * S::LDA + ty * 4, a[k]);
+          lds4(as + (k2 + k) * S::LDA + 64 + ty * 4, a[k] + 4);
+        }
+        uint64_t b[4];
+        const ulonglong2 b0 = *reinterpret_cast<const ulonglong2 *>(bs + (k2 + k) * S::LDB + tx * 4);
+        const ulonglong2 b1 = *reinterpret_cast<const ulonglong2 *>(bs + (k2 + k) * S::LDB + 64 + tx * 4);
+        b[0] = b0.x, b[1] = b0.y, b[2] = b1.x, b[3] = b1.y;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const uint64_t aa = pack2(a[k][r], a[k][r]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) fma2(acc[r][c], aa, b[c]);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < PER_STEP; ++c)   // a few of a later slab's copies between the multiplications
+        slab.copy(k2 / 2 * PER_STEP + c, fill * S::A_STAGE, fill * S::B_STAGE, A, Bm);
     }
-    multiply_slab<T>(As[buf], Bs[buf], acc, ty, tx);
-    if (more) {
-      if constexpr (A_KMAJOR) store_km<T, VEC>(As[buf ^ 1], ra);
-      else store_mn<T, VEC>(As[buf ^ 1], ra);
-      store_mn<T, VEC>(Bs[buf ^ 1], rb);
-    }
-    __syncthreads();
-    buf ^= 1;
+    slab.advance();
+    cp_async_commit();
+    fill = cur;
+    cur = cur + 1 < S::STAGES ? cur + 1 : 0;
   }
-  ep(acc, m0, n0, ty, tx, (int)blockIdx.z);
+  cp_async_wait<0>();
+  float out[8][8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      out[r][2 * c] = __uint_as_float((uint32_t)acc[r][c]);
+      out[r][2 * c + 1] = __uint_as_float((uint32_t)(acc[r][c] >> 32));
+    }
+  ep(out, m0, n0, ty, tx, (int)blockIdx.z);
 }
 
 // The same contraction for float32 outputs of few 128 x 128 tiles: a 32 x 64 tile per CTA of four warps, each 8 rows x 64
@@ -325,47 +231,22 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1)
 // row length, and its reads of A are broadcasts).  Such launches are bound by latency and by the SMs they leave idle, not by
 // arithmetic: the slabs arrive by 4-byte cp.async (any alignment) with three of four stages in flight, and what the epilogue
 // reads is requested before the main loop.  Each output is the same chain of FMAs over ascending k as in the kernel above.
-struct SmallTile {
+template <bool A_KMAJOR>
+struct SmallShape {
+  static constexpr bool KMAJOR = A_KMAJOR;
   static constexpr int BM = 32, BN = 64, BK = 32, STAGES = 4, THREADS = 128;
-  static constexpr int LDA = 32 + 4;   // K-major A as [m][k], MN-major as [k][m]: 16-byte rows
-  static constexpr int A_STAGE = 32 * LDA, B_STAGE = BK * BN;
+  static constexpr int LDA = 32 + 4, LDB = BN;   // K-major A as [m][k], MN-major as [k][m]: 16-byte rows
+  static constexpr int A_STAGE = 32 * LDA, B_STAGE = BK * LDB;
   static constexpr size_t SMEM_BYTES = (size_t)STAGES * (A_STAGE + B_STAGE) * sizeof(float);
 };
-__device__ __forceinline__ void cp_async4(float *dst, const float *src, bool valid) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(valid ? 4 : 0) : "memory");
-}
-
-template <bool A_KMAJOR>
-__device__ __forceinline__ void load_small_slab(float *As, float *Bs, const float *__restrict__ A, long lda,
-                                                const float *__restrict__ Bm, long ldb, long m0, long Mdim, long n0,
-                                                long Ndim, int k0, int kend) {
-  const int w8 = (threadIdx.x >> 5) * 8, lane = threadIdx.x & 31;
-#pragma unroll
-  for (int t = 0; t < 8; ++t) {
-    const long m = m0 + (A_KMAJOR ? w8 + t : lane);
-    const int k = k0 + (A_KMAJOR ? lane : w8 + t);
-    const bool ok = m < Mdim && k < kend;
-    cp_async4(As + (w8 + t) * SmallTile::LDA + lane, ok ? A + (A_KMAJOR ? m * lda + k : (long)k * lda + m) : A, ok);
-  }
-#pragma unroll
-  for (int t = 0; t < 8; ++t) {
-    const int k = k0 + w8 + t;
-    const float *row = Bm + (long)k * ldb + n0 + lane;
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const bool ok = k < kend && n0 + lane + 32 * c < Ndim;
-      cp_async4(Bs + (w8 + t) * SmallTile::BN + lane + 32 * c, ok ? row + 32 * c : Bm, ok);
-    }
-  }
-}
 
 // grid.x = column tiles, grid.y = row tiles, grid.z = k-splits
 template <bool A_KMAJOR, class Epilogue>
-__global__ void __launch_bounds__(SmallTile::THREADS)
+__global__ void __launch_bounds__(SmallShape<A_KMAJOR>::THREADS)
     small_contraction_kernel(const float *__restrict__ A, long lda, const float *__restrict__ Bm, long ldb, long Mdim,
                              long Ndim, int K, int kper, Epilogue ep) {
-  using S = SmallTile;
+  using S = SmallShape<A_KMAJOR>;
+  using L = Slab<float, S, 1>;
   extern __shared__ __align__(16) float small_smem[];
   float *As = small_smem, *Bs = small_smem + S::STAGES * S::A_STAGE;
   const int w8 = (threadIdx.x >> 5) * 8, lane = threadIdx.x & 31;
@@ -373,25 +254,31 @@ __global__ void __launch_bounds__(SmallTile::THREADS)
   const int kbeg = blockIdx.z * kper;
   const int kend = min(K, kbeg + kper);
   const int nk = kend > kbeg ? (kend - kbeg + S::BK - 1) / S::BK : 0;
+  L slab(A, lda, Bm, ldb, m0, Mdim, n0, Ndim, kbeg, kend, As, Bs);
 #pragma unroll
   for (int s = 0; s < S::STAGES - 1; ++s) {
-    if (s < nk)
-      load_small_slab<A_KMAJOR>(As + s * S::A_STAGE, Bs + s * S::B_STAGE, A, lda, Bm, ldb, m0, Mdim, n0, Ndim,
-                                kbeg + s * S::BK, kend);
-    f64mma::cp_async_commit();
+    if (s < nk) {
+#pragma unroll
+      for (int c = 0; c < L::N; ++c) slab.copy(c, s * S::A_STAGE, s * S::B_STAGE, A, Bm);
+      slab.advance();
+    }
+    cp_async_commit();
   }
   typename Epilogue::Strip strip(ep, m0 + w8, n0 + lane, lane);
   float acc[8][2];
 #pragma unroll
   for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = 0.f;
   for (int kt = 0; kt < nk; ++kt) {
-    f64mma::cp_async_wait<S::STAGES - 2>();   // slab kt has landed
-    __syncthreads();                          // ... for every thread, and the stage refilled below is free
+    cp_async_wait<S::STAGES - 2>();   // slab kt has landed
+    __syncthreads();                  // ... for every thread, and the stage refilled below is free
     const int nx = kt + S::STAGES - 1;
-    if (nx < nk)
-      load_small_slab<A_KMAJOR>(As + nx % S::STAGES * S::A_STAGE, Bs + nx % S::STAGES * S::B_STAGE, A, lda, Bm, ldb, m0,
-                                Mdim, n0, Ndim, kbeg + nx * S::BK, kend);
-    f64mma::cp_async_commit();
+    if (nx < nk) {
+#pragma unroll
+      for (int c = 0; c < L::N; ++c)
+        slab.copy(c, nx % S::STAGES * S::A_STAGE, nx % S::STAGES * S::B_STAGE, A, Bm);
+      slab.advance();
+    }
+    cp_async_commit();
     const float *as = As + kt % S::STAGES * S::A_STAGE, *bs = Bs + kt % S::STAGES * S::B_STAGE + lane;
 #pragma unroll
     for (int k4 = 0; k4 < S::BK; k4 += 4) {
@@ -411,7 +298,7 @@ __global__ void __launch_bounds__(SmallTile::THREADS)
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const float b0 = bs[(k4 + k) * S::BN], b1 = bs[(k4 + k) * S::BN + 32];
+        const float b0 = bs[(k4 + k) * S::LDB], b1 = bs[(k4 + k) * S::LDB + 32];
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
           acc[r][0] = fmaf(a[r][k], b0, acc[r][0]);
@@ -420,7 +307,7 @@ __global__ void __launch_bounds__(SmallTile::THREADS)
       }
     }
   }
-  f64mma::cp_async_wait<0>();
+  cp_async_wait<0>();
   strip.finish(ep, acc, m0 + w8, n0 + lane, (int)blockIdx.z);
 }
 
@@ -432,6 +319,7 @@ struct StoreEpilogue {
   long ld;           // row stride of out
   long zstride;      // elements between k-split slices
   bool vec;
+  // The micro-tiles of the large-tile kernel.
   __device__ __forceinline__ void operator()(T (&acc)[8][8], long m0, long n0, int ty, int tx, int z) const {
     T *base = out + (long)z * zstride;
 #pragma unroll
@@ -439,12 +327,11 @@ struct StoreEpilogue {
       const long m = m0 + micro_index(ty, r);
       if (m >= rows) continue;
 #pragma unroll
-      for (int g = 0; g < MicroCols<T>::NG; ++g) {
-        constexpr int GW = MicroCols<T>::GW;
-        const long n = n0 + MicroCols<T>::group_start(tx, g);
+      for (int g = 0; g < 2; ++g) {
+        const long n = n0 + g * 64 + tx * 4;
         const long left = cols - n;
         if (left <= 0) continue;
-        storeg(base + m * ld + n, &acc[r][g * GW], vec, left >= GW ? GW : (int)left);
+        store4(base + m * ld + n, &acc[r][g * 4], vec, left >= 4 ? 4 : (int)left);
       }
     }
   }
@@ -483,7 +370,7 @@ struct TraceEpilogue {
     bool cj_low[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-      const long j = n0 + MicroCols<T>::col(tx, c);
+      const long j = n0 + micro_index(tx, c);
       const bool in = j < M;
       cj[c] = in ? Cj[j] : (T)1;
       cj_low[c] = cj[c] < p.cthr;
@@ -497,14 +384,14 @@ struct TraceEpilogue {
       const bool skip = ci < p.cthr;
       const uint8_t *mrow = wmask ? wmask + i * H : nullptr;
 #pragma unroll
-      for (int g = 0; g < MicroCols<T>::NG; ++g) {
-        constexpr int GW = MicroCols<T>::GW;
-        const long j = n0 + MicroCols<T>::group_start(tx, g);
+      for (int g = 0; g < 2; ++g) {
+        constexpr int GW = 4;
+        const long j = n0 + g * 64 + tx * 4;
         const long left = M - j;
         if (left <= 0) continue;
         const int valid = left >= GW ? GW : (int)left;
         T c4[GW], w4[GW];
-        loadg(Cij + i * M + j, c4, vec, valid);
+        load4(Cij + i * M + j, c4, vec, valid);
 #pragma unroll
         for (int c = 0; c < GW; ++c) {
           if (c < valid) {
@@ -516,8 +403,8 @@ struct TraceEpilogue {
             w4[c] = w;
           }
         }
-        storeg(Cij + i * M + j, c4, vec, valid);
-        storeg(W + i * M + j, w4, vec, valid);
+        store4(Cij + i * M + j, c4, vec, valid);
+        store4(W + i * M + j, w4, vec, valid);
       }
     }
   }
@@ -768,6 +655,17 @@ static TracePairs to_pairs(const TraceEpilogue<double> &e) {
 
 static int sm_count();
 
+// More than 48 KB of dynamic shared memory is asked for once per kernel and device.
+template <class K>
+static cudaError_t allow_smem(K kernel, size_t bytes, bool (&configured)[64]) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && configured[dev]) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess && dev >= 0 && dev < 64) configured[dev] = true;
+  return e;
+}
+
 template <bool A_KMAJOR, int BM, bool DEEP, int V, class Pairs>
 static cudaError_t launch_f64_mma_tiles(const double *A, long lda, const double *Bm, long ldb, long Mdim, long Ndim,
                                         int K, int splits, bool cols_fastest, Pairs ep, cudaStream_t st) {
@@ -775,13 +673,8 @@ static cudaError_t launch_f64_mma_tiles(const double *A, long lda, const double 
   using C = F::Cfg<BM, DEEP>;
   auto kernel = F::contraction_kernel<A_KMAJOR, BM, DEEP, V, Pairs>;
   static bool configured[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 64) configured[dev] = true;
-  }
+  const cudaError_t e = allow_smem(kernel, C::SMEM_BYTES, configured);
+  if (e != cudaSuccess) return e;
   const unsigned mt = (unsigned)((Mdim + BM - 1) / BM), nt = (unsigned)((Ndim + F::BN - 1) / F::BN);
   if (cols_fastest && mt > 65535u) cols_fastest = false;
   dim3 grid(cols_fastest ? nt : mt, cols_fastest ? mt : nt, (unsigned)splits);
@@ -822,44 +715,47 @@ static bool small_tiles(long tiles, bool forward) {
 template <bool A_KMAJOR, class Ep>
 static cudaError_t launch_small_contraction(const float *A, long lda, const float *Bm, long ldb, long Mdim, long Ndim,
                                             int K, int splits, int kper, Ep ep, cudaStream_t st) {
-  using S = SmallTile;
+  using S = SmallShape<A_KMAJOR>;
   auto kernel = small_contraction_kernel<A_KMAJOR, Ep>;
   static bool configured[64] = {false};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 64) configured[dev] = true;
-  }
+  const cudaError_t e = allow_smem(kernel, S::SMEM_BYTES, configured);
+  if (e != cudaSuccess) return e;
   const dim3 grid((unsigned)((Ndim + S::BN - 1) / S::BN), (unsigned)((Mdim + S::BM - 1) / S::BM), (unsigned)splits);
   if (grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
   kernel<<<grid, S::THREADS, S::SMEM_BYTES, st>>>(A, lda, Bm, ldb, Mdim, Ndim, K, kper, ep);
   return launched();
 }
 
+template <bool A_KMAJOR, int V, class Ep>
+static cudaError_t launch_tiles(const float *A, long lda, const float *Bm, long ldb, long Mdim, long Ndim, int K,
+                                int splits, int kper, bool cols_fastest, Ep ep, cudaStream_t st) {
+  auto kernel = contraction_kernel<A_KMAJOR, V, Ep>;
+  static bool configured[64] = {false};
+  const cudaError_t e = allow_smem(kernel, Tile::SMEM_BYTES, configured);
+  if (e != cudaSuccess) return e;
+  const unsigned mt = (unsigned)((Mdim + 127) / 128), nt = (unsigned)((Ndim + 127) / 128);
+  if (cols_fastest && mt > 65535u) cols_fastest = false;
+  const dim3 grid(cols_fastest ? nt : mt, cols_fastest ? mt : nt, (unsigned)splits);
+  if (grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
+  kernel<<<grid, Tile::THREADS, Tile::SMEM_BYTES, st>>>(A, lda, Bm, ldb, Mdim, Ndim, K, kper, cols_fastest, ep);
+  return launched();
+}
+
 template <typename T, bool A_KMAJOR, class Ep>
 static cudaError_t launch_contraction(const T *A, long lda, const T *Bm, long ldb, long Mdim, long Ndim, int K,
                                       int splits, int kper, bool vec, bool cols_fastest, Ep ep, cudaStream_t st) {
-  const unsigned mt = (unsigned)((Mdim + 127) / 128), nt = (unsigned)((Ndim + 127) / 128);
-  if (mt == 0 || nt == 0 || K <= 0) return cudaSuccess;
+  const long mt = (Mdim + 127) / 128, nt = (Ndim + 127) / 128;
+  if (mt <= 0 || nt <= 0 || K <= 0) return cudaSuccess;
+  // `vec`: every operand row starts on a 16-byte boundary and holds a whole number of 16-byte pieces
   if constexpr (std::is_same<T, double>::value) {
-    // `vec`: every operand row starts on a 16-byte boundary and holds an even number of elements
     if (vec && lda % 2 == 0 && ldb % 2 == 0)
       return launch_f64_mma<A_KMAJOR, 2>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, to_pairs(ep), st);
     return launch_f64_mma<A_KMAJOR, 1>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, to_pairs(ep), st);
   } else {
-  if (small_tiles((long)mt * nt * splits, A_KMAJOR))
-    return launch_small_contraction<A_KMAJOR>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, ep, st);
-  if (cols_fastest && mt > 65535u) cols_fastest = false;
-  dim3 grid(cols_fastest ? nt : mt, cols_fastest ? mt : nt, (unsigned)splits);
-  if (grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
-  constexpr int V = Vec16<T>::N;
-  if (vec)
-    contraction_kernel<T, A_KMAJOR, V, Ep><<<grid, 256, 0, st>>>(A, lda, Bm, ldb, Mdim, Ndim, K, kper, cols_fastest, ep);
-  else
-    contraction_kernel<T, A_KMAJOR, 1, Ep><<<grid, 256, 0, st>>>(A, lda, Bm, ldb, Mdim, Ndim, K, kper, cols_fastest, ep);
-  return launched();
+    if (small_tiles(mt * nt * splits, A_KMAJOR))
+      return launch_small_contraction<A_KMAJOR>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, ep, st);
+    if (vec) return launch_tiles<A_KMAJOR, 4>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, cols_fastest, ep, st);
+    return launch_tiles<A_KMAJOR, 1>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, cols_fastest, ep, st);
   }
 }
 
@@ -900,7 +796,7 @@ int forward_splits(long B, long N, long M) {
   const long tiles = ((B + 127) / 128) * ((M + 127) / 128);
   const long want = 2 * sms;
   long s = tiles >= want ? 1 : want / (tiles > 0 ? tiles : 1);
-  const long slabs = (N + Tile<T>::BK - 1) / Tile<T>::BK;
+  const long slabs = (N + Tile::BK - 1) / Tile::BK;
   const long max_s = slabs / 8 > 0 ? slabs / 8 : 1;
   if (s > max_s) s = max_s;
   if (s > 64) s = 64;
@@ -914,8 +810,8 @@ template <typename T>
 cudaError_t launch_forward_product(const T *x, const T *w, T *partial, long B, long N, long M, int splits,
                                    cudaStream_t st) {
   constexpr int V = Vec16<T>::N;
-  const long slabs = (N + Tile<T>::BK - 1) / Tile<T>::BK;
-  const int kper = (int)((slabs + splits - 1) / splits) * Tile<T>::BK;
+  const long slabs = (N + Tile::BK - 1) / Tile::BK;
+  const int kper = (int)((slabs + splits - 1) / splits) * Tile::BK;
   const bool vec = (N % V == 0) && (M % V == 0) && aligned16(x) && aligned16(w);
   StoreEpilogue<T> ep{partial, B, M, M, B * M, (M % V == 0) && aligned16(partial)};
   return launch_contraction<T, true>(x, N, w, M, B, M, (int)N, splits, kper, vec, false, ep, st);
@@ -1287,7 +1183,7 @@ cudaError_t launch_trace_update_fused(const T *x, const T *y, long B, long N, lo
                    aligned16(x) && aligned16(y);
   TraceEpilogue<T> ep{Ci, Cj, Cij, w, wmask, row_begin, row_end, M, H, Mc, p,
                       (M % V == 0) && aligned16(Cij) && aligned16(w), rci, rcj};
-  const int kper = (int)((B + Tile<T>::BK - 1) / Tile<T>::BK) * Tile<T>::BK;
+  const int kper = (int)((B + Tile::BK - 1) / Tile::BK) * Tile::BK;
   return launch_contraction<T, false>(x + row_begin, N, y, M, row_end - row_begin, M, (int)B, 1, kper, vec, true, ep, st);
 }
 template cudaError_t launch_trace_update_fused<float>(const float *, const float *, long, long, long, long, long,
@@ -1307,7 +1203,7 @@ cudaError_t launch_outer_product(const T *x, const T *y, long B, long N, long M,
   const bool vec = (N % V == 0) && (M % V == 0) && (row_begin % V == 0) && ((row_end - row_begin) % V == 0) &&
                    aligned16(x) && aligned16(y);
   StoreEpilogue<T> ep{delta + row_begin * M, row_end - row_begin, M, M, 0, (M % V == 0) && aligned16(delta)};
-  const int kper = (int)((B + Tile<T>::BK - 1) / Tile<T>::BK) * Tile<T>::BK;
+  const int kper = (int)((B + Tile::BK - 1) / Tile::BK) * Tile::BK;
   return launch_contraction<T, false>(x + row_begin, N, y, M, row_end - row_begin, M, (int)B, 1, kper, vec, true, ep, st);
 }
 template cudaError_t launch_outer_product<float>(const float *, const float *, long, long, long, float *, long, long,
