@@ -115,6 +115,8 @@ static inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t
 // are conflict-free 16-byte loads and global stores are 16 bytes per thread, 256 contiguous bytes per half-warp.  The slabs
 // arrive by cp.async, three of four stages in flight, and the multiplications are the two-wide FMA (two columns; each half
 // rounds like a single FMA): one issue slot for two leaves the others to the operand reads and copies.
+// 1001 x 6001 -> 2257, odd rows: forward 690 -> 586 us, trace 778 -> 570 us against register-staged slabs (46 TFLOP/s; a
+// warp of 4 x 8 threads, which halves the shared-memory passes, changes nothing).
 // ----------------------------------------------------------------------------
 struct Tile {
   static constexpr int BM = 128, BN = 128, BK = 16, THREADS = 256, STAGES = 4;
@@ -704,13 +706,10 @@ static cudaError_t launch_f64_mma(const double *A, long lda, const double *Bm, l
   return launch_f64_mma_tiles<A_KMAJOR, 128, false, V>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, ep, st);
 }
 
-// When the 32 x 64 tiles take over.  Forward products (no epilogue to speak of): below two thirds of an SM's worth of 128 x
-// 128 tiles; 28 tiles 21.6 -> 10.0 us, 92 tiles 22.0 -> 20.8, but 112 tiles 23.3 -> 27.7.  Trace steps, whose epilogue is a
-// logarithm and a division per output: below one wave of the large kernel's CTAs (two per SM); 32 tiles 40.5 -> 13.1 us,
-// 96 tiles 41.4 -> 28.9, 216 tiles 59.6 -> 57.0, but 800 tiles 144 -> 156.
-static bool small_tiles(long tiles, bool forward) {
-  return forward ? 3 * tiles < 2L * sm_count() : tiles < 2L * sm_count();
-}
+// When the 32 x 64 tiles take over, in 128 x 128 tiles.  Forward products: below half an SM's worth; 28 tiles 18.5 -> 9.1
+// us, but 92 tiles 19.0 -> 20.6.  Trace steps, whose epilogue is a logarithm and a division per output: below one per SM; 32
+// tiles 35.6 -> 12.8 us, 96 tiles 36.5 -> 28.3, but 216 tiles 55.0 -> 54.7 at batch 97 and 125 -> 136 at batch 512.
+static bool small_tiles(long tiles, bool forward) { return (forward ? 2 : 1) * tiles < sm_count(); }
 
 template <bool A_KMAJOR, class Ep>
 static cudaError_t launch_small_contraction(const float *A, long lda, const float *Bm, long ldb, long Mdim, long Ndim,
