@@ -11,6 +11,7 @@
 // are padded so that a half-warp's fragment loads (four rows of four consecutive doubles) fall into
 // 16 different bank pairs.
 #pragma once
+#include "sbb_launch.cuh"
 #include "sbb_slab.cuh"
 
 namespace sbb {
@@ -144,6 +145,7 @@ template <bool A_KMAJOR, int BM, bool DEEP, int V, class Epilogue>
 __global__ void __launch_bounds__(Cfg<BM>::THREADS, Cfg<BM, DEEP>::CTAS_PER_SM)
     contraction_kernel(const double *__restrict__ A, long lda, const double *__restrict__ Bm, long ldb, long Mdim,
                        long Ndim, int K, int kper, bool cols_fastest, Epilogue ep) {
+  after_previous();
   constexpr int A_STAGE = Cfg<BM>::A_STAGE, LDA_M = Cfg<BM>::LDA_M, STAGES = Cfg<BM, DEEP>::STAGES;
   extern __shared__ __align__(16) double smem[];
   double *As = smem, *Bs = smem + STAGES * A_STAGE;

@@ -6,6 +6,7 @@
 // 16-byte pieces of the weights with sixteen of them in flight, and the block that finishes a group of hypercolumns last
 // adds up the ranges and takes the softmax.
 #include "sbb_kernels.cuh"
+#include "sbb_launch.cuh"
 #include "sbb_math.cuh"
 
 namespace sbb {
@@ -26,6 +27,7 @@ template <typename T, int V, int R>
 __global__ void __launch_bounds__(kFewThreads)
     few_forward_kernel(const T *__restrict__ x, const T *__restrict__ W, const T *__restrict__ bias, T *__restrict__ out,
                        T *partial, int *tickets, int N, int M, int Mc, int cols, int lanes, int range) {
+  after_previous();
   __shared__ T s_sum[kFewThreads * V * R];
   __shared__ int s_last;
   T *s_support = s_sum;   // (the sums have been read by then)
@@ -172,7 +174,7 @@ cudaError_t launch_few_forward(const T *x, const T *W, const T *bias, T *out, lo
   const dim3 grid((unsigned)p.chunks, (unsigned)p.ranges);
   constexpr int V = 16 / (int)sizeof(T);
 #define SBB_FEW(VV, R) \
-  few_forward_kernel<T, VV, R><<<grid, kFewThreads, 0, st>>>(x, W, bias, out, partial, tickets, (int)N, (int)(H * Mc), (int)Mc, \
+  launch_next(few_forward_kernel<T, VV, R>, grid, kFewThreads, 0, st, x, W, bias, out, partial, tickets, (int)N, (int)(H * Mc), (int)Mc, \
                                                             p.cols, p.lanes, p.range)
 #define SBB_FEW_R(R) \
   if (p.vec == 1) SBB_FEW(1, R); \

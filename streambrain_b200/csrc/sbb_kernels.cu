@@ -12,6 +12,7 @@
 // transposed on its way into shared memory.
 #include "sbb_kernels.cuh"
 #include "sbb_f64_mma.cuh"
+#include "sbb_launch.cuh"
 #include "sbb_math.cuh"
 
 #include <atomic>
@@ -149,6 +150,7 @@ template <bool A_KMAJOR, int V, class Epilogue>
 __global__ void __launch_bounds__(Tile::THREADS, 2)
     contraction_kernel(const float *__restrict__ A, long lda, const float *__restrict__ Bm, long ldb, long Mdim, long Ndim,
                        int K, int kper, bool cols_fastest, Epilogue ep) {
+  after_previous();
   using S = TileShape<A_KMAJOR>;
   using L = Slab<float, S, V>;
   extern __shared__ __align__(16) float tile_smem[];
@@ -247,6 +249,7 @@ template <bool A_KMAJOR, class Epilogue>
 __global__ void __launch_bounds__(SmallShape<A_KMAJOR>::THREADS)
     small_contraction_kernel(const float *__restrict__ A, long lda, const float *__restrict__ Bm, long ldb, long Mdim,
                              long Ndim, int K, int kper, Epilogue ep) {
+  after_previous();
   using S = SmallShape<A_KMAJOR>;
   using L = Slab<float, S, 1>;
   extern __shared__ __align__(16) float small_smem[];
@@ -683,7 +686,7 @@ static cudaError_t launch_f64_mma_tiles(const double *A, long lda, const double 
   if (grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
   const int slabs = (K + F::BK - 1) / F::BK;
   const int kper = (slabs + splits - 1) / splits * F::BK;
-  kernel<<<grid, C::THREADS, C::SMEM_BYTES, st>>>(A, lda, Bm, ldb, Mdim, Ndim, K, kper, cols_fastest, ep);
+  launch_next(kernel, grid, C::THREADS, C::SMEM_BYTES, st, A, lda, Bm, ldb, Mdim, Ndim, K, kper, cols_fastest, ep);
   return launched();
 }
 
@@ -721,7 +724,7 @@ static cudaError_t launch_small_contraction(const float *A, long lda, const floa
   if (e != cudaSuccess) return e;
   const dim3 grid((unsigned)((Ndim + S::BN - 1) / S::BN), (unsigned)((Mdim + S::BM - 1) / S::BM), (unsigned)splits);
   if (grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
-  kernel<<<grid, S::THREADS, S::SMEM_BYTES, st>>>(A, lda, Bm, ldb, Mdim, Ndim, K, kper, ep);
+  launch_next(kernel, grid, S::THREADS, S::SMEM_BYTES, st, A, lda, Bm, ldb, Mdim, Ndim, K, kper, ep);
   return launched();
 }
 
@@ -736,7 +739,7 @@ static cudaError_t launch_tiles(const float *A, long lda, const float *Bm, long 
   if (cols_fastest && mt > 65535u) cols_fastest = false;
   const dim3 grid(cols_fastest ? nt : mt, cols_fastest ? mt : nt, (unsigned)splits);
   if (grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
-  kernel<<<grid, Tile::THREADS, Tile::SMEM_BYTES, st>>>(A, lda, Bm, ldb, Mdim, Ndim, K, kper, cols_fastest, ep);
+  launch_next(kernel, grid, Tile::THREADS, Tile::SMEM_BYTES, st, A, lda, Bm, ldb, Mdim, Ndim, K, kper, cols_fastest, ep);
   return launched();
 }
 
@@ -844,6 +847,7 @@ template <typename T, int CACHE>
 __global__ void __launch_bounds__(256)
     reduce_bias_softmax_kernel(const T *partial, int splits, long slice, const T *__restrict__ bias, T *out,
                                long groups, long H, long Mc, int width) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   const int sub = lane % width;
   const long warp = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -914,6 +918,7 @@ template <typename T, int NC, bool SPLIT>
 __global__ void __launch_bounds__(256)
     softmax_warp_kernel(const T *partial, int splits, long slice, const T *__restrict__ bias, T *out, long groups,
                         int H, int Mc) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   const long g = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (g >= groups) return;   // whole warps leave together
@@ -986,6 +991,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
     reduce_bias_kernel(const T *partial, int splits, long slice, const T *__restrict__ bias, T *out, long total,
                        long M) {
+  after_previous();
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   T s = partial[idx];
@@ -1002,7 +1008,7 @@ cudaError_t launch_reduce_bias_softmax(const T *partial, int splits, const T *bi
   if (total == 0) return cudaSuccess;
   if (!softmax) {
     if (splits == 1 && bias == nullptr && partial == out) return cudaSuccess;
-    reduce_bias_kernel<T><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(partial, splits, total, bias, out, total, M);
+    launch_next(reduce_bias_kernel<T>, (unsigned)((total + 255) / 256), 256, 0, st, partial, splits, total, bias, out, total, M);
     return launched();
   }
   int width = 32;
@@ -1017,10 +1023,10 @@ cudaError_t launch_reduce_bias_softmax(const T *partial, int splits, const T *bi
 #define SBB_SOFTMAX_WARP(NC)                                                                                      \
   do {                                                                                                            \
     if (splits > 1)                                                                                               \
-      softmax_warp_kernel<T, NC, true><<<(unsigned)((groups + 7) / 8), 256, 0, st>>>(partial, splits, total, bias, out, \
+      launch_next(softmax_warp_kernel<T, NC, true>, (unsigned)((groups + 7) / 8), 256, 0, st, partial, splits, total, bias, out, \
                                                                                     groups, (int)H, (int)Mc);    \
     else                                                                                                          \
-      softmax_warp_kernel<T, NC, false><<<(unsigned)((groups + 7) / 8), 256, 0, st>>>(partial, splits, total, bias, out, \
+      launch_next(softmax_warp_kernel<T, NC, false>, (unsigned)((groups + 7) / 8), 256, 0, st, partial, splits, total, bias, out, \
                                                                                      groups, (int)H, (int)Mc);   \
   } while (0)
     if (per_lane <= 4) SBB_SOFTMAX_WARP(4);
@@ -1031,15 +1037,15 @@ cudaError_t launch_reduce_bias_softmax(const T *partial, int splits, const T *bi
     return launched();
   }
   if (per_lane <= 4)
-    reduce_bias_softmax_kernel<T, 4><<<blocks, 256, 0, st>>>(partial, splits, total, bias, out, groups, H, Mc, width);
+    launch_next(reduce_bias_softmax_kernel<T, 4>, blocks, 256, 0, st, partial, splits, total, bias, out, groups, H, Mc, width);
   else if (per_lane <= 8)
-    reduce_bias_softmax_kernel<T, 8><<<blocks, 256, 0, st>>>(partial, splits, total, bias, out, groups, H, Mc, width);
+    launch_next(reduce_bias_softmax_kernel<T, 8>, blocks, 256, 0, st, partial, splits, total, bias, out, groups, H, Mc, width);
   else if (per_lane <= 12)
-    reduce_bias_softmax_kernel<T, 12><<<blocks, 256, 0, st>>>(partial, splits, total, bias, out, groups, H, Mc, width);
+    launch_next(reduce_bias_softmax_kernel<T, 12>, blocks, 256, 0, st, partial, splits, total, bias, out, groups, H, Mc, width);
   else if (per_lane <= 16)
-    reduce_bias_softmax_kernel<T, 16><<<blocks, 256, 0, st>>>(partial, splits, total, bias, out, groups, H, Mc, width);
+    launch_next(reduce_bias_softmax_kernel<T, 16>, blocks, 256, 0, st, partial, splits, total, bias, out, groups, H, Mc, width);
   else
-    reduce_bias_softmax_kernel<T, 0><<<blocks, 256, 0, st>>>(partial, splits, total, bias, out, groups, H, Mc, width);
+    launch_next(reduce_bias_softmax_kernel<T, 0>, blocks, 256, 0, st, partial, splits, total, bias, out, groups, H, Mc, width);
   return launched();
 }
 template cudaError_t launch_reduce_bias_softmax<float>(const float *, int, const float *, float *, long, long, long,
@@ -1054,6 +1060,7 @@ template cudaError_t launch_reduce_bias_softmax<double>(const double *, int, con
 template <typename T>
 __global__ void __launch_bounds__(256)
     colsum_kernel(const T *__restrict__ a, long B, long cols, T *sums, T *lo) {
+  after_previous();
   __shared__ T part[8][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const long col = (long)blockIdx.x * 32 + tx;
@@ -1090,7 +1097,7 @@ __global__ void __launch_bounds__(256)
 template <typename T>
 cudaError_t launch_colsum(const T *a, long B, long cols, T *sums, cudaStream_t st, T *lo) {
   if (cols == 0) return cudaSuccess;
-  colsum_kernel<T><<<(unsigned)((cols + 31) / 32), 256, 0, st>>>(a, B, cols, sums, lo);
+  launch_next(colsum_kernel<T>, (unsigned)((cols + 31) / 32), 256, 0, st, a, B, cols, sums, lo);
   return launched();
 }
 template cudaError_t launch_colsum<float>(const float *, long, long, float *, cudaStream_t, float *);
@@ -1104,6 +1111,7 @@ template cudaError_t launch_colsum<double>(const double *, long, long, double *,
 template <typename T>
 __global__ void __launch_bounds__(256)
     column_vectors_kernel(ColumnVectors<T> x, ColumnVectors<T> y, long B, TraceParams<T> p, BiasParams<T> nb, unsigned x_blocks) {
+  after_previous();
   __shared__ T part[8][33];
   const bool is_x = blockIdx.x < x_blocks;
   const ColumnVectors<T> &o = is_x ? x : y;
@@ -1146,7 +1154,7 @@ cudaError_t launch_column_vectors(const ColumnVectors<T> &x, const ColumnVectors
                                   BiasParams<T> bias, cudaStream_t st) {
   const unsigned xb = (unsigned)((x.cols + 31) / 32), yb = (unsigned)((y.cols + 31) / 32);
   if (xb + yb == 0) return cudaSuccess;
-  column_vectors_kernel<T><<<xb + yb, 256, 0, st>>>(x, y, B, p, bias, xb);
+  launch_next(column_vectors_kernel<T>, xb + yb, 256, 0, st, x, y, B, p, bias, xb);
   return launched();
 }
 template cudaError_t launch_column_vectors<float>(const ColumnVectors<float> &, const ColumnVectors<float> &, long,
@@ -1410,6 +1418,7 @@ template cudaError_t launch_apply_mask<double>(double *, const uint8_t *, long, 
 template <typename T>
 __global__ void count_correct_kernel(const T *__restrict__ pred, const T *__restrict__ labels, long rows, long classes,
                                      unsigned long long *count) {
+  after_previous();
   const long r = (long)blockIdx.x * blockDim.x + threadIdx.x;
   bool hit = false;
   if (r < rows) {
@@ -1429,7 +1438,7 @@ template <typename T>
 cudaError_t launch_count_correct(const T *pred, const T *labels, long rows, long classes, unsigned long long *count,
                                  cudaStream_t st) {
   if (rows == 0) return cudaSuccess;
-  count_correct_kernel<T><<<(unsigned)((rows + 255) / 256), 256, 0, st>>>(pred, labels, rows, classes, count);
+  launch_next(count_correct_kernel<T>, (unsigned)((rows + 255) / 256), 256, 0, st, pred, labels, rows, classes, count);
   return launched();
 }
 template cudaError_t launch_count_correct<float>(const float *, const float *, long, long, unsigned long long *,
@@ -1446,6 +1455,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
     gather_rows_kernel(const T *__restrict__ src, const long *__restrict__ order, long first, long rows, long cols,
                        T *__restrict__ dst, int vec16) {
+  after_previous();
   const long warp = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
@@ -1470,7 +1480,7 @@ cudaError_t launch_gather_rows(const T *src, const long *order, long first, long
   const int vec16 = (cols * (long)sizeof(T)) % 16 == 0 && aligned16(src) && aligned16(dst);
   const long blocks = (rows + 7) / 8;   // eight warps per block, one row per warp and pass
   const int cap = sm_count() * 8;
-  gather_rows_kernel<T><<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(src, order, first, rows, cols, dst,
+  launch_next(gather_rows_kernel<T>, (unsigned)(blocks < cap ? blocks : cap), 256, 0, st, src, order, first, rows, cols, dst,
                                                                                  vec16);
   return launched();
 }

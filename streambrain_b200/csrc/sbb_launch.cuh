@@ -1,0 +1,32 @@
+// Launches that begin while the kernel before them in the stream drains (programmatic stream serialization).
+#pragma once
+#include <cuda_runtime.h>
+
+namespace sbb {
+
+// First statement of a kernel that launch_next starts, ahead of every access to global memory: waits until the kernels
+// before it in the stream have ended and what they wrote is visible, then lets the next kernel's blocks take the places that
+// this kernel's leave.  Every kernel of a chain waits, so each has all its predecessors behind it.
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// A training step is five kernels of 3 to 30 us; starting each only when the one before had ended cost 1.1 to 2.5 us a
+// launch.
+template <class... P, class... A>
+inline cudaError_t launch_next(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
+}
+
+}  // namespace sbb

@@ -1,6 +1,7 @@
 // Structural plasticity: the mutual-information score of every connection of one hypercolumn, the swaps of silent
 // and active connections it decides, and the weights of the rows a swap touched.
 #include "sbb_kernels.cuh"
+#include "sbb_launch.cuh"
 #include "sbb_math.cuh"
 
 #include <math.h>
@@ -524,6 +525,7 @@ __device__ __forceinline__ void replay_swaps(const uint32_t (&row)[NS], int (&cl
 // already).
 template <typename T, bool SCORE>
 __global__ void __launch_bounds__(kMaskThreads, sizeof(T) == 4 ? 2 : 1) mask_update_kernel(const MaskArgs<T> a) {
+  after_previous();
   __shared__ TopShared<T> sh;
   __shared__ unsigned long long s_best[2][kGroups];
   __shared__ uint32_t low_row[2][64], changed[6 * 32];
@@ -872,7 +874,7 @@ static cudaError_t launch_mask(uint8_t *wmask, const T *weights, const T *Ci, co
     a.block_rows = SCORE ? kMaskThreads / a.width : kMaskThreads / 8;
     while ((1 << a.rows_log2) < a.block_rows) a.rows_log2 += 1;
     const long rows = a.block_rows;
-    mask_update_kernel<T, SCORE><<<(unsigned)((N + rows - 1) / rows), kMaskThreads, 0, st>>>(a);
+    launch_next(mask_update_kernel<T, SCORE>, (unsigned)((N + rows - 1) / rows), kMaskThreads, 0, st, a);
     return launched();
   }
   if constexpr (SCORE) {

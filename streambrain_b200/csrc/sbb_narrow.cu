@@ -6,6 +6,7 @@
 // own: the 3000 -> 10 layer at batch 128 took 20.4 + 5.7 us for the forward pass and 31.0 + 2 x 2.6 us for the train
 // step.  Here every thread has all its loads of the inputs in flight at once.
 #include "sbb_kernels.cuh"
+#include "sbb_launch.cuh"
 #include "sbb_math.cuh"
 
 namespace sbb {
@@ -27,6 +28,7 @@ template <typename T, int MP, int R, int WARPS>
 __global__ void __launch_bounds__(256)
     narrow_forward_kernel(const T *__restrict__ x, const T *__restrict__ W, const T *__restrict__ bias, T *__restrict__ out,
                           long B, int N, int M, int Mc) {
+  after_previous();
   constexpr int SETS = 8 / WARPS;   // groups of R samples per block
   __shared__ T part[8][R][MP];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -104,6 +106,7 @@ template <typename T, int MP>
 __global__ void __launch_bounds__(256)
     narrow_train_kernel(const T *__restrict__ x, const T *__restrict__ y, long B, int N, int M, int H, int Mc, T *Ci, T *Cj,
                         T *Cij, T *W, const uint8_t *__restrict__ wmask, TraceParams<T> p, BiasParams<T> nb, int *ticket) {
+  after_previous();
   constexpr int STAGE = NarrowTrain<T, MP>::STAGE, CH = NarrowTrain<T, MP>::CH;
   constexpr int NCH = MP / CH, E = 32 * CH / 256;   // outputs per thread: NCH chunks of E
   __shared__ __align__(16) T ys[STAGE][MP];
@@ -234,9 +237,9 @@ cudaError_t forward_mp(const T *x, const T *W, const T *bias, T *out, long B, lo
 #define SBB_NARROW_FWD(R)                                                                                              \
   do {                                                                                                                 \
     if (N <= 512) /* not enough inputs to share among the warps of a block */                                          \
-      narrow_forward_kernel<T, MP, R, 1><<<(unsigned)((B + 8 * R - 1) / (8 * R)), 256, 0, st>>>(x, W, bias, out, B, (int)N, (int)M, (int)Mc); \
+      launch_next(narrow_forward_kernel<T, MP, R, 1>, (unsigned)((B + 8 * R - 1) / (8 * R)), 256, 0, st, x, W, bias, out, B, (int)N, (int)M, (int)Mc); \
     else                                                                                                               \
-      narrow_forward_kernel<T, MP, R, 8><<<(unsigned)((B + R - 1) / R), 256, 0, st>>>(x, W, bias, out, B, (int)N, (int)M, (int)Mc); \
+      launch_next(narrow_forward_kernel<T, MP, R, 8>, (unsigned)((B + R - 1) / R), 256, 0, st, x, W, bias, out, B, (int)N, (int)M, (int)Mc); \
   } while (0)
   if (per <= 1 || RMAX == 1) SBB_NARROW_FWD(1);
   else if (per <= 2 || RMAX == 2) SBB_NARROW_FWD((RMAX < 2 ? RMAX : 2));
@@ -273,7 +276,7 @@ cudaError_t launch_narrow_train(const T *x, const T *y, long B, long N, long M, 
                                 const uint8_t *wmask, TraceParams<T> p, BiasParams<T> nb, int *ticket, cudaStream_t st) {
   const unsigned blocks = (unsigned)((N + 31) / 32);
 #define SBB_NARROW_TRAIN(MP)                                                                                            \
-  narrow_train_kernel<T, MP><<<blocks, 256, 0, st>>>(x, y, B, (int)N, (int)M, (int)H, (int)Mc, Ci, Cj, Cij, W, wmask, p, nb, ticket)
+  launch_next(narrow_train_kernel<T, MP>, blocks, 256, 0, st, x, y, B, (int)N, (int)M, (int)H, (int)Mc, Ci, Cj, Cij, W, wmask, p, nb, ticket)
   if (M <= 8) SBB_NARROW_TRAIN(8);
   else if (M <= 16) SBB_NARROW_TRAIN(16);
   else SBB_NARROW_TRAIN(32);

@@ -40,6 +40,7 @@
 #include <cstdlib>
 #include <mutex>
 
+#include "sbb_launch.cuh"
 #include "sbb_math.cuh"
 
 namespace sbb {
@@ -191,6 +192,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  after_previous();   // (barriers and tensor memory are set up while the kernel before ends)
 
   // PAIR: the work items are pairs of row tiles, and the two CTAs of a cluster walk them together
   const int m_units = PAIR ? (wk.m_tiles + 1) / 2 : wk.m_tiles;
@@ -793,9 +795,8 @@ cudaError_t launch_tc(const TcMaps &tm, const TcWork &wk, const TcEpilogue &ep, 
   int sms = g_sm_count_tc[dev] - (leave_reserved_sms ? tc_get_reserved_sms() : 0);
   if (sms < 1) sms = 1;
   const unsigned grid = (unsigned)(total < sms ? total : sms);
-  kernel<<<grid, kThreads, SM::TOTAL, st>>>(tm.a, tm.b, tm.a3, tm.b3, tm.c, tm.alo, tm.blo, tm.a3lo, tm.b3lo, wk, ep,
-                                            status);
-  return cudaGetLastError();
+  return launch_next(kernel, grid, kThreads, SM::TOTAL, st, tm.a, tm.b, tm.a3, tm.b3, tm.c, tm.alo, tm.blo, tm.a3lo, tm.b3lo,
+                     wk, ep, status);
 }
 
 // SBB_TC_PAIR=0 keeps one CTA per tile (read once).
@@ -824,7 +825,7 @@ cudaError_t launch_tc_pair(const TcMaps &tm, const TcWork &wk, const TcEpilogue 
   const long pairs = (long)((wk.m_tiles + 1) / 2) * wk.n_tiles * wk.splits;
   if (pairs <= 0) return cudaSuccess;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
@@ -845,6 +846,9 @@ cudaError_t launch_tc_pair(const TcMaps &tm, const TcWork &wk, const TcEpilogue 
   long clusters = max_clusters[dev] < g_sm_count_tc[dev] / 2 ? max_clusters[dev] : g_sm_count_tc[dev] / 2;
   if (clusters > pairs) clusters = pairs;
   cfg.gridDim = dim3((unsigned)(2 * clusters), 1, 1);
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // as launch_next
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kernel, tm.a, tm.b, tm.a3, tm.b3, tm.c, tm.alo, tm.blo, tm.a3lo, tm.b3lo, wk, ep,
                             status);
 }

@@ -22,6 +22,7 @@
 
 #include <atomic>
 
+#include "sbb_launch.cuh"
 #include "sbb_math.cuh"
 
 namespace sbb {
@@ -117,6 +118,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   cluster_sync_all();   // the peer's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  after_previous();   // (barriers and tensor memory are set up while the kernel before ends)
 
   // The clusters walk the tiles side by side, columns fastest (rows fastest where the columns are the longer side): at any
   // time they share the operands of a few row tiles.
@@ -523,7 +525,7 @@ cudaError_t launch_trace_update_tc(const float *x, const float *y, long B, long 
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
@@ -544,6 +546,9 @@ cudaError_t launch_trace_update_tc(const float *x, const float *y, long B, long 
   const long pairs = (long)g.m_units * g.n_tiles;
   const long clusters = pairs < max_clusters[dev].load() ? pairs : max_clusters[dev].load();
   cfg.gridDim = dim3((unsigned)(2 * clusters), 1, 1);
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // as launch_next
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, trace_kernel, ma, mb, ma3, mb3, mc, g, host.status);
   if (e == cudaSuccess) count_launches(1);
   return e;
