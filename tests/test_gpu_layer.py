@@ -647,3 +647,29 @@ def test_forward_of_few_samples_vs_oracle(port_kernels, tag, dtype, B, N, H, Mc)
     want = ref.compute_activation(x)
     for _ in range(2):   # the tickets are zero again after a launch
         assert rel_inf(dev.compute_activation(x), want) < TOL[np.dtype(dtype)]
+
+
+@pytest.mark.parametrize("tag,dtype", DTYPES)
+@pytest.mark.parametrize("B,N,H,Mc", [(5, 1, 1, 33), (33, 31, 5, 13), (97, 65, 7, 19), (128, 129, 3, 43), (131, 1601, 8, 63),
+                                      (257, 2051, 11, 127), (1025, 517, 27, 39), (64, 1600, 47, 64), (320, 1602, 19, 33)])
+def test_contractions_of_odd_rows_vs_oracle(port_kernels, tag, dtype, B, N, H, Mc):
+    """Rows of any length: small and large output tiles and their edges, one slab and many, one k-split and several, 8-byte
+    and 16-byte copies of float64, one deep block per SM and several."""
+    import streambrain_b200 as B200
+    init = (0.5, 1 / Mc, 0.5 / Mc)
+    np.random.seed(4)
+    dev = B200.StructuralPlasticityLayer(N, H, Mc, 0.1, -100.0, 0.05, 0.02, 0.5, 16, init, dtype=dtype)
+    ref = oracle.OracleLayer(port_kernels, "plastic", N, H, Mc, 0.1, init, dtype, khalf=-100.0, pmin=0.05, taubdt=0.02, density=0.5)
+    rs = np.random.RandomState(B + N)
+    dev.weights = (0.05 * rs.randn(N, H * Mc)).astype(dtype)
+    for name in ("weights", "bias", "wmask"):
+        setattr(ref, name, getattr(dev, name))
+    x = rs.rand(B, N).astype(dtype)
+    tol = TOL[np.dtype(dtype)]
+    assert rel_inf(dev.compute_activation(x), ref.compute_activation(x)) < 10 * tol
+    y = rs.dirichlet(np.ones(Mc), size=(B, H)).reshape(B, H * Mc).astype(dtype)
+    ref.train_step(x, y, None)
+    dev.train_step(x, y, None)
+    for name in ("Ci", "Cj", "Cij", "bias"):
+        assert rel_inf(getattr(dev, name), getattr(ref, name)) < tol, name
+    assert weight_err(dev.weights, ref.weights) < 10 * tol
