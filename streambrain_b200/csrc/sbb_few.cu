@@ -160,7 +160,7 @@ template <typename T>
 bool few_samples(const T *W, long B, long N, long H, long Mc, size_t *scratch_elems) {
   FewPlan p;
   if (!few_plan<T>(W, B, N, H, Mc, p)) return false;
-  *scratch_elems = (size_t)p.ranges * kFewSamples * (size_t)(H * Mc);
+  *scratch_elems = (size_t)p.ranges * (size_t)B * (size_t)(H * Mc);
   return true;
 }
 template bool few_samples<float>(const float *, long, long, long, long, size_t *);

@@ -13,7 +13,7 @@ __device__ __forceinline__ void after_previous() {
 }
 
 // A training step is five kernels of 3 to 30 us; starting each only when the one before had ended cost 1.1 to 2.5 us a
-// launch.
+// launch.  1001 x 481 at batch 97: 49 -> 40 us a step; 1568 x 3000 at 128: 74 -> 68; a fit of 5000 samples: 6.7 -> 5.4 ms.
 template <class... P, class... A>
 inline cudaError_t launch_next(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchAttribute attr[1];
