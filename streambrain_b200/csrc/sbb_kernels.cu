@@ -779,17 +779,18 @@ static int sm_count() {
 
 // k-splits of the forward product.  float32: output tiles of 128 x 128 until two CTAs per SM are busy, at least eight slabs
 // each.  float64 (128 x 64 tiles, slabs of 16): the split whose fullest SM has the least to do, in slabs, counting each
-// partial sum's way to memory and back (16 bytes per output at about 4 TB/s against about 1.05 us per slab of a tile); 47
+// partial sum's way to memory and back (16 bytes per output at about 4 TB/s against about 1.05 us per slab of a tile, and a
+// fifth of that for its turn in the sum); 47
 // tiles of 98 slabs: three splits on 141 SMs, 33 slabs each, half of the partial sums that two CTAs per SM need for 34.
 template <typename T>
 int forward_splits(long B, long N, long M) {
   const long sms = sm_count();
   if (sizeof(T) == 8) {
     const long tiles = ((B + 127) / 128) * ((M + f64mma::BN - 1) / f64mma::BN), slabs = (N + f64mma::BK - 1) / f64mma::BK;
-    const double per_split = (double)B * M / 262144.0;
+    const double per_split = (double)B * M / 262144.0 + 0.2;
     int best = 1;
     double least = 0;
-    for (long s = 1; s <= 16 && (s == 1 || slabs / s >= 4); ++s) {
+    for (long s = 1; s <= 64 && (s == 1 || slabs / s >= 4); ++s) {
       const double cost = (double)((tiles * s + sms - 1) / sms) * ((slabs + s - 1) / s) + per_split * s;
       if (s == 1 || cost < least) least = cost, best = (int)s;
     }
@@ -865,6 +866,7 @@ __global__ void __launch_bounds__(256)
       T s = -INFINITY;
       if (live && j < Mc) {
         s = partial[base + j];
+#pragma unroll 8
         for (int z = 1; z < splits; ++z) s += partial[(long)z * slice + base + j];
         if (bias) s += bias[col0 + j];
       }
@@ -937,7 +939,8 @@ __global__ void __launch_bounds__(256)
     if (!SPLIT && bs && e * 32 < left) v[e] += bs[e * 32];
   }
   if (SPLIT) {
-#pragma unroll 2
+    constexpr int AHEAD = NC <= 4 ? 8 : NC <= 8 ? 4 : 2;
+#pragma unroll AHEAD
     for (int z = 1; z < splits; ++z) {
       const T *sz = src + (long)z * slice;
       T d[NC];
