@@ -5,8 +5,8 @@
 //
 // CTA tile 128 x 64 (eight warps, two CTAs per SM) or 64 x 64 (four warps, three CTAs per SM: for
 // launches whose 128-row tiles would leave most of a last wave of CTAs empty), k-slabs of 16 in a
-// three-stage cp.async pipeline, warp tile 32 x 32 (4 x 4 instruction tiles).  A launch of no more
-// 128-row tiles than SMs has one CTA per SM and takes six stages instead.  The copies are 16 bytes
+// three-stage cp.async pipeline, warp tile 32 x 32 (4 x 4 instruction tiles).  A forward product of no
+// more tiles than SMs has one CTA per SM and takes six stages instead.  The copies are 16 bytes
 // wide where rows start on 16-byte boundaries and one element otherwise.  Shared-memory rows
 // are padded so that a half-warp's fragment loads (four rows of four consecutive doubles) fall into
 // 16 different bank pairs.

@@ -691,7 +691,7 @@ static cudaError_t launch_f64_mma_tiles(const double *A, long lda, const double 
 }
 
 // Row tiles of 128 unless the fullest SM has fewer rows to do in tiles of 64: 1568 x 3000 outputs are 611 tiles of 128
-// rows, five on some SMs, or 1175 tiles of 64 rows, at most eight.  The forward product's 128-row tiles on as many SMs
+// rows, five on some SMs, or 1175 tiles of 64 rows, at most eight.  The forward product's tiles on as many SMs
 // take the deep pipeline (the trace step's few-tile launches have one short chain of slabs, which it does not help).
 template <bool A_KMAJOR, int V, class Pairs>
 static cudaError_t launch_f64_mma(const double *A, long lda, const double *Bm, long ldb, long Mdim, long Ndim, int K,
@@ -700,8 +700,13 @@ static cudaError_t launch_f64_mma(const double *A, long lda, const double *Bm, l
   const long nt = (Ndim + F::BN - 1) / F::BN, sms = sm_count();
   auto ctas = [&](long bm) { return ((Mdim + bm - 1) / bm) * nt * splits; };
   auto rows = [&](long bm) { return (ctas(bm) + sms - 1) / sms * bm; };
-  if (rows(64) < rows(128))
+  if (rows(64) < rows(128)) {
+    if constexpr (A_KMAJOR) {
+      if (ctas(64) <= sms)
+        return launch_f64_mma_tiles<A_KMAJOR, 64, true, V>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, ep, st);
+    }
     return launch_f64_mma_tiles<A_KMAJOR, 64, false, V>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, ep, st);
+  }
   if constexpr (A_KMAJOR) {
     if (ctas(128) <= sms)
       return launch_f64_mma_tiles<A_KMAJOR, 128, true, V>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, ep, st);
@@ -788,10 +793,11 @@ int forward_splits(long B, long N, long M) {
   if (sizeof(T) == 8) {
     const long tiles = ((B + 127) / 128) * ((M + f64mma::BN - 1) / f64mma::BN), slabs = (N + f64mma::BK - 1) / f64mma::BK;
     const double per_split = (double)B * M / 262144.0 + 0.2;
+    const long slots = B <= 64 ? 2 * sms : sms;   // batches of one 64-row tile: two of its four-warp CTAs keep an SM busy
     int best = 1;
     double least = 0;
     for (long s = 1; s <= 64 && (s == 1 || slabs / s >= 4); ++s) {
-      const double cost = (double)((tiles * s + sms - 1) / sms) * ((slabs + s - 1) / s) + per_split * s;
+      const double cost = (double)((tiles * s + slots - 1) / slots) * ((slabs + s - 1) / s) + per_split * s;
       if (s == 1 || cost < least) least = cost, best = (int)s;
     }
     return best;
