@@ -784,15 +784,15 @@ static int sm_count() {
 
 // k-splits of the forward product.  float32: output tiles of 128 x 128 until two CTAs per SM are busy, at least eight slabs
 // each.  float64 (128 x 64 tiles, slabs of 16): the split whose fullest SM has the least to do, in slabs, counting each
-// partial sum's way to memory and back (16 bytes per output at about 4 TB/s against about 1.05 us per slab of a tile, and a
-// fifth of that for its turn in the sum); 47
+// partial sum's way to memory and back (16 bytes per output at about 4 TB/s against about 1.05 us per slab of a tile, and
+// two fifths of that for its turn in the sum); 47
 // tiles of 98 slabs: three splits on 141 SMs, 33 slabs each, half of the partial sums that two CTAs per SM need for 34.
 template <typename T>
 int forward_splits(long B, long N, long M) {
   const long sms = sm_count();
   if (sizeof(T) == 8) {
     const long tiles = ((B + 127) / 128) * ((M + f64mma::BN - 1) / f64mma::BN), slabs = (N + f64mma::BK - 1) / f64mma::BK;
-    const double per_split = (double)B * M / 262144.0 + 0.2;
+    const double per_split = (double)B * M / 262144.0 + 0.4;
     const long slots = B <= 64 ? 2 * sms : sms;   // batches of one 64-row tile: two of its four-warp CTAs keep an SM busy
     int best = 1;
     double least = 0;
@@ -945,15 +945,19 @@ __global__ void __launch_bounds__(256)
     if (!SPLIT && bs && e * 32 < left) v[e] += bs[e * 32];
   }
   if (SPLIT) {
-    constexpr int AHEAD = NC <= 4 ? 8 : NC <= 8 ? 4 : 2;
-#pragma unroll AHEAD
-    for (int z = 1; z < splits; ++z) {
+    constexpr int AHEAD = NC <= 4 ? 8 : NC <= 12 ? 4 : 2;
+    T d[AHEAD][NC];
+#pragma unroll 1
+    for (int z = 1; z < splits; z += AHEAD) {
       const T *sz = src + (long)z * slice;
-      T d[NC];
 #pragma unroll
-      for (int e = 0; e < NC; ++e) d[e] = e * 32 < left ? sz[e * 32] : (T)0;
+      for (int a = 0; a < AHEAD; ++a)
 #pragma unroll
-      for (int e = 0; e < NC; ++e) v[e] += d[e];
+        for (int e = 0; e < NC; ++e) d[a][e] = z + a < splits && e * 32 < left ? sz[a * slice + e * 32] : (T)0;
+#pragma unroll
+      for (int a = 0; a < AHEAD; ++a)
+#pragma unroll
+        for (int e = 0; e < NC; ++e) v[e] += d[a][e];
     }
   }
 #pragma unroll
