@@ -980,8 +980,8 @@ __global__ void __launch_bounds__(256)
   mx = subwarp_max(mx, 32);
   T sum = (T)0;
   if constexpr (sizeof(T) == 8) {
-    // one copy of the float64 exponential (the entries rotate through slot 0) and one division: unrolled, a kernel of a
-    // few microseconds spends most of them fetching instructions
+    // one copy of the float64 exponential (the entries rotate through slot 0): unrolled, a kernel of a few microseconds
+    // spends most of them fetching instructions
 #pragma unroll 1
     for (int e = 0; e < NC; ++e) {
       const T x = e * 32 < left ? sbb_exp(v[0] - mx) : (T)0;
@@ -998,13 +998,26 @@ __global__ void __launch_bounds__(256)
     }
   }
   sum = subwarp_sum(sum, 32);
+  const DivideBy<T> by(sum);
   if constexpr (sizeof(T) == 8) {
-    const T scale = (T)1 / sum;
+    // (128 samples, 784 -> 15 x 200: the forward pass takes 27.5 us, and 28.8 with a multiplication by 1 / sum, which rounds
+    // once more than the division)
+    bool covered = true;
+#pragma unroll
+    for (int e = 0; e < NC; ++e) covered = covered && by.covers(v[e]);
+    if (!covered) {   // rare: one copy of the division, as of the exponential
+#pragma unroll 1
+      for (int e = 0; e < NC; ++e) {
+        if (e * 32 < left) dst[e * 32] = v[0] / sum;
+#pragma unroll
+        for (int q = 0; q + 1 < NC; ++q) v[q] = v[q + 1];
+      }
+      return;
+    }
 #pragma unroll
     for (int e = 0; e < NC; ++e)
-      if (e * 32 < left) dst[e * 32] = v[e] * scale;
-  } else {   // (a NaN sum: the method's NaN is the division's)
-    const DivideBy by(sum);
+      if (e * 32 < left) dst[e * 32] = by.quotient(v[e]);
+  } else {
 #pragma unroll
     for (int e = 0; e < NC; ++e)
       if (e * 32 < left) dst[e * 32] = by(v[e]);

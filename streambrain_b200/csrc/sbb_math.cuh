@@ -30,21 +30,30 @@ __device__ __forceinline__ T log_ratio(T cij, T ci, T cj, T cthr4) {
   return sbb_log(num / (ci * cj));
 }
 
-// v / d for many v in [0, 1] and one d >= 1, correctly rounded, from the rounded reciprocal of d: Markstein's method (IBM
-// J. Res. Dev. 34, 1990): with y = RN(1/d), q = RN(v y) and the exact remainder r = v - q d, RN(q + r y) is RN(v / d)
-// unless d's significand is all ones; the remainder is exact for v >= 2^-100.  Three instructions for the division's dozen.
+// v / d for many v in [0, 1] and one d in [1, 2^20], correctly rounded, from the rounded reciprocal of d: Markstein's method
+// (IBM J. Res. Dev. 34, 1990): with y = RN(1/d), q = RN(v y) and the remainder r = v - q d, RN(q + r y) is RN(v / d) unless
+// d's significand is all ones; nothing underflows on the way for v >= MIN.  Three instructions for the division's dozen or
+// more.
+template <typename T>
 struct DivideBy {
-  float d, y;
+  static constexpr T MIN = sizeof(T) == 4 ? (T)0x1p-100 : (T)0x1p-900;
+  T d, y;
   bool plain;   // the one significand the method does not cover
-  __device__ __forceinline__ explicit DivideBy(float divisor) : d(divisor) {
-    y = __frcp_rn(divisor);
-    plain = (__float_as_uint(divisor) & 0x7FFFFFu) == 0x7FFFFFu;
+  __device__ __forceinline__ explicit DivideBy(T divisor) : d(divisor) {
+    if constexpr (sizeof(T) == 4) {
+      y = __frcp_rn(divisor);
+      plain = (__float_as_uint(divisor) & 0x7FFFFFu) == 0x7FFFFFu;
+    } else {
+      y = __drcp_rn(divisor);
+      plain = (__double_as_longlong(divisor) & 0xFFFFFFFFFFFFFll) == 0xFFFFFFFFFFFFFll;
+    }
   }
-  __device__ __forceinline__ float operator()(float v) const {
-    if (plain || (v < 0x1p-100f && v > 0.f)) return v / d;
-    const float q = __fmul_rn(v, y);
-    return fmaf(fmaf(-q, d, v), y, q);
+  __device__ __forceinline__ bool covers(T v) const { return !(plain || (v < MIN && v > (T)0)); }
+  __device__ __forceinline__ T quotient(T v) const {   // (a NaN divisor: the method's NaN is the division's)
+    const T q = v * y;
+    return fma(fma(-q, d, v), y, q);
   }
+  __device__ __forceinline__ T operator()(T v) const { return covers(v) ? quotient(v) : v / d; }
 };
 
 // One unit's gain and bias from its new trace (kernels_openmp_internal.cc:221-246); k = (khalf - 1) pmin4^2.

@@ -92,6 +92,27 @@ def test_forward_and_softmax_vs_oracle(k, port_kernels, tag, dtype, B, N, H, Mc)
 
 
 @pytest.mark.parametrize("tag,dtype", DTYPES)
+@pytest.mark.parametrize("Mc", [17, 33, 100, 129, 200, 256, 300, 384, 400, 512])
+def test_softmax_rounds_like_the_division(k, tag, dtype, Mc):
+    """Groups of 17 to 512 units divide by their sum through its reciprocal; wider ones divide.  Padding a group with
+    units at minus infinity, whose exponentials add exact zeros, sends the same numbers through the other kernel: the
+    results are the same to the bit, exponentials near the smallest numbers included."""
+    rs = np.random.RandomState(Mc)
+    rows = 1500
+    a = rs.randn(rows, Mc) * np.exp(rs.uniform(-2, 5, (rows, 1)))
+    deep = {"f32": (-104, -60), "f64": (-745, -600)}[tag]
+    a[::7, 1:] = rs.uniform(*deep, (len(a[::7]), Mc - 1))   # one strong unit, the others around the smallest numbers
+    a[::7, 0] = 0
+    a = a.astype(dtype)
+    wide = np.full((rows, 544), -np.inf, dtype=dtype)
+    wide[:, :Mc] = a
+    got = k.softmax_minicolumns(a, 1, Mc)
+    want = k.softmax_minicolumns(wide, 1, 544)
+    assert not want[:, Mc:].any()
+    assert np.array_equal(got, want[:, :Mc])
+
+
+@pytest.mark.parametrize("tag,dtype", DTYPES)
 @pytest.mark.parametrize("B,N,H,Mc", SHAPES)
 def test_trace_update_vs_oracle(k, port_kernels, tag, dtype, B, N, H, Mc):
     rs = np.random.RandomState(B * 11 + N)
