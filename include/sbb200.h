@@ -457,6 +457,8 @@ int sbb_measure_fp64_rates(double *dfma_tflops, double *dmma_tflops);
 
 /* Number of kernels this library has launched in this process (all threads). */
 unsigned long long sbb_kernel_launches(void);
+/* How many of them were tensor-core kernels that worked in CTA pairs (none with SBB_TC_PAIR=0 in the environment). */
+unsigned long long sbb_cta_pair_launches(void);
 
 /* Block until all work on `stream` has finished. */
 int sbb_stream_sync(void *stream);

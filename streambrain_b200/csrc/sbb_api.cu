@@ -445,6 +445,7 @@ int sbb_version(void) { return 100; }
 const char *sbb_last_error(void) { return g_error.c_str(); }
 int sbb_device_count(void) { return device_count(); }
 unsigned long long sbb_kernel_launches(void) { return sbb::kernel_launches(); }
+unsigned long long sbb_cta_pair_launches(void) { return sbb::tc_pair_launches(); }
 
 int sbb_set_contraction_path(int path) {
   ARG(path == SBB_PATH_GENERAL || path == SBB_PATH_TENSOR, "invalid contraction path %d", path);

@@ -56,10 +56,15 @@ struct TcHost {
   int *status;   // status word of the bounded waits on the current device
   int sms, lose_arrive;
   long long wait_limit;
+  bool pairs;    // false: SBB_TC_PAIR=0
 };
 bool tc_host(TcHost *out);
 bool tc_map_2d(void *map, const float *base, long inner, long outer, int box_inner, int box_outer, bool mn_major);
 bool tc_map_chunks(void *map, const float *base, long cols, long rows, int box_rows, int box_chunks);
+
+// Launches so far whose CTAs worked in pairs.
+void tc_count_pair_launch();
+unsigned long long tc_pair_launches();
 
 // Status word of the bounded device-side waits on the current device: 0 = all
 // waits completed, otherwise the code of the first wait that gave up.

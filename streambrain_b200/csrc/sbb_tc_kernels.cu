@@ -631,6 +631,7 @@ int g_sm_count_tc[64] = {0};
 std::atomic<int> g_reserved_sms{-1};   // -1: not set yet (the environment decides on first use)
 std::atomic<long long> g_wait_limit{kWaitLimitCycles};
 std::atomic<int> g_lose_arrive{0};     // launches that still have to lose one arrival (test hook)
+std::atomic<unsigned long long> g_pair_launches{0};
 long long wait_limit_now() { return g_wait_limit.load(); }
 int take_lose_arrive() {
   int n = g_lose_arrive.load();
@@ -799,7 +800,7 @@ cudaError_t launch_tc(const TcMaps &tm, const TcWork &wk, const TcEpilogue &ep, 
                      wk, ep, status);
 }
 
-// SBB_TC_PAIR=0 keeps one CTA per tile (read once).
+// SBB_TC_PAIR=0 keeps one CTA per tile, in the forward product and in the trace update (read once).
 bool pairs_enabled() {
   static const bool on = [] {
     const char *e = getenv("SBB_TC_PAIR");
@@ -849,17 +850,23 @@ cudaError_t launch_tc_pair(const TcMaps &tm, const TcWork &wk, const TcEpilogue 
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // as launch_next
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, kernel, tm.a, tm.b, tm.a3, tm.b3, tm.c, tm.alo, tm.blo, tm.a3lo, tm.b3lo, wk, ep,
-                            status);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tm.a, tm.b, tm.a3, tm.b3, tm.c, tm.alo, tm.blo, tm.a3lo, tm.b3lo, wk,
+                                           ep, status);
+  if (e == cudaSuccess) tc_count_pair_launch();
+  return e;
 }
 
 }  // namespace
+
+void tc_count_pair_launch() { g_pair_launches += 1; }
+unsigned long long tc_pair_launches() { return g_pair_launches.load(); }
 
 bool tc_host(TcHost *out) {
   out->status = status_word();
   out->sms = g_sm_count_tc[current_device()];
   out->wait_limit = wait_limit_now();
   out->lose_arrive = out->status != nullptr ? take_lose_arrive() : 0;
+  out->pairs = pairs_enabled();
   return out->status != nullptr && init_once();
 }
 bool tc_map_2d(void *map, const float *base, long inner, long outer, int box_inner, int box_outer, bool mn_major) {

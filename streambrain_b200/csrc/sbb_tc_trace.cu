@@ -4,7 +4,11 @@
 //
 // float32 operands as split TF32 products (hi*hi + hi*lo + lo*hi, see sbb_tc_kernels.cu): A's parts go to tensor memory,
 // B's low part beside the raw tile in shared memory.  A cluster of two CTAs works on 256 rows x 192 columns
-// (tcgen05.mma.cta_group::2); each CTA stages and splits its own 128 rows of A and half of the columns of B.
+// (tcgen05.mma.cta_group::2); each CTA stages and splits its own 128 rows of A and half of the columns of B.  (!PAIR, what
+// SBB_TC_PAIR=0 selects: one CTA works on 128 rows x 192 columns by itself and stages all columns of B, which leaves room
+// for three stages; the products, chains and sums are the same.  It is there to compare with and for
+// devices that cannot place pairs.  Train step without a mask update: 1568 -> 30 x 100 at batch 128 32.1 us in pairs, 33.2
+// without; 55296 -> 30 x 100 at 256 565 and 686 us.)
 // Roles in a CTA (672 threads, one CTA per SM, tiles walked persistently):
 //   warps 0-11   epilogue: accumulator, old trace (by TMA, the whole tile's blocks one tile ahead), arithmetic, stores
 //   warps 12-15  A converters (one tile row, that is one tensor-memory lane, per thread)
@@ -33,29 +37,35 @@ namespace {
 
 constexpr int kEpi = 12, kConv = 12, kTma = 16, kMma = 17, kVec = 18, kConvB = 19, kBWarps = 2;
 constexpr int kThreads = (kConvB + kBWarps) * 32;
-constexpr int kBN = 192, kBNH = kBN / 2, kBK = 16, kStages = 4;   // (tensor memory holds the A parts of four stages)
+constexpr int kBN = 192, kBK = 16;
 constexpr int kChainKb = 16;                     // k-blocks per accumulation chain
 constexpr int kGroups = kBN / (kEpi / 4) / 32;   // 32-column groups per epilogue warp
-constexpr int kABytes = 128 * kBK * 4, kBBytes = kBNH * kBK * 4;
-constexpr int kTx = kABytes + kBBytes, kStage = kTx + kBBytes;   // [A | B | B lo]
+constexpr int kABytes = 128 * kBK * 4;
 constexpr int kTmemA = 2 * kBN;                  // two accumulators, then per stage kBK columns of A hi and as many of A lo
-static_assert(kTmemA + kStages * 2 * kBK <= 512, "tensor memory budget");
-static_assert(kStage % 1024 == 0 && kABytes % 1024 == 0 && kTx % 1024 == 0, "swizzle alignment");
 constexpr int kSlab = 32 * 32 * 4;               // a 32 x 32 block of the trace matrix
 struct TileVectors {
   float rci[128], rcj[kBN];     // reciprocals of Ci and Cj, 0 below the threshold
   uint32_t bits[128];           // per row: bit k = mask of hypercolumn (the tile's first) + k
 };
-constexpr int kSlabOffset = kStages * kStage;
-constexpr int kVecOffset = kSlabOffset + kEpi * kGroups * kSlab;
-constexpr int kBarOffset = kVecOffset + 2 * (int)sizeof(TileVectors);
-// full, converted, empty per stage; acc_full[2], acc_empty[2], drain, vec_full[2], vec_empty[2]; one per block of the tile
-constexpr int kBars = 3 * kStages + 9 + kEpi * kGroups;
-constexpr int kSmem = kBarOffset + kBars * 8 + 24 + 1024;
-static_assert(kBarOffset % 8 == 0 && kSmem <= 232448, "shared memory budget");
+template <bool PAIR>
+struct Layout {
+  static constexpr int BNH = PAIR ? kBN / 2 : kBN;   // columns of B a CTA stages
+  static constexpr int STAGES = PAIR ? 4 : 3;        // (tensor memory holds the A parts of four stages)
+  static constexpr int B_BYTES = BNH * kBK * 4;
+  static constexpr int TX = kABytes + B_BYTES, STAGE = TX + B_BYTES;   // [A | B | B lo]
+  static_assert(kTmemA + STAGES * 2 * kBK <= 512, "tensor memory budget");
+  static_assert(STAGE % 1024 == 0 && kABytes % 1024 == 0 && TX % 1024 == 0, "swizzle alignment");
+  static constexpr int SLAB_OFFSET = STAGES * STAGE;
+  static constexpr int VEC_OFFSET = SLAB_OFFSET + kEpi * kGroups * kSlab;
+  static constexpr int BAR_OFFSET = VEC_OFFSET + 2 * (int)sizeof(TileVectors);
+  // full, converted, empty per stage; acc_full[2], acc_empty[2], drain, vec_full[2], vec_empty[2]; one per block of the tile
+  static constexpr int BARS = 3 * STAGES + 9 + kEpi * kGroups;
+  static constexpr int SMEM = BAR_OFFSET + BARS * 8 + 24 + 1024;
+  static_assert(BAR_OFFSET % 8 == 0 && SMEM <= 232448, "shared memory budget");
+};
 
 struct Trace {
-  int m_units, n_tiles, kblocks, m_fastest;
+  int m_units, n_tiles, kblocks, m_fastest;   // m_units: row tiles, or pairs of them
   int a_box3, b_box3_tiles;   // A, and column tiles below the limit of B, come in one 3-D box per stage
   int lose_arrive;            // test hook: converter thread 0 of CTA 0 skips its arrival for the first stage
   long long wait_limit;
@@ -69,15 +79,19 @@ struct Trace {
   float one_minus, cthr4, ema_scale;
 };
 
+template <bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
     trace_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmA3, const __grid_constant__ CUtensorMap tmB3,
                  const __grid_constant__ CUtensorMap tmC, const Trace g, int *status) {
+  using L = Layout<PAIR>;
+  constexpr int kStages = L::STAGES, kStage = L::STAGE, kBNH = L::BNH, kBBytes = L::B_BYTES, kTx = L::TX;
+  constexpr int kSlabOffset = L::SLAB_OFFSET, kVecOffset = L::VEC_OFFSET;
   extern __shared__ uint8_t smem_dyn[];
   const uint32_t dyn_base = smem_u32(smem_dyn);
   const uint32_t base = (dyn_base + 1023u) & ~1023u;   // swizzle atoms need 1024-byte alignment
   uint8_t *smem = smem_dyn + (base - dyn_base);
-  const uint32_t bars = base + kBarOffset;
+  const uint32_t bars = base + L::BAR_OFFSET;
   auto bar_full = [&](int s) { return bars + 8u * s; };
   auto bar_conv = [&](int s) { return bars + 8u * (kStages + s); };
   auto bar_empty = [&](int s) { return bars + 8u * (2 * kStages + s); };
@@ -86,21 +100,29 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t bar_drain = bars + 8u * (3 * kStages + 4);
   auto bar_vec_full = [&](int b) { return bars + 8u * (3 * kStages + 5 + b); };
   auto bar_vec_empty = [&](int b) { return bars + 8u * (3 * kStages + 7 + b); };
+  auto leader_arrive = [&](uint32_t bar) {   // (PAIR: the leader's barrier counts both CTAs' threads)
+    if constexpr (PAIR) mbar_arrive_rank(bar, 0);
+    else mbar_arrive(bar);
+  };
+  auto commit = [&](uint32_t bar) {   // (PAIR: to both CTAs' barriers)
+    if constexpr (PAIR) mma_commit_pair(bar);
+    else mma_commit(bar);
+  };
   auto bar_slab = [&](int e, int gr) { return bars + 8u * (3 * kStages + 9 + kGroups * e + gr); };
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + kBarOffset + kBars * 8);
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L::BAR_OFFSET + L::BARS * 8);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_ctarank();
+  const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(bar_full(s), 1);
-      mbar_init(bar_conv(s), 2 * (4 + kBWarps) * 32);   // the leader's counts both CTAs' converters
+      mbar_init(bar_conv(s), (PAIR ? 2 : 1) * (4 + kBWarps) * 32);   // the leader's counts both CTAs' converters
       mbar_init(bar_empty(s), 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(bar_acc_full(b), 1);
-      mbar_init(bar_acc_empty(b), 2 * kEpi);
+      mbar_init(bar_acc_empty(b), (PAIR ? 2 : 1) * kEpi);
       mbar_init(bar_vec_full(b), 32);
       mbar_init(bar_vec_empty(b), kEpi);
     }
@@ -111,11 +133,17 @@ __global__ void __launch_bounds__(kThreads, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kMma) {
-    tmem_alloc_pair(smem_u32(tmem_slot), 512);
-    tmem_relinquish_pair();
+    if constexpr (PAIR) {
+      tmem_alloc_pair(smem_u32(tmem_slot), 512);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(smem_u32(tmem_slot), 512);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
-  cluster_sync_all();   // the peer's barriers exist before anything arrives on them
+  if constexpr (PAIR) cluster_sync_all();   // the peer's barriers exist before anything arrives on them
+  else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   after_previous();   // (barriers and tensor memory are set up while the kernel before ends)
@@ -123,7 +151,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   // The clusters walk the tiles side by side, columns fastest (rows fastest where the columns are the longer side): at any
   // time they share the operands of a few row tiles.
   const long total = (long)g.m_units * g.n_tiles;
-  const long w_first = blockIdx.x >> 1, w_step = gridDim.x >> 1;
+  const long w_first = PAIR ? blockIdx.x >> 1 : blockIdx.x, w_step = PAIR ? gridDim.x >> 1 : gridDim.x;
   auto decode = [&](long w, int &mt, int &nt) {
     if (g.m_fastest) {
       mt = (int)(w % g.m_units);
@@ -132,7 +160,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       nt = (int)(w % g.n_tiles);
       mt = (int)(w / g.n_tiles);
     }
-    mt = 2 * mt + (int)rank;   // may be one past the last row tile: such a CTA stages zeros and stores nothing
+    if (PAIR) mt = 2 * mt + (int)rank;   // may be one past the last row tile: such a CTA stages zeros and stores nothing
   };
   auto hc_of = [&](long n) -> int { return g.hc_magic ? (int)__umulhi((uint32_t)n, g.hc_magic) : (int)(n / g.Mc); };
   auto first_hc = [&](int nt) -> int { return g.wmask ? hc_of((long)nt * kBN) : 0; };
@@ -178,9 +206,13 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else if (warp == kMma) {
     // ------------------------------------------------------------ MMA issuer
     if (lane == 0 && rank == 0) {
-      // D float32, A (tensor memory) and B (shared memory, MN-major) TF32; 256 rows over the pair, kBN columns
-      constexpr uint32_t idesc =
-          (1u << 4) | (2u << 7) | (2u << 10) | (1u << 16) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+      // D float32, A (tensor memory) and B (shared memory, MN-major) TF32; 256 rows over the pair (or 128), kBN columns
+      constexpr uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | (1u << 16) | ((uint32_t)(kBN >> 3) << 17) |
+                                 ((uint32_t)((PAIR ? 256 : 128) >> 4) << 24);
+      auto mma = [&](uint32_t d, uint32_t ta, uint64_t db, uint32_t accumulate) {
+        if constexpr (PAIR) mma_tf32_ts_pair(d, ta, db, idesc, accumulate);
+        else mma_tf32_ts(d, ta, db, idesc, accumulate);
+      };
       uint32_t it = 0, chain = 0;
       bool ok = true;
       for (long w = w_first; w < total && ok; w += w_step) {
@@ -199,21 +231,21 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (int kk = 0; kk < kBK / 8; ++kk) {   // eight 128-byte rows (two 4-row swizzle atoms) of B per instruction
               const uint64_t db_hi = smem_desc_mn(b_hi + kk * 1024, kBK * 128), db_lo = smem_desc_mn(b_lo + kk * 1024, kBK * 128);
-              mma_tf32_ts_pair(d_tmem, ta + kBK + kk * 8, db_hi, idesc, first && kk == 0 ? 0u : 1u);
-              mma_tf32_ts_pair(d_tmem, ta + kk * 8, db_lo, idesc, 1u);
-              mma_tf32_ts_pair(d_tmem, ta + kk * 8, db_hi, idesc, 1u);
+              mma(d_tmem, ta + kBK + kk * 8, db_hi, first && kk == 0 ? 0u : 1u);
+              mma(d_tmem, ta + kk * 8, db_lo, 1u);
+              mma(d_tmem, ta + kk * 8, db_hi, 1u);
             }
             first = false;
-            mma_commit_pair(bar_empty(s));   // the stage may be refilled, in both CTAs, once these MMAs have read it
+            commit(bar_empty(s));   // the stage may be refilled, in both CTAs, once these MMAs have read it
           }
           if (ok) {
-            mma_commit_pair(bar_acc_full(buf));
+            commit(bar_acc_full(buf));
             ++chain;
           }
         }
       }
       // nothing may still be running in the tensor pipe when its memory is freed (bounded by time alone)
-      mma_commit_pair(bar_drain);
+      commit(bar_drain);
       if (!mbar_try_wait(bar_drain, 0)) mbar_wait_slow(bar_drain, 0, abort_flag, status, kWaitDrain, false);
     }
   } else if (warp >= kConv && warp < kConv + 4) {
@@ -239,7 +271,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         tmem_st_32x32b<kBK>(ta + kBK, r);
         tmem_wait_st();
         tc_fence_before();
-        if (!(g.lose_arrive && it == 0 && threadIdx.x == kConv * 32 && blockIdx.x == 0)) mbar_arrive_rank(bar_conv(s), 0);
+        if (!(g.lose_arrive && it == 0 && threadIdx.x == kConv * 32 && blockIdx.x == 0)) leader_arrive(bar_conv(s));
       }
   } else if (warp >= kConvB) {
     // ------------------------------------------------------------ B's low part beside the raw tile
@@ -254,14 +286,19 @@ __global__ void __launch_bounds__(kThreads, 1)
         float4 *low = reinterpret_cast<float4 *>(smem + s * kStage + kTx);
         constexpr int kPieces = kBBytes / 16 / (kBWarps * 32);
         static_assert(kBBytes % (16 * kBWarps * 32) == 0, "a whole number of 16-byte pieces per thread");
-        float4 v[kPieces];   // every load is issued before the first store
+        constexpr int kAhead = 6;   // loads issued before the first store: all of a pair's share
+        static_assert(kPieces % kAhead == 0, "whole groups of pieces");
 #pragma unroll
-        for (int i = 0; i < kPieces; ++i) v[i] = raw[t + i * (kBWarps * 32)];
+        for (int i0 = 0; i0 < kPieces; i0 += kAhead) {
+          float4 v[kAhead];
 #pragma unroll
-        for (int i = 0; i < kPieces; ++i)
-          low[t + i * (kBWarps * 32)] = make_float4(tf32_lo(v[i].x), tf32_lo(v[i].y), tf32_lo(v[i].z), tf32_lo(v[i].w));
+          for (int i = 0; i < kAhead; ++i) v[i] = raw[t + (i0 + i) * (kBWarps * 32)];
+#pragma unroll
+          for (int i = 0; i < kAhead; ++i)
+            low[t + (i0 + i) * (kBWarps * 32)] = make_float4(tf32_lo(v[i].x), tf32_lo(v[i].y), tf32_lo(v[i].z), tf32_lo(v[i].w));
+        }
         fence_async_smem();   // make the generic-proxy writes visible to the tensor pipe
-        mbar_arrive_rank(bar_conv(s), 0);
+        leader_arrive(bar_conv(s));
       }
   } else if (warp == kVec) {
     // ------------------------------------------------------------ row and column data, one tile ahead
@@ -448,7 +485,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
-          mbar_arrive_rank(bar_acc_empty(buf), 0);
+          leader_arrive(bar_acc_empty(buf));
           if (last_chain) mbar_arrive(bar_vec_empty(tile & 1u));
         }
       }
@@ -458,10 +495,12 @@ __global__ void __launch_bounds__(kThreads, 1)
   // ------------------------------------------------------------ tear-down
   __syncwarp();
   tc_fence_before();
-  cluster_sync_all();   // neither CTA retires while the other may still signal it or read its operands
+  if constexpr (PAIR) cluster_sync_all();   // neither CTA retires while the other may still signal it or read its operands
+  else __syncthreads();
   if (warp == kMma) {
     tc_fence_after();
-    tmem_dealloc_pair(tmem_base, 512);
+    if constexpr (PAIR) tmem_dealloc_pair(tmem_base, 512);
+    else tmem_dealloc(tmem_base, 512);
   }
 }
 
@@ -494,11 +533,11 @@ cudaError_t launch_trace_update_tc(const float *x, const float *y, long B, long 
   if (!tc_map_2d(&ma, x, N, B, 32, kBK, true) || !tc_map_2d(&mb, y, M, B, 32, kBK, true) ||
       !tc_map_2d(&mc, Cij, M, N, 32, 32, false))
     return cudaErrorInvalidValue;
-  const bool a3 = N % 32 == 0 && tc_map_chunks(&ma3, x, N, B, kBK, 4), b3 = tc_map_chunks(&mb3, y, M, B, kBK, kBNH / 32);
+  const bool a3 = N % 32 == 0 && tc_map_chunks(&ma3, x, N, B, kBK, 4), b3 = tc_map_chunks(&mb3, y, M, B, kBK, (host.pairs ? Layout<true>::BNH : Layout<false>::BNH) / 32);
   if (!a3) ma3 = ma;
   if (!b3) mb3 = mb;
   Trace g{};
-  g.m_units = (int)((N + 255) / 256);
+  g.m_units = (int)(host.pairs ? (N + 255) / 256 : (N + 127) / 128);
   g.n_tiles = (int)((M + kBN - 1) / kBN);
   g.kblocks = (int)((B + kBK - 1) / kBK);
   g.m_fastest = M > N ? 1 : 0;   // consecutive tiles re-use the larger operand
@@ -524,33 +563,50 @@ cudaError_t launch_trace_update_tc(const float *x, const float *y, long B, long 
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  const long units = (long)g.m_units * g.n_tiles;
+  if (!host.pairs) {
+    using L = Layout<false>;
+    static std::atomic<bool> configured[64];
+    if (!configured[dev].load()) {
+      const cudaError_t e = cudaFuncSetAttribute(trace_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
+      if (e != cudaSuccess) return e;
+      configured[dev].store(true);
+    }
+    const cudaError_t e = launch_next(trace_kernel<false>, (unsigned)(units < host.sms ? units : host.sms), kThreads, L::SMEM, st,
+                                      ma, mb, ma3, mb3, mc, g, host.status);
+    if (e == cudaSuccess) count_launches(1);
+    return e;
+  }
+  using L = Layout<true>;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.dynamicSmemBytes = kSmem;
+  cfg.dynamicSmemBytes = L::SMEM;
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   static std::atomic<int> max_clusters[64];   // resident pairs (one CTA per SM; pairs must share a GPC's SMs)
   if (max_clusters[dev].load() == 0) {
-    cudaError_t e = cudaFuncSetAttribute(trace_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    cudaError_t e = cudaFuncSetAttribute(trace_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
     if (e != cudaSuccess) return e;
     cfg.gridDim = dim3((unsigned)(host.sms / 2 * 2), 1, 1);
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, trace_kernel, &cfg) != cudaSuccess || n <= 0 || n > host.sms / 2) n = host.sms / 2;
+    if (cudaOccupancyMaxActiveClusters(&n, trace_kernel<true>, &cfg) != cudaSuccess || n <= 0 || n > host.sms / 2) n = host.sms / 2;
     max_clusters[dev].store(n);
   }
-  const long pairs = (long)g.m_units * g.n_tiles;
-  const long clusters = pairs < max_clusters[dev].load() ? pairs : max_clusters[dev].load();
+  const long clusters = units < max_clusters[dev].load() ? units : max_clusters[dev].load();
   cfg.gridDim = dim3((unsigned)(2 * clusters), 1, 1);
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // as launch_next
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.numAttrs = 2;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, trace_kernel, ma, mb, ma3, mb3, mc, g, host.status);
-  if (e == cudaSuccess) count_launches(1);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, trace_kernel<true>, ma, mb, ma3, mb3, mc, g, host.status);
+  if (e == cudaSuccess) {
+    count_launches(1);
+    tc_count_pair_launch();
+  }
   return e;
 }
 

@@ -279,7 +279,7 @@ def test_a_wait_that_runs_out_is_reported_and_the_device_stays_usable(k):
 def test_one_cta_form_of_the_tensor_kernels(port_kernels, tmp_path):
     """The tensor-core contractions run as CTA pairs by default; SBB_TC_PAIR=0 (read once per process, hence the
     child process) keeps one CTA per tile.  Both forms of the forward product, of the single-chain and of the
-    multi-chain trace update must agree with the oracle."""
+    multi-chain trace update must agree with the oracle, and must be the ones that ran."""
     import os
     import subprocess
     import sys
@@ -292,15 +292,19 @@ from streambrain_b200 import kernels_b200 as k
 from streambrain_b200._lib import check, lib
 check(lib.sbb_set_contraction_path(1))
 out = {}
-for tag, (B, N, H, Mc) in {"single": (256, 388, 3, 44), "multi": (600, 260, 2, 130)}.items():
+for tag, (B, N, H, Mc) in {"single": (256, 388, 3, 44), "multi": (700, 260, 2, 130)}.items():
     rs = np.random.RandomState(B + N)
     M = H * Mc
     x, y = rs.rand(B, N).astype(np.float32), rs.rand(B, M).astype(np.float32)
     st = [rs.rand(N).astype(np.float32), rs.rand(M).astype(np.float32), rs.rand(N, M).astype(np.float32)]
     w = rs.randn(N, M).astype(np.float32)
     b = rs.randn(M).astype(np.float32)
+    pairs = [lib.sbb_cta_pair_launches()]
     out[tag + "_fwd"] = k.update_state(np.zeros((B, M), dtype=np.float32), w, b, x)
+    pairs.append(lib.sbb_cta_pair_launches())
     got = k.update_weights(*[v.copy() for v in st], x, y, 0.05, np.zeros((N, M), dtype=np.float32), 0.025)
+    pairs.append(lib.sbb_cta_pair_launches())
+    out[tag + "_pairs"] = np.diff(np.array(pairs, dtype=np.int64))
     for name, v in zip(("Ci", "Cj", "Cij", "W"), got):
         out[tag + "_" + name] = v
 np.savez(sys.argv[1], **out)
@@ -312,7 +316,7 @@ np.savez(sys.argv[1], **out)
         subprocess.run([sys.executable, "-c", script, path], check=True, env=env, timeout=300)
         results[pair] = np.load(path)
     tol = TOL[np.dtype(np.float32)]
-    for tag, (B, N, H, Mc) in {"single": (256, 388, 3, 44), "multi": (600, 260, 2, 130)}.items():
+    for tag, (B, N, H, Mc) in {"single": (256, 388, 3, 44), "multi": (700, 260, 2, 130)}.items():
         rs = np.random.RandomState(B + N)
         M = H * Mc
         x, y = rs.rand(B, N).astype(np.float32), rs.rand(B, M).astype(np.float32)
@@ -323,10 +327,13 @@ np.savez(sys.argv[1], **out)
         want = port_kernels.update_weights(*[v.copy() for v in st], x, y, 0.05, np.zeros((N, M), dtype=np.float32), 0.025)
         for pair in ("0", "1"):
             r = results[pair]
+            assert list(r[tag + "_pairs"]) == [int(pair)] * 2, (tag, pair)   # one launch of each, in pairs or not
             assert rel_inf(r[tag + "_fwd"], fwd) < tol, (tag, pair)
             for name, v in zip(("Ci", "Cj", "Cij"), want):
                 assert rel_inf(r[tag + "_" + name], v) < tol, (tag, pair, name)
             assert weight_err(r[tag + "_W"], want[3]) < 10 * tol, (tag, pair)
+        for name in ("fwd", "Cij", "W"):   # the same products, chains and sums
+            assert np.array_equal(results["0"][tag + "_" + name], results["1"][tag + "_" + name]), (tag, name)
 
 
 @pytest.mark.parametrize("n,mc", [(600, 6), (2048, 40), (2049, 40), (20000, 5)])
