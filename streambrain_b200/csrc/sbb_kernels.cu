@@ -17,6 +17,8 @@
 
 #include <atomic>
 #include <math.h>
+#include <stdlib.h>
+#include <string.h>
 
 namespace sbb {
 
@@ -132,6 +134,10 @@ struct TileShape : Tile {
 };
 
 __device__ __forceinline__ void lds4(const float *p, float *r) { unpack(*reinterpret_cast<const float4 *>(p), r); }
+__device__ __forceinline__ void lds4(const double *p, double *r) {
+  unpack(*reinterpret_cast<const double2 *>(p), r);
+  unpack(*reinterpret_cast<const double2 *>(p + 2), r + 2);
+}
 
 // Row / column of micro-tile entry e (0..7) inside the 128-wide tile.
 __device__ __forceinline__ int micro_index(int t, int e) { return (e < 4 ? 0 : 64) + t * 4 + (e & 3); }
@@ -235,25 +241,28 @@ __global__ void __launch_bounds__(Tile::THREADS, 2)
 // row length, and its reads of A are broadcasts).  Such launches are bound by latency and by the SMs they leave idle, not by
 // arithmetic: the slabs arrive by 4-byte cp.async (any alignment) with three of four stages in flight, and what the epilogue
 // reads is requested before the main loop.  Each output is the same chain of FMAs over ascending k as in the kernel above.
-template <bool A_KMAJOR>
+// (In float64 it is what SBB_F64_CONTRACTION=dfma runs, with the general epilogue's division and library logarithm, to
+// compare the FP64 tensor-core kernels with: 1568 -> 30 x 100 at batch 128, forward pass 82 us against 43, train step without
+// a mask update 136 against 72.)
+template <typename T, bool A_KMAJOR>
 struct SmallShape {
   static constexpr bool KMAJOR = A_KMAJOR;
   static constexpr int BM = 32, BN = 64, BK = 32, STAGES = 4, THREADS = 128;
   static constexpr int LDA = 32 + 4, LDB = BN;   // K-major A as [m][k], MN-major as [k][m]: 16-byte rows
   static constexpr int A_STAGE = 32 * LDA, B_STAGE = BK * LDB;
-  static constexpr size_t SMEM_BYTES = (size_t)STAGES * (A_STAGE + B_STAGE) * sizeof(float);
+  static constexpr size_t SMEM_BYTES = (size_t)STAGES * (A_STAGE + B_STAGE) * sizeof(T);
 };
 
 // grid.x = column tiles, grid.y = row tiles, grid.z = k-splits
-template <bool A_KMAJOR, class Epilogue>
-__global__ void __launch_bounds__(SmallShape<A_KMAJOR>::THREADS)
-    small_contraction_kernel(const float *__restrict__ A, long lda, const float *__restrict__ Bm, long ldb, long Mdim,
-                             long Ndim, int K, int kper, Epilogue ep) {
+template <typename T, bool A_KMAJOR, class Epilogue>
+__global__ void __launch_bounds__(SmallShape<T, A_KMAJOR>::THREADS)
+    small_contraction_kernel(const T *__restrict__ A, long lda, const T *__restrict__ Bm, long ldb, long Mdim, long Ndim, int K,
+                             int kper, Epilogue ep) {
   after_previous();
-  using S = SmallShape<A_KMAJOR>;
-  using L = Slab<float, S, 1>;
-  extern __shared__ __align__(16) float small_smem[];
-  float *As = small_smem, *Bs = small_smem + S::STAGES * S::A_STAGE;
+  using S = SmallShape<T, A_KMAJOR>;
+  using L = Slab<T, S, 1>;
+  extern __shared__ __align__(16) unsigned char small_smem[];
+  T *As = reinterpret_cast<T *>(small_smem), *Bs = As + S::STAGES * S::A_STAGE;
   const int w8 = (threadIdx.x >> 5) * 8, lane = threadIdx.x & 31;
   const long m0 = (long)blockIdx.y * S::BM, n0 = (long)blockIdx.x * S::BN;
   const int kbeg = blockIdx.z * kper;
@@ -270,9 +279,9 @@ __global__ void __launch_bounds__(SmallShape<A_KMAJOR>::THREADS)
     cp_async_commit();
   }
   typename Epilogue::Strip strip(ep, m0 + w8, n0 + lane, lane);
-  float acc[8][2];
+  T acc[8][2];
 #pragma unroll
-  for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = 0.f;
+  for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = (T)0;
   for (int kt = 0; kt < nk; ++kt) {
     cp_async_wait<S::STAGES - 2>();   // slab kt has landed
     __syncthreads();                  // ... for every thread, and the stage refilled below is free
@@ -284,17 +293,17 @@ __global__ void __launch_bounds__(SmallShape<A_KMAJOR>::THREADS)
       slab.advance();
     }
     cp_async_commit();
-    const float *as = As + kt % S::STAGES * S::A_STAGE, *bs = Bs + kt % S::STAGES * S::B_STAGE + lane;
+    const T *as = As + kt % S::STAGES * S::A_STAGE, *bs = Bs + kt % S::STAGES * S::B_STAGE + lane;
 #pragma unroll
     for (int k4 = 0; k4 < S::BK; k4 += 4) {
-      float a[8][4];   // [row][k]
+      T a[8][4];   // [row][k]
       if constexpr (A_KMAJOR) {
 #pragma unroll
         for (int r = 0; r < 8; ++r) lds4(as + (w8 + r) * S::LDA + k4, a[r]);
       } else {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          float v[8];
+          T v[8];
           lds4(as + (k4 + k) * S::LDA + w8, v);
           lds4(as + (k4 + k) * S::LDA + w8 + 4, v + 4);
 #pragma unroll
@@ -303,11 +312,11 @@ __global__ void __launch_bounds__(SmallShape<A_KMAJOR>::THREADS)
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const float b0 = bs[(k4 + k) * S::LDB], b1 = bs[(k4 + k) * S::LDB + 32];
+        const T b0 = bs[(k4 + k) * S::LDB], b1 = bs[(k4 + k) * S::LDB + 32];
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
-          acc[r][0] = fmaf(a[r][k], b0, acc[r][0]);
-          acc[r][1] = fmaf(a[r][k], b1, acc[r][1]);
+          acc[r][0] = fma(a[r][k], b0, acc[r][0]);
+          acc[r][1] = fma(a[r][k], b1, acc[r][1]);
         }
       }
     }
@@ -719,11 +728,11 @@ static cudaError_t launch_f64_mma(const double *A, long lda, const double *Bm, l
 // tiles 35.6 -> 12.8 us, 96 tiles 36.5 -> 28.3, but 216 tiles 55.0 -> 54.7 at batch 97 and 125 -> 136 at batch 512.
 static bool small_tiles(long tiles, bool forward) { return (forward ? 2 : 1) * tiles < sm_count(); }
 
-template <bool A_KMAJOR, class Ep>
-static cudaError_t launch_small_contraction(const float *A, long lda, const float *Bm, long ldb, long Mdim, long Ndim,
-                                            int K, int splits, int kper, Ep ep, cudaStream_t st) {
-  using S = SmallShape<A_KMAJOR>;
-  auto kernel = small_contraction_kernel<A_KMAJOR, Ep>;
+template <typename T, bool A_KMAJOR, class Ep>
+static cudaError_t launch_small_contraction(const T *A, long lda, const T *Bm, long ldb, long Mdim, long Ndim, int K,
+                                            int splits, int kper, Ep ep, cudaStream_t st) {
+  using S = SmallShape<T, A_KMAJOR>;
+  auto kernel = small_contraction_kernel<T, A_KMAJOR, Ep>;
   static bool configured[64] = {false};
   const cudaError_t e = allow_smem(kernel, S::SMEM_BYTES, configured);
   if (e != cudaSuccess) return e;
@@ -748,6 +757,15 @@ static cudaError_t launch_tiles(const float *A, long lda, const float *Bm, long 
   return launched();
 }
 
+// SBB_F64_CONTRACTION=dfma keeps float64 off the FP64 tensor-core instruction (read once).
+static bool f64_mma_enabled() {
+  static const bool on = [] {
+    const char *e = getenv("SBB_F64_CONTRACTION");
+    return !(e != nullptr && strcmp(e, "dfma") == 0);
+  }();
+  return on;
+}
+
 template <typename T, bool A_KMAJOR, class Ep>
 static cudaError_t launch_contraction(const T *A, long lda, const T *Bm, long ldb, long Mdim, long Ndim, int K,
                                       int splits, int kper, bool vec, bool cols_fastest, Ep ep, cudaStream_t st) {
@@ -755,12 +773,14 @@ static cudaError_t launch_contraction(const T *A, long lda, const T *Bm, long ld
   if (mt <= 0 || nt <= 0 || K <= 0) return cudaSuccess;
   // `vec`: every operand row starts on a 16-byte boundary and holds a whole number of 16-byte pieces
   if constexpr (std::is_same<T, double>::value) {
+    if (!f64_mma_enabled() && Mdim <= 65535L * SmallShape<T, A_KMAJOR>::BM)   // (its row tiles are grid.y)
+      return launch_small_contraction<T, A_KMAJOR>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, ep, st);
     if (vec && lda % 2 == 0 && ldb % 2 == 0)
       return launch_f64_mma<A_KMAJOR, 2>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, to_pairs(ep), st);
     return launch_f64_mma<A_KMAJOR, 1>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, to_pairs(ep), st);
   } else {
     if (small_tiles(mt * nt * splits, A_KMAJOR))
-      return launch_small_contraction<A_KMAJOR>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, ep, st);
+      return launch_small_contraction<T, A_KMAJOR>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, ep, st);
     if (vec) return launch_tiles<A_KMAJOR, 4>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, cols_fastest, ep, st);
     return launch_tiles<A_KMAJOR, 1>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, cols_fastest, ep, st);
   }

@@ -336,6 +336,64 @@ np.savez(sys.argv[1], **out)
             assert np.array_equal(results["0"][tag + "_" + name], results["1"][tag + "_" + name]), (tag, name)
 
 
+def test_float64_contractions_without_the_tensor_core_instruction(k, port_kernels, tmp_path):
+    """SBB_F64_CONTRACTION=dfma (read once per process, hence the child processes) runs the float64 contractions on plain
+    FMAs, with divisions and the library's logarithm in the trace update.  Both settings must agree with the oracle, and
+    must differ in the weights' last digits: otherwise the setting changed nothing."""
+    import os
+    import subprocess
+    import sys
+    from conftest import REPO
+    cases = [(97, 1001, 3, 37), (128, 260, 2, 130), (33, 31, 1, 65)]
+
+    def inputs(B, N, H, Mc):
+        rs = np.random.RandomState(B + N)
+        M = H * Mc
+        x, y = rs.rand(B, N), rs.rand(B, M)
+        return x, y, [rs.rand(N), rs.rand(M), rs.rand(N, M)], rs.randn(N, M), rs.randn(M)
+
+    script = r'''
+import sys
+import numpy as np
+sys.path.insert(0, %r)
+from streambrain_b200 import kernels_b200 as k
+data = np.load(sys.argv[1])
+out = {}
+for c in range(%d):
+    x, y, Ci, Cj, Cij, w, b = (data["%%d_%%d" %% (c, q)] for q in range(7))
+    out["%%d_fwd" %% c] = k.update_state(np.zeros((len(x), len(b))), w, b, x)
+    got = k.update_weights(Ci.copy(), Cj.copy(), Cij.copy(), x, y, 0.05, np.zeros_like(w), 0.025)
+    for name, v in zip(("Ci", "Cj", "Cij", "W"), got):
+        out["%%d_%%s" %% (c, name)] = v
+np.savez(sys.argv[2], **out)
+''' % (REPO, len(cases))
+    data, want = {}, {}
+    for c, case in enumerate(cases):
+        x, y, st, w, b = inputs(*case)
+        for q, v in enumerate([x, y, *st, w, b]):
+            data["%d_%d" % (c, q)] = v
+        want["%d_fwd" % c] = port_kernels.update_state(np.zeros((len(x), len(b))), w, b, x)
+        for name, v in zip(("Ci", "Cj", "Cij", "W"), port_kernels.update_weights(*[v.copy() for v in st], x, y, 0.05,
+                                                                              np.zeros_like(w), 0.025)):
+            want["%d_%s" % (c, name)] = v
+    np.savez(str(tmp_path / "in.npz"), **data)
+    results = {}
+    for setting in ("dfma", ""):
+        path = str(tmp_path / ("out%s.npz" % setting))
+        subprocess.run([sys.executable, "-c", script, str(tmp_path / "in.npz"), path], check=True, timeout=300,
+                       env=dict(os.environ, SBB_F64_CONTRACTION=setting))
+        results[setting] = np.load(path)
+        for name, v in want.items():
+            got = results[setting][name]
+            if name.endswith("_W"):
+                assert weight_err(got, v) < 1e-11, (setting, name)
+            else:
+                assert rel_inf(got, v) < 1e-12, (setting, name)
+    for c in range(len(cases)):
+        name = "%d_W" % c
+        assert not np.array_equal(results["dfma"][name], results[""][name]), name
+
+
 @pytest.mark.parametrize("n,mc", [(600, 6), (2048, 40), (2049, 40), (20000, 5)])
 @pytest.mark.parametrize("case", ["equal rows", "one group of rows"])
 def test_update_mask_with_crowded_lists(k, port_kernels, n, mc, case):
