@@ -28,7 +28,7 @@ def sources() -> list[str]:
 
 
 def _deps() -> list[str]:
-    return sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(INCLUDE, "*.h"))
+    return sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(INCLUDE, "*.h"))
 
 
 def up_to_date() -> bool:

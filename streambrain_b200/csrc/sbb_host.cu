@@ -6,108 +6,14 @@
 // while the next is filled or drained.
 #include "sbb_host.cuh"
 
-#include <atomic>
-#include <chrono>
-#include <condition_variable>
 #include <cstdint>
-#include <cstring>
 #include <mutex>
-#include <thread>
-#include <vector>
+#include <new>
+
+#include "sbb_copy_threads.h"
 
 namespace sbb {
 namespace {
-
-// ---- memcpy by several threads ------------------------------------------------------------------
-// One job at a time, cut into pieces that the caller and the workers claim one by one: whoever is late, for a worker still
-// waking up, finds nothing left.  Workers spin for a while after a job (a copy is a series of jobs) before they sleep.
-class CopyThreads {
- public:
-  static CopyThreads &get() {
-    static CopyThreads t;
-    return t;
-  }
-  void copy(void *dst, const void *src, size_t bytes) {
-    if (bytes <= 2 * kPiece || workers_.empty() || !mutex_.try_lock()) {   // (busy with another thread's job)
-      std::memcpy(dst, src, bytes);
-      return;
-    }
-    const uint32_t pieces = (uint32_t)((bytes + kPiece - 1) / kPiece);
-    const uint64_t generation = (next_.load(std::memory_order_relaxed) >> 32) + 1;
-    dst_.store(static_cast<char *>(dst), std::memory_order_relaxed);
-    src_.store(static_cast<const char *>(src), std::memory_order_relaxed);
-    bytes_.store(bytes, std::memory_order_relaxed);
-    done_.store(0, std::memory_order_relaxed);
-    next_.store(generation << 32, std::memory_order_release);
-    if (asleep_.load() > 0) {
-      { std::lock_guard<std::mutex> l(sleep_mutex_); }
-      wake_.notify_all();
-    }
-    while (take_piece()) {
-    }
-    while (done_.load(std::memory_order_acquire) < pieces) std::this_thread::yield();
-    next_.store(generation << 32 | kClosed, std::memory_order_release);   // before the fields change again
-    mutex_.unlock();
-  }
-
- private:
-  static constexpr size_t kPiece = 128 << 10;
-  static constexpr uint32_t kClosed = 0xFFFFFFFFu;
-  CopyThreads() {
-    unsigned n = std::thread::hardware_concurrency() / 2;
-    if (n > 8) n = 8;
-    for (unsigned k = 1; k < n; ++k) workers_.emplace_back([this] { work(); });
-  }
-  ~CopyThreads() {
-    {
-      std::lock_guard<std::mutex> l(sleep_mutex_);
-      stop_.store(true);
-    }
-    wake_.notify_all();
-    for (auto &w : workers_) w.join();
-  }
-  // The fields change only while the job is closed, and a claim fails when the job number or its next piece has changed
-  // since they were read: fields read before a successful claim belong to the claimed job.
-  bool take_piece() {
-    uint64_t v = next_.load(std::memory_order_acquire);
-    while (true) {
-      char *dst = dst_.load(std::memory_order_relaxed);
-      const char *src = src_.load(std::memory_order_relaxed);
-      const size_t bytes = bytes_.load(std::memory_order_relaxed), at = (size_t)(uint32_t)v * kPiece;
-      if ((uint32_t)v == kClosed || at >= bytes) return false;
-      if (!next_.compare_exchange_weak(v, v + 1, std::memory_order_acq_rel)) continue;
-      std::memcpy(dst + at, src + at, bytes - at < kPiece ? bytes - at : kPiece);
-      done_.fetch_add(1, std::memory_order_release);
-      return true;
-    }
-  }
-  void work() {
-    while (!stop_.load(std::memory_order_relaxed)) {
-      const uint64_t seen = next_.load() >> 32;
-      bool any = false;
-      while (take_piece()) any = true;
-      const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(any ? 200 : 0);
-      while ((next_.load(std::memory_order_relaxed) >> 32) == seen && !stop_.load(std::memory_order_relaxed) &&
-             std::chrono::steady_clock::now() < until)
-        std::this_thread::yield();
-      if ((next_.load() >> 32) != seen) continue;
-      std::unique_lock<std::mutex> l(sleep_mutex_);
-      asleep_.fetch_add(1);
-      wake_.wait(l, [&] { return stop_.load() || (next_.load() >> 32) != seen; });
-      asleep_.fetch_sub(1);
-    }
-  }
-  std::vector<std::thread> workers_;
-  std::mutex mutex_, sleep_mutex_;
-  std::condition_variable wake_;
-  std::atomic<int> asleep_{0};
-  std::atomic<bool> stop_{false};
-  std::atomic<char *> dst_{nullptr};
-  std::atomic<const char *> src_{nullptr};
-  std::atomic<size_t> bytes_{0};
-  std::atomic<uint64_t> next_{kClosed};   // job number << 32 | next piece to claim
-  std::atomic<uint32_t> done_{0};
-};
 
 constexpr int kSlots = 4, kKept = 4;      // contexts kept for later calls: 32 MB of pinned memory at most
 constexpr size_t kSlotBytes = 2 << 20;
@@ -158,7 +64,8 @@ struct HostContext {
 
 namespace {
 std::mutex g_contexts_mutex;
-std::vector<HostContext *> g_contexts;   // free ones, at most kKept; the process's end gives them back
+HostContext *g_contexts[kKept];   // free ones; the process's end gives them back
+int g_free_contexts = 0;
 }  // namespace
 
 HostCall::HostCall() {
@@ -167,23 +74,23 @@ HostCall::HostCall() {
   if (error_ != cudaSuccess) return;
   {
     std::lock_guard<std::mutex> l(g_contexts_mutex);
-    for (size_t k = 0; k < g_contexts.size(); ++k)
+    for (int k = 0; k < g_free_contexts; ++k)
       if (g_contexts[k]->device == dev) {
         ctx_ = g_contexts[k];
-        g_contexts.erase(g_contexts.begin() + (long)k);
+        g_contexts[k] = g_contexts[--g_free_contexts];
         return;
       }
   }
-  ctx_ = new HostContext();
-  error_ = ctx_->create(dev);
+  ctx_ = new (std::nothrow) HostContext();
+  error_ = ctx_ != nullptr ? ctx_->create(dev) : cudaErrorMemoryAllocation;
 }
 
 HostCall::~HostCall() {
   if (ctx_ == nullptr) return;
   if (error_ == cudaSuccess) {
     std::lock_guard<std::mutex> l(g_contexts_mutex);
-    if ((int)g_contexts.size() < kKept) {
-      g_contexts.push_back(ctx_);
+    if (g_free_contexts < kKept) {
+      g_contexts[g_free_contexts++] = ctx_;
       return;
     }
   }
