@@ -149,6 +149,8 @@ class _DeviceLayer:
         if on_device:
             x = self._dev_input(inputs, self.in_features)
             y = self._dev_input(outputs, self.out_features)
+            if y.shape[0] < x.shape[0]:
+                raise ValueError("train_step: %d samples but %d outputs" % (x.shape[0], y.shape[0]))
             rc = lib.sbb_layer_train_step(self._handle, x.data_ptr(), y.data_ptr(), x.shape[0], h, _stream_ptr())
             if rc:
                 check(rc)
@@ -168,6 +170,8 @@ class _DeviceLayer:
         B = inputs.shape[0]
         x = np.ascontiguousarray(inputs, dtype=self.dtype)
         t = None if targets is None else np.ascontiguousarray(targets, dtype=self.dtype)
+        if x.size != B * self.in_features or (t is not None and t.size < B * self.out_features):
+            raise ValueError("step_host: shape mismatch")
         y = np.empty((B, self.out_features), dtype=self.dtype) if want_activation else None
         h = -1 if hypercolumn is None else int(hypercolumn)
         check(lib.sbb_layer_step_host(self._handle, host_ptr(x), None if t is None else host_ptr(t), B, h,
@@ -250,6 +254,8 @@ class _DeviceLayer:
             raise ValueError("the layer is row-sharded: its forward pass and train step run as one sharded_step")
         x = self._dev_input(inputs, self.in_features)
         y = self._dev_input(outputs, self.out_features)
+        if y.shape[0] < x.shape[0]:
+            raise ValueError("dp_train_step: %d samples but %d outputs" % (x.shape[0], y.shape[0]))
         pipelined_dp_step(_DeviceDPOps(self), x, y, hypercolumn, x.shape[0], world_size, all_reduce, row_blocks)
 
     # -- row-sharded layer over peer-mapped memory ----------------------------

@@ -533,6 +533,26 @@ def test_errors_are_reported_not_fatal(B200):
     assert _lib.lib.sbb_kernel_launches() > 0
 
 
+def test_outputs_too_short_for_the_samples_are_refused(B200):
+    """The native calls read batch rows of every operand: arrays that hold fewer are refused before anything runs."""
+    import torch
+    layer = B200.DenseLayer(12, 2, 4, 0.01, (0.1, 0.1, 0.01), np.float32)
+    before = layer.Cij
+    x, y = torch.rand((6, 12), device="cuda"), torch.rand((6, 8), device="cuda")
+    with pytest.raises(ValueError):
+        layer.train_step(x, y[:5])
+    with pytest.raises(ValueError):
+        layer.dp_train_step(x, y[:5], None, 1, lambda t: None)
+    xh, yh = x.cpu().numpy(), y.cpu().numpy()
+    for bad_x, bad_y in ((xh[:, :11], yh), (xh.ravel(), yh), (xh, yh[:5]), (xh, yh[:, :7])):
+        with pytest.raises(ValueError):
+            layer.step_host(bad_x, bad_y)
+    assert np.array_equal(layer.Cij, before)
+    layer.train_step(x, y)
+    layer.step_host(xh.reshape(6, 3, 4), yh)   # (any shape that holds the samples)
+    assert not np.array_equal(layer.Cij, before)
+
+
 @pytest.mark.parametrize("tag,dtype", [("f32", np.float32), ("f64", np.float64)])
 @pytest.mark.parametrize("kind", ["dense", "plastic"])
 @pytest.mark.parametrize("B,N,H,Mc", [(1, 1, 1, 2), (3, 31, 1, 8), (64, 33, 3, 3), (65, 512, 2, 8), (129, 513, 1, 10),
