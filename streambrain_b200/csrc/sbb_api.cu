@@ -168,7 +168,7 @@ struct sbb_layer {
   void *state[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   size_t state_bytes[7] = {0, 0, 0, 0, 0, 0, 0};
   Scratch fwd_partial;   // k-split partial sums of the forward product
-  Scratch score;         // mask-update scratch: per-row score, active count, candidate lists
+  Scratch score;         // mask-update scratch: per-row score, active count, filter key, old bit; best keys per block
   Scratch hx, hy, ht;    // staging for the host-buffer entry points
   Scratch ticket;        // finished blocks of a launch: [whole launch][per hypercolumn]; zero between launches
   Scratch rc;            // reciprocals of Ci and Cj (0 below the threshold) for the tensor-core trace update

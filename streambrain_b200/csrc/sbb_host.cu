@@ -2,8 +2,8 @@
 //
 // What bounds them is the copy by the CPU: a pageable cudaMemcpy stages the data through the driver's pinned buffer with
 // one thread (12 GB/s up, 21 GB/s down measured here, against some 55 GB/s of the link).  Here the pieces of a copy pass
-// through four pinned slots, several threads copy between the slots and the caller's memory, and the link moves one slot
-// while the next is filled or drained.
+// through four pinned slots, and the link moves one slot while the next is filled or drained; pieces of more than 256 KB,
+// that is copies of more than 1 MB, are copied between the slots and the caller's memory by several threads.
 #include "sbb_host.cuh"
 
 #include <cstdint>

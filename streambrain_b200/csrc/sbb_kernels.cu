@@ -1,15 +1,16 @@
 // General-shape CUDA kernels of the BCPNN layer train step (float and double).
 //
-// These are the kernels that accept any N, M, B (odd sizes, unaligned rows, the
-// 10-column classifier) and the float64 path; the tcgen05 tile kernels for
-// aligned float32 shapes live in their own translation unit and share the
-// arithmetic helpers below.
+// These are the contractions for any N, M, B (odd sizes, unaligned rows) and for
+// float64, and the softmax, the column vectors and the element-wise kernels of
+// every path.  The tcgen05 tile kernels for aligned float32 shapes, the kernels
+// for layers of few units or forward passes of few samples, and the mask update
+// have files of their own.
 //
 // Data layout: every matrix is row-major and contiguous.  x[B,N], y[B,M],
 // weights/Cij[N,M], wmask[N,H] bytes.  Both contractions of the step read their
 // operands "MN-major" (contiguous along the output dimension) except the forward
-// product's x, which is contiguous along the reduction dimension and is
-// transposed on its way into shared memory.
+// product's x, which is contiguous along the reduction dimension in memory and in
+// shared memory alike.
 #include "sbb_kernels.cuh"
 #include "sbb_f64_mma.cuh"
 #include "sbb_launch.cuh"

@@ -123,7 +123,8 @@ cudaError_t launch_apply_mask(T *w, const uint8_t *wmask, long N, long M, long H
 
 // Mask update for hypercolumn h.  `weights` null => the un-masked weight is
 // recomputed from the traces.  `scratch` holds mask_scratch_bytes(N, sizeof(T))
-// bytes (256-byte aligned): per-row score, active count and previous mask bit, candidate lists.  mask_scratch_init
+// bytes (256-byte aligned): per-row score, active count, filter key and previous mask bit, best keys per block of rows.
+// mask_scratch_init
 // prepares it once; every launch leaves it ready for the next.
 // `rewrite_w` non-null => the weights of hypercolumn h are recomputed from the traces, under the
 // new mask, for every row whose mask bit a swap changed.

@@ -124,7 +124,7 @@ struct TcSmem {
 // (the forward pass sums over in_features) are cut into short chains whose
 // results the epilogue warps add in full float32.
 template <bool A_KMAJOR, int BN, int BK, int STAGES, int CHAIN, bool PRESPLIT = false, bool PAIR = false>
-// 14 warps are allocated registers as 16: 128 registers per thread is the most that fits one CTA per SM.
+// (16 warps of 128 registers per thread: the whole register file, one CTA per SM)
 __global__ void __launch_bounds__(kThreads, 1)
     tc_contraction_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                           const __grid_constant__ CUtensorMap tmA3, const __grid_constant__ CUtensorMap tmB3,

@@ -112,7 +112,7 @@ def _oracle_mask_update(port_kernels, dev, hp, h, mask_before):
 
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 def test_stl10_full_size_mask_update_vs_oracle(B200, port_kernels, contraction_path, dtype):
-    """55296 input rows: the candidate-list search over 64 row chunks, from finite scores (the start state
+    """55296 input rows: the lists from some 860 blocks of 64 rows, from finite scores (the start state
     of the benchmark), must pick the connections the oracle picks from the same traces."""
     from streambrain_b200 import synthetic
     if dtype == np.float64 and contraction_path == "tensor":

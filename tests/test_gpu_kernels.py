@@ -169,7 +169,7 @@ def _mask_case(rs, n, hc, mc, dtype, density=0.3):
 
 
 @pytest.mark.parametrize("n,hc,mc", [(1, 1, 2), (53, 4, 6), (128, 2, 64), (700, 3, 100), (2500, 30, 10),
-                                     # 1024 rows and more take the candidate-list search instead of the full scan
+                                     # 2049 rows and more: listed from the blocks that have a row near the top
                                      (1024, 2, 8), (4096, 2, 8), (5000, 3, 20), (30011, 2, 10)])
 def test_update_mask_f64_identical_to_oracle(k, port_kernels, n, hc, mc):
     rs = np.random.RandomState(n)
@@ -204,7 +204,7 @@ def test_update_mask_edge_cases(k, port_kernels):
 def test_update_mask_with_nan_scores_at_the_head_of_a_class(k, port_kernels, n, iterations):
     """Always-on inputs (Ci == 1 and Cij == Cj) give NaN scores.  The reference's scan picks a NaN
     row exactly when it is the lowest-index row of its class, which can repeat swap after swap
-    (the row heads the other class next) -- the candidate-list search must follow it move by move.
+    (the row heads the other class next) -- the replay of the swaps must follow it move by move.
     Several low rows of both classes are made NaN, among them row 0 and the first silent row."""
     rs = np.random.RandomState(7 * n + iterations)
     wmask, w, Ci, Cj, Cij = _mask_case(rs, n, 3, 6, np.float64, density=0.5)
@@ -225,7 +225,7 @@ def test_update_mask_with_nan_scores_at_the_head_of_a_class(k, port_kernels, n, 
 def test_update_mask_with_nan_and_inf_scores(k, port_kernels, n):
     """Rows whose Ci is exactly 1 (an input that is always on) divide by zero in the score:
     +-inf and NaN scores must be ranked exactly as the reference's front-to-back scan ranks
-    them, in the full scan (small n) and in the candidate-list search."""
+    them, whether all rows are listed (small n) or those of the blocks with a row near the top."""
     rs = np.random.RandomState(n)
     wmask, w, Ci, Cj, Cij = _mask_case(rs, n, 3, 6, np.float64, density=0.4)
     for variant in range(3):
