@@ -773,9 +773,9 @@ def run_b200(args, wl, p, batch):
                     # DRAM bytes are not measured by this program: the ncu capture of this kernel is summarised
                     # in the named profile
                     "traffic": None,
-                    "traffic_source": "profiles/tc_contraction_kernels_stl10_f32.txt (dram__bytes_read.sum + "
-                                      "dram__bytes_write.sum of one launch under ncu)" if tensor_path else
-                                      "profiles/trace_update_simt_stl10_f32.txt",
+                    "traffic_source": "profiles/%s (dram__bytes_read.sum + dram__bytes_write.sum of one launch under ncu)" %
+                                      ("tc_contraction_kernels_stl10_f32.txt" if tensor_path else
+                                       "general_path_kernels_stl10_f32.txt"),
                     "peak_source": peak_kind, "algorithmic_bytes": upd_b,
                     "ms_per_launch": per_step_trace,
                     "forward_ms": (sum(fwd_ms) / len(fwd_ms)) if fwd_ms else None,
