@@ -140,6 +140,25 @@ def test_trace_update_vs_oracle(k, port_kernels, tag, dtype, B, N, H, Mc):
     assert weight_err(w1, w2) < 10 * tol
 
 
+def test_float64_logarithm_of_the_trace_update(k):
+    """The float64 trace update's own logarithm (a table of 128 and a series).  With Ci = Cj = 1 the weight is the logarithm
+    of the new Cij as returned.  Bound: two roundings below 2^-54 on the way to ln m, the series' remainder and r's rounding
+    below 1e-17, the last rounding 2^-53 |ln x|, and e times the rounding of ln 2 (2.4e-17): within 3e-16 max(1, |ln x|)."""
+    rs = np.random.RandomState(11)
+    N, M = 257, 130
+    x = 2.0 ** rs.uniform(-390, 990, (N, M))
+    x[:64] = rs.uniform(0.5, 2.0, (64, M))                       # both sides of one
+    x[64:128] = 1 + rs.uniform(-1, 1, (64, M)) * 10.0 ** rs.uniform(-16, -2, (64, M))
+    edges = 1 + (np.arange(128) + rs.choice([-1, 0, 1], 128) * 2.0 ** -45) / 128   # ends of the table's intervals
+    x[128:138, :128] = edges * 2.0 ** rs.randint(-20, 20, (10, 128))
+    Ci, Cj, Cij, W = k.update_weights(np.ones(N), np.full(M, 2.0), 2 * x, np.ones((1, N)), np.zeros((1, M)), 0.5,
+                                      np.zeros((N, M)), 1e-30)
+    assert np.all(Ci == 1) and np.all(Cj == 1) and np.array_equal(Cij, x)
+    want = np.log(x.astype(np.longdouble))
+    err = np.abs(W.astype(np.longdouble) - want) / np.maximum(1, np.abs(want))
+    assert float(err.max()) < 3e-16, float(err.max())
+
+
 @pytest.mark.parametrize("tag,dtype", DTYPES)
 def test_bias_kernels_vs_oracle(k, port_kernels, tag, dtype):
     rs = np.random.RandomState(5)
