@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   auto bar_slab = [&](int e, int gr) { return bars + 8u * (3 * kStages + 9 + kGroups * e + gr); };
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L::BAR_OFFSET + L::BARS * 8);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // (uniform)
   const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
 
   if (threadIdx.x == 0) {
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (warp == kTma) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (long w = w_first; w < total && ok; w += w_step) {
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == kMma) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       // D float32, A (tensor memory) and B (shared memory, MN-major) TF32; 256 rows over the pair (or 128), kBN columns
       constexpr uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | (1u << 16) | ((uint32_t)(kBN >> 3) << 17) |
                                  ((uint32_t)((PAIR ? 256 : 128) >> 4) << 24);
