@@ -59,7 +59,10 @@ struct TcHost {
   bool pairs;    // false: SBB_TC_PAIR=0
 };
 bool tc_host(TcHost *out);
-bool tc_map_2d(void *map, const float *base, long inner, long outer, int box_inner, int box_outer, bool mn_major);
+// How a box lands in shared memory: rows of 128 or of 64 bytes under the swizzle of that width, or rows of 128 bytes under
+// the flavour of the 128-byte swizzle (32-byte base) that MN-major 32-bit operands need.
+enum { kMapRows = 0, kMapMnMajor = 1, kMapRows64 = 2 };
+bool tc_map_2d(void *map, const float *base, long inner, long outer, int box_inner, int box_outer, int layout);
 bool tc_map_chunks(void *map, const float *base, long cols, long rows, int box_rows, int box_chunks);
 
 // Launches so far whose CTAs worked in pairs.

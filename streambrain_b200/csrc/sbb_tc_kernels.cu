@@ -105,7 +105,9 @@ struct TcSmem {
   // tensor memory: two accumulators, then (not PRESPLIT) per stage BK columns of A hi and BK of A lo
   static constexpr int TMEM_A_COL = 2 * BN;
   static constexpr int TMEM_COLS = 512;
-  static_assert(2 * BN + (PRESPLIT ? 0 : STAGES * 2 * BK) <= TMEM_COLS, "tensor memory budget");
+  // A's parts of this many k-blocks fit beside the accumulators; shared memory may hold more stages than that
+  static constexpr int SLOTS = (TMEM_COLS - 2 * BN) / (2 * BK) < STAGES ? (TMEM_COLS - 2 * BN) / (2 * BK) : STAGES;
+  static_assert(PRESPLIT || SLOTS >= 2, "tensor memory budget");
   static_assert(STAGE_BYTES % 1024 == 0, "stages keep the 1024-byte swizzle alignment");
   static constexpr int SLAB_OFFSET = STAGES * STAGE_BYTES;
   // two 32 x 32 block buffers per epilogue warp: staging for the TMA stores of the raw product
@@ -320,7 +322,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             tc_fence_after();
             const uint32_t b_hi = base + s * SM::STAGE_BYTES + SM::A_BYTES;
             const uint32_t b_lo = base + s * SM::STAGE_BYTES + SM::RAW_BYTES;
-            const uint32_t ta_hi = tmem_base + SM::TMEM_A_COL + s * (2 * BK);
+            const uint32_t ta_hi = tmem_base + SM::TMEM_A_COL + (it % SM::SLOTS) * (2 * BK);
 #pragma unroll
             for (int kk = 0; kk < BK / 8; ++kk) {
               // One MMA consumes 8 k-values: 8 columns of A in tensor memory, eight 128-byte rows
@@ -373,7 +375,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int kb = 0; kb < nkb; ++kb, ++it) {
         const int s = it % STAGES;
         const uint32_t ph = (it / STAGES) & 1u;
-        if (!mbar_wait(bar_full(s), ph, abort_flag, status, kWaitFull)) { ok = false; break; }
+        if (!mbar_wait_warp(bar_full(s), ph, abort_flag, status, kWaitFull)) { ok = false; break; }
         if (threadIdx.x == 0 && kb == 0) TC_TRACE((w - w_first) / w_step, 5);
         if (threadIdx.x == 0 && kb == nkb - 1) TC_TRACE((w - w_first) / w_step, 9);
         static_assert(kConvWarps == 4, "one A row (tensor-memory lane) per converter thread");
@@ -397,7 +399,14 @@ __global__ void __launch_bounds__(kThreads, 1)
           for (int k = 0; k < BK; ++k)
             r[k] = *reinterpret_cast<const uint32_t *>(acol + k * 128 + ((((lane >> 3) ^ (k & 3))) << 5));
         }
-        const uint32_t ta = tmem_base + SM::TMEM_A_COL + s * (2 * BK) + ((uint32_t)(warp * 32) << 16);
+        if constexpr (SM::SLOTS < STAGES) {   // the k-block whose place in tensor memory this one takes has been multiplied
+          if (it >= SM::SLOTS) {
+            const uint32_t old = it - SM::SLOTS;
+            if (!mbar_wait_warp(bar_empty(old % STAGES), (old / STAGES) & 1u, abort_flag, status, kWaitEmpty)) { ok = false; break; }
+            tc_fence_after();
+          }
+        }
+        const uint32_t ta = tmem_base + SM::TMEM_A_COL + (it % SM::SLOTS) * (2 * BK) + ((uint32_t)(warp * 32) << 16);
         tmem_st_32x32b<BK>(ta, r);
 #pragma unroll
         for (int k = 0; k < BK; ++k) r[k] = __float_as_uint(tf32_lo(__uint_as_float(r[k])));
@@ -442,7 +451,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int kb = 0; kb < nkb; ++kb, ++it) {
         const int s = it % STAGES;
         const uint32_t ph = (it / STAGES) & 1u;
-        if (!mbar_wait(bar_full(s), ph, abort_flag, status, kWaitFull)) { ok = false; break; }
+        if (!mbar_wait_warp(bar_full(s), ph, abort_flag, status, kWaitFull)) { ok = false; break; }
         // lo parts beside the raw tile in shared memory; every load is issued before the first store
         constexpr int kBThreads = kBConvWarps * 32;
         const float4 *rawb = reinterpret_cast<const float4 *>(smem + s * SM::STAGE_BYTES + SM::A_BYTES);
@@ -526,7 +535,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int nchains = (nkb + CHAIN - 1) / CHAIN;
         for (int c = 0; c < nchains && ok; ++c, ++chain) {
           const uint32_t buf = chain & 1u, aph = (chain >> 1) & 1u;
-          if (!mbar_wait(bar_acc_full(buf), aph, abort_flag, status, kWaitAccFull)) { ok = false; break; }
+          if (!mbar_wait_warp(bar_acc_full(buf), aph, abort_flag, status, kWaitAccFull)) { ok = false; break; }
           __syncwarp();
           tc_fence_after();
 #pragma unroll
@@ -565,7 +574,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       } else {
         const uint32_t buf = chain & 1u, aph = (chain >> 1) & 1u;
-        if (!mbar_wait(bar_acc_full(buf), aph, abort_flag, status, kWaitAccFull)) { ok = false; break; }
+        if (!mbar_wait_warp(bar_acc_full(buf), aph, abort_flag, status, kWaitAccFull)) { ok = false; break; }
         if (threadIdx.x == kConvWarps * 32) TC_TRACE(chain, 3);
         __syncwarp();
         tc_fence_after();
@@ -722,21 +731,20 @@ struct MapCache {
 thread_local MapCache g_map_cache;
 
 bool make_map_uncached(CUtensorMap *map, const float *base, long inner, long outer, int box_inner, int box_outer,
-                       bool mn_major);
+                       int layout);
 bool make_map_chunks_uncached(CUtensorMap *map, const float *base, long cols, long rows, int box_rows, int box_chunks);
 
-// 2-D float32 tensor map over a row-major [outer, inner] matrix, zero fill.  `mn_major` selects the
-// 32-byte-base flavour of the 128-byte swizzle that MN-major 32-bit operands need.
+// 2-D float32 tensor map over a row-major [outer, inner] matrix, zero fill.
 bool make_map(CUtensorMap *map, const float *base, long inner, long outer, int box_inner, int box_outer,
-              bool mn_major) {
-  const MapKey k{base, inner, outer, box_inner, box_outer, mn_major ? 1 : 0};
+              int layout) {
+  const MapKey k{base, inner, outer, box_inner, box_outer, layout};
   if (g_map_cache.find(k, map)) return true;
-  if (!make_map_uncached(map, base, inner, outer, box_inner, box_outer, mn_major)) return false;
+  if (!make_map_uncached(map, base, inner, outer, box_inner, box_outer, layout)) return false;
   g_map_cache.put(k, *map);
   return true;
 }
 bool make_map_chunks(CUtensorMap *map, const float *base, long cols, long rows, int box_rows, int box_chunks) {
-  const MapKey k{base, cols, rows, box_rows, box_chunks, 2};
+  const MapKey k{base, cols, rows, box_rows, box_chunks, -1};
   if (g_map_cache.find(k, map)) return true;
   if (!make_map_chunks_uncached(map, base, cols, rows, box_rows, box_chunks)) return false;
   g_map_cache.put(k, *map);
@@ -744,14 +752,16 @@ bool make_map_chunks(CUtensorMap *map, const float *base, long cols, long rows, 
 }
 
 bool make_map_uncached(CUtensorMap *map, const float *base, long inner, long outer, int box_inner, int box_outer,
-                       bool mn_major) {
+                       int layout) {
   cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
   cuuint64_t strides[1] = {(cuuint64_t)inner * sizeof(float)};
   cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer};
   cuuint32_t estr[2] = {1, 1};
   const CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims, strides, box,
                               estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              mn_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
+                              layout == kMapMnMajor ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B
+                              : layout == kMapRows64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                                     : CU_TENSOR_MAP_SWIZZLE_128B,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
@@ -869,8 +879,8 @@ bool tc_host(TcHost *out) {
   out->pairs = pairs_enabled();
   return out->status != nullptr && init_once();
 }
-bool tc_map_2d(void *map, const float *base, long inner, long outer, int box_inner, int box_outer, bool mn_major) {
-  return make_map(static_cast<CUtensorMap *>(map), base, inner, outer, box_inner, box_outer, mn_major);
+bool tc_map_2d(void *map, const float *base, long inner, long outer, int box_inner, int box_outer, int layout) {
+  return make_map(static_cast<CUtensorMap *>(map), base, inner, outer, box_inner, box_outer, layout);
 }
 bool tc_map_chunks(void *map, const float *base, long cols, long rows, int box_rows, int box_chunks) {
   return make_map_chunks(static_cast<CUtensorMap *>(map), base, cols, rows, box_rows, box_chunks);
@@ -892,11 +902,14 @@ bool tc_available() {
 
 bool tc_shape_ok(const void *x, const void *y_or_w, long N, long M) {
   return N % 4 == 0 && M % 4 == 0 && N >= 4 && M >= 4 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 &&
-         (reinterpret_cast<uintptr_t>(y_or_w) & 15u) == 0 && N < 2147483647L && M < 2147483647L;
+         (reinterpret_cast<uintptr_t>(y_or_w) & 15u) == 0 && N < 2147483136L && M < 2147483136L;   // (tile coordinates in 32 bits)
 }
 
 namespace {
-constexpr int kFwdBN = 128, kFwdBK = 32, kFwdStages = 4;
+// A stage of a pair is 32 KB and its MMAs take 0.39 us: six of them cover the 2 us from asking for a k-block until its place is
+// free again (fetch, split, multiply), four did not; tensor memory has room for the split rows of four.  Forward pass with four
+// and with six: 55296 -> 30 x 100 at batch 256 356 and 338 us, 1568 -> 100 x 300 at 1024 418 and 386.
+constexpr int kFwdBN = 128, kFwdBK = 32, kFwdStages = 4, kFwdPairStages = 6;
 constexpr int kFwdPrefetch = 0;  // k-blocks of W requested into L2 ahead of the shared-memory pipeline (measured: no gain at 4-16)
 constexpr int kFwdChain = 4;  // 4 k-blocks of 32 = 128 k-values (48 MMAs) per tensor-memory accumulation chain
 constexpr int kTrBN = 192, kTrBK = 16, kTrStages = 4;
@@ -964,7 +977,7 @@ cudaError_t launch_forward_product_tc(const float *x, const float *w, float *par
   forward_split_plan(B, N, M, plan_splits, k_per_split);
   if (plan_splits != splits) return cudaErrorInvalidValue;
   TcMaps tm;
-  if (!make_map(&tm.a, x, N, B, 32, 128, false) || !make_map(&tm.b, w, M, N, 32, kFwdBK, true)) return cudaErrorInvalidValue;
+  if (!make_map(&tm.a, x, N, B, 32, 128, kMapRows) || !make_map(&tm.b, w, M, N, 32, kFwdBK, kMapMnMajor)) return cudaErrorInvalidValue;
   tm.a3 = tm.a;
   tm.c = tm.a;
   // CTA pairs when the row tiles pair up: the two CTAs that need the same tile of W each fetch half of it
@@ -982,7 +995,7 @@ cudaError_t launch_forward_product_tc(const float *x, const float *w, float *par
   ep.rows = B;
   ep.cols = M;
   ep.ld = M;
-  cudaError_t e = pair ? launch_tc_pair<true, kFwdBN, kFwdBK, kFwdStages, kFwdChain>(tm, wk, ep, st)
+  cudaError_t e = pair ? launch_tc_pair<true, kFwdBN, kFwdBK, kFwdPairStages, kFwdChain>(tm, wk, ep, st)
                        : launch_tc<true, kFwdBN, kFwdBK, kFwdStages, kFwdChain>(tm, wk, ep, st);
   if (e == cudaSuccess) count_launches(1);
   return e;
@@ -993,7 +1006,7 @@ namespace {
 // (pre != 0) of their low-part planes.  a3 / b3 report whether the one-box 3-D forms exist.
 bool batch_operand_maps(TcMaps &tm, const float *x, const float *y, const float *x_lo, const float *y_lo, bool pre,
                         long B, long N, long M, int bn, bool &a3, bool &b3) {
-  if (!make_map(&tm.a, x, N, B, 32, kTrBK, true) || !make_map(&tm.b, y, M, B, 32, kTrBK, true)) return false;
+  if (!make_map(&tm.a, x, N, B, 32, kTrBK, kMapMnMajor) || !make_map(&tm.b, y, M, B, 32, kTrBK, kMapMnMajor)) return false;
   a3 = N % 32 == 0 && make_map_chunks(&tm.a3, x, N, B, kTrBK, 4);
   if (!a3) tm.a3 = tm.a;
   b3 = make_map_chunks(&tm.b3, y, M, B, kTrBK, bn / 32);
@@ -1003,7 +1016,7 @@ bool batch_operand_maps(TcMaps &tm, const float *x, const float *y, const float 
   tm.a3lo = tm.a3;
   tm.b3lo = tm.b3;
   if (pre) {
-    if (!make_map(&tm.alo, x_lo, N, B, 32, kTrBK, true) || !make_map(&tm.blo, y_lo, M, B, 32, kTrBK, true)) return false;
+    if (!make_map(&tm.alo, x_lo, N, B, 32, kTrBK, kMapMnMajor) || !make_map(&tm.blo, y_lo, M, B, 32, kTrBK, kMapMnMajor)) return false;
     if (a3 && !make_map_chunks(&tm.a3lo, x_lo, N, B, kTrBK, 4)) return false;
     if (b3 && !make_map_chunks(&tm.b3lo, y_lo, M, B, kTrBK, bn / 32)) return false;
   }
@@ -1041,7 +1054,7 @@ cudaError_t launch_outer_product_tc(const float *x, const float *y, long B, long
     ep.rows = rows;
     ep.cols = M;
     ep.ld = M;
-    ep.tma_store = (reinterpret_cast<uintptr_t>(ep.out) & 15u) == 0 && make_map(&tm.c, ep.out, M, rows, 32, 32, false);
+    ep.tma_store = (reinterpret_cast<uintptr_t>(ep.out) & 15u) == 0 && make_map(&tm.c, ep.out, M, rows, 32, 32, kMapRows);
     if (!ep.tma_store) tm.c = tm.a;
     cudaError_t e = pre ? launch_tc<false, kLongBN, kTrBK, kLongStages, kTrChainKb, true>(tm, wk, ep, st, true)
                         : launch_tc<false, kLongBN, kTrBK, kLongStages, kTrChainKb>(tm, wk, ep, st, true);
@@ -1057,7 +1070,7 @@ cudaError_t launch_outer_product_tc(const float *x, const float *y, long B, long
   ep.rows = rows;
   ep.cols = M;
   ep.ld = M;
-  ep.tma_store = (reinterpret_cast<uintptr_t>(ep.out) & 15u) == 0 && make_map(&tm.c, ep.out, M, rows, 32, 32, false);
+  ep.tma_store = (reinterpret_cast<uintptr_t>(ep.out) & 15u) == 0 && make_map(&tm.c, ep.out, M, rows, 32, 32, kMapRows);
   if (!ep.tma_store) tm.c = tm.a;
   // the one contraction that runs beside a collective (the reduction of the previous row block)
   cudaError_t e = pre ? launch_tc<false, kTrBN, kTrBK, kTrStages, 0, true>(tm, wk, ep, st, true)
