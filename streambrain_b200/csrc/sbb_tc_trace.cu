@@ -10,7 +10,8 @@
 // devices that cannot place pairs.  Train step without a mask update: 1568 -> 30 x 100 at batch 128 32.1 us in pairs, 33.2
 // without; 55296 -> 30 x 100 at 256 565 and 686 us.)
 // Roles in a CTA (672 threads, one CTA per SM, tiles walked persistently):
-//   warps 0-11   epilogue: accumulator, old trace (by TMA, the whole tile's blocks one tile ahead), arithmetic, stores
+//   warps 0-11   epilogue: accumulator, old trace (by TMA, the whole tile's blocks one tile ahead), arithmetic; new traces
+//                and weights leave by TMA
 //   warps 12-15  A converters (one tile row, that is one tensor-memory lane, per thread)
 //   warp 16      TMA producer (one lane)
 //   warp 17      MMA issuer (one lane of the pair's leader) and owner of the tensor-memory allocation
@@ -43,6 +44,7 @@ constexpr int kGroups = kBN / (kEpi / 4) / 32;   // 32-column groups per epilogu
 constexpr int kABytes = 128 * kBK * 4;
 constexpr int kTmemA = 2 * kBN;                  // two accumulators, then per stage kBK columns of A hi and as many of A lo
 constexpr int kSlab = 32 * 32 * 4;               // a 32 x 32 block of the trace matrix
+constexpr int kHalf = kSlab / 2;                 // 32 rows x 16 columns of weights
 struct TileVectors {
   float rci[128], rcj[kBN];     // reciprocals of Ci and Cj, 0 below the threshold
   uint32_t bits[128];           // per row: bit k = mask of hypercolumn (the tile's first) + k
@@ -50,13 +52,15 @@ struct TileVectors {
 template <bool PAIR>
 struct Layout {
   static constexpr int BNH = PAIR ? kBN / 2 : kBN;   // columns of B a CTA stages
-  static constexpr int STAGES = PAIR ? 4 : 3;        // (tensor memory holds the A parts of four stages)
+  static constexpr int STAGES = PAIR ? 5 : 3;        // stages in shared memory
+  static constexpr int SLOTS = PAIR ? 4 : 3;         // k-blocks whose A parts tensor memory holds
   static constexpr int B_BYTES = BNH * kBK * 4;
   static constexpr int TX = kABytes + B_BYTES, STAGE = TX + B_BYTES;   // [A | B | B lo]
-  static_assert(kTmemA + STAGES * 2 * kBK <= 512, "tensor memory budget");
+  static_assert(SLOTS <= STAGES && kTmemA + SLOTS * 2 * kBK <= 512, "tensor memory budget");
   static_assert(STAGE % 1024 == 0 && kABytes % 1024 == 0 && TX % 1024 == 0, "swizzle alignment");
   static constexpr int SLAB_OFFSET = STAGES * STAGE;
-  static constexpr int VEC_OFFSET = SLAB_OFFSET + kEpi * kGroups * kSlab;
+  static constexpr int W_OFFSET = SLAB_OFFSET + kEpi * kGroups * kSlab;   // weights on their way out
+  static constexpr int VEC_OFFSET = W_OFFSET + kEpi * kHalf;
   static constexpr int BAR_OFFSET = VEC_OFFSET + 2 * (int)sizeof(TileVectors);
   // full, converted, empty per stage; acc_full[2], acc_empty[2], drain, vec_full[2], vec_empty[2]; one per block of the tile
   static constexpr int BARS = 3 * STAGES + 9 + kEpi * kGroups;
@@ -69,13 +73,12 @@ struct Trace {
   int a_box3, b_box3_tiles;   // A, and column tiles below the limit of B, come in one 3-D box per stage
   int lose_arrive;            // test hook: converter thread 0 of CTA 0 skips its arrival for the first stage
   long long wait_limit;
-  long rows, cols;            // N, M
+  int rows, cols;             // N, M
   const float *rci, *rcj;
-  float *Cij, *W;
   const uint8_t *wmask;
   uint32_t hc_magic;          // ceil(2^32 / Mc) where that divides every column exactly, else 0
-  long H, Mc;
-  int fast_ok;                // select words usable: Mc >= 32 (or no mask) and cthr^4 a normal float
+  int H, Mc;
+  int normal;                 // cthr^4 is a normal float: every logarithm's argument is
   float one_minus, cthr4, ema_scale;
 };
 
@@ -83,10 +86,10 @@ template <bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
     trace_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmA3, const __grid_constant__ CUtensorMap tmB3,
-                 const __grid_constant__ CUtensorMap tmC, const Trace g, int *status) {
+                 const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmW, const Trace g, int *status) {
   using L = Layout<PAIR>;
   constexpr int kStages = L::STAGES, kStage = L::STAGE, kBNH = L::BNH, kBBytes = L::B_BYTES, kTx = L::TX;
-  constexpr int kSlabOffset = L::SLAB_OFFSET, kVecOffset = L::VEC_OFFSET;
+  constexpr int kSlots = L::SLOTS, kSlabOffset = L::SLAB_OFFSET, kVecOffset = L::VEC_OFFSET;
   extern __shared__ uint8_t smem_dyn[];
   const uint32_t dyn_base = smem_u32(smem_dyn);
   const uint32_t base = (dyn_base + 1023u) & ~1023u;   // swizzle atoms need 1024-byte alignment
@@ -150,31 +153,24 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   // The clusters walk the tiles side by side, columns fastest (rows fastest where the columns are the longer side): at any
   // time they share the operands of a few row tiles.
-  const long total = (long)g.m_units * g.n_tiles;
-  const long w_first = PAIR ? blockIdx.x >> 1 : blockIdx.x, w_step = PAIR ? gridDim.x >> 1 : gridDim.x;
-  auto decode = [&](long w, int &mt, int &nt) {
-    if (g.m_fastest) {
-      mt = (int)(w % g.m_units);
-      nt = (int)(w / g.m_units);
-    } else {
-      nt = (int)(w % g.n_tiles);
-      mt = (int)(w / g.n_tiles);
-    }
+  const uint32_t total = (uint32_t)g.m_units * (uint32_t)g.n_tiles;
+  const uint32_t w_first = PAIR ? blockIdx.x >> 1 : blockIdx.x, w_step = PAIR ? gridDim.x >> 1 : gridDim.x;
+  auto decode = [&](uint32_t w, int &mt, int &nt) {
+    const uint32_t fast = g.m_fastest ? g.m_units : g.n_tiles, slow_at = w / fast, fast_at = w - slow_at * fast;
+    mt = (int)(g.m_fastest ? fast_at : slow_at);
+    nt = (int)(g.m_fastest ? slow_at : fast_at);
     if (PAIR) mt = 2 * mt + (int)rank;   // may be one past the last row tile: such a CTA stages zeros and stores nothing
   };
-  auto hc_of = [&](long n) -> int { return g.hc_magic ? (int)__umulhi((uint32_t)n, g.hc_magic) : (int)(n / g.Mc); };
-  auto first_hc = [&](int nt) -> int { return g.wmask ? hc_of((long)nt * kBN) : 0; };
-  auto last_hc = [&](int nt) -> int {
-    const long n = (long)nt * kBN + kBN - 1;
-    return g.wmask ? hc_of(n < g.cols ? n : g.cols - 1) : 0;
-  };
+  auto hc_of = [&](int n) -> int { return (int)(g.hc_magic ? __umulhi((uint32_t)n, g.hc_magic) : (uint32_t)n / (uint32_t)g.Mc); };
+  auto first_hc = [&](int nt) -> int { return g.wmask ? hc_of(nt * kBN) : 0; };
+  auto last_hc = [&](int nt) -> int { return g.wmask ? hc_of(min(nt * kBN + kBN, g.cols) - 1) : 0; };
 
   if (warp == kTma) {
     // ------------------------------------------------------------ TMA producer
     if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
-      for (long w = w_first; w < total && ok; w += w_step) {
+      for (uint32_t w = w_first; w < total && ok; w += w_step) {
         int mt, nt;
         decode(w, mt, nt);
         for (int kb = 0; kb < g.kblocks; ++kb, ++it) {
@@ -215,7 +211,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       };
       uint32_t it = 0, chain = 0;
       bool ok = true;
-      for (long w = w_first; w < total && ok; w += w_step) {
+      for (uint32_t w = w_first; w < total && ok; w += w_step) {
         for (int kb = 0; kb < g.kblocks && ok;) {
           const uint32_t buf = chain & 1u;
           if (!mbar_wait(bar_acc_empty(buf), ((chain >> 1) & 1u) ^ 1u, abort_flag, status, kWaitAccEmpty)) { ok = false; break; }
@@ -227,7 +223,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (!mbar_wait(bar_conv(s), (it / kStages) & 1u, abort_flag, status, kWaitConv)) { ok = false; break; }
             tc_fence_after();
             const uint32_t b_hi = base + s * kStage + kABytes, b_lo = base + s * kStage + kTx;
-            const uint32_t ta = tmem_base + kTmemA + s * (2 * kBK);
+            const uint32_t ta = tmem_base + kTmemA + (it % kSlots) * (2 * kBK);
 #pragma unroll
             for (int kk = 0; kk < kBK / 8; ++kk) {   // eight 128-byte rows (two 4-row swizzle atoms) of B per instruction
               const uint64_t db_hi = smem_desc_mn(b_hi + kk * 1024, kBK * 128), db_lo = smem_desc_mn(b_lo + kk * 1024, kBK * 128);
@@ -253,10 +249,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint32_t it = 0;
     bool ok = true;
     const int cw = warp - kConv;   // tensor-memory lane quarter (kConv is a multiple of four)
-    for (long w = w_first; w < total && ok; w += w_step)
+    for (uint32_t w = w_first; w < total && ok; w += w_step)
       for (int kb = 0; kb < g.kblocks; ++kb, ++it) {
         const int s = it % kStages;
-        if (!mbar_wait(bar_full(s), (it / kStages) & 1u, abort_flag, status, kWaitFull)) { ok = false; break; }
+        if (!mbar_wait_warp(bar_full(s), (it / kStages) & 1u, abort_flag, status, kWaitFull)) { ok = false; break; }
         // MN-major tile [32-row chunk][k][32 rows]: element (k, m) of chunk m / 32 sits in the 128-byte line k at 32-byte
         // piece ((m % 32) / 8) ^ (k % 4); a warp reads one line per k
         const uint8_t *acol = smem + s * kStage + cw * (kBK * 128) + ((lane & 7) << 2);
@@ -264,7 +260,14 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
         for (int k = 0; k < kBK; ++k)
           r[k] = *reinterpret_cast<const uint32_t *>(acol + k * 128 + (((lane >> 3) ^ (k & 3)) << 5));
-        const uint32_t ta = tmem_base + kTmemA + s * (2 * kBK) + ((uint32_t)(cw * 32) << 16);
+        if constexpr (kSlots < kStages) {   // the k-block whose place in tensor memory this one takes has been multiplied
+          if (it >= kSlots) {
+            const uint32_t old = it - kSlots;
+            if (!mbar_wait_warp(bar_empty(old % kStages), (old / kStages) & 1u, abort_flag, status, kWaitEmpty)) { ok = false; break; }
+            tc_fence_after();
+          }
+        }
+        const uint32_t ta = tmem_base + kTmemA + (it % kSlots) * (2 * kBK) + ((uint32_t)(cw * 32) << 16);
         tmem_st_32x32b<kBK>(ta, r);
 #pragma unroll
         for (int k = 0; k < kBK; ++k) r[k] = __float_as_uint(tf32_lo(__uint_as_float(r[k])));
@@ -278,10 +281,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint32_t it = 0;
     bool ok = true;
     const int t = threadIdx.x - kConvB * 32;
-    for (long w = w_first; w < total && ok; w += w_step)
+    for (uint32_t w = w_first; w < total && ok; w += w_step)
       for (int kb = 0; kb < g.kblocks; ++kb, ++it) {
         const int s = it % kStages;
-        if (!mbar_wait(bar_full(s), (it / kStages) & 1u, abort_flag, status, kWaitFull)) { ok = false; break; }
+        if (!mbar_wait_warp(bar_full(s), (it / kStages) & 1u, abort_flag, status, kWaitFull)) { ok = false; break; }
         const float4 *raw = reinterpret_cast<const float4 *>(smem + s * kStage + kABytes);
         float4 *low = reinterpret_cast<float4 *>(smem + s * kStage + kTx);
         constexpr int kPieces = kBBytes / 16 / (kBWarps * 32);
@@ -303,7 +306,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else if (warp == kVec) {
     // ------------------------------------------------------------ row and column data, one tile ahead
     uint32_t t = 0;
-    for (long w = w_first; w < total; w += w_step, ++t) {
+    for (uint32_t w = w_first; w < total; w += w_step, ++t) {
       int mt, nt;
       decode(w, mt, nt);
       const uint32_t b = t & 1u;
@@ -342,141 +345,133 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else {
     // ------------------------------------------------------------ epilogue
-    // Thread (lane) owns four tile rows (16*hh + lane/4 + 8*rr) of its warp's TMEM lane quarter and, per 32-column group,
-    // the column pairs 8*rep + 2*(lane%4) + {0,1}: four lanes cover 32 contiguous bytes of a row.
+    // A thread owns one row of the tile and 16 of its columns at a time: what belongs to the row (reciprocal, mask bits) is
+    // one register, what belongs to a column the same word for all lanes, and the trace block is read and written back in
+    // 16-byte pieces of the thread's own row; the arithmetic is two-wide.  New traces leave from where the old ones landed,
+    // weights from a buffer of the warp's own, both by TMA.  With four rows and eight scattered column pairs to a thread it
+    // was 37 instructions an element and 5 million store requests of eight bytes a lane at 55296 x 3000; a tile took longer
+    // here than in the tensor core.  Train step without a mask update, before and now: 1568 -> 30 x 100 at batch 128 30.8
+    // and 23.3 us, 1568 -> 100 x 300 at 1024 541 and 494; 55296 -> 30 x 100 at 256 546 both (there it is memory, and the
+    // fetches that wait for it).
     const int q = warp & 3, ch = warp >> 2;     // lane quarter, third of the tile's columns
-    const int lr = lane >> 2, lc = (lane & 3) * 2;
-    uint32_t swz[4];                            // byte offset of column pair `rep` inside a swizzled 128-byte row
-#pragma unroll
-    for (int rep = 0; rep < 4; ++rep) swz[rep] = ((uint32_t)((2 * rep + (lc >> 2)) ^ lr) << 4) + (uint32_t)(lc & 3) * 4u;
-    const long w_minus_c = g.W - g.Cij;         // the weight of an element sits this far from its trace
     const int nchains = (g.kblocks + kChainKb - 1) / kChainKb;
-    const bool has_mask = g.wmask != nullptr;
+    const uint32_t slabs = base + kSlabOffset + warp * kGroups * kSlab, wbuf = base + L::W_OFFSET + warp * kHalf;
+    uint8_t *slab_row = smem + kSlabOffset + warp * kGroups * kSlab + lane * 128;
+    uint8_t *w_row = smem + L::W_OFFSET + warp * kHalf + lane * 64;
+    const uint64_t scale2 = pair_of(g.ema_scale, g.ema_scale), ln2 = pair_of(kLn2, kLn2);
     uint32_t chain = 0, tile = 0;
     bool ok = true;
-    // this warp's block of the old trace: column group gr of tile (mt, nt)
-    auto issue_slab = [&](int mt, int nt, int gr) {
-      mbar_arrive_expect_tx(bar_slab(warp, gr), kSlab);
-      tma_load_2d(base + kSlabOffset + (warp * kGroups + gr) * kSlab, &tmC, nt * kBN + (ch * kGroups + gr) * 32, mt * 128 + 32 * q,
-                  bar_slab(warp, gr));
-    };
-    if (lane == 0 && w_first < total) {
+    // this warp's block of the old trace: column group gr of tile w
+    auto issue_slab = [&](uint32_t w, int gr) {
       int mt, nt;
-      decode(w_first, mt, nt);
-#pragma unroll
-      for (int gr = 0; gr < kGroups; ++gr) issue_slab(mt, nt, gr);
-    }
-    for (long w = w_first; w < total && ok; w += w_step, ++tile) {
-      int mt, nt, mt_next = 0, nt_next = 0;
       decode(w, mt, nt);
-      if (w + w_step < total) decode(w + w_step, mt_next, nt_next);
+      mbar_arrive_expect_tx(bar_slab(warp, gr), kSlab);
+      tma_load_2d(slabs + gr * kSlab, &tmC, nt * kBN + (ch * kGroups + gr) * 32, mt * 128 + 32 * q, bar_slab(warp, gr));
+    };
+    if (w_first < total && elect_one()) {
+#pragma unroll
+      for (int gr = 0; gr < kGroups; ++gr) issue_slab(w_first, gr);
+    }
+    for (uint32_t w = w_first; w < total && ok; w += w_step, ++tile) {
+      int mt, nt;
+      decode(w, mt, nt);
+      const bool more = total - w > w_step;
       const int hc_first = first_hc(nt);
       const bool bits_ok = last_hc(nt) - hc_first < 32;
-      const bool tile_fast = g.fast_ok && (long)mt * 128 + 128 <= g.rows;
+      const int row0 = mt * 128 + 32 * q;
       const TileVectors *v = reinterpret_cast<const TileVectors *>(smem + kVecOffset) + (tile & 1u);
-      if (!mbar_wait(bar_vec_full(tile & 1u), (tile >> 1) & 1u, abort_flag, status, kWaitSlab)) { ok = false; break; }
+      if (!mbar_wait_warp(bar_vec_full(tile & 1u), (tile >> 1) & 1u, abort_flag, status, kWaitSlab)) { ok = false; break; }
+      const float r = v->rci[32 * q + lane];
+      const uint64_t r2 = pair_of(r, r);
       for (int cc = 0; cc < nchains && ok; ++cc, ++chain) {
         const uint32_t buf = chain & 1u;
-        if (!mbar_wait(bar_acc_full(buf), (chain >> 1) & 1u, abort_flag, status, kWaitAccFull)) { ok = false; break; }
+        if (!mbar_wait_warp(bar_acc_full(buf), (chain >> 1) & 1u, abort_flag, status, kWaitAccFull)) { ok = false; break; }
         __syncwarp();
         tc_fence_after();
         const uint32_t tacc = tmem_base + buf * kBN + ch * (kGroups * 32) + ((uint32_t)(32 * q) << 16);
         const bool last_chain = cc == nchains - 1;
         const float decay = cc == 0 ? g.one_minus : 1.f;   // the old trace decays once
+        const uint64_t decay2 = pair_of(decay, decay);
 #pragma unroll 1
         for (int gr = 0; gr < kGroups; ++gr) {
-          if (cc == 0 && !mbar_wait(bar_slab(warp, gr), tile & 1u, abort_flag, status, kWaitSlab)) { ok = false; break; }
-          uint8_t *sl = smem + kSlabOffset + (warp * kGroups + gr) * kSlab + lr * 128;
+          if (cc == 0 && !mbar_wait_warp(bar_slab(warp, gr), tile & 1u, abort_flag, status, kWaitSlab)) { ok = false; break; }
           const int vc = (ch * kGroups + gr) * 32;           // first column of the group, in the tile
-          const long gs = (long)nt * kBN + vc;
-          // whole blocks with at most two hypercolumns: one select word per row, bit 8*rep + e = "element e of column
-          // pair rep keeps its weight"
-          const bool g_fast = tile_fast && gs + 32 <= g.cols;
-          uint32_t live32 = 0, first32 = 0xFFFFFFFFu;   // columns at or above the threshold; of the first hypercolumn
-          int k0 = 0;
-          if (last_chain && g_fast) {
-            live32 = __ballot_sync(0xFFFFFFFFu, v->rcj[vc + lane] != 0.f);
-            if (has_mask) {
-              const int hc0 = hc_of(gs);
-              const long bnd = (long)(hc0 + 1) * g.Mc - gs;
-              if (bnd < 32) first32 = (1u << bnd) - 1u;
-              k0 = hc0 - hc_first;
+          const int gs = nt * kBN + vc;
+          const bool inside = row0 < g.rows && gs < g.cols;   // (what lies past the edges of a block is clipped by TMA)
+          uint32_t word = 0;   // bit k: the element in column k of the group keeps its weight
+          if (last_chain && inside) {
+            word = 0xFFFFFFFFu;
+            if (g.wmask != nullptr) {
+              word = 0;
+              const uint32_t mb = v->bits[32 * q + lane];
+              const int h1 = hc_of(min(gs + 32, g.cols) - 1);
+              for (int h = hc_of(gs); h <= h1; ++h) {
+                const int from = h * g.Mc - gs, to = from + g.Mc;   // the hypercolumn's columns in the group
+                const uint32_t seg = (to < 32 ? (1u << to) - 1u : 0xFFFFFFFFu) & ~(from > 0 ? (1u << from) - 1u : 0u);
+                const bool on = bits_ok ? (mb >> (h - hc_first)) & 1u
+                                        : row0 + lane < g.rows && __ldg(g.wmask + (long)(row0 + lane) * g.H + h) != 0;
+                if (on) word |= seg;
+              }
             }
+            const uint32_t live = __ballot_sync(0xFFFFFFFFu, v->rcj[vc + lane] != 0.f);   // columns at or above the threshold
+            word = r != 0.f ? word & live : 0u;
           }
-#pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
+          uint8_t *sl = slab_row + gr * kSlab;
+#pragma unroll 1
+          for (int half = 0; half < 2; ++half) {
             float a[16];
             __syncwarp();   // tcgen05.ld is warp-collective
-            tmem_ld_16x256b_x4(tacc + gr * 32 + ((uint32_t)(16 * hh) << 16), a);
-            float2 c[2][4];
+            tmem_ld_32x32b_x16(tacc + gr * 32 + half * 16, a);
+            uint64_t c[8];   // pairs of neighbouring columns
 #pragma unroll
-            for (int rr = 0; rr < 2; ++rr)
-#pragma unroll
-              for (int rep = 0; rep < 4; ++rep) {
-                float2 c2 = *reinterpret_cast<const float2 *>(sl + (16 * hh + 8 * rr) * 128 + swz[rep]);
-                c2.x = fmaf(c2.x, decay, a[rep * 4 + rr * 2 + 0] * g.ema_scale);
-                c2.y = fmaf(c2.y, decay, a[rep * 4 + rr * 2 + 1] * g.ema_scale);
-                c[rr][rep] = c2;
-              }
+            for (int k = 0; k < 4; ++k) {
+              const ulonglong2 old = *reinterpret_cast<const ulonglong2 *>(sl + (((half * 4 + k) ^ (lane & 7)) << 4));
+              c[2 * k] = fma_pair(old.x, decay2, mul_pair(pair_of(a[4 * k], a[4 * k + 1]), scale2));
+              c[2 * k + 1] = fma_pair(old.y, decay2, mul_pair(pair_of(a[4 * k + 2], a[4 * k + 3]), scale2));
+            }
             if (!last_chain) {   // the running sum stays in shared memory
 #pragma unroll
-              for (int rr = 0; rr < 2; ++rr)
-#pragma unroll
-                for (int rep = 0; rep < 4; ++rep)
-                  *reinterpret_cast<float2 *>(sl + (16 * hh + 8 * rr) * 128 + swz[rep]) = c[rr][rep];
+              for (int k = 0; k < 4; ++k)
+                *reinterpret_cast<ulonglong2 *>(sl + (((half * 4 + k) ^ (lane & 7)) << 4)) = make_ulonglong2(c[2 * k], c[2 * k + 1]);
               continue;
             }
-            if (hh == 1) {
-              // the block is about to be overwritten by TMA: every lane's accesses must have been performed, not merely issued
-              fence_async_smem();
-              __syncwarp();
-              if (lane == 0 && w + w_step < total) issue_slab(mt_next, nt_next, gr);
-            }
+            const uint32_t sel = word >> (16 * half);
+            float wv[16];
 #pragma unroll
-            for (int rr = 0; rr < 2; ++rr) {
-              const int vr = 32 * q + 16 * hh + 8 * rr + lr;
-              const long i = (long)mt * 128 + vr;
-              float *cp = g.Cij + i * g.cols + gs + lc;
-              const float r = v->rci[vr];
-              const uint32_t mb = v->bits[vr];
-              if (g_fast) {
-                const uint32_t m0 = 0u - ((mb >> k0) & 1u), m1 = 0u - ((mb >> (k0 + 1)) & 1u);
-                const uint32_t word = ((m0 & first32) | (m1 & ~first32)) & live32;
-                const uint32_t sel = r != 0.f ? (word >> lc) & 0x03030303u : 0u;
-#pragma unroll
-                for (int rep = 0; rep < 4; ++rep) {
-                  const float2 rcj = *reinterpret_cast<const float2 *>(v->rcj + vc + lc + rep * 8);
-                  float2 c2 = c[rr][rep];
-                  c2.x = fmaxf(c2.x, 0.f);
-                  c2.y = fmaxf(c2.y, 0.f);
-                  const float wx = lg2_ftz(fmaxf(c2.x, g.cthr4) * (r * rcj.x)) * kLn2;
-                  const float wy = lg2_ftz(fmaxf(c2.y, g.cthr4) * (r * rcj.y)) * kLn2;
-                  __stcs(reinterpret_cast<float2 *>(cp + rep * 8), c2);
-                  __stcs(reinterpret_cast<float2 *>(cp + w_minus_c + rep * 8),
-                         make_float2((sel & (1u << (8 * rep))) ? wx : 0.f, (sel & (2u << (8 * rep))) ? wy : 0.f));
-                }
-              } else if (i < g.rows) {   // edges, narrow hypercolumns: every element checked
-#pragma unroll
-                for (int rep = 0; rep < 4; ++rep) {
-                  const long n = gs + lc + rep * 8;
-                  if (!(n < g.cols)) continue;   // cols is even: n + 1 is in range too
-                  const float2 rcj = *reinterpret_cast<const float2 *>(v->rcj + vc + lc + rep * 8);
-                  float2 c2 = c[rr][rep];
-                  c2.x = fmaxf(c2.x, 0.f);
-                  c2.y = fmaxf(c2.y, 0.f);
-                  bool on0 = r != 0.f && rcj.x != 0.f, on1 = r != 0.f && rcj.y != 0.f;
-                  if (has_mask) {
-                    const uint8_t *mr = g.wmask + i * g.H;
-                    const int h0 = hc_of(n), h1 = hc_of(n + 1);
-                    on0 = on0 && (bits_ok ? (mb >> (h0 - hc_first)) & 1u : (uint32_t)__ldg(mr + h0)) != 0;
-                    on1 = on1 && (bits_ok ? (mb >> (h1 - hc_first)) & 1u : (uint32_t)__ldg(mr + h1)) != 0;
-                  }
-                  const float wx = __logf(fmaxf(c2.x, g.cthr4) * (r * rcj.x));
-                  const float wy = __logf(fmaxf(c2.y, g.cthr4) * (r * rcj.y));
-                  __stcs(reinterpret_cast<float2 *>(cp + rep * 8), c2);
-                  __stcs(reinterpret_cast<float2 *>(cp + w_minus_c + rep * 8), make_float2(on0 ? wx : 0.f, on1 ? wy : 0.f));
-                }
+            for (int k = 0; k < 8; ++k) {
+              float2 t = halves(c[k]);
+              t.x = fmaxf(t.x, 0.f);
+              t.y = fmaxf(t.y, 0.f);
+              c[k] = pair_of(t.x, t.y);
+              const uint64_t rc = mul_pair(r2, *reinterpret_cast<const uint64_t *>(v->rcj + vc + half * 16 + 2 * k));
+              const float2 arg = halves(mul_pair(pair_of(fmaxf(t.x, g.cthr4), fmaxf(t.y, g.cthr4)), rc));
+              float2 l;
+              if (g.normal) {
+                l = halves(mul_pair(pair_of(lg2_ftz(arg.x), lg2_ftz(arg.y)), ln2));
+              } else {
+                l = make_float2(__logf(arg.x), __logf(arg.y));
               }
+              wv[2 * k] = sel & (1u << (2 * k)) ? l.x : 0.f;
+              wv[2 * k + 1] = sel & (2u << (2 * k)) ? l.y : 0.f;
+            }
+            if (elect_one()) {   // the weights before these have left their buffer, and the traces the block before this one
+              bulk_wait_read_0();
+              if (half == 0 && gr > 0 && more) issue_slab(w + w_step, gr - 1);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              *reinterpret_cast<ulonglong2 *>(sl + (((half * 4 + k) ^ (lane & 7)) << 4)) = make_ulonglong2(c[2 * k], c[2 * k + 1]);
+              *reinterpret_cast<float4 *>(w_row + ((k ^ (lane >> 1 & 3)) << 4)) =
+                  make_float4(wv[4 * k], wv[4 * k + 1], wv[4 * k + 2], wv[4 * k + 3]);
+            }
+            // every lane's accesses must have been performed, not merely issued, before TMA reads or overwrites the blocks
+            fence_async_smem();
+            __syncwarp();
+            if (inside && elect_one()) {
+              tma_store_2d(&tmW, wbuf, gs + half * 16, row0);
+              if (half == 1) tma_store_2d(&tmC, slabs + gr * kSlab, gs, row0);
+              bulk_commit();
             }
           }
         }
@@ -484,12 +479,19 @@ __global__ void __launch_bounds__(kThreads, 1)
         // the accumulator may be overwritten (the leader's MMA warp waits for both CTAs' epilogue warps)
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) {
+        if (elect_one()) {
           leader_arrive(bar_acc_empty(buf));
-          if (last_chain) mbar_arrive(bar_vec_empty(tile & 1u));
+          if (last_chain) {
+            mbar_arrive(bar_vec_empty(tile & 1u));
+            if (more) {
+              bulk_wait_read_0();
+              issue_slab(w + w_step, kGroups - 1);
+            }
+          }
         }
       }
     }
+    if (elect_one()) bulk_wait_all();   // what this warp has sent by TMA has landed before the CTA retires
   }
 
   // ------------------------------------------------------------ tear-down
@@ -525,13 +527,13 @@ uint32_t exact_division_magic(long d, long limit) {
 cudaError_t launch_trace_update_tc(const float *x, const float *y, long B, long N, long M, long H, const float *rci,
                                    const float *rcj, float *Cij, float *w, const uint8_t *wmask, TraceParams<float> p,
                                    cudaStream_t st) {
-  if (!tc_available() || !tc_shape_ok(x, y, N, M) || !tc_shape_ok(Cij, Cij, N, M) || (reinterpret_cast<uintptr_t>(w) & 7u))
+  if (!tc_available() || !tc_shape_ok(x, y, N, M) || !tc_shape_ok(Cij, w, N, M))
     return cudaErrorNotSupported;
   TcHost host;
   if (!tc_host(&host)) return cudaErrorMemoryAllocation;
-  CUtensorMap ma, mb, ma3, mb3, mc;
-  if (!tc_map_2d(&ma, x, N, B, 32, kBK, true) || !tc_map_2d(&mb, y, M, B, 32, kBK, true) ||
-      !tc_map_2d(&mc, Cij, M, N, 32, 32, false))
+  CUtensorMap ma, mb, ma3, mb3, mc, mw;
+  if (!tc_map_2d(&ma, x, N, B, 32, kBK, kMapMnMajor) || !tc_map_2d(&mb, y, M, B, 32, kBK, kMapMnMajor) ||
+      !tc_map_2d(&mc, Cij, M, N, 32, 32, kMapRows) || !tc_map_2d(&mw, w, M, N, 16, 32, kMapRows64))
     return cudaErrorInvalidValue;
   const bool a3 = N % 32 == 0 && tc_map_chunks(&ma3, x, N, B, kBK, 4), b3 = tc_map_chunks(&mb3, y, M, B, kBK, (host.pairs ? Layout<true>::BNH : Layout<false>::BNH) / 32);
   if (!a3) ma3 = ma;
@@ -545,17 +547,15 @@ cudaError_t launch_trace_update_tc(const float *x, const float *y, long B, long 
   g.b_box3_tiles = b3 ? (int)(M / 32 * 32 / kBN) : 0;
   g.lose_arrive = host.lose_arrive;
   g.wait_limit = host.wait_limit;
-  g.rows = N;
-  g.cols = M;
+  g.rows = (int)N;
+  g.cols = (int)M;
   g.rci = rci;
   g.rcj = rcj;
-  g.Cij = Cij;
-  g.W = w;
   g.wmask = wmask;
-  g.H = H;
-  g.Mc = H > 0 ? M / H : M;
+  g.H = (int)H;
+  g.Mc = (int)(H > 0 ? M / H : M);
   g.hc_magic = wmask ? exact_division_magic(g.Mc, M + 2) : 0;
-  g.fast_ok = (wmask == nullptr || g.Mc >= 32) && p.cthr4 >= 1e-30f;
+  g.normal = p.cthr4 >= 1e-30f;
   g.one_minus = p.one_minus;
   g.cthr4 = p.cthr4;
   g.ema_scale = p.taupdt / p.batch;
@@ -573,7 +573,7 @@ cudaError_t launch_trace_update_tc(const float *x, const float *y, long B, long 
       configured[dev].store(true);
     }
     const cudaError_t e = launch_next(trace_kernel<false>, (unsigned)(units < host.sms ? units : host.sms), kThreads, L::SMEM, st,
-                                      ma, mb, ma3, mb3, mc, g, host.status);
+                                      ma, mb, ma3, mb3, mc, mw, g, host.status);
     if (e == cudaSuccess) count_launches(1);
     return e;
   }
@@ -602,7 +602,7 @@ cudaError_t launch_trace_update_tc(const float *x, const float *y, long B, long 
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // as launch_next
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.numAttrs = 2;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, trace_kernel<true>, ma, mb, ma3, mb3, mc, g, host.status);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, trace_kernel<true>, ma, mb, ma3, mb3, mc, mw, g, host.status);
   if (e == cudaSuccess) {
     count_launches(1);
     tc_count_pair_launch();
