@@ -149,7 +149,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  after_previous();   // (barriers and tensor memory are set up while the kernel before ends)
+  // Only the warp that reads what the kernel before this one in the stream computed (column_vectors_kernel: the reciprocals)
+  // waits for its end, and the epilogue, which writes, waits for that warp.  x, y and the old traces come by TMA and were
+  // complete before that kernel let any of these blocks start: every kernel does so only after its own predecessors.
+  // Train step without a mask update, 1568 -> 30 x 100 at batch 128: 23.3 -> 20.0 us.
 
   // The clusters walk the tiles side by side, columns fastest (rows fastest where the columns are the longer side): at any
   // time they share the operands of a few row tiles.
@@ -306,6 +309,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else if (warp == kVec) {
     // ------------------------------------------------------------ row and column data, one tile ahead
     uint32_t t = 0;
+    after_previous();
     for (uint32_t w = w_first; w < total; w += w_step, ++t) {
       int mt, nt;
       decode(w, mt, nt);
