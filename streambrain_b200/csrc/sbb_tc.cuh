@@ -27,8 +27,8 @@ cudaError_t launch_forward_product_tc(const float *x, const float *w, float *par
                                       int splits, cudaStream_t st);
 
 // Fused trace step: Cij = moving average of x^T y / B, w = log(Cij / (Ci Cj)) under the mask (null: none), from the
-// reciprocals of the new Ci and Cj (0 where the trace is below the threshold).
-cudaError_t launch_trace_update_tc(const float *x, const float *y, long B, long N, long M, long H, const float *rci,
+// reciprocals of the new Ci and Cj (0 where the trace is below the threshold).  x: N columns of rows `ldx` apart.
+cudaError_t launch_trace_update_tc(const float *x, long ldx, const float *y, long B, long N, long M, long H, const float *rci,
                                    const float *rcj, float *Cij, float *w, const uint8_t *wmask, TraceParams<float> p,
                                    cudaStream_t st);
 
@@ -62,8 +62,9 @@ bool tc_host(TcHost *out);
 // How a box lands in shared memory: rows of 128 or of 64 bytes under the swizzle of that width, or rows of 128 bytes under
 // the flavour of the 128-byte swizzle (32-byte base) that MN-major 32-bit operands need.
 enum { kMapRows = 0, kMapMnMajor = 1, kMapRows64 = 2 };
-bool tc_map_2d(void *map, const float *base, long inner, long outer, int box_inner, int box_outer, int layout);
-bool tc_map_chunks(void *map, const float *base, long cols, long rows, int box_rows, int box_chunks);
+// (pitch: elements from row to row)
+bool tc_map_2d(void *map, const float *base, long inner, long outer, long pitch, int box_inner, int box_outer, int layout);
+bool tc_map_chunks(void *map, const float *base, long cols, long rows, long pitch, int box_rows, int box_chunks);
 
 // Launches so far whose CTAs worked in pairs.
 void tc_count_pair_launch();

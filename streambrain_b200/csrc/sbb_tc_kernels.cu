@@ -698,10 +698,10 @@ int *status_word() {
 // costs about a microsecond each, which is a tenth of the step of a small layer.
 struct MapKey {
   const void *base;
-  long inner, outer;
+  long inner, outer, pitch;
   int box_a, box_b, kind;
   bool operator==(const MapKey &o) const {
-    return base == o.base && inner == o.inner && outer == o.outer && box_a == o.box_a && box_b == o.box_b && kind == o.kind;
+    return base == o.base && inner == o.inner && outer == o.outer && pitch == o.pitch && box_a == o.box_a && box_b == o.box_b && kind == o.kind;
   }
 };
 struct MapCache {
@@ -711,7 +711,7 @@ struct MapCache {
   bool used[kSlots] = {false};
   static unsigned slot(const MapKey &k) {
     uint64_t h = reinterpret_cast<uintptr_t>(k.base) * 0x9E3779B97F4A7C15ull;
-    h ^= (uint64_t)k.inner * 0xC2B2AE3D27D4EB4Full + (uint64_t)k.outer * 0x165667B19E3779F9ull +
+    h ^= (uint64_t)k.inner * 0xC2B2AE3D27D4EB4Full + (uint64_t)(k.outer ^ k.pitch << 20) * 0x165667B19E3779F9ull +
          (uint64_t)(k.box_a * 131 + k.box_b * 17 + k.kind);
     return (unsigned)(h >> 40) % kSlots;
   }
@@ -730,37 +730,15 @@ struct MapCache {
 };
 thread_local MapCache g_map_cache;
 
-bool make_map_uncached(CUtensorMap *map, const float *base, long inner, long outer, int box_inner, int box_outer,
-                       int layout);
-bool make_map_chunks_uncached(CUtensorMap *map, const float *base, long cols, long rows, int box_rows, int box_chunks);
-
-// 2-D float32 tensor map over a row-major [outer, inner] matrix, zero fill.
-bool make_map(CUtensorMap *map, const float *base, long inner, long outer, int box_inner, int box_outer,
-              int layout) {
-  const MapKey k{base, inner, outer, box_inner, box_outer, layout};
-  if (g_map_cache.find(k, map)) return true;
-  if (!make_map_uncached(map, base, inner, outer, box_inner, box_outer, layout)) return false;
-  g_map_cache.put(k, *map);
-  return true;
-}
-bool make_map_chunks(CUtensorMap *map, const float *base, long cols, long rows, int box_rows, int box_chunks) {
-  const MapKey k{base, cols, rows, box_rows, box_chunks, -1};
-  if (g_map_cache.find(k, map)) return true;
-  if (!make_map_chunks_uncached(map, base, cols, rows, box_rows, box_chunks)) return false;
-  g_map_cache.put(k, *map);
-  return true;
-}
-
-bool make_map_uncached(CUtensorMap *map, const float *base, long inner, long outer, int box_inner, int box_outer,
-                       int layout) {
-  cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
-  cuuint64_t strides[1] = {(cuuint64_t)inner * sizeof(float)};
-  cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer};
+bool make_map_uncached(CUtensorMap *map, const MapKey &k) {
+  cuuint64_t dims[2] = {(cuuint64_t)k.inner, (cuuint64_t)k.outer};
+  cuuint64_t strides[1] = {(cuuint64_t)k.pitch * sizeof(float)};
+  cuuint32_t box[2] = {(cuuint32_t)k.box_a, (cuuint32_t)k.box_b};
   cuuint32_t estr[2] = {1, 1};
-  const CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims, strides, box,
+  const CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(k.base), dims, strides, box,
                               estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              layout == kMapMnMajor ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B
-                              : layout == kMapRows64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                              k.kind == kMapMnMajor ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B
+                              : k.kind == kMapRows64 ? CU_TENSOR_MAP_SWIZZLE_64B
                                                      : CU_TENSOR_MAP_SWIZZLE_128B,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
@@ -768,15 +746,37 @@ bool make_map_uncached(CUtensorMap *map, const float *base, long inner, long out
 
 // 3-D view {32, rows, cols/32} of a row-major [rows, cols] float32 matrix (element (i, r, c) = m[r][32c + i]);
 // a box {32, box_rows, box_chunks} lands in shared memory as [chunk][row][32], the MN-major stage layout.
-bool make_map_chunks_uncached(CUtensorMap *map, const float *base, long cols, long rows, int box_rows, int box_chunks) {
-  if (cols < 32) return false;
-  cuuint64_t dims[3] = {32, (cuuint64_t)rows, (cuuint64_t)(cols / 32)};
-  cuuint64_t strides[2] = {(cuuint64_t)cols * sizeof(float), 128};
-  cuuint32_t box[3] = {32, (cuuint32_t)box_rows, (cuuint32_t)box_chunks};
+bool make_map_chunks_uncached(CUtensorMap *map, const MapKey &k) {
+  if (k.inner < 32) return false;
+  cuuint64_t dims[3] = {32, (cuuint64_t)k.outer, (cuuint64_t)(k.inner / 32)};
+  cuuint64_t strides[2] = {(cuuint64_t)k.pitch * sizeof(float), 128};
+  cuuint32_t box[3] = {32, (cuuint32_t)k.box_a, (cuuint32_t)k.box_b};
   cuuint32_t estr[3] = {1, 1, 1};
-  return g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(base), dims, strides, box, estr,
+  return g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void *>(k.base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// 2-D float32 tensor map over a row-major [outer, inner] matrix with rows `pitch` elements apart, zero fill.
+bool make_map(CUtensorMap *map, const float *base, long inner, long outer, long pitch, int box_inner, int box_outer, int layout) {
+  const MapKey k{base, inner, outer, pitch, box_inner, box_outer, layout};
+  if (g_map_cache.find(k, map)) return true;
+  if (!make_map_uncached(map, k)) return false;
+  g_map_cache.put(k, *map);
+  return true;
+}
+bool make_map(CUtensorMap *map, const float *base, long inner, long outer, int box_inner, int box_outer, int layout) {
+  return make_map(map, base, inner, outer, inner, box_inner, box_outer, layout);
+}
+bool make_map_chunks(CUtensorMap *map, const float *base, long cols, long rows, long pitch, int box_rows, int box_chunks) {
+  const MapKey k{base, cols, rows, pitch, box_rows, box_chunks, -1};
+  if (g_map_cache.find(k, map)) return true;
+  if (!make_map_chunks_uncached(map, k)) return false;
+  g_map_cache.put(k, *map);
+  return true;
+}
+bool make_map_chunks(CUtensorMap *map, const float *base, long cols, long rows, int box_rows, int box_chunks) {
+  return make_map_chunks(map, base, cols, rows, cols, box_rows, box_chunks);
 }
 
 // Column tiles of width bn whose every 32-column group lies inside the matrix.
@@ -879,11 +879,11 @@ bool tc_host(TcHost *out) {
   out->pairs = pairs_enabled();
   return out->status != nullptr && init_once();
 }
-bool tc_map_2d(void *map, const float *base, long inner, long outer, int box_inner, int box_outer, int layout) {
-  return make_map(static_cast<CUtensorMap *>(map), base, inner, outer, box_inner, box_outer, layout);
+bool tc_map_2d(void *map, const float *base, long inner, long outer, long pitch, int box_inner, int box_outer, int layout) {
+  return make_map(static_cast<CUtensorMap *>(map), base, inner, outer, pitch, box_inner, box_outer, layout);
 }
-bool tc_map_chunks(void *map, const float *base, long cols, long rows, int box_rows, int box_chunks) {
-  return make_map_chunks(static_cast<CUtensorMap *>(map), base, cols, rows, box_rows, box_chunks);
+bool tc_map_chunks(void *map, const float *base, long cols, long rows, long pitch, int box_rows, int box_chunks) {
+  return make_map_chunks(static_cast<CUtensorMap *>(map), base, cols, rows, pitch, box_rows, box_chunks);
 }
 
 // Launch counter shared with the general-shape kernels (defined in sbb_kernels.cu).

@@ -528,18 +528,18 @@ uint32_t exact_division_magic(long d, long limit) {
 
 }  // namespace
 
-cudaError_t launch_trace_update_tc(const float *x, const float *y, long B, long N, long M, long H, const float *rci,
+cudaError_t launch_trace_update_tc(const float *x, long ldx, const float *y, long B, long N, long M, long H, const float *rci,
                                    const float *rcj, float *Cij, float *w, const uint8_t *wmask, TraceParams<float> p,
                                    cudaStream_t st) {
-  if (!tc_available() || !tc_shape_ok(x, y, N, M) || !tc_shape_ok(Cij, w, N, M))
+  if (!tc_available() || !tc_shape_ok(x, y, N, M) || ldx % 4 != 0 || !tc_shape_ok(Cij, w, N, M))
     return cudaErrorNotSupported;
   TcHost host;
   if (!tc_host(&host)) return cudaErrorMemoryAllocation;
   CUtensorMap ma, mb, ma3, mb3, mc, mw;
-  if (!tc_map_2d(&ma, x, N, B, 32, kBK, kMapMnMajor) || !tc_map_2d(&mb, y, M, B, 32, kBK, kMapMnMajor) ||
-      !tc_map_2d(&mc, Cij, M, N, 32, 32, kMapRows) || !tc_map_2d(&mw, w, M, N, 16, 32, kMapRows64))
+  if (!tc_map_2d(&ma, x, N, B, ldx, 32, kBK, kMapMnMajor) || !tc_map_2d(&mb, y, M, B, M, 32, kBK, kMapMnMajor) ||
+      !tc_map_2d(&mc, Cij, M, N, M, 32, 32, kMapRows) || !tc_map_2d(&mw, w, M, N, M, 16, 32, kMapRows64))
     return cudaErrorInvalidValue;
-  const bool a3 = N % 32 == 0 && tc_map_chunks(&ma3, x, N, B, kBK, 4), b3 = tc_map_chunks(&mb3, y, M, B, kBK, (host.pairs ? Layout<true>::BNH : Layout<false>::BNH) / 32);
+  const bool a3 = N % 32 == 0 && tc_map_chunks(&ma3, x, N, B, ldx, kBK, 4), b3 = tc_map_chunks(&mb3, y, M, B, M, kBK, (host.pairs ? Layout<true>::BNH : Layout<false>::BNH) / 32);
   if (!a3) ma3 = ma;
   if (!b3) mb3 = mb;
   Trace g{};

@@ -28,11 +28,11 @@ extern "C" int pthread_create(pthread_t *t, const pthread_attr_t *a, void *(*f)(
 static bool copies(unsigned seed) {
   std::vector<unsigned char> src(6 << 20), dst(src.size() + 2);
   for (size_t k = 0; k < src.size(); ++k) src[k] = (unsigned char)((k * 2654435761u + seed) >> 13);
-  const size_t sizes[] = {0, 1, 4095, 131072, 262143, 262144, 262145, 262144 + 131072, 1000001, 3 << 20, (6 << 20) - 7};
+  const size_t sizes[] = {0, 1, 4095, 65536, 65537, 131072, 524287, 524288, 524288 + 32768 + 15, 262143, 262144, 262145, 262144 + 131072, 1000001, 3 << 20, (6 << 20) - 7};
   for (int round = 0; round < 6; ++round)
     for (size_t n : sizes) {
       std::memset(dst.data(), 0xEE, n + 2);
-      sbb::CopyThreads::get().copy(dst.data() + 1, src.data(), n);
+      sbb::CopyThreads::get().copy(dst.data() + 1, src.data(), n, round & 1);
       if (std::memcmp(dst.data() + 1, src.data(), n) != 0 || dst[0] != 0xEE || dst[n + 1] != 0xEE) {
         std::printf("wrong copy of %zu bytes\n", n);
         return false;

@@ -140,6 +140,34 @@ def test_trace_update_vs_oracle(k, port_kernels, tag, dtype, B, N, H, Mc):
     assert weight_err(w1, w2) < 10 * tol
 
 
+@pytest.mark.parametrize("tag,dtype", DTYPES)
+@pytest.mark.parametrize("N,M", [(1100, 1000), (1001, 1153), (65, 20000), (130, 300004), (4096, 256)])
+def test_trace_update_in_blocks_of_rows(k, port_kernels, tag, dtype, N, M):
+    """Host arrays of more than two pinned slots go through in blocks of rows: whole and ragged blocks, a block of one slot
+    and of many, rows longer than a slot, pageable and page-locked arrays; and not where the weights are the array of the
+    joint trace, which is still to be read then: that array ends with the weights."""
+    import torch
+    rs = np.random.RandomState(N + M)
+    B = 9
+    x, y = rs.rand(B, N).astype(dtype), rs.rand(B, M).astype(dtype)
+    Ci, Cj, Cij = rs.rand(N).astype(dtype), rs.rand(M).astype(dtype), rs.rand(N, M).astype(dtype)
+    got = k.update_weights(Ci.copy(), Cj.copy(), Cij.copy(), x, y, 0.1, np.empty((N, M), dtype=dtype), 0.05)
+    rows = np.unique(np.r_[0, 63, 64, 127, N - 1, rs.randint(0, N, 8)])
+    rows = rows[rows < N]
+    want = port_kernels.update_weights(Ci[rows].copy(), Cj.copy(), Cij[rows].copy(), np.ascontiguousarray(x[:, rows]), y, 0.1,
+                                       np.empty((len(rows), M), dtype=dtype), 0.05)
+    tol = TOL[np.dtype(dtype)]
+    assert rel_inf(got[0][rows], want[0]) < tol and rel_inf(got[1], want[1]) < tol and rel_inf(got[2][rows], want[2]) < tol
+    assert weight_err(got[3][rows], want[3]) < 10 * tol
+    one = Cij.copy()
+    k.update_weights(Ci.copy(), Cj.copy(), one, x, y, 0.1, one, 0.05)
+    assert np.array_equal(one, got[3])
+    pinned = [torch.from_numpy(a).pin_memory() for a in (Ci, Cj, Cij, x, y, np.zeros((N, M), dtype=dtype))]
+    p = [t.numpy() for t in pinned]
+    k.update_weights(p[0], p[1], p[2], p[3], p[4], 0.1, p[5], 0.05)
+    assert all(np.array_equal(a, b) for a, b in zip((p[0], p[1], p[2], p[5]), got))
+
+
 def test_float64_logarithm_of_the_trace_update(k):
     """The float64 trace update's own logarithm (a table of 128 and a series).  With Ci = Cj = 1 the weight is the logarithm
     of the new Cij as returned.  Bound: two roundings below 2^-54 on the way to ln m, the series' remainder and r's rounding
