@@ -28,7 +28,7 @@ class CopyThreads {
   // first, as a store to a line that is not in the cache does: 153 against 66 GB/s by eight threads).
   void copy(void *dst, const void *src, size_t bytes, bool past_cache = false) {
     past_cache = past_cache && bytes >= kPastCache;
-    if (bytes <= 2 * kPiece || workers_.empty() || !mutex_.try_lock()) {   // (busy with another thread's job)
+    if (bytes <= kAlone || workers_.empty() || !mutex_.try_lock()) {   // (busy with another thread's job)
       move(static_cast<char *>(dst), static_cast<const char *>(src), bytes, past_cache);
       return;
     }
@@ -53,6 +53,7 @@ class CopyThreads {
 
  private:
   static constexpr size_t kPiece = 32 << 10;   // (half a microsecond to copy in cache, two from memory)
+  static constexpr size_t kAlone = 128 << 10;   // up to here the workers cost more than they save (84 KB: 4 us)
   static constexpr size_t kPastCache = 512 << 10;
   static constexpr uint32_t kClosed = 0xFFFFFFFFu;
   static void move(char *dst, const char *src, size_t bytes, bool past_cache) {
