@@ -293,6 +293,35 @@ template <typename T>
 __device__ __forceinline__ void top_rows(const MaskArgs<T> &a, int groups, TopShared<T> &sh) {
   typedef typename ScoreKey<T>::type K;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  // What the selection reads is asked for in as few rounds as there are dependences: each is a trip through L2.
+  struct Rows {
+    uint32_t f[4];
+    uint8_t m[4];
+    T nom[4];
+    int cs[4];
+  } rows;
+  auto fetch = [&](const int (&e)[4]) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool in = e[u] < (int)a.N;
+      rows.f[u] = in ? __ldcg(a.ms.filter + e[u]) : 0u;
+      rows.m[u] = in ? __ldcg(a.ms.old_col + e[u]) : 0;
+      rows.nom[u] = in ? __ldcg(a.ms.score + e[u]) : (T)0;
+      rows.cs[u] = in ? __ldcg(a.ms.csum + e[u]) : 0;
+    }
+  };
+  // all rows where that is a round trip to memory less; the rows of the blocks that have one that passes otherwise
+  const bool all = a.N <= 4 * kMaskThreads;
+  uint2 block_best[2];
+  int e[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) e[u] = (int)threadIdx.x + u * kMaskThreads;
+  if (all) {
+    fetch(e);
+  } else {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) block_best[u] = e[u] < (int)gridDim.x ? __ldcg(a.ms.block_best + e[u]) : make_uint2(0, 0);
+  }
   if (wid < 2) {
     // (exact keys: equal top words of float64 keys do not decide)
     const unsigned long long g = lane < groups ? __ldcg(&a.ms.header->best[wid][lane]) : ~0ull;
@@ -313,22 +342,22 @@ __device__ __forceinline__ void top_rows(const MaskArgs<T> &a, int groups, TopSh
   }
   __syncthreads();
   const uint32_t f0 = filter_key(sh.bound_key[0]), f1 = filter_key(sh.bound_key[1]);
-  auto consider = [&](int e, uint32_t f, int c) {
+  auto consider = [&](int u) {
+    const uint32_t f = rows.f[u];
+    const int c = rows.m[u];
     if (f == 0 || f < (c == 0 ? f0 : f1)) return;
-    if (f == (c == 0 ? f0 : f1)) {
-      const K k = sizeof(T) == 4 ? (K)f : class_key<T>(c, swap_score(__ldcg(a.ms.score + e), __ldcg(a.ms.csum + e)));
-      if (before(sh.bound_key[c], sh.bound_row[c], k, (uint32_t)(e + 1))) return;
-    }
+    const K k = sizeof(T) == 4 ? (K)f : class_key<T>(c, swap_score(rows.nom[u], rows.cs[u]));
+    if (f == (c == 0 ? f0 : f1) && before(sh.bound_key[c], sh.bound_row[c], k, (uint32_t)(e[u] + 1))) return;
     const int at = atomicAdd(&sh.count[c], 1);
     if (at >= kTopSlots) return;
-    sh.row[c][at] = (uint32_t)e;
-    if (sizeof(T) == 4) sh.key[c][at] = (K)f;
+    sh.row[c][at] = (uint32_t)e[u];
+    sh.key[c][at] = k;
+    sh.nom[c][at] = rows.nom[u];
+    sh.cs[c][at] = rows.cs[u];
   };
-  // the rows of the blocks that have one that passes; all rows where that is a round trip to memory less
-  const bool all = a.N <= 4 * kMaskThreads;
   if (!all) {
     for (int k = threadIdx.x; k < (int)gridDim.x; k += kMaskThreads) {
-      const uint2 best = __ldcg(a.ms.block_best + k);
+      const uint2 best = k < kMaskThreads ? block_best[0] : k < 2 * kMaskThreads ? block_best[1] : __ldcg(a.ms.block_best + k);
       if ((best.x == 0 || best.x < f0) && (best.y == 0 || best.y < f1)) continue;
       const int at = atomicAdd(&sh.blocks, 1);
       if (at < kTopSlots) sh.block[at] = k;
@@ -336,23 +365,20 @@ __device__ __forceinline__ void top_rows(const MaskArgs<T> &a, int groups, TopSh
     __syncthreads();
   }
   const bool some = !all && sh.blocks <= kTopSlots;
-  const int rows = some ? sh.blocks * a.block_rows : (int)a.N;
+  const int nrows = some ? sh.blocks * a.block_rows : (int)a.N;
 #pragma unroll 1
-  for (int t0 = threadIdx.x; t0 < rows; t0 += 4 * kMaskThreads) {
-    int e[4];
-    uint32_t f[4];
-    uint8_t m[4];
+  for (int t0 = threadIdx.x; t0 < nrows; t0 += 4 * kMaskThreads) {
+    if (!all) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int t = t0 + u * kMaskThreads;
-      e[u] = some && t < rows ? sh.block[t >> a.rows_log2] * a.block_rows + (t & (a.block_rows - 1)) : t;
-      const bool in = t < rows && e[u] < (int)a.N;
-      f[u] = in ? __ldcg(a.ms.filter + e[u]) : 0u;
-      m[u] = in ? __ldcg(a.ms.old_col + e[u]) : 0;
+      for (int u = 0; u < 4; ++u) {
+        const int t = t0 + u * kMaskThreads;
+        e[u] = t >= nrows ? (int)a.N : some ? sh.block[t >> a.rows_log2] * a.block_rows + (t & (a.block_rows - 1)) : t;
+      }
+      fetch(e);
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (f[u] >= (f0 < f1 ? f0 : f1)) consider(e[u], f[u], m[u]);
+      if (rows.f[u] >= (f0 < f1 ? f0 : f1)) consider(u);
   }
   __syncthreads();
   const int c = threadIdx.x / kTopSlots, i = threadIdx.x % kTopSlots;
@@ -363,16 +389,10 @@ __device__ __forceinline__ void top_rows(const MaskArgs<T> &a, int groups, TopSh
   int cs = 0;
   if (i < n && n <= kTopSlots) {
     row = sh.row[c][i];
-    nom = __ldcg(a.ms.score + row);
-    cs = __ldcg(a.ms.csum + row);
-    if constexpr (sizeof(T) == 4) {
-      k = sh.key[c][i];
-    } else {
-      k = class_key<T>(c, swap_score(nom, cs));
-      sh.key[c][i] = k;
-    }
+    nom = sh.nom[c][i];
+    cs = sh.cs[c][i];
+    k = sh.key[c][i];
   }
-  if (sizeof(T) != 4) __syncthreads();
   if (i < n && n <= kTopSlots) {
     int rank = 0;
 #pragma unroll 4
@@ -525,7 +545,6 @@ __device__ __forceinline__ void replay_swaps(const uint32_t (&row)[NS], int (&cl
 // already).
 template <typename T, bool SCORE>
 __global__ void __launch_bounds__(kMaskThreads, sizeof(T) == 4 ? 2 : 1) mask_update_kernel(const MaskArgs<T> a) {
-  after_previous();
   __shared__ TopShared<T> sh;
   __shared__ unsigned long long s_best[2][kGroups];
   __shared__ uint32_t low_row[2][64], changed[6 * 32];
@@ -535,6 +554,7 @@ __global__ void __launch_bounds__(kMaskThreads, sizeof(T) == 4 ? 2 : 1) mask_upd
   if (threadIdx.x == 0) s_nan = 0;
   if (threadIdx.x < 2 * kGroups) s_best[threadIdx.x / kGroups][threadIdx.x % kGroups] = 0;
   __syncthreads();
+  after_previous();   // (no access to global memory before it)
   // what the last block selects by: the filter key of a scored row, and the best one of its group
   auto leave_key = [&](long i, T nom, int cnt, int m) {
     const T sc = swap_score(nom, cnt);
@@ -615,8 +635,8 @@ __global__ void __launch_bounds__(kMaskThreads, sizeof(T) == 4 ? 2 : 1) mask_upd
     const long i = (long)blockIdx.x * a.block_rows + threadIdx.x;
     if ((int)threadIdx.x < a.block_rows && i < a.N) leave_key(i, a.ms.score[i], a.ms.csum[i], a.ms.old_col[i]);
   }
-  // ---- the block that finishes last goes on
-  __threadfence();
+  // ---- the block that finishes last goes on (the fence of the thread that counts the block covers what the barrier has put
+  // before it)
   __syncthreads();
   if (threadIdx.x < 2 * kGroups) {
     const unsigned long long best = s_best[threadIdx.x / kGroups][threadIdx.x % kGroups];
@@ -624,10 +644,12 @@ __global__ void __launch_bounds__(kMaskThreads, sizeof(T) == 4 ? 2 : 1) mask_upd
     const uint32_t f = __reduce_max_sync(0xffffffffu, (uint32_t)(best >> 32));
     if (lane == 0) reinterpret_cast<uint32_t *>(a.ms.block_best + blockIdx.x)[wid] = f;
     if (threadIdx.x == 0 && s_nan) atomicOr(&a.ms.header->nan, 1);
-    __threadfence();
   }
   __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(&a.ms.header->ticket, 1) == (int)gridDim.x - 1;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(&a.ms.header->ticket, 1) == (int)gridDim.x - 1;
+  }
   __syncthreads();
   if (!s_last) return;
   __threadfence();
@@ -665,6 +687,18 @@ __global__ void __launch_bounds__(kMaskThreads, sizeof(T) == 4 ? 2 : 1) mask_upd
         for (int w = 0; w < kMaskWarps; ++w) low_cnt[threadIdx.x] += win_cnt[w][threadIdx.x];
       __syncthreads();
       if (low_cnt[0] >= want && low_cnt[1] >= want) break;   // uniform: read after the barrier
+    }
+  }
+  if (wid != 0 && a.rewrite_w != nullptr) {
+    // most rows that will move are on the lists: their traces come to this SM while the swaps are decided
+    const int lines = (int)((a.Mc * sizeof(T) + 127) / 128) + 1;   // of a row's traces in hypercolumn h, and its Ci
+    for (int t = threadIdx.x - 32; t < 2 * a.iterations * (lines + 1); t += kMaskThreads - 32) {
+      const int slot = t / (lines + 1), k = t % (lines + 1);
+      const uint32_t r = sh.top_row[slot & 1][slot >> 1];
+      if (r == kNoRow) continue;
+      const long col = k * (long)(128 / sizeof(T));
+      const T *p = k == lines ? a.Ci + r : a.Cij + (long)r * a.M + a.h * a.Mc + (col < a.Mc ? col : a.Mc - 1);
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
     }
   }
   if (wid == 0) {
@@ -729,34 +763,36 @@ __global__ void __launch_bounds__(kMaskThreads, sizeof(T) == 4 ? 2 : 1) mask_upd
     if (lane == 0) n_changed = a.rewrite_w != nullptr ? n : 0;
   }
   __syncthreads();
-  // the weights of hypercolumn h of the rows whose mask bit changed follow the new bit: four entries per thread in flight
-  const int elems = n_changed * (int)a.Mc;
+  // the weights of hypercolumn h of the rows whose mask bit changed follow the new bit: a warp per row, the rows that became
+  // active (they come first) spread over the warps, four entries per lane in flight
 #pragma unroll 1
-  for (int t0 = threadIdx.x; t0 < elems; t0 += 4 * kMaskThreads) {
-    T ci[4], cj[4], cij[4];
-    long at[4];
-    uint32_t on[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int t = t0 + u * kMaskThreads < elems ? t0 + u * kMaskThreads : t0;
-      const uint32_t ch = changed[t / (int)a.Mc];
-      const long col = a.h * a.Mc + t % (int)a.Mc;
-      at[u] = (long)(ch >> 1) * a.M + col;
-      on[u] = ch & 1u;
-      ci[u] = a.Ci[ch >> 1];
-      cj[u] = a.Cj[col];
-      cij[u] = a.Cij[at[u]];
+  for (int q = wid; q < n_changed; q += kMaskWarps) {
+    const long row = changed[q] >> 1;
+    const T ci = a.Ci[row];
+    const T *cj = a.Cj + a.h * a.Mc + lane, *cij = a.Cij + row * a.M + a.h * a.Mc + lane;
+    T *w = a.rewrite_w + row * a.M + a.h * a.Mc + lane;
+    const int left = (int)a.Mc - lane;   // entry e of this lane exists when 32 * e < left
+    if (!(changed[q] & 1u) || ci < a.cthr) {
+      for (int e = 0; e < left; e += 32) w[e] = (T)0;
+      continue;
     }
 #pragma unroll 1
-    for (int u = 0; u < 4 && t0 + u * kMaskThreads < elems; ++u) {
-      a.rewrite_w[at[0]] = on[0] && !(ci[0] < a.cthr) && !(cj[0] < a.cthr) ? log_ratio(cij[0], ci[0], cj[0], a.cthr4) : (T)0;
+    for (int e0 = 0; e0 < left; e0 += 128) {
+      T pj[4], pij[4];
 #pragma unroll
-      for (int v = 0; v < 3; ++v) {
-        ci[v] = ci[v + 1];
-        cj[v] = cj[v + 1];
-        cij[v] = cij[v + 1];
-        at[v] = at[v + 1];
-        on[v] = on[v + 1];
+      for (int u = 0; u < 4; ++u) {
+        const bool in = e0 + 32 * u < left;
+        pj[u] = in ? cj[e0 + 32 * u] : (T)0;
+        pij[u] = in ? cij[e0 + 32 * u] : (T)0;
+      }
+#pragma unroll 1
+      for (int e = e0; e < left && e < e0 + 128; e += 32) {
+        w[e] = !(pj[0] < a.cthr) ? log_ratio(pij[0], ci, pj[0], a.cthr4) : (T)0;
+#pragma unroll
+        for (int v = 0; v < 3; ++v) {
+          pj[v] = pj[v + 1];
+          pij[v] = pij[v + 1];
+        }
       }
     }
   }
