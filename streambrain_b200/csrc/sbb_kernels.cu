@@ -670,13 +670,26 @@ static TracePairs to_pairs(const TraceEpilogue<double> &e) {
 
 static int sm_count();
 
+constexpr size_t kMostSmem = 232448;   // of one block; an SM has 1 KB more, and every block takes 1 KB besides its own
+
+// Dynamic shared memory to ask for, so that no SM gets more blocks than an even spread over the SMs gives it: blocks are
+// placed while the kernel before still runs on some of them (programmatic launches), and with room for two or more on an SM
+// some got two while others got none.  float64 trace step 2048 -> 8 x 64 at batch 1024, 128 blocks: 86 or 156 us, by the device
+// and the state of the SMs, without it; 86 with it.
+static size_t spread_smem(size_t own, long blocks) {
+  const long sms = sm_count(), per = (blocks + sms - 1) / sms;
+  if (per < 1 || per > 8) return own;
+  const size_t least = ((kMostSmem + 1024) / (size_t)(per + 1) - 1024) / 128 * 128 + 128;   // (no more than that: other kernels' blocks
+  return least > own ? least : own;                                                          // still fit beside them)
+}
+
 // More than 48 KB of dynamic shared memory is asked for once per kernel and device.
 template <class K>
-static cudaError_t allow_smem(K kernel, size_t bytes, bool (&configured)[64]) {
+static cudaError_t allow_smem(K kernel, bool (&configured)[64]) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && configured[dev]) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostSmem);
   if (e == cudaSuccess && dev >= 0 && dev < 64) configured[dev] = true;
   return e;
 }
@@ -688,7 +701,7 @@ static cudaError_t launch_f64_mma_tiles(const double *A, long lda, const double 
   using C = F::Cfg<BM, DEEP>;
   auto kernel = F::contraction_kernel<A_KMAJOR, BM, DEEP, V, Pairs>;
   static bool configured[64] = {false};
-  const cudaError_t e = allow_smem(kernel, C::SMEM_BYTES, configured);
+  const cudaError_t e = allow_smem(kernel, configured);
   if (e != cudaSuccess) return e;
   const unsigned mt = (unsigned)((Mdim + BM - 1) / BM), nt = (unsigned)((Ndim + F::BN - 1) / F::BN);
   if (cols_fastest && mt > 65535u) cols_fastest = false;
@@ -696,7 +709,7 @@ static cudaError_t launch_f64_mma_tiles(const double *A, long lda, const double 
   if (grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
   const int slabs = (K + F::BK - 1) / F::BK;
   const int kper = (slabs + splits - 1) / splits * F::BK;
-  launch_next(kernel, grid, C::THREADS, C::SMEM_BYTES, st, A, lda, Bm, ldb, Mdim, Ndim, K, kper, cols_fastest, ep);
+  launch_next(kernel, grid, C::THREADS, spread_smem(C::SMEM_BYTES, (long)mt * nt * splits), st, A, lda, Bm, ldb, Mdim, Ndim, K, kper, cols_fastest, ep);
   return launched();
 }
 
@@ -735,11 +748,11 @@ static cudaError_t launch_small_contraction(const T *A, long lda, const T *Bm, l
   using S = SmallShape<T, A_KMAJOR>;
   auto kernel = small_contraction_kernel<T, A_KMAJOR, Ep>;
   static bool configured[64] = {false};
-  const cudaError_t e = allow_smem(kernel, S::SMEM_BYTES, configured);
+  const cudaError_t e = allow_smem(kernel, configured);
   if (e != cudaSuccess) return e;
   const dim3 grid((unsigned)((Ndim + S::BN - 1) / S::BN), (unsigned)((Mdim + S::BM - 1) / S::BM), (unsigned)splits);
   if (grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
-  launch_next(kernel, grid, S::THREADS, S::SMEM_BYTES, st, A, lda, Bm, ldb, Mdim, Ndim, K, kper, ep);
+  launch_next(kernel, grid, S::THREADS, spread_smem(S::SMEM_BYTES, (long)grid.x * grid.y * splits), st, A, lda, Bm, ldb, Mdim, Ndim, K, kper, ep);
   return launched();
 }
 
@@ -748,13 +761,13 @@ static cudaError_t launch_tiles(const float *A, long lda, const float *Bm, long 
                                 int splits, int kper, bool cols_fastest, Ep ep, cudaStream_t st) {
   auto kernel = contraction_kernel<A_KMAJOR, V, Ep>;
   static bool configured[64] = {false};
-  const cudaError_t e = allow_smem(kernel, Tile::SMEM_BYTES, configured);
+  const cudaError_t e = allow_smem(kernel, configured);
   if (e != cudaSuccess) return e;
   const unsigned mt = (unsigned)((Mdim + 127) / 128), nt = (unsigned)((Ndim + 127) / 128);
   if (cols_fastest && mt > 65535u) cols_fastest = false;
   const dim3 grid(cols_fastest ? nt : mt, cols_fastest ? mt : nt, (unsigned)splits);
   if (grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
-  launch_next(kernel, grid, Tile::THREADS, Tile::SMEM_BYTES, st, A, lda, Bm, ldb, Mdim, Ndim, K, kper, cols_fastest, ep);
+  launch_next(kernel, grid, Tile::THREADS, spread_smem(Tile::SMEM_BYTES, (long)mt * nt * splits), st, A, lda, Bm, ldb, Mdim, Ndim, K, kper, cols_fastest, ep);
   return launched();
 }
 
