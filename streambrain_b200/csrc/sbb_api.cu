@@ -344,7 +344,17 @@ int train_rows(sbb_layer *L, const T *x, const T *y, long B, long N, long M, lon
   SBB_CUDA(sbb::launch_column_vectors<T>(sbb::ColumnVectors<T>{x, N, Ci, rci}, sbb::ColumnVectors<T>{y, M, Cj, rcj}, B, p, bias, st));
   if (N == 0) return SBB_OK;
   PhaseTimer timer(L, SBB_PHASE_TRACE, st);
-  if (tc) {
+  const int splits = L == nullptr ? 1 : tc ? sbb::trace_splits_tc(B, N, M) : sbb::trace_splits<T>(B, N, M);
+  if (splits > 1) {
+    SBB_TRY(L->fwd_partial.reserve((size_t)splits * (size_t)(N * M) * sizeof(T)));   // (the forward pass has done with it)
+    T *const partial = static_cast<T *>(L->fwd_partial.d);
+    if (tc) {
+      if constexpr (std::is_same<T, float>::value) SBB_CUDA(sbb::launch_split_product_tc(x, y, B, N, M, splits, partial, st));
+    } else {
+      SBB_CUDA(sbb::launch_split_product<T>(x, y, B, N, M, splits, partial, st));
+    }
+    SBB_CUDA(sbb::launch_split_trace<T>(partial, splits, N, M, H, M / H, Ci, Cj, rci, rcj, Cij, W, wmask, p, tc, st));
+  } else if (tc) {
     if constexpr (std::is_same<T, float>::value)
       SBB_CUDA(sbb::launch_trace_update_tc(x, N, y, B, N, M, wmask ? H : 0, rci, rcj, Cij, W, wmask, p, st));
   } else {

@@ -1386,6 +1386,150 @@ template cudaError_t launch_trace_apply<double>(const double *, long, long, long
                                                 const double *, double *, double *, const uint8_t *,
                                                 TraceParams<double>, int, long, long, cudaStream_t, bool);
 
+// ----------------------------------------------------------------------------
+// The trace step of a long batch whose outputs are few tiles: the batch is cut into `splits` parts, whose products are
+// formed side by side (a fused launch would sum each output over the whole batch on a few SMs), and this adds them up and does
+// what the fused epilogues do.  The arithmetic is that of the path: reciprocals and lg2 behind the tensor-core product
+// (FAST), the reciprocals and logarithm of the float64 kernel, divisions and the library's logarithm otherwise.
+// 88 -> 2 x 264 at batch 5851, train step: float32 165 us fused, 31 so; float64 235 and 50.
+// ----------------------------------------------------------------------------
+template <typename T, int V, bool FAST>
+__global__ void __launch_bounds__(256)
+    split_trace_kernel(const T *__restrict__ partial, int splits, long slice, int M, int H, int Mc, const T *__restrict__ Ci,
+                       const T *__restrict__ Cj, const T *__restrict__ rci, const T *__restrict__ rcj, T *Cij, T *W,
+                       const uint8_t *__restrict__ wmask, TraceParams<T> p) {
+  after_previous();
+  const long at = ((long)blockIdx.x * 256 + threadIdx.x) * V;
+  if (at >= slice) return;
+  const long i = at / M;
+  const int j = (int)(at - i * M);
+  struct alignas(sizeof(T) * V) Piece {
+    T v[V];
+  };
+  Piece c = *reinterpret_cast<const Piece *>(Cij + at), w;
+  const uint8_t *mrow = wmask ? wmask + i * H : nullptr;
+  bool on[V];
+  T cj[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    on[v] = mrow == nullptr || mrow[(unsigned)(j + v) / (unsigned)Mc] != 0;
+    cj[v] = (FAST || sizeof(T) == 8 ? rcj : Cj)[j + v];
+  }
+  const T ci = (FAST || sizeof(T) == 8 ? rci : Ci)[i];
+  T s[V];
+#pragma unroll
+  for (int v = 0; v < V; ++v) s[v] = (T)0;
+  constexpr int U = 8;   // parts in flight
+  for (int z = 0; z < splits; z += U) {
+    Piece d[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (z + u < splits) d[u] = *reinterpret_cast<const Piece *>(partial + (long)(z + u) * slice + at);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (z + u < splits)
+#pragma unroll
+        for (int v = 0; v < V; ++v) s[v] += d[u].v[v];
+  }
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    T x;
+    if constexpr (FAST) {
+      x = trace_ema_fast(c.v[v], s[v], p.one_minus, p.taupdt / p.batch);
+      w.v[v] = on[v] && ci != 0.f && cj[v] != 0.f ? log_ratio_fast(x, ci, cj[v], p.cthr4) : 0.f;
+    } else if constexpr (sizeof(T) == 8) {
+      x = fma(c.v[v], p.one_minus, s[v] * (1.0 / p.batch * p.taupdt));
+      x = x > 0.0 ? x : 0.0;
+      w.v[v] = on[v] && ci != 0.0 && cj[v] != 0.0 ? f64mma::log_positive((x < p.cthr4 ? p.cthr4 : x) * (ci * cj[v])) : 0.0;
+    } else {
+      x = trace_ema(c.v[v], s[v], p);
+      w.v[v] = on[v] && !(ci < p.cthr) && !(cj[v] < p.cthr) ? log_ratio(x, ci, cj[v], p.cthr4) : (T)0;
+    }
+    c.v[v] = x;
+  }
+  *reinterpret_cast<Piece *>(Cij + at) = c;
+  *reinterpret_cast<Piece *>(W + at) = w;
+}
+
+template <typename T>
+cudaError_t launch_split_trace(const T *partial, int splits, long N, long M, long H, long Mc, const T *Ci, const T *Cj,
+                               const T *rci, const T *rcj, T *Cij, T *w, const uint8_t *wmask, TraceParams<T> p, bool fast,
+                               cudaStream_t st) {
+  const long slice = N * M;
+  constexpr int V = Vec16<T>::N;
+  const bool vec = M % V == 0 && aligned16(partial) && aligned16(Cij) && aligned16(w);
+  auto launch = [&](auto kernel, int v) {
+    launch_next(kernel, (unsigned)((slice / v + 255) / 256), 256, 0, st, partial, splits, slice, (int)M, (int)H, (int)Mc, Ci, Cj, rci,
+                rcj, Cij, w, wmask, p);
+  };
+  if constexpr (sizeof(T) == 4) {
+    if (fast) {   // (the tensor-core path's rows are multiples of 16 bytes)
+      launch(split_trace_kernel<T, V, true>, V);
+      return launched();
+    }
+  }
+  if (vec) launch(split_trace_kernel<T, V, false>, V);
+  else launch(split_trace_kernel<T, 1, false>, 1);
+  return launched();
+}
+template cudaError_t launch_split_trace<float>(const float *, int, long, long, long, long, const float *, const float *,
+                                               const float *, const float *, float *, float *, const uint8_t *,
+                                               TraceParams<float>, bool, cudaStream_t);
+template cudaError_t launch_split_trace<double>(const double *, int, long, long, long, long, const double *, const double *,
+                                                const double *, const double *, double *, double *, const uint8_t *,
+                                                TraceParams<double>, bool, cudaStream_t);
+
+// partial[s, N, M]: the products of the parts of the batch.
+template <typename T>
+cudaError_t launch_split_product(const T *x, const T *y, long B, long N, long M, int splits, T *partial, cudaStream_t st) {
+  constexpr int V = Vec16<T>::N;
+  const bool vec = N % V == 0 && M % V == 0 && aligned16(x) && aligned16(y);
+  StoreEpilogue<T> ep{partial, N, M, M, N * M, M % V == 0 && aligned16(partial)};
+  const long slabs = (B + Tile::BK - 1) / Tile::BK;
+  return launch_contraction<T, false>(x, N, y, M, N, M, (int)B, splits, (int)((slabs + splits - 1) / splits) * Tile::BK, vec, true,
+                                      ep, st);
+}
+template cudaError_t launch_split_product<float>(const float *, const float *, long, long, long, int, float *, cudaStream_t);
+template cudaError_t launch_split_product<double>(const double *, const double *, long, long, long, int, double *, cudaStream_t);
+
+// Parts the batch of a trace step is cut into (1: the fused kernel), from what a launch takes in microseconds: slabs of a part
+// times the time of one with so many blocks to an SM, and for the parts the second launch and the way of the partial sums to
+// memory and back.  Measured (train step without a mask update, fused -> best of 2 to 48 parts -> the rule's): float32 501 x 301
+// at batch 1001 41 -> 23 -> 24, 207 x 9 at 4000 136 -> 22 -> 21; float64 88 x 528 at 5851 235 -> 50 -> 50, 501 x 301 at 1001 54 ->
+// 24 -> 24, 256 x 256 at 2048 90 -> 24 -> 26, 5000 x 50 at 3000 148 -> 101 -> 103.  With more tiles than blocks fit it loses:
+// float64 2048 x 512 at 1024 86 -> 90.  Its sums are the more exact ones (1843 x 424 at 5485: 5e-8 of the trace against 2e-7).
+template <typename T>
+int trace_splits(long B, long N, long M) {
+  // (float32 layers of many inputs keep the order of their sums, as few_plan's: 1843 x 424 at batch 5485 moved single weights by
+  // 7e-4 of their mean square in two steps, 12566 x 102 at 1444 the activations by 2e-5)
+  if (B < 128 || (sizeof(T) == 4 && N > 1024)) return 1;
+  const long sms = sm_count();
+  auto ceil_div = [](long a, long b) { return (a + b - 1) / b; };
+  auto per_slab = [&](long blocks, long per_sm, double one, double two, double full) {   // us, by the blocks an SM has
+    if (blocks <= sms) return one;
+    if (blocks <= 2 * sms) return two;
+    return full * (double)ceil_div(blocks, per_sm * sms);
+  };
+  auto cost = [&](long s) {
+    if (sizeof(T) == 8) return ceil_div(ceil_div(B, 16), s) * per_slab(ceil_div(N, 64) * ceil_div(M, 64) * s, 3, 0.9, 1.0, 1.5);
+    const long tiles = ceil_div(N, 128) * ceil_div(M, 128) * s;
+    if (small_tiles(tiles, false)) return ceil_div(ceil_div(B, 32), s) * per_slab(ceil_div(N, 32) * ceil_div(M, 64) * s, 4, 1.2, 1.5, 2.0);
+    return ceil_div(ceil_div(B, 16), s) * per_slab(tiles, 2, 1.9, 3.4, 3.4);
+  };
+  int best = 1;
+  const double fused = cost(1);
+  double least = 0.85 * fused;
+  for (long s = 2; s <= 48 && B / s >= 64; ++s) {
+    if (s * N * M > (1l << 26)) break;
+    const double c = cost(s) + 4.0 + (double)(s * N * M) * (2 * sizeof(T)) / 3e6;
+    if (c < least) least = c, best = (int)s;
+  }
+  const long slabs = ceil_div(B, Tile::BK);
+  return (int)ceil_div(slabs, ceil_div(slabs, best));   // no empty part
+}
+template int trace_splits<float>(long, long, long);
+template int trace_splits<double>(long, long, long);
+
 // Un-fused trace update in the NumPy operation order: (1-t)*C + t*(sum/B).
 template <typename T>
 __global__ void counters_apply_kernel(T *c, const T *__restrict__ sums, long n, T taupdt, T batch) {

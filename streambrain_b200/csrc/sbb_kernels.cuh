@@ -104,6 +104,17 @@ cudaError_t launch_trace_apply(const T *delta, long N, long M, long H, long Mc, 
                                T *w, const uint8_t *wmask, TraceParams<T> p, int ema, long row_begin, long row_end,
                                cudaStream_t st, bool fast = false);
 
+// A trace step in two launches: the products of `splits` parts of the batch (partial[s, N, M]), then sums, traces and weights.
+template <typename T>
+int trace_splits(long B, long N, long M);   // 1: the fused kernel is the better one
+template <typename T>
+cudaError_t launch_split_product(const T *x, const T *y, long B, long N, long M, int splits, T *partial, cudaStream_t st);
+// fast: the sums come from the tensor-core product; rci, rcj are read then and for float64
+template <typename T>
+cudaError_t launch_split_trace(const T *partial, int splits, long N, long M, long H, long Mc, const T *Ci, const T *Cj,
+                               const T *rci, const T *rcj, T *Cij, T *w, const uint8_t *wmask, TraceParams<T> p, bool fast,
+                               cudaStream_t st);
+
 // Un-fused Cij update with the numpy operation order: (1-t)*C + t*(sum/B).
 template <typename T>
 cudaError_t launch_counters_apply(T *c, const T *sums, long n, T taupdt, T batch, cudaStream_t st);

@@ -32,6 +32,11 @@ cudaError_t launch_trace_update_tc(const float *x, long ldx, const float *y, lon
                                    const float *rcj, float *Cij, float *w, const uint8_t *wmask, TraceParams<float> p,
                                    cudaStream_t st);
 
+// The split form of the trace step (sbb_kernels.cuh): parts of the batch, and their products partial[s, N, M].
+int trace_splits_tc(long B, long N, long M);
+cudaError_t launch_split_product_tc(const float *x, const float *y, long B, long N, long M, int splits, float *partial,
+                                    cudaStream_t st);
+
 // delta[i, j] = sum_b x[b, i] y[b, j] for rows [row_begin,row_end)
 // x_lo / y_lo (both or neither): planes of the operands' low parts as launch_colsum writes them; with them the
 // kernel takes both halves of both operands by TMA and converts nothing itself.

@@ -1079,6 +1079,58 @@ cudaError_t launch_outer_product_tc(const float *x, const float *y, long B, long
   return e;
 }
 
+// Parts the batch of a trace step is cut into (1: the fused kernel), as trace_splits: both kernels take about 0.42 us per
+// k-block of 16 samples, in rounds of 74 pairs of SMs with 256 x 192 outputs or of 148 SMs with 128 x 128.  Measured (column
+// vectors included, fused -> best of 2 to 48 parts -> the rule's): 88 x 528 at batch 5851 165 -> 31 -> 31 us, 256 x 256 at 2048 63 ->
+// 19 -> 21, 512 x 1024 at 4096 116 -> 46 -> 46, 664 x 16 at 5453 153 -> 30 -> 30, 128 x 96 at 512 22 -> 13 -> 13; 2048 x 1024 at 2048 (48
+// pairs) 64 -> 74 with two parts, 20000 x 64 at 1024 (79 pairs) 69 -> 66.
+namespace {
+// k-blocks of a part.  Parts of more than 1024 samples in all are whole accumulation chains, so that their sums are those of the
+// fused kernel's chains to the bit; cut elsewhere, the chains' truncation differs from its by up to 4e-6 of the sum, of which a
+// layer with a large taupdt and its own activations for outputs makes 1e-5 in two steps (1024 -> 128 at batch 8192).
+long part_kblocks(long kblocks, long splits) {
+  const long unit = kblocks > 64 ? kTrChainKb : 1, units = (kblocks + unit - 1) / unit;
+  return (units + splits - 1) / splits * unit;
+}
+}  // namespace
+
+int trace_splits_tc(long B, long N, long M) {
+  const long kblocks = (B + kTrBK - 1) / kTrBK, pairs = ((N + 255) / 256) * ((M + kTrBN - 1) / kTrBN);
+  const long tiles = ((N + 127) / 128) * ((M + kLongBN - 1) / kLongBN);
+  if (kblocks < 16 || N > 4096) return 1;   // (many inputs: they keep the order of their sums, as few_plan's)
+  status_word();   // fills the SM count
+  const long sms = g_sm_count_tc[current_device()];
+  auto ceil_div = [](long a, long b) { return (a + b - 1) / b; };
+  int best = 1;
+  double least = 0.85 * (double)(ceil_div(pairs, sms / 2 > 0 ? sms / 2 : 1) * kblocks) * 0.42;
+  for (long s = 2; s <= 48 && kblocks / s >= 4; ++s) {
+    if (s * N * M > (1l << 26)) break;
+    const long per = part_kblocks(kblocks, s), parts = ceil_div(kblocks, per);
+    const double c = (double)(ceil_div(tiles * parts, sms) * per) * 0.42 + 5.0 + (double)(parts * N * M) * 8.0 / 3e6;
+    if (c < least) least = c, best = (int)s;
+  }
+  return (int)ceil_div(kblocks, part_kblocks(kblocks, best));   // no empty part
+}
+
+cudaError_t launch_split_product_tc(const float *x, const float *y, long B, long N, long M, int splits, float *partial,
+                                    cudaStream_t st) {
+  if (!tc_available() || !tc_shape_ok(x, y, N, M) || (reinterpret_cast<uintptr_t>(partial) & 7u)) return cudaErrorNotSupported;
+  TcMaps tm;
+  bool a3 = false, b3 = false;
+  if (!batch_operand_maps(tm, x, y, nullptr, nullptr, false, B, N, M, kLongBN, a3, b3)) return cudaErrorInvalidValue;
+  tm.c = tm.a;
+  const long kblocks = (B + kTrBK - 1) / kTrBK;
+  TcWork wk{(int)((N + 127) / 128), (int)((M + kLongBN - 1) / kLongBN), splits, (int)B, (int)part_kblocks(kblocks, splits) * kTrBK,
+            M > N ? 1 : 0, 0, a3 ? 1 : 0, b3 ? full_chunk_tiles(M, kLongBN) : 0, 0, wait_limit_now(), take_lose_arrive()};
+  TcEpilogue ep{};
+  ep.out = partial;
+  ep.rows = N;
+  ep.cols = M;
+  ep.ld = M;
+  const cudaError_t e = launch_tc<false, kLongBN, kTrBK, kLongStages, kTrChainKb>(tm, wk, ep, st);
+  if (e == cudaSuccess) count_launches(1);
+  return e;
+}
 
 #ifdef SBB_TC_TRACE
 extern "C" int sbb_tc_trace_read(unsigned long long *out) {

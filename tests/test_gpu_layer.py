@@ -693,3 +693,43 @@ def test_contractions_of_odd_rows_vs_oracle(port_kernels, tag, dtype, B, N, H, M
     for name in ("Ci", "Cj", "Cij", "bias"):
         assert rel_inf(getattr(dev, name), getattr(ref, name)) < tol, name
     assert weight_err(dev.weights, ref.weights) < 10 * tol
+
+
+@pytest.mark.parametrize("tag,dtype", DTYPES)
+@pytest.mark.parametrize("kind,B,N,H,Mc", [("plastic", 512, 128, 2, 48), ("plastic", 1500, 88, 2, 66), ("plastic", 1030, 207, 5, 9),
+                                           ("plastic", 2049, 65, 3, 13), ("plastic", 700, 260, 1, 300), ("plastic", 5000, 129, 40, 1),
+                                           ("plastic", 600, 104, 1, 9), ("plastic", 1025, 300, 2, 16), ("dense", 1024, 300, 1, 10),
+                                           ("dense", 2050, 1100, 1, 30), ("dense", 513, 2300, 1, 3)])
+def test_long_batches_of_few_outputs_vs_oracle(port_kernels, tag, dtype, kind, B, N, H, Mc):
+    """Batches whose trace step is few tiles are cut into parts whose sums a second launch adds up; layers of few units share
+    a batch over a cluster of two, four or eight blocks: whole and ragged parts, vector and scalar rows, masks with many
+    hypercolumns to a row, units on both sides of the limits."""
+    import streambrain_b200 as B200
+    hp = dict(khalf=-100.0, pmin=0.05, taubdt=0.02, density=0.5)
+    init = (0.5, 1 / Mc, 0.5 / Mc)
+    np.random.seed(5)
+    if kind == "dense":
+        dev = B200.DenseLayer(N, H, Mc, 0.1, init, dtype=dtype)
+        ref = oracle.OracleLayer(port_kernels, kind, N, H, Mc, 0.1, init, dtype)
+    else:
+        dev = B200.StructuralPlasticityLayer(N, H, Mc, 0.1, hp["khalf"], hp["pmin"], hp["taubdt"], hp["density"], 16, init, dtype=dtype)
+        ref = oracle.OracleLayer(port_kernels, kind, N, H, Mc, 0.1, init, dtype, **hp)
+        ref.wmask = dev.wmask
+    rs = np.random.RandomState(B + N)
+    dev.weights = (0.05 * rs.randn(N, H * Mc)).astype(dtype)
+    for name in ("weights", "bias"):
+        setattr(ref, name, getattr(dev, name))
+    tol = TOL[np.dtype(dtype)]
+    for step in range(2):   # the tickets are zero again after a launch
+        x = rs.rand(B, N).astype(dtype)
+        y = rs.dirichlet(np.ones(Mc), size=(B, H)).reshape(B, H * Mc).astype(dtype)
+        assert rel_inf(dev.compute_activation(x), ref.compute_activation(x)) < 10 * tol, step
+        for layer in (ref, dev):
+            layer.train_step(x, y, *(() if kind == "dense" else (None,)))
+        for name in ("Ci", "Cj", "Cij", "bias"):
+            assert rel_inf(getattr(dev, name), getattr(ref, name)) < tol, (name, step)
+        assert weight_err(dev.weights, ref.weights) < 10 * tol, step
+        if kind == "plastic":
+            assert not dev.weights[np.repeat(ref.wmask == 0, Mc, axis=1)].any()
+        for name in ("weights", "bias", "Ci", "Cj", "Cij"):
+            setattr(dev, name, getattr(ref, name))
