@@ -1180,7 +1180,7 @@ template cudaError_t launch_colsum<double>(const double *, long, long, double *,
 // order of colsum_kernel.  Bound by latency for small layers, by HBM otherwise: sixteen loads per thread in flight.  (The two
 // column sums, the reciprocals and the bias were four launches, 2 x 3.3 + 1.9 + 1.9 us at 1568 + 3000 columns, batch 128;
 // 3.7 us now.  1568 + 30000 columns, batch 1024: 67 -> 28 us.)
-template <typename T>
+template <typename T, bool few>
 __global__ void __launch_bounds__(256)
     column_vectors_kernel(ColumnVectors<T> x, ColumnVectors<T> y, long B, TraceParams<T> p, BiasParams<T> nb, unsigned x_blocks) {
   after_previous();
@@ -1194,6 +1194,17 @@ __global__ void __launch_bounds__(256)
     constexpr int U = 16;
     const T *src = o.a + col;
     long b = ty;
+    if (few) {   // long batches of few columns: sixteen loads of each of few blocks do not keep memory busy (88 + 528 columns at
+                 // batch 5851: 20.7 -> 12 us)
+      constexpr int D = 64;
+      for (; b + 8 * (D - 1) < B; b += 8 * D) {
+        T v[D];
+#pragma unroll
+        for (int u = 0; u < D; ++u) v[u] = __ldg(src + (b + 8 * u) * o.cols);
+#pragma unroll
+        for (int u = 0; u < D; ++u) s += v[u];
+      }
+    }
     for (; b + 8 * (U - 1) < B; b += 8 * U) {
       T v[U];
 #pragma unroll
@@ -1226,7 +1237,8 @@ cudaError_t launch_column_vectors(const ColumnVectors<T> &x, const ColumnVectors
                                   BiasParams<T> bias, cudaStream_t st) {
   const unsigned xb = (unsigned)((x.cols + 31) / 32), yb = (unsigned)((y.cols + 31) / 32);
   if (xb + yb == 0) return cudaSuccess;
-  launch_next(column_vectors_kernel<T>, xb + yb, 256, 0, st, x, y, B, p, bias, xb);
+  if (B >= 1024 && xb + yb <= 2 * (unsigned)sm_count()) launch_next(column_vectors_kernel<T, true>, xb + yb, 256, 0, st, x, y, B, p, bias, xb);
+  else launch_next(column_vectors_kernel<T, false>, xb + yb, 256, 0, st, x, y, B, p, bias, xb);
   return launched();
 }
 template cudaError_t launch_column_vectors<float>(const ColumnVectors<float> &, const ColumnVectors<float> &, long,
