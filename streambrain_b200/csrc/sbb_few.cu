@@ -16,6 +16,11 @@ void count_launches(int n);   // sbb_kernels.cu
 namespace {
 
 constexpr int kFewThreads = 256;
+// Inputs of a thread beyond which its weights stream, two batches of eight in flight, and the inputs wait in shared memory: in
+// registers, one per weight in flight and sample, they leave room for one block on an SM.  Three float64 samples 3370 -> 75 x
+// 213 206 -> 131 us; the one or two batches of a smaller range lose by the inputs' own trip (one sample 1568 -> 30 x 100 8.8 ->
+// 12.4 us).
+constexpr int kFewStream = 64;
 
 template <typename T, int V>
 struct alignas(sizeof(T) * V) Piece {
@@ -23,7 +28,7 @@ struct alignas(sizeof(T) * V) Piece {
 };
 
 // `cols` = columns of a block (whole hypercolumns), `lanes` = threads across them, kFewThreads / lanes inputs at a time.
-template <typename T, int V, int R>
+template <typename T, int V, int R, bool STREAM>
 __global__ void __launch_bounds__(kFewThreads)
     few_forward_kernel(const T *__restrict__ x, const T *__restrict__ W, const T *__restrict__ bias, T *__restrict__ out,
                        T *partial, int *tickets, int N, int M, int Mc, int cols, int lanes, int range) {
@@ -39,8 +44,46 @@ __global__ void __launch_bounds__(kFewThreads)
   for (int r = 0; r < R; ++r)
 #pragma unroll
     for (int v = 0; v < V; ++v) acc[r][v] = (T)0;
-  if (g < groups && c < width) {
-    constexpr int U = 16;
+  const bool active = g < groups && c < width;
+  if constexpr (STREAM) {
+    constexpr int U = 8;
+    constexpr int KT = sizeof(T) * R <= 16 ? 1024 : 512;   // inputs in shared memory at a time
+    __shared__ T s_x[R][KT];
+    for (int t0 = k0; t0 < k1; t0 += KT) {
+      const int t1 = min(k1, t0 + KT);
+      const T *wp = W + c0 + c;
+      auto load = [&](Piece<T, V> (&w)[U], int k) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (k + u * groups < t1) w[u] = *reinterpret_cast<const Piece<T, V> *>(wp + (long)(k + u * groups) * M);
+      };
+      auto multiply = [&](const Piece<T, V> (&w)[U], int k) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (k + u * groups < t1)
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+              for (int v = 0; v < V; ++v) acc[r][v] = fma(s_x[r][k + u * groups - t0], w[u].v[v], acc[r][v]);
+      };
+      Piece<T, V> a[U], b[U];
+      int k = t0 + g;
+      if (active) load(a, k);
+      if (t0 > k0) __syncthreads();   // the inputs before these have been read
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        for (int t = threadIdx.x; t < t1 - t0; t += kFewThreads) s_x[r][t] = x[(long)r * N + t0 + t];
+      __syncthreads();
+      if (active)
+        for (; k < t1; k += 2 * U * groups) {
+          load(b, k + U * groups);
+          multiply(a, k);
+          load(a, k + 2 * U * groups);
+          multiply(b, k + U * groups);
+        }
+    }
+  } else if (active) {
+    constexpr int U = R <= 2 ? 16 : 8;   // (as registers allow with two blocks on an SM: four float32 samples 1568 -> 30 x 100 19.3 -> 17.5 us)
     const T *wp = W + c0 + c;
     for (int k = k0 + g; k < k1; k += U * groups) {
       Piece<T, V> w[U];
@@ -66,11 +109,12 @@ __global__ void __launch_bounds__(kFewThreads)
 #pragma unroll
           for (int v = 0; v < V; ++v) acc[r][v] = fma(xv[u][r], w[u].v[v], acc[r][v]);
     }
+  }
+  if (active)
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
       for (int v = 0; v < V; ++v) s_sum[(g * R + r) * lanes * V + c + v] = acc[r][v];
-  }
   __syncthreads();
   for (int t = threadIdx.x; t < R * width; t += kFewThreads) {
     const int r = t / width, j = t % width;
@@ -117,6 +161,7 @@ __global__ void __launch_bounds__(kFewThreads)
 
 struct FewPlan {
   int vec, cols, lanes, chunks, ranges, range;
+  bool stream;
 };
 template <typename T>
 bool few_plan(const void *W, long B, long N, long H, long Mc, FewPlan &p) {
@@ -153,6 +198,7 @@ bool few_plan(const void *W, long B, long N, long H, long Mc, FewPlan &p) {
   if (ranges > 64) ranges = 64;
   p.range = (int)((N + ranges - 1) / ranges);
   p.ranges = (int)((N + p.range - 1) / p.range);
+  p.stream = p.range / groups > kFewStream;
   return true;
 }
 
@@ -175,12 +221,14 @@ cudaError_t launch_few_forward(const T *x, const T *W, const T *bias, T *out, lo
   if (!few_plan<T>(W, B, N, H, Mc, p)) return cudaErrorNotSupported;
   const dim3 grid((unsigned)p.chunks, (unsigned)p.ranges);
   constexpr int V = 16 / (int)sizeof(T);
-#define SBB_FEW(VV, R) \
-  launch_next(few_forward_kernel<T, VV, R>, grid, kFewThreads, 0, st, x, W, bias, out, partial, tickets, (int)N, (int)(H * Mc), (int)Mc, \
-                                                            p.cols, p.lanes, p.range)
+#define SBB_FEW(VV, R, S) \
+  launch_next(few_forward_kernel<T, VV, R, S>, grid, kFewThreads, 0, st, x, W, bias, out, partial, tickets, (int)N, (int)(H * Mc), (int)Mc, \
+              p.cols, p.lanes, p.range)
 #define SBB_FEW_R(R) \
-  if (p.vec == 1) SBB_FEW(1, R); \
-  else SBB_FEW(V, R)
+  if (p.vec == 1 && p.stream) SBB_FEW(1, R, true); \
+  else if (p.vec == 1) SBB_FEW(1, R, false); \
+  else if (p.stream) SBB_FEW(V, R, true); \
+  else SBB_FEW(V, R, false)
   if (B == 1) {
     SBB_FEW_R(1);
   } else if (B == 2) {

@@ -651,10 +651,11 @@ def test_state_round_trip_through_the_copy_slots(n, m):
 @pytest.mark.parametrize("tag,dtype", DTYPES)
 @pytest.mark.parametrize("B", [1, 2, 3, 4, 5])
 @pytest.mark.parametrize("N,H,Mc", [(1, 1, 33), (17, 3, 37), (1568, 30, 100), (4096, 2, 256), (4097, 5, 64), (700, 13, 4), (333, 2, 300),
-                                    (260, 1, 1024)])
+                                    (260, 1, 1024), (9001, 3, 7), (3000, 150, 4), (300, 75, 251)])
 def test_forward_of_few_samples_vs_oracle(port_kernels, tag, dtype, B, N, H, Mc):
     """One to four samples take a kernel of their own: vector and scalar columns, one and many hypercolumns per block, wide
-    hypercolumns, inputs that do and do not divide into ranges, and the first sizes that do not take it."""
+    hypercolumns, inputs that do and do not divide into ranges, ranges whose weights stream, and the first sizes that do not
+    take it."""
     import streambrain_b200 as B200
     np.random.seed(2)
     args = (N, H, Mc, 0.01, -100.0, 0.05, 0.02, 0.5, 16, (0.5, 1 / Mc, 0.5 / Mc))
@@ -665,8 +666,21 @@ def test_forward_of_few_samples_vs_oracle(port_kernels, tag, dtype, B, N, H, Mc)
         setattr(ref, name, getattr(dev, name))
     x = np.random.rand(B, N).astype(dtype)
     want = ref.compute_activation(x)
-    for _ in range(2):   # the tickets are zero again after a launch
+    for _ in range(2):
         assert rel_inf(dev.compute_activation(x), want) < TOL[np.dtype(dtype)]
+
+
+def test_forward_of_few_samples_with_several_fills_of_shared_memory(port_kernels):
+    """Ranges of more inputs than the streaming form holds at a time."""
+    import streambrain_b200 as B200
+    N, H, Mc = 1030, 149, 129
+    rs = np.random.RandomState(3)
+    dev = B200.DenseLayer(N, H, Mc, 0.01, (0.5, 1 / Mc, 0.5 / Mc), dtype=np.float64)
+    x = rs.rand(3, N)
+    support = x @ dev.weights + dev.bias
+    e = np.exp(support.reshape(3, H, Mc) - support.reshape(3, H, Mc).max(axis=2, keepdims=True))
+    want = (e / e.sum(axis=2, keepdims=True)).reshape(3, H * Mc)
+    assert rel_inf(dev.compute_activation(x), want) < TOL[np.dtype(np.float64)]
 
 
 @pytest.mark.parametrize("tag,dtype", DTYPES)
