@@ -865,10 +865,7 @@ template cudaError_t launch_forward_product<double>(const double *, const double
                                                     cudaStream_t);
 
 // ----------------------------------------------------------------------------
-// out = sum_s partial[s] + bias, then softmax per hypercolumn.
-// One sub-warp of `width` lanes per (row, hypercolumn) group.  A lane owns the
-// entries sub, sub+width, ... of its group; with CACHE > 0 they stay in registers
-// (Mc <= CACHE*width), otherwise they are re-read from `out`.
+// out = sum_s partial[s] + bias, then softmax per hypercolumn: one warp or part of a warp per (row, hypercolumn) group.
 // ----------------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ T subwarp_max(T v, int width) {
@@ -884,7 +881,9 @@ __device__ __forceinline__ T subwarp_sum(T v, int width) {
   return v;
 }
 
-template <typename T, int CACHE>
+// Groups of any size (what the kernels below do not take): a lane owns the entries sub, sub + width, ... of its group and keeps
+// them in `out`.
+template <typename T>
 __global__ void __launch_bounds__(256)
     reduce_bias_softmax_kernel(const T *partial, int splits, long slice, const T *__restrict__ bias, T *out,
                                long groups, long H, long Mc, int width) {
@@ -896,121 +895,35 @@ __global__ void __launch_bounds__(256)
   const bool live = g < groups;
   const long base = g * Mc;            // offset of the group inside [rows, H*Mc]
   const long col0 = (g % H) * Mc;      // first column of the group
-  constexpr int NC = CACHE > 0 ? CACHE : 1;
-  T v[NC];
   T mx = -INFINITY;
-  if (CACHE > 0) {
-#pragma unroll
-    for (int e = 0; e < NC; ++e) {
-      const long j = sub + (long)e * width;
-      T s = -INFINITY;
-      if (live && j < Mc) {
-        s = partial[base + j];
-#pragma unroll 8
-        for (int z = 1; z < splits; ++z) s += partial[(long)z * slice + base + j];
-        if (bias) s += bias[col0 + j];
-      }
-      v[e] = s;
+  if (live)
+    for (long j = sub; j < Mc; j += width) {
+      T s = partial[base + j];
+      for (int z = 1; z < splits; ++z) s += partial[(long)z * slice + base + j];
+      if (bias) s += bias[col0 + j];
+      out[base + j] = s;
       mx = s > mx ? s : mx;
     }
-    mx = subwarp_max(mx, width);
-    T sum = (T)0;
-#pragma unroll
-    for (int e = 0; e < NC; ++e) {
-      const long j = sub + (long)e * width;
-      if (live && j < Mc) {
-        v[e] = sbb_exp(v[e] - mx);
-        sum += v[e];
-      }
+  mx = subwarp_max(mx, width);
+  T sum = (T)0;
+  if (live)
+    for (long j = sub; j < Mc; j += width) {
+      const T e = sbb_exp(out[base + j] - mx);
+      out[base + j] = e;
+      sum += e;
     }
-    sum = subwarp_sum(sum, width);
-#pragma unroll
-    for (int e = 0; e < NC; ++e) {
-      const long j = sub + (long)e * width;
-      if (live && j < Mc) out[base + j] = v[e] / sum;
-    }
-  } else {
-    if (live)
-      for (long j = sub; j < Mc; j += width) {
-        T s = partial[base + j];
-        for (int z = 1; z < splits; ++z) s += partial[(long)z * slice + base + j];
-        if (bias) s += bias[col0 + j];
-        out[base + j] = s;
-        mx = s > mx ? s : mx;
-      }
-    mx = subwarp_max(mx, width);
-    T sum = (T)0;
-    if (live)
-      for (long j = sub; j < Mc; j += width) {
-        const T e = sbb_exp(out[base + j] - mx);
-        out[base + j] = e;
-        sum += e;
-      }
-    sum = subwarp_sum(sum, width);
-    if (live)
-      for (long j = sub; j < Mc; j += width) out[base + j] = out[base + j] / sum;
-  }
+  sum = subwarp_sum(sum, width);
+  if (live)
+    for (long j = sub; j < Mc; j += width) out[base + j] = out[base + j] / sum;
 }
 
-// The same for groups of more than 16 entries (one whole warp per group) with every per-element index a
-// compile-time multiple of 32 from three pointers formed once: the general kernel above spends most of its
-// instructions on 64-bit index arithmetic (about 100 per element at Mc = 300, which made it issue-bound: 183 us
-// for 246 MB at the 1568 -> 100 x 300 layer).
-template <typename T, int NC, bool SPLIT>
-__global__ void __launch_bounds__(256)
-    softmax_warp_kernel(const T *partial, int splits, long slice, const T *__restrict__ bias, T *out, long groups,
-                        int H, int Mc) {
-  after_previous();
-  const int lane = threadIdx.x & 31;
-  const long g = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (g >= groups) return;   // whole warps leave together
-  const T *src = partial + g * Mc + lane;
-  const T *bs = bias ? bias + (g % H) * (long)Mc + lane : nullptr;
-  T *dst = out + g * Mc + lane;
-  const int left = Mc - lane;   // entry e of this lane exists when e * 32 < left
-  T v[NC];
+// Softmax of a group of up to 32 * NC entries by one warp: lane l holds entries l, l + 32, ..., entry e of it exists when
+// e * 32 < left (-inf otherwise), and dst points at its first one.
+template <typename T, int NC>
+__device__ __forceinline__ void warp_softmax(T (&v)[NC], int left, T *dst) {
   T mx = -INFINITY;
-  // (entries inside, partial sums outside: all entries' loads are in flight at once.  With the loops the other way round
-  // each partial sum was a round trip to memory of its own: 11.2 us for 128 x 15 groups of 200 doubles in six partial
-  // sums)
 #pragma unroll
-  for (int e = 0; e < NC; ++e) {
-    v[e] = e * 32 < left ? src[e * 32] : -INFINITY;
-    if (!SPLIT && bs && e * 32 < left) v[e] += bs[e * 32];
-  }
-  if (SPLIT) {
-    if constexpr (sizeof(T) == 4) {
-#pragma unroll 2
-      for (int z = 1; z < splits; ++z) {
-        const T *sz = src + (long)z * slice;
-        T d[NC];
-#pragma unroll
-        for (int e = 0; e < NC; ++e) d[e] = e * 32 < left ? sz[e * 32] : (T)0;
-#pragma unroll
-        for (int e = 0; e < NC; ++e) v[e] += d[e];
-      }
-    } else {   // (more registers, for the many parts of a float64 batch; in float32, seven parts, a 1001 x 481 step took 45.7 us with them, 41.0 so)
-      constexpr int AHEAD = NC <= 4 ? 8 : NC <= 12 ? 4 : 2;
-      T d[AHEAD][NC];
-#pragma unroll 1
-      for (int z = 1; z < splits; z += AHEAD) {
-        const T *sz = src + (long)z * slice;
-#pragma unroll
-        for (int a = 0; a < AHEAD; ++a)
-#pragma unroll
-          for (int e = 0; e < NC; ++e) d[a][e] = z + a < splits && e * 32 < left ? sz[a * slice + e * 32] : (T)0;
-#pragma unroll
-        for (int a = 0; a < AHEAD; ++a)
-#pragma unroll
-          for (int e = 0; e < NC; ++e) v[e] += d[a][e];
-      }
-    }
-  }
-#pragma unroll
-  for (int e = 0; e < NC; ++e) {
-    if (SPLIT && bs && e * 32 < left) v[e] += bs[e * 32];
-    mx = v[e] > mx ? v[e] : mx;
-  }
+  for (int e = 0; e < NC; ++e) mx = v[e] > mx ? v[e] : mx;
   mx = subwarp_max(mx, 32);
   T sum = (T)0;
   if constexpr (sizeof(T) == 8) {
@@ -1058,6 +971,132 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// The same for groups of more than 16 entries (one whole warp per group) with every per-element index a
+// compile-time multiple of 32 from three pointers formed once: the general kernel above spends most of its
+// instructions on 64-bit index arithmetic (about 100 per element at Mc = 300, which made it issue-bound: 183 us
+// for 246 MB at the 1568 -> 100 x 300 layer).
+template <typename T, int NC, bool SPLIT>
+__global__ void __launch_bounds__(256)
+    softmax_warp_kernel(const T *partial, int splits, long slice, const T *__restrict__ bias, T *out, long groups,
+                        int H, int Mc) {
+  after_previous();
+  const int lane = threadIdx.x & 31;
+  const long g = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (g >= groups) return;   // whole warps leave together
+  const T *src = partial + g * Mc + lane;
+  const T *bs = bias ? bias + (g % H) * (long)Mc + lane : nullptr;
+  T *dst = out + g * Mc + lane;
+  const int left = Mc - lane;   // entry e of this lane exists when e * 32 < left
+  T v[NC];
+  // (entries inside, partial sums outside: all entries' loads are in flight at once.  With the loops the other way round
+  // each partial sum was a round trip to memory of its own: 11.2 us for 128 x 15 groups of 200 doubles in six partial
+  // sums)
+#pragma unroll
+  for (int e = 0; e < NC; ++e) {
+    v[e] = e * 32 < left ? src[e * 32] : -INFINITY;
+    if (!SPLIT && bs && e * 32 < left) v[e] += bs[e * 32];
+  }
+  if (SPLIT) {
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll 2
+      for (int z = 1; z < splits; ++z) {
+        const T *sz = src + (long)z * slice;
+        T d[NC];
+#pragma unroll
+        for (int e = 0; e < NC; ++e) d[e] = e * 32 < left ? sz[e * 32] : (T)0;
+#pragma unroll
+        for (int e = 0; e < NC; ++e) v[e] += d[e];
+      }
+    } else {   // (more registers, for the many parts of a float64 batch; in float32, seven parts, a 1001 x 481 step took 45.7 us with them, 41.0 so)
+      constexpr int AHEAD = NC <= 4 ? 8 : NC <= 12 ? 4 : 2;
+      T d[AHEAD][NC];
+#pragma unroll 1
+      for (int z = 1; z < splits; z += AHEAD) {
+        const T *sz = src + (long)z * slice;
+#pragma unroll
+        for (int a = 0; a < AHEAD; ++a)
+#pragma unroll
+          for (int e = 0; e < NC; ++e) d[a][e] = z + a < splits && e * 32 < left ? sz[a * slice + e * 32] : (T)0;
+#pragma unroll
+        for (int a = 0; a < AHEAD; ++a)
+#pragma unroll
+          for (int e = 0; e < NC; ++e) v[e] += d[a][e];
+      }
+    }
+  }
+  if (SPLIT && bs) {
+#pragma unroll
+    for (int e = 0; e < NC; ++e)
+      if (e * 32 < left) v[e] += bs[e * 32];
+  }
+  warp_softmax<T, NC>(v, left, dst);
+}
+
+// The same for few groups with many partial sums: a block per group, a thread per entry while the partial sums are added (in
+// the same order), then the group's softmax by the first warp as above.  With a warp per group, 64 groups of 207 entries in 64
+// partial sums took 24.8 us, two dependent rounds of loads per pair of partial sums; 8.6 us so.
+template <typename T, int NC>
+__global__ void __launch_bounds__(256)
+    softmax_block_kernel(const T *__restrict__ partial, int splits, long slice, const T *__restrict__ bias, T *__restrict__ out, int H,
+                         int Mc) {
+  after_previous();
+  __shared__ T support[NC * 32];
+  const long base = (long)blockIdx.x * Mc;
+  const T *bs = bias ? bias + (blockIdx.x % (unsigned)H) * (long)Mc : nullptr;
+  for (int j = threadIdx.x; j < Mc; j += 256) {
+    constexpr int U = 16;
+    const T *p = partial + base + j;
+    T s = p[0];
+    for (int z = 1; z < splits; z += U) {
+      T d[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) d[u] = z + u < splits ? p[(z + u) * slice] : (T)0;
+#pragma unroll
+      for (int u = 0; u < U; ++u) s = z + u < splits ? s + d[u] : s;
+    }
+    support[j] = bs ? s + bs[j] : s;
+  }
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  const int left = Mc - (int)threadIdx.x;
+  T v[NC];
+#pragma unroll
+  for (int e = 0; e < NC; ++e) v[e] = e * 32 < left ? support[threadIdx.x + e * 32] : -INFINITY;
+  warp_softmax<T, NC>(v, left, out + base + threadIdx.x);
+}
+
+// And for groups of up to 16 entries, one to a lane: 2^log2 lanes per group.  1524 x 82 groups of 5 doubles took 15.3 us in the
+// general kernel, most of it index arithmetic in 64 bits, 8.7 us here; 627 x 96 groups of 16 floats 16.7 and 14.0.
+template <typename T>
+__global__ void __launch_bounds__(256)
+    softmax_lanes_kernel(const T *partial, int splits, long slice, const T *__restrict__ bias, T *out,   // (may be the same)
+                         uint32_t groups, uint32_t H, uint32_t Mc, int log2) {
+  after_previous();
+  const int width = 1 << log2;
+  const uint32_t at = blockIdx.x * 256u + threadIdx.x, g = at >> log2, sub = at & (uint32_t)(width - 1);
+  const bool live = g < groups && sub < Mc;
+  const uint32_t i = g * Mc + sub;
+  T v = -INFINITY;
+  if (live) {
+    constexpr int U = 8;
+    const T *p = partial + i;
+    v = p[0];
+    for (int z = 1; z < splits; z += U) {
+      T d[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) d[u] = z + u < splits ? p[(z + u) * slice] : (T)0;
+#pragma unroll
+      for (int u = 0; u < U; ++u) v = z + u < splits ? v + d[u] : v;
+    }
+    if (bias) v += bias[g % H * Mc + sub];
+  }
+  T mx = v > -INFINITY ? v : -INFINITY;
+  mx = subwarp_max(mx, width);
+  const T e = live ? sbb_exp(v - mx) : (T)0;
+  const T sum = subwarp_sum(e, width);
+  if (live) out[i] = e / sum;
+}
+
 // out[r, j] = sum_s partial[s, r, j] + bias[j]   (no softmax)
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -1086,11 +1125,14 @@ cudaError_t launch_reduce_bias_softmax(const T *partial, int splits, const T *bi
   int width = 32;
   while (width > 1 && (width >> 1) >= Mc) width >>= 1;
   const long groups = rows * H;
-  const long per_warp = 32 / width;
-  const long warps = (groups + per_warp - 1) / per_warp;
-  const unsigned blocks = (unsigned)((warps + 7) / 8);
   const long per_lane = (Mc + width - 1) / width;
   if (width == 32 && per_lane <= 16 && H < (1l << 31) && Mc < (1l << 31)) {
+    // few groups, many partial sums: a block per group.  (128 x 30 groups of 100 in six parts stay with a warp each.)
+    if (splits >= 8 && groups <= 4 * sm_count()) {
+      if (per_lane <= 8) launch_next(softmax_block_kernel<T, 8>, (unsigned)groups, 256, 0, st, partial, splits, total, bias, out, (int)H, (int)Mc);
+      else launch_next(softmax_block_kernel<T, 16>, (unsigned)groups, 256, 0, st, partial, splits, total, bias, out, (int)H, (int)Mc);
+      return launched();
+    }
     // one warp per group: the lean kernel (same arithmetic, same summation order)
 #define SBB_SOFTMAX_WARP(NC)                                                                                      \
   do {                                                                                                            \
@@ -1108,16 +1150,15 @@ cudaError_t launch_reduce_bias_softmax(const T *partial, int splits, const T *bi
 #undef SBB_SOFTMAX_WARP
     return launched();
   }
-  if (per_lane <= 4)
-    launch_next(reduce_bias_softmax_kernel<T, 4>, blocks, 256, 0, st, partial, splits, total, bias, out, groups, H, Mc, width);
-  else if (per_lane <= 8)
-    launch_next(reduce_bias_softmax_kernel<T, 8>, blocks, 256, 0, st, partial, splits, total, bias, out, groups, H, Mc, width);
-  else if (per_lane <= 12)
-    launch_next(reduce_bias_softmax_kernel<T, 12>, blocks, 256, 0, st, partial, splits, total, bias, out, groups, H, Mc, width);
-  else if (per_lane <= 16)
-    launch_next(reduce_bias_softmax_kernel<T, 16>, blocks, 256, 0, st, partial, splits, total, bias, out, groups, H, Mc, width);
-  else
-    launch_next(reduce_bias_softmax_kernel<T, 0>, blocks, 256, 0, st, partial, splits, total, bias, out, groups, H, Mc, width);
+  if (width < 32 && groups * width < (1l << 31) && total < (1l << 31)) {
+    int log2 = 0;
+    while ((1 << log2) < width) ++log2;
+    launch_next(softmax_lanes_kernel<T>, (unsigned)((groups * width + 255) / 256), 256, 0, st, partial, splits, total, bias, out,
+                (uint32_t)groups, (uint32_t)H, (uint32_t)Mc, log2);
+    return launched();
+  }
+  const long per_warp = 32 / width, warps = (groups + per_warp - 1) / per_warp;
+  launch_next(reduce_bias_softmax_kernel<T>, (unsigned)((warps + 7) / 8), 256, 0, st, partial, splits, total, bias, out, groups, H, Mc, width);
   return launched();
 }
 template cudaError_t launch_reduce_bias_softmax<float>(const float *, int, const float *, float *, long, long, long,
