@@ -245,26 +245,30 @@ __global__ void __launch_bounds__(Tile::THREADS, 2)
 // (In float64 it is what SBB_F64_CONTRACTION=dfma runs, with the general epilogue's division and library logarithm, to
 // compare the FP64 tensor-core kernels with: 1568 -> 30 x 100 at batch 128, forward pass 82 us against 43, train step without
 // a mask update 136 against 72.)
-template <typename T, bool A_KMAJOR>
+// ROWS: rows of a warp.  Eight; four, and twice the warps, in trace steps that leave the schedulers idle, up to two blocks to an SM,
+// or four and few slabs (an element's logarithm and division are some hundred dependent instructions, and a thread has two of
+// them per row): 1001 x 481 at batch 97 13.2 -> 10.7 us, 1211 x 39 at 40 8.0 -> 5.6, 231 x 3108 at 47 (392 blocks) 11.2 -> 9.5; 1843 x 424 at
+// 5485 (406 blocks) 328 -> 372, so not there.  The forward product gains nothing (9.1 and 9.4).
+template <typename T, bool A_KMAJOR, int ROWS>
 struct SmallShape {
   static constexpr bool KMAJOR = A_KMAJOR;
-  static constexpr int BM = 32, BN = 64, BK = 32, STAGES = 4, THREADS = 128;
+  static constexpr int BM = 32, BN = 64, BK = 32, STAGES = 4, THREADS = 32 / ROWS * 32;
   static constexpr int LDA = 32 + 4, LDB = BN;   // K-major A as [m][k], MN-major as [k][m]: 16-byte rows
   static constexpr int A_STAGE = 32 * LDA, B_STAGE = BK * LDB;
   static constexpr size_t SMEM_BYTES = (size_t)STAGES * (A_STAGE + B_STAGE) * sizeof(T);
 };
 
 // grid.x = column tiles, grid.y = row tiles, grid.z = k-splits
-template <typename T, bool A_KMAJOR, class Epilogue>
-__global__ void __launch_bounds__(SmallShape<T, A_KMAJOR>::THREADS)
+template <typename T, bool A_KMAJOR, int ROWS, class Epilogue>
+__global__ void __launch_bounds__(SmallShape<T, A_KMAJOR, ROWS>::THREADS)
     small_contraction_kernel(const T *__restrict__ A, long lda, const T *__restrict__ Bm, long ldb, long Mdim, long Ndim, int K,
                              int kper, Epilogue ep) {
   after_previous();
-  using S = SmallShape<T, A_KMAJOR>;
+  using S = SmallShape<T, A_KMAJOR, ROWS>;
   using L = Slab<T, S, 1>;
   extern __shared__ __align__(16) unsigned char small_smem[];
   T *As = reinterpret_cast<T *>(small_smem), *Bs = As + S::STAGES * S::A_STAGE;
-  const int w8 = (threadIdx.x >> 5) * 8, lane = threadIdx.x & 31;
+  const int w8 = (threadIdx.x >> 5) * ROWS, lane = threadIdx.x & 31;
   const long m0 = (long)blockIdx.y * S::BM, n0 = (long)blockIdx.x * S::BN;
   const int kbeg = blockIdx.z * kper;
   const int kend = min(K, kbeg + kper);
@@ -279,10 +283,10 @@ __global__ void __launch_bounds__(SmallShape<T, A_KMAJOR>::THREADS)
     }
     cp_async_commit();
   }
-  typename Epilogue::Strip strip(ep, m0 + w8, n0 + lane, lane);
-  T acc[8][2];
+  typename Epilogue::template Strip<ROWS> strip(ep, m0 + w8, n0 + lane, lane);
+  T acc[ROWS][2];
 #pragma unroll
-  for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = (T)0;
+  for (int r = 0; r < ROWS; ++r) acc[r][0] = acc[r][1] = (T)0;
   for (int kt = 0; kt < nk; ++kt) {
     cp_async_wait<S::STAGES - 2>();   // slab kt has landed
     __syncthreads();                  // ... for every thread, and the stage refilled below is free
@@ -297,25 +301,25 @@ __global__ void __launch_bounds__(SmallShape<T, A_KMAJOR>::THREADS)
     const T *as = As + kt % S::STAGES * S::A_STAGE, *bs = Bs + kt % S::STAGES * S::B_STAGE + lane;
 #pragma unroll
     for (int k4 = 0; k4 < S::BK; k4 += 4) {
-      T a[8][4];   // [row][k]
+      T a[ROWS][4];   // [row][k]
       if constexpr (A_KMAJOR) {
 #pragma unroll
-        for (int r = 0; r < 8; ++r) lds4(as + (w8 + r) * S::LDA + k4, a[r]);
+        for (int r = 0; r < ROWS; ++r) lds4(as + (w8 + r) * S::LDA + k4, a[r]);
       } else {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          T v[8];
-          lds4(as + (k4 + k) * S::LDA + w8, v);
-          lds4(as + (k4 + k) * S::LDA + w8 + 4, v + 4);
+          T v[ROWS];
 #pragma unroll
-          for (int r = 0; r < 8; ++r) a[r][k] = v[r];
+          for (int r = 0; r < ROWS; r += 4) lds4(as + (k4 + k) * S::LDA + w8 + r, v + r);
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r) a[r][k] = v[r];
         }
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const T b0 = bs[(k4 + k) * S::LDB], b1 = bs[(k4 + k) * S::LDB + 32];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
+        for (int r = 0; r < ROWS; ++r) {
           acc[r][0] = fma(a[r][k], b0, acc[r][0]);
           acc[r][1] = fma(a[r][k], b1, acc[r][1]);
         }
@@ -350,13 +354,14 @@ struct StoreEpilogue {
       }
     }
   }
-  // Rows m .. m + 7, columns n and n + 32 of the small-tile kernel.
+  // ROWS rows from m on, columns n and n + 32 of the small-tile kernel.
+  template <int ROWS>
   struct Strip {
     __device__ __forceinline__ Strip(const StoreEpilogue &, long, long, int) {}
-    __device__ __forceinline__ void finish(const StoreEpilogue &e, T (&acc)[8][2], long m, long n, int z) const {
+    __device__ __forceinline__ void finish(const StoreEpilogue &e, T (&acc)[ROWS][2], long m, long n, int z) const {
       T *p = e.out + (long)z * e.zstride + m * e.ld + n;
 #pragma unroll
-      for (int r = 0; r < 8; ++r, p += e.ld) {
+      for (int r = 0; r < ROWS; ++r, p += e.ld) {
         if (m + r < e.rows && n < e.cols) p[0] = acc[r][0];
         if (m + r < e.rows && n + 32 < e.cols) p[32] = acc[r][1];
       }
@@ -423,14 +428,15 @@ struct TraceEpilogue {
       }
     }
   }
-  // Rows m .. m + 7, columns n and n + 32 of the small-tile kernel: everything the epilogue reads is requested before the
+  // ROWS rows from m on, columns n and n + 32 of the small-tile kernel: everything the epilogue reads is requested before the
   // main loop, and its arithmetic (the same as above) is one row at a time from one copy of the code, the rows rotating
   // through slot 0: unrolled, sixteen logarithms and divisions come from a cold instruction cache.
+  template <int ROWS>
   struct Strip {
-    T old[8][2], ci, cj[2];   // ci: lane r holds row r's
+    T old[ROWS][2], ci, cj[2];   // ci: lane r holds row r's
     unsigned on = 0;          // bit 2 * r + c: the mask keeps the element's weight
     __device__ __forceinline__ Strip(const TraceEpilogue &e, long m, long n, int lane) {
-      const long i0 = e.row0 + m, i = i0 + (lane & 7);
+      const long i0 = e.row0 + m, i = i0 + (lane & (ROWS - 1));
       ci = i < e.row_end ? e.Ci[i] : (T)0;
       const T *src = e.Cij + i0 * e.M + n;
       const uint8_t *mrow[2];
@@ -441,7 +447,7 @@ struct TraceEpilogue {
         mrow[c] = e.wmask ? e.wmask + i0 * e.H + (unsigned)j / (unsigned)e.Mc : nullptr;
       }
 #pragma unroll
-      for (int r = 0; r < 8; ++r, src += e.M)
+      for (int r = 0; r < ROWS; ++r, src += e.M)
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           const bool in = i0 + r < e.row_end && n + 32 * c < e.M;
@@ -449,9 +455,9 @@ struct TraceEpilogue {
           if (in && (mrow[c] == nullptr || mrow[c][r * e.H] != 0)) on |= 1u << (2 * r + c);
         }
     }
-    __device__ __forceinline__ void finish(const TraceEpilogue &e, T (&acc)[8][2], long m, long n, int) {
+    __device__ __forceinline__ void finish(const TraceEpilogue &e, T (&acc)[ROWS][2], long m, long n, int) {
       const long i0 = e.row0 + m;
-      const int rows = (int)min(8L, e.row_end - i0);
+      const int rows = (int)min((long)ROWS, e.row_end - i0);
       T *pc = e.Cij + i0 * e.M + n, *pw = e.W + i0 * e.M + n;
 #pragma unroll 1
       for (int r = 0; r < rows; ++r, pc += e.M, pw += e.M) {
@@ -466,7 +472,7 @@ struct TraceEpilogue {
             pw[32 * c] = w;
           }
 #pragma unroll
-          for (int k = 0; k < 7; ++k) {
+          for (int k = 0; k < ROWS - 1; ++k) {
             acc[k][c] = acc[k + 1][c];
             old[k][c] = old[k + 1][c];
           }
@@ -742,11 +748,11 @@ static cudaError_t launch_f64_mma(const double *A, long lda, const double *Bm, l
 // tiles 35.6 -> 12.8 us, 96 tiles 36.5 -> 28.3, but 216 tiles 55.0 -> 54.7 at batch 97 and 125 -> 136 at batch 512.
 static bool small_tiles(long tiles, bool forward) { return (forward ? 2 : 1) * tiles < sm_count(); }
 
-template <typename T, bool A_KMAJOR, class Ep>
-static cudaError_t launch_small_contraction(const T *A, long lda, const T *Bm, long ldb, long Mdim, long Ndim, int K,
+template <typename T, bool A_KMAJOR, int ROWS, class Ep>
+static cudaError_t launch_small_tiles(const T *A, long lda, const T *Bm, long ldb, long Mdim, long Ndim, int K,
                                             int splits, int kper, Ep ep, cudaStream_t st) {
-  using S = SmallShape<T, A_KMAJOR>;
-  auto kernel = small_contraction_kernel<T, A_KMAJOR, Ep>;
+  using S = SmallShape<T, A_KMAJOR, ROWS>;
+  auto kernel = small_contraction_kernel<T, A_KMAJOR, ROWS, Ep>;
   static bool configured[64] = {false};
   const cudaError_t e = allow_smem(kernel, configured);
   if (e != cudaSuccess) return e;
@@ -754,6 +760,16 @@ static cudaError_t launch_small_contraction(const T *A, long lda, const T *Bm, l
   if (grid.y > 65535u || grid.z > 65535u) return cudaErrorInvalidConfiguration;
   launch_next(kernel, grid, S::THREADS, spread_smem(S::SMEM_BYTES, (long)grid.x * grid.y * splits), st, A, lda, Bm, ldb, Mdim, Ndim, K, kper, ep);
   return launched();
+}
+template <typename T, bool A_KMAJOR, class Ep>
+static cudaError_t launch_small_contraction(const T *A, long lda, const T *Bm, long ldb, long Mdim, long Ndim, int K,
+                                            int splits, int kper, Ep ep, cudaStream_t st) {
+  using S = SmallShape<T, A_KMAJOR, 8>;
+  const long blocks = ((Ndim + S::BN - 1) / S::BN) * ((Mdim + S::BM - 1) / S::BM) * splits;
+  if constexpr (!A_KMAJOR) {
+    if (blocks <= 2 * sm_count() || (blocks <= 4 * sm_count() && K <= 512)) return launch_small_tiles<T, A_KMAJOR, 4>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, ep, st);
+  }
+  return launch_small_tiles<T, A_KMAJOR, 8>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, ep, st);
 }
 
 template <bool A_KMAJOR, int V, class Ep>
@@ -787,7 +803,7 @@ static cudaError_t launch_contraction(const T *A, long lda, const T *Bm, long ld
   if (mt <= 0 || nt <= 0 || K <= 0) return cudaSuccess;
   // `vec`: every operand row starts on a 16-byte boundary and holds a whole number of 16-byte pieces
   if constexpr (std::is_same<T, double>::value) {
-    if (!f64_mma_enabled() && Mdim <= 65535L * SmallShape<T, A_KMAJOR>::BM)   // (its row tiles are grid.y)
+    if (!f64_mma_enabled() && Mdim <= 65535L * SmallShape<T, A_KMAJOR, 8>::BM)   // (its row tiles are grid.y)
       return launch_small_contraction<T, A_KMAJOR>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, ep, st);
     if (vec && lda % 2 == 0 && ldb % 2 == 0)
       return launch_f64_mma<A_KMAJOR, 2>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, to_pairs(ep), st);
