@@ -253,16 +253,21 @@ struct PhaseTimer {
 
 // Whether the kernels for layers of few units may take the layer: they sum in another order than the tiled ones.  In a
 // float32 layer that learns from its own activations a difference in the last digit of an activation reaches the weights
-// of all its inputs alike and adds up over tens of thousands of them in the next forward pass, so those keep their order.
+// of all its inputs alike and adds up over them in the next forward pass, by a factor of some N taupdt / 10, and taupdt grows
+// with the root of the batch.  Where that is large those keep their order (4096 -> 32 at batch 512 moved 6e-5 in two steps), and
+// where the forward pass is the slower one: its reads of the weights take M lines of memory for each of M units.  (Two launches
+// a step instead of four: 206 -> 9 units at batch 44 27 -> 17 us, 72 -> 16 at 41 33 -> 18, 1024 -> 24 at 58 42 -> 27; but 1211 -> 30
+// at 400 44 -> 40, 3333 -> 32 at 57 42 -> 113.)
 template <typename T>
-bool narrow(const sbb_layer *L) {
-  return std::is_same<T, double>::value || L->desc.kind == SBB_LAYER_DENSE;
+bool narrow(const sbb_layer *L, long B) {
+  if (std::is_same<T, double>::value || L->desc.kind == SBB_LAYER_DENSE) return true;
+  return L->N <= 4096 && L->M <= 32 && L->N * L->N * B <= (1l << 28) && L->M * L->M * (L->N / 256 + 1) <= 3000;
 }
 
 template <typename T>
 int layer_forward(sbb_layer *L, const T *x, long B, T *y, cudaStream_t st) {
   const T *W = static_cast<const T *>(L->state[SBB_STATE_WEIGHTS]);
-  if (narrow<T>(L) && sbb::narrow_forward(B, L->N, L->M, sizeof(T))) {
+  if (narrow<T>(L, B) && sbb::narrow_forward(B, L->N, L->M, sizeof(T))) {
     PhaseTimer timer(L, SBB_PHASE_FORWARD, st);
     SBB_CUDA(sbb::launch_narrow_forward<T>(x, W, static_cast<const T *>(L->state[SBB_STATE_BIAS]), y, B, L->N, L->M, L->Mc, st));
     timer.stop();
@@ -369,7 +374,7 @@ int layer_train_step(sbb_layer *L, const T *x, const T *y, long B, long h, cudaS
   const sbb::TraceParams<T> p = sbb::make_trace_params<T>(L->desc.taupdt, L->desc.taupdt / 2, B);
   T *Ci = static_cast<T *>(L->state[SBB_STATE_CI]);
   T *Cj = static_cast<T *>(L->state[SBB_STATE_CJ]);
-  if (narrow<T>(L) && sbb::narrow_layer(L->N, L->M)) {
+  if (narrow<T>(L, B) && sbb::narrow_layer(L->N, L->M)) {
     PhaseTimer timer(L, SBB_PHASE_TRACE, st);
     SBB_CUDA(sbb::launch_narrow_train<T>(x, y, B, L->N, L->M, L->H, L->Mc, Ci, Cj, static_cast<T *>(L->state[SBB_STATE_CIJ]),
                                          static_cast<T *>(L->state[SBB_STATE_WEIGHTS]),

@@ -308,9 +308,10 @@ cudaError_t forward_mp(const T *x, const T *W, const T *bias, T *out, long B, lo
   constexpr int RMAX = narrow_samples(MP, sizeof(T));
   // few samples: one per block (or warp), so that all SMs take part; more of them share each read of the weights
   const long per = (B + 295) / 296;
+  const bool alone = N <= 64 || (N <= 512 && per > 1);   // (500 -> 31 at batch 128, a step: 37 us alone, 25 shared)
 #define SBB_NARROW_FWD(R)                                                                                              \
   do {                                                                                                                 \
-    if (N <= 512) /* not enough inputs to share among the warps of a block */                                          \
+    if (alone) /* not enough inputs to share among the warps of a block, or samples enough without */                  \
       launch_next(narrow_forward_kernel<T, MP, R, 1>, (unsigned)((B + 8 * R - 1) / (8 * R)), 256, 0, st, x, W, bias, out, B, (int)N, (int)M, (int)Mc); \
     else                                                                                                               \
       launch_next(narrow_forward_kernel<T, MP, R, 8>, (unsigned)((B + R - 1) / R), 256, 0, st, x, W, bias, out, B, (int)N, (int)M, (int)Mc); \
