@@ -140,12 +140,17 @@ __device__ __forceinline__ double log_positive(double x) {
 // grid.x = row tiles of the output, grid.y = column tiles (swapped when cols_fastest), grid.z = k-splits.
 // k-split z covers [z*kper, min(K, (z+1)*kper)), kper a multiple of BK.  The epilogue receives the thread's
 // accumulators: ep.tile(acc, m, n, z) with acc[mi][ni][e] = output element (m + 8*mi, n + 8*ni + e), n even;
-// ep.prefetch(m, n, lane) is called before the main loop with the first element of the warp's 32 x 32 block.
+// ep.prefetch(m, n, lane) is called before the main loop with the first element of the warp's 32 x 32 block.  Epilogue::LATE:
+// the kernel before this one in the stream does not write what the main loop reads.
 template <bool A_KMAJOR, int BM, bool DEEP, int V, class Epilogue>
 __global__ void __launch_bounds__(Cfg<BM>::THREADS, Cfg<BM, DEEP>::CTAS_PER_SM)
     contraction_kernel(const double *__restrict__ A, long lda, const double *__restrict__ Bm, long ldb, long Mdim,
                        long Ndim, int K, int kper, bool cols_fastest, Epilogue ep) {
-  after_previous();
+  // 16-byte copies go past L1, so a kernel whose operands were complete before the kernel ahead of it let it start (see
+  // trace_kernel) waits only ahead of its epilogue: train step 1568 -> 30 x 100 at batch 128 73.1 -> 70.2 us, 784 -> 30 x 100 at 32
+  // 33.9 -> 31.3.  (Four blocks of 64 rows on an SM: 73.2 and 28.6.)
+  constexpr bool LATE = Epilogue::LATE && V == 2;
+  if constexpr (!LATE) after_previous();
   constexpr int A_STAGE = Cfg<BM>::A_STAGE, LDA_M = Cfg<BM>::LDA_M, STAGES = Cfg<BM, DEEP>::STAGES;
   extern __shared__ __align__(16) double smem[];
   double *As = smem, *Bs = smem + STAGES * A_STAGE;
@@ -219,6 +224,7 @@ __global__ void __launch_bounds__(Cfg<BM>::THREADS, Cfg<BM, DEEP>::CTAS_PER_SM)
     cur = next;
   }
   cp_async_wait<0>();
+  if constexpr (LATE) after_previous();
   ep.tile(acc, m0 + wm + g, n0 + wn + 2 * t, (int)blockIdx.z);
 }
 

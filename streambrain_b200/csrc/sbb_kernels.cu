@@ -487,6 +487,7 @@ struct TraceEpilogue {
 // accumulator pairs of the mma.sync fragment layout (element (m, n) and (m, n + 1), n even).
 // ----------------------------------------------------------------------------
 struct StorePairs {
+  static constexpr bool LATE = false;
   double *out;
   long rows, cols, ld, zstride;
   bool vec;
@@ -520,6 +521,7 @@ struct StorePairs {
 // from one copy of the code (the accumulators rotate): unrolled it was 32 logarithms long and ran from a cold instruction
 // cache.  1568 x 3000, batch 128: 96 us with that, a 64-bit division per column and a float64 division per row and column.
 struct TracePairs {
+  static constexpr bool LATE = true;   // that kernel is column_vectors_kernel, which writes the reciprocals, or a copy of old traces
   const double *rci, *rcj;   // reciprocals of Ci and Cj, 0 below the threshold
   double *Cij, *W;
   const uint8_t *wmask;
