@@ -995,15 +995,15 @@ __device__ __forceinline__ void warp_softmax(T (&v)[NC], int left, T *dst) {
 // for 246 MB at the 1568 -> 100 x 300 layer).
 template <typename T, int NC, bool SPLIT>
 __global__ void __launch_bounds__(256)
-    softmax_warp_kernel(const T *partial, int splits, long slice, const T *__restrict__ bias, T *out, long groups,
-                        int H, int Mc) {
+    softmax_warp_kernel(const T *partial, int splits, long slice, const T *__restrict__ bias, T *out, uint32_t groups,
+                        uint32_t H, int Mc) {
   after_previous();
   const int lane = threadIdx.x & 31;
-  const long g = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const uint32_t g = blockIdx.x * 8u + (threadIdx.x >> 5);
   if (g >= groups) return;   // whole warps leave together
-  const T *src = partial + g * Mc + lane;
-  const T *bs = bias ? bias + (g % H) * (long)Mc + lane : nullptr;
-  T *dst = out + g * Mc + lane;
+  const T *src = partial + (long)g * Mc + lane;
+  const T *bs = bias ? bias + (long)(g % H) * Mc + lane : nullptr;
+  T *dst = out + (long)g * Mc + lane;
   const int left = Mc - lane;   // entry e of this lane exists when e * 32 < left
   T v[NC];
   // (entries inside, partial sums outside: all entries' loads are in flight at once.  With the loops the other way round
@@ -1144,7 +1144,7 @@ cudaError_t launch_reduce_bias_softmax(const T *partial, int splits, const T *bi
   while (width > 1 && (width >> 1) >= Mc) width >>= 1;
   const long groups = rows * H;
   const long per_lane = (Mc + width - 1) / width;
-  if (width == 32 && per_lane <= 16 && H < (1l << 31) && Mc < (1l << 31)) {
+  if (width == 32 && per_lane <= 16 && groups < (1l << 31)) {
     // few groups, many partial sums: a block per group.  (128 x 30 groups of 100 in six parts stay with a warp each.)
     if (splits >= 8 && groups <= 4 * sm_count()) {
       if (per_lane <= 8) launch_next(softmax_block_kernel<T, 8>, (unsigned)groups, 256, 0, st, partial, splits, total, bias, out, (int)H, (int)Mc);
@@ -1156,12 +1156,13 @@ cudaError_t launch_reduce_bias_softmax(const T *partial, int splits, const T *bi
   do {                                                                                                            \
     if (splits > 1)                                                                                               \
       launch_next(softmax_warp_kernel<T, NC, true>, (unsigned)((groups + 7) / 8), 256, 0, st, partial, splits, total, bias, out, \
-                                                                                    groups, (int)H, (int)Mc);    \
+                                                                                    (uint32_t)groups, (uint32_t)H, (int)Mc);    \
     else                                                                                                          \
       launch_next(softmax_warp_kernel<T, NC, false>, (unsigned)((groups + 7) / 8), 256, 0, st, partial, splits, total, bias, out, \
-                                                                                     groups, (int)H, (int)Mc);   \
+                                                                                     (uint32_t)groups, (uint32_t)H, (int)Mc);   \
   } while (0)
-    if (per_lane <= 4) SBB_SOFTMAX_WARP(4);
+    if (per_lane <= 2) SBB_SOFTMAX_WARP(2);
+    else if (per_lane <= 4) SBB_SOFTMAX_WARP(4);
     else if (per_lane <= 8) SBB_SOFTMAX_WARP(8);
     else if (per_lane <= 12) SBB_SOFTMAX_WARP(12);
     else SBB_SOFTMAX_WARP(16);
