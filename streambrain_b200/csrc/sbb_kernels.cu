@@ -746,7 +746,8 @@ static cudaError_t launch_f64_mma(const double *A, long lda, const double *Bm, l
 }
 
 // When the 32 x 64 tiles take over, in 128 x 128 tiles.  Forward products: below half an SM's worth; 28 tiles 18.5 -> 9.1
-// us, but 92 tiles 19.0 -> 20.6.  Trace steps, whose epilogue is a logarithm and a division per output: below one per SM; 32
+// us, but 92 tiles 19.0 -> 20.6.  And up to 64 samples (launch_contraction), of whose large tiles half or more is padding: 4999 x
+// 2989 at batch 32 92 -> 42 us, at 64 93 -> 72, at 96 94 -> 105; 42265 x 150 74 -> 35, 75 -> 47, 76 -> 60.  Trace steps, whose epilogue is a logarithm and a division per output: below one per SM; 32
 // tiles 35.6 -> 12.8 us, 96 tiles 36.5 -> 28.3, but 216 tiles 55.0 -> 54.7 at batch 97 and 125 -> 136 at batch 512.
 static bool small_tiles(long tiles, bool forward) { return (forward ? 2 : 1) * tiles < sm_count(); }
 
@@ -811,7 +812,7 @@ static cudaError_t launch_contraction(const T *A, long lda, const T *Bm, long ld
       return launch_f64_mma<A_KMAJOR, 2>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, to_pairs(ep), st);
     return launch_f64_mma<A_KMAJOR, 1>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, cols_fastest, to_pairs(ep), st);
   } else {
-    if (small_tiles(mt * nt * splits, A_KMAJOR))
+    if (small_tiles(mt * nt * splits, A_KMAJOR) || (A_KMAJOR && Mdim <= 64))
       return launch_small_contraction<T, A_KMAJOR>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, ep, st);
     if (vec) return launch_tiles<A_KMAJOR, 4>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, cols_fastest, ep, st);
     return launch_tiles<A_KMAJOR, 1>(A, lda, Bm, ldb, Mdim, Ndim, K, splits, kper, cols_fastest, ep, st);
