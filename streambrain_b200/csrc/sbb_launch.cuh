@@ -29,16 +29,17 @@ inline cudaError_t launch_next(void (*kernel)(P...), dim3 grid, unsigned threads
   return cudaLaunchKernelEx(&cfg, kernel, (P)args...);
 }
 
-// The same in clusters of `cluster` blocks.
+// The same in clusters of blocks.
 template <class... P, class... A>
-inline cudaError_t launch_clusters(void (*kernel)(P...), dim3 grid, unsigned cluster, unsigned threads, size_t smem, cudaStream_t st,
+inline cudaError_t launch_clusters(void (*kernel)(P...), dim3 grid, dim3 cluster, unsigned threads, size_t smem, cudaStream_t st,
                                    A... args) {
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = cluster;
-  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  attr[1].val.clusterDim.x = cluster.x;
+  attr[1].val.clusterDim.y = cluster.y;
+  attr[1].val.clusterDim.z = cluster.z;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads, 1, 1);
