@@ -185,6 +185,7 @@ struct sbb_layer {
   void *state[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   size_t state_bytes[7] = {0, 0, 0, 0, 0, 0, 0};
   Scratch fwd_partial;   // k-split partial sums of the forward product
+  Scratch split_partial; // products of the parts of a long batch (trace steps of few output tiles)
   Scratch score;         // mask-update scratch: per-row score, active count, filter key, old bit; best keys per block
   Scratch hx, hy, ht;    // staging for the host-buffer entry points
   Scratch ticket;        // finished blocks of a launch: [whole launch][per hypercolumn]; zero between launches
@@ -351,8 +352,8 @@ int train_rows(sbb_layer *L, const T *x, const T *y, long B, long N, long M, lon
   PhaseTimer timer(L, SBB_PHASE_TRACE, st);
   const int splits = L == nullptr ? 1 : tc ? sbb::trace_splits_tc(B, N, M) : sbb::trace_splits<T>(B, N, M);
   if (splits > 1) {
-    SBB_TRY(L->fwd_partial.reserve((size_t)splits * (size_t)(N * M) * sizeof(T)));   // (the forward pass has done with it)
-    T *const partial = static_cast<T *>(L->fwd_partial.d);
+    SBB_TRY(L->split_partial.reserve((size_t)splits * (size_t)(N * M) * sizeof(T)));
+    T *const partial = static_cast<T *>(L->split_partial.d);
     if (tc) {
       if constexpr (std::is_same<T, float>::value) SBB_CUDA(sbb::launch_split_product_tc(x, y, B, N, M, splits, partial, st));
     } else {
@@ -880,6 +881,7 @@ int sbb_layer_destroy(sbb_layer *L) {
   for (int k = 0; k < 7; ++k)
     if (L->state[k]) cudaFree(L->state[k]);
   L->fwd_partial.release();
+  L->split_partial.release();
   L->score.release();
   L->hx.release();
   L->hy.release();
