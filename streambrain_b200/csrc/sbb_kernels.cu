@@ -15,6 +15,7 @@
 #include "sbb_f64_mma.cuh"
 #include "sbb_launch.cuh"
 #include "sbb_math.cuh"
+#include "sbb_tc_ptx.cuh"
 
 #include <atomic>
 #include <math.h>
@@ -937,15 +938,15 @@ __global__ void __launch_bounds__(256)
 }
 
 // Softmax of a group of up to 32 * NC entries by one warp: lane l holds entries l, l + 32, ..., entry e of it exists when
-// e * 32 < left (-inf otherwise), and dst points at its first one.
-template <typename T, int NC>
+// e < FULL or e * 32 < left (-inf otherwise), and dst points at its first one.
+template <typename T, int NC, int FULL>
 __device__ __forceinline__ void warp_softmax(T (&v)[NC], int left, T *dst) {
-  T mx = -INFINITY;
-#pragma unroll
-  for (int e = 0; e < NC; ++e) mx = v[e] > mx ? v[e] : mx;
-  mx = subwarp_max(mx, 32);
-  T sum = (T)0;
   if constexpr (sizeof(T) == 8) {
+    T mx = -INFINITY;
+#pragma unroll
+    for (int e = 0; e < NC; ++e) mx = v[e] > mx ? v[e] : mx;
+    mx = subwarp_max(mx, 32);
+    T sum = (T)0;
     // one copy of the float64 exponential (the entries rotate through slot 0): unrolled, a kernel of a few microseconds
     // spends most of them fetching instructions
 #pragma unroll 1
@@ -956,16 +957,8 @@ __device__ __forceinline__ void warp_softmax(T (&v)[NC], int left, T *dst) {
       for (int q = 0; q + 1 < NC; ++q) v[q] = v[q + 1];
       v[NC - 1] = x;
     }
-  } else {
-#pragma unroll
-    for (int e = 0; e < NC; ++e) {
-      v[e] = e * 32 < left ? sbb_exp(v[e] - mx) : (T)0;
-      sum += v[e];
-    }
-  }
-  sum = subwarp_sum(sum, 32);
-  const DivideBy<T> by(sum);
-  if constexpr (sizeof(T) == 8) {
+    sum = subwarp_sum(sum, 32);
+    const DivideBy<T> by(sum);
     // (128 samples, 784 -> 15 x 200: the forward pass takes 27.5 us, and 28.8 with a multiplication by 1 / sum, which rounds
     // once more than the division)
     bool covered = true;
@@ -982,19 +975,51 @@ __device__ __forceinline__ void warp_softmax(T (&v)[NC], int left, T *dst) {
     }
 #pragma unroll
     for (int e = 0; e < NC; ++e)
-      if (e * 32 < left) dst[e * 32] = by.quotient(v[e]);
+      if (e < FULL || e * 32 < left) dst[e * 32] = by.quotient(v[e]);
   } else {
+    // What bounds the kernel in float32 is the issue of instructions, so each entry gets as few as it can: no test for the
+    // entries that every lane has, the maximum of the lanes in one instruction, one test for all entries of whether the
+    // short division covers them, and that division two entries at a time (100 groups of 300 at batch 1024: 520 instructions
+    // a group of 300 and 68.0 us without these, 37.6 us so).
+    float mx = -INFINITY;
 #pragma unroll
-    for (int e = 0; e < NC; ++e)
-      if (e * 32 < left) dst[e * 32] = by(v[e]);
+    for (int e = 0; e < NC; ++e) mx = fmaxf(v[e], mx);   // (NaNs lose, and of -0 and 0 either will do)
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(mx) : "f"(mx));
+    float sum = 0.f;
+    uint32_t least = 0xffffffffu;   // of bits(v) - 1: zeros wrap to the top
+#pragma unroll
+    for (int e = 0; e < NC; ++e) {
+      v[e] = e < FULL || e * 32 < left ? sbb_exp(v[e] - mx) : 0.f;
+      sum += v[e];
+      least = min(least, __float_as_uint(v[e]) - 1u);
+    }
+    sum = subwarp_sum(sum, 32);
+    const DivideBy<float> by(sum);
+    if (by.plain || least < __float_as_uint(DivideBy<float>::MIN) - 1u) {   // rare
+#pragma unroll 1
+      for (int e = 0; e < NC; ++e) {
+        if (e * 32 < left) dst[e * 32] = by(v[0]);
+#pragma unroll
+        for (int q = 0; q + 1 < NC; ++q) v[q] = v[q + 1];
+      }
+      return;
+    }
+    const uint64_t y = pair_of(by.y, by.y), minus_d = pair_of(-by.d, -by.d);
+#pragma unroll
+    for (int e = 0; e < NC; e += 2) {
+      const uint64_t p = pair_of(v[e], v[e + 1]), q = mul_pair(p, y);
+      const float2 r = halves(fma_pair(fma_pair(q, minus_d, p), y, q));   // DivideBy::quotient
+      if (e < FULL || e * 32 < left) dst[e * 32] = r.x;
+      if (e + 1 < FULL || (e + 1) * 32 < left) dst[(e + 1) * 32] = r.y;
+    }
   }
 }
 
 // The same for groups of more than 16 entries (one whole warp per group) with every per-element index a
 // compile-time multiple of 32 from three pointers formed once: the general kernel above spends most of its
 // instructions on 64-bit index arithmetic (about 100 per element at Mc = 300, which made it issue-bound: 183 us
-// for 246 MB at the 1568 -> 100 x 300 layer).
-template <typename T, int NC, bool SPLIT>
+// for 246 MB at the 1568 -> 100 x 300 layer at batch 1024; 37.6 us here, 6.5 TB/s).
+template <typename T, int NC, int FULL, bool SPLIT>
 __global__ void __launch_bounds__(256)
     softmax_warp_kernel(const T *partial, int splits, long slice, const T *__restrict__ bias, T *out, uint32_t groups,
                         uint32_t H, int Mc) {
@@ -1005,15 +1030,15 @@ __global__ void __launch_bounds__(256)
   const T *src = partial + (long)g * Mc + lane;
   const T *bs = bias ? bias + (long)(g % H) * Mc + lane : nullptr;
   T *dst = out + (long)g * Mc + lane;
-  const int left = Mc - lane;   // entry e of this lane exists when e * 32 < left
+  const int left = Mc - lane;   // entry e of this lane exists when e < FULL or e * 32 < left
   T v[NC];
   // (entries inside, partial sums outside: all entries' loads are in flight at once.  With the loops the other way round
   // each partial sum was a round trip to memory of its own: 11.2 us for 128 x 15 groups of 200 doubles in six partial
   // sums)
 #pragma unroll
   for (int e = 0; e < NC; ++e) {
-    v[e] = e * 32 < left ? src[e * 32] : -INFINITY;
-    if (!SPLIT && bs && e * 32 < left) v[e] += bs[e * 32];
+    v[e] = e < FULL || e * 32 < left ? src[e * 32] : -INFINITY;
+    if (!SPLIT && bs && (e < FULL || e * 32 < left)) v[e] += bs[e * 32];
   }
   if (SPLIT) {
     if constexpr (sizeof(T) == 4) {
@@ -1022,7 +1047,7 @@ __global__ void __launch_bounds__(256)
         const T *sz = src + (long)z * slice;
         T d[NC];
 #pragma unroll
-        for (int e = 0; e < NC; ++e) d[e] = e * 32 < left ? sz[e * 32] : (T)0;
+        for (int e = 0; e < NC; ++e) d[e] = e < FULL || e * 32 < left ? sz[e * 32] : (T)0;
 #pragma unroll
         for (int e = 0; e < NC; ++e) v[e] += d[e];
       }
@@ -1035,7 +1060,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
         for (int a = 0; a < AHEAD; ++a)
 #pragma unroll
-          for (int e = 0; e < NC; ++e) d[a][e] = z + a < splits && e * 32 < left ? sz[a * slice + e * 32] : (T)0;
+          for (int e = 0; e < NC; ++e) d[a][e] = z + a < splits && (e < FULL || e * 32 < left) ? sz[a * slice + e * 32] : (T)0;
 #pragma unroll
         for (int a = 0; a < AHEAD; ++a)
 #pragma unroll
@@ -1046,9 +1071,9 @@ __global__ void __launch_bounds__(256)
   if (SPLIT && bs) {
 #pragma unroll
     for (int e = 0; e < NC; ++e)
-      if (e * 32 < left) v[e] += bs[e * 32];
+      if (e < FULL || e * 32 < left) v[e] += bs[e * 32];
   }
-  warp_softmax<T, NC>(v, left, dst);
+  warp_softmax<T, NC, FULL>(v, left, dst);
 }
 
 // The same for few groups with many partial sums: a block per group, a thread per entry while the partial sums are added (in
@@ -1081,7 +1106,7 @@ __global__ void __launch_bounds__(256)
   T v[NC];
 #pragma unroll
   for (int e = 0; e < NC; ++e) v[e] = e * 32 < left ? support[threadIdx.x + e * 32] : -INFINITY;
-  warp_softmax<T, NC>(v, left, out + base + threadIdx.x);
+  warp_softmax<T, NC, 0>(v, left, out + base + threadIdx.x);
 }
 
 // And for groups of up to 16 entries, one to a lane: 2^log2 lanes per group.  1524 x 82 groups of 5 doubles took 15.3 us in the
@@ -1153,20 +1178,25 @@ cudaError_t launch_reduce_bias_softmax(const T *partial, int splits, const T *bi
       return launched();
     }
     // one warp per group: the lean kernel (same arithmetic, same summation order)
-#define SBB_SOFTMAX_WARP(NC)                                                                                      \
+#define SBB_SOFTMAX_WARP(NC, FULL)                                                                                     \
   do {                                                                                                            \
     if (splits > 1)                                                                                               \
-      launch_next(softmax_warp_kernel<T, NC, true>, (unsigned)((groups + 7) / 8), 256, 0, st, partial, splits, total, bias, out, \
+      launch_next(softmax_warp_kernel<T, NC, FULL, true>, (unsigned)((groups + 7) / 8), 256, 0, st, partial, splits, total, bias, out, \
                                                                                     (uint32_t)groups, (uint32_t)H, (int)Mc);    \
     else                                                                                                          \
-      launch_next(softmax_warp_kernel<T, NC, false>, (unsigned)((groups + 7) / 8), 256, 0, st, partial, splits, total, bias, out, \
+      launch_next(softmax_warp_kernel<T, NC, FULL, false>, (unsigned)((groups + 7) / 8), 256, 0, st, partial, splits, total, bias, out, \
                                                                                      (uint32_t)groups, (uint32_t)H, (int)Mc);   \
   } while (0)
-    if (per_lane <= 2) SBB_SOFTMAX_WARP(2);
-    else if (per_lane <= 4) SBB_SOFTMAX_WARP(4);
-    else if (per_lane <= 8) SBB_SOFTMAX_WARP(8);
-    else if (per_lane <= 12) SBB_SOFTMAX_WARP(12);
-    else SBB_SOFTMAX_WARP(16);
+    // (float32: slots in pairs, and a test for the last pair's entries alone.  100 groups of 300 at batch 1024, 10 slots: 68.0 us
+    // with 12 slots and a test in each, 37.6 so.  In float64 more kernels than these gain nothing: the exponential takes the time)
+    constexpr bool F32 = sizeof(T) == 4;
+    if (per_lane <= 2) SBB_SOFTMAX_WARP(2, 0);
+    else if (per_lane <= 4) SBB_SOFTMAX_WARP(4, F32 ? 2 : 0);
+    else if (F32 && per_lane <= 6) SBB_SOFTMAX_WARP(F32 ? 6 : 8, F32 ? 4 : 0);
+    else if (per_lane <= 8) SBB_SOFTMAX_WARP(8, F32 ? 6 : 0);
+    else if (F32 && per_lane <= 10) SBB_SOFTMAX_WARP(F32 ? 10 : 12, F32 ? 8 : 0);
+    else if (per_lane <= 12) SBB_SOFTMAX_WARP(12, F32 ? 10 : 0);
+    else SBB_SOFTMAX_WARP(16, F32 ? 12 : 0);
 #undef SBB_SOFTMAX_WARP
     return launched();
   }

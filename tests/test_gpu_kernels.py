@@ -113,6 +113,29 @@ def test_softmax_rounds_like_the_division(k, tag, dtype, Mc):
 
 
 @pytest.mark.parametrize("tag,dtype", DTYPES)
+@pytest.mark.parametrize("Mc", [17, 32, 64, 65, 128, 129, 192, 193, 256, 257, 320, 321, 384, 385, 511, 512])
+def test_softmax_at_the_edges_of_its_slots(k, tag, dtype, Mc):
+    """The smallest and largest group of every kernel that holds a group in one warp, with zeros, infinities and NaNs
+    among the entries: the same to the bit as the kernel for groups of any size."""
+    rs = np.random.RandomState(Mc)
+    a = (rs.randn(64, Mc) * 3).astype(dtype)
+    a[1] = 0
+    a[2, ::2], a[2, 1::2] = 0, -0.0
+    a[3, -1] = np.inf
+    a[4, 0] = np.nan
+    a[5] = -np.inf
+    a[6, :-1] = -np.inf
+    a[7] = 1e30
+    a[8, Mc // 2] = -np.nan
+    a[9, 1:] = -np.inf
+    wide = np.full((64, 544), -np.inf, dtype=dtype)
+    wide[:, :Mc] = a
+    got = k.softmax_minicolumns(a, 1, Mc)
+    want = k.softmax_minicolumns(wide, 1, 544)[:, :Mc]
+    assert np.array_equal(got, want, equal_nan=True)
+
+
+@pytest.mark.parametrize("tag,dtype", DTYPES)
 @pytest.mark.parametrize("B,N,H,Mc", SHAPES)
 def test_trace_update_vs_oracle(k, port_kernels, tag, dtype, B, N, H, Mc):
     rs = np.random.RandomState(B * 11 + N)
