@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(Tile::THREADS, 2)
 // reads is requested before the main loop.  Each output is the same chain of FMAs over ascending k as in the kernel above.
 // (In float64 it is what SBB_F64_CONTRACTION=dfma runs, with the general epilogue's division and library logarithm, to
 // compare the FP64 tensor-core kernels with: 1568 -> 30 x 100 at batch 128, forward pass 82 us against 43, train step without
-// a mask update 136 against 72.)
+// a mask update 142 against 70.)
 // ROWS: rows of a warp.  Eight; four, and twice the warps, in trace steps that leave the schedulers idle, up to two blocks to an SM,
 // or four and few slabs (an element's logarithm and division are some hundred dependent instructions, and a thread has two of
 // them per row): 1001 x 481 at batch 97 13.2 -> 10.7 us, 1211 x 39 at 40 8.0 -> 5.6, 231 x 3108 at 47 (392 blocks) 11.2 -> 9.5; 1843 x 424 at
@@ -1355,6 +1355,94 @@ template cudaError_t launch_vector_ema<double>(double *, const double *, long, T
 // Trace step: fused (x^T y in the contraction, traces and weights in its
 // epilogue) and split (raw x^T y, then an element-wise tail).
 // ----------------------------------------------------------------------------
+// The float32 trace step of few samples: no tile of products to form, so a warp walks `rows` rows of 32 columns.  A lane owns a
+// column, whose activations (and column data) stay in registers; lane r loads row r's inputs, which reach the others by
+// shuffles.  Four rows' old traces are in flight while the four before are worked on, one after the other from one copy of the
+// arithmetic.  Each sum is the chain of FMAs over ascending samples that the tile kernels form.
+template <int NB>
+__global__ void __launch_bounds__(256)
+    trace_few_kernel(const float *__restrict__ x, long ldx, const float *__restrict__ y, int B, TraceEpilogue<float> e, unsigned column_warps,
+                     int rows) {
+  after_previous();
+  const int lane = threadIdx.x & 31;
+  const unsigned warp = blockIdx.x * 8u + (threadIdx.x >> 5);
+  const long i0 = e.row0 + (long)(warp / column_warps) * rows;
+  if (i0 >= e.row_end) return;
+  const int here = e.row_end - i0 < rows ? (int)(e.row_end - i0) : rows;
+  const unsigned j = warp % column_warps * 32u + lane;
+  const bool live = j < (unsigned)e.M;
+  const unsigned col = live ? j : 0u;   // (loads need no branch)
+  float yv[NB], xv[NB];
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    yv[b] = b < B ? y[(long)b * e.M + col] : 0.f;
+    xv[b] = b < B && lane < here ? x[(long)b * ldx + i0 + lane] : 0.f;
+  }
+  const float my_ci = lane < here ? e.Ci[i0 + lane] : 0.f, cj = e.Cj[col];
+  const bool column_on = !(cj < e.p.cthr);
+  float *c = e.Cij + i0 * e.M + col, *w = e.W + i0 * e.M + col;
+  const uint8_t *mask = e.wmask ? e.wmask + i0 * e.H + col / (unsigned)e.Mc : nullptr;
+  constexpr int U = 4;
+  float old[U], next[U];
+  bool on[U], next_on[U];
+  auto fetch = [&](int r0) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool in = r0 + u < here;
+      next[u] = in ? c[(long)(r0 + u) * e.M] : 0.f;
+      next_on[u] = mask == nullptr || (in && mask[(long)(r0 + u) * e.H] != 0);
+    }
+  };
+  fetch(0);
+#pragma unroll 1
+  for (int r0 = 0; r0 < here; r0 += U) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      old[u] = next[u];
+      on[u] = next_on[u];
+    }
+    fetch(r0 + U);
+    const int last = here < r0 + U ? here : r0 + U;
+#pragma unroll 1
+    for (int r = r0; r < last; ++r) {
+      float sum = 0.f;
+#pragma unroll
+      for (int b = 0; b < NB; ++b) sum = fmaf(__shfl_sync(0xffffffffu, xv[b], r), yv[b], sum);
+      const float ci = __shfl_sync(0xffffffffu, my_ci, r);
+      const float v = trace_ema(old[0], sum, e.p);
+      const float g = on[0] && column_on && !(ci < e.p.cthr) ? log_ratio(v, ci, cj, e.p.cthr4) : 0.f;
+      if (live) {
+        c[(long)r * e.M] = v;
+        w[(long)r * e.M] = g;
+      }
+#pragma unroll
+      for (int u = 0; u + 1 < U; ++u) {
+        old[u] = old[u + 1];
+        on[u] = on[u + 1];
+      }
+    }
+  }
+}
+// What bounds it is the issue of instructions, some hundred for the two divisions and the logarithm of an element, and two more for
+// each sample.  Train step without a mask update, tiles -> this, at 4, 8 and 16 samples: 3202 x 7398 177 -> 95, 178 -> 116,
+// 178 -> 154 us; 2217 x 1425 35.9 -> 21.0, 36.0 -> 23.2, 36.0 -> 27.1; 26849 x 49 23.1 -> 16.3, 23.2 -> 16.4, 23.2 -> 15.9; 1211 x 39
+// 7.2 -> 7.1, 7.3 -> 6.9, 7.2 -> 6.9.  The same kernel for 24 samples loses: 190 -> 254, 38.7 -> 49.4, 26.2 -> 26.0, 7.2 -> 7.0.
+constexpr long kFewTrace = 16;   // most samples
+static bool few_trace_fits(long B, long rows, long M) {
+  return B >= 1 && B <= kFewTrace && M < (1l << 31) && ((M + 31) / 32) * ((rows + 3) / 4) < (1l << 31);
+}
+static cudaError_t launch_trace_few(const float *x, long ldx, const float *y, long B, const TraceEpilogue<float> &e, cudaStream_t st) {
+  const long n = e.row_end - e.row0, column_warps = (e.M + 31) / 32;
+  int rows = 32;   // (fewer where that leaves fewer than sixteen warps to an SM)
+  while (rows > 4 && ((n + rows - 1) / rows) * column_warps < 16l * sm_count()) rows >>= 1;
+  const unsigned blocks = (unsigned)((((n + rows - 1) / rows) * column_warps + 7) / 8);
+  auto launch = [&](auto kernel) { launch_next(kernel, blocks, 256, 0, st, x, ldx, y, (int)B, e, (unsigned)column_warps, rows); };
+  if (B <= 4) launch(trace_few_kernel<4>);
+  else if (B <= 8) launch(trace_few_kernel<8>);
+  else launch(trace_few_kernel<16>);
+  return launched();
+}
+
 template <typename T>
 cudaError_t launch_trace_update_fused(const T *x, const T *y, long B, long N, long M, long H, long Mc, const T *Ci,
                                       const T *Cj, const T *rci, const T *rcj, T *Cij, T *w, const uint8_t *wmask,
@@ -1365,6 +1453,8 @@ cudaError_t launch_trace_update_fused(const T *x, const T *y, long B, long N, lo
                    aligned16(x) && aligned16(y);
   TraceEpilogue<T> ep{Ci, Cj, Cij, w, wmask, row_begin, row_end, M, H, Mc, p,
                       (M % V == 0) && aligned16(Cij) && aligned16(w), rci, rcj};
+  if constexpr (std::is_same<T, float>::value)
+    if (few_trace_fits(B, row_end - row_begin, M)) return launch_trace_few(x, N, y, B, ep, st);
   const int kper = (int)((B + Tile::BK - 1) / Tile::BK) * Tile::BK;
   return launch_contraction<T, false>(x + row_begin, N, y, M, row_end - row_begin, M, (int)B, 1, kper, vec, true, ep, st);
 }

@@ -7,8 +7,8 @@
 // (tcgen05.mma.cta_group::2); each CTA stages and splits its own 128 rows of A and half of the columns of B.  (!PAIR, what
 // SBB_TC_PAIR=0 selects: one CTA works on 128 rows x 192 columns by itself and stages all columns of B, which leaves room
 // for three stages; the products, chains and sums are the same.  It is there to compare with and for
-// devices that cannot place pairs.  Train step without a mask update: 1568 -> 30 x 100 at batch 128 32.1 us in pairs, 33.2
-// without; 55296 -> 30 x 100 at 256 565 and 686 us.)
+// devices that cannot place pairs.  Train step without a mask update: 1568 -> 30 x 100 at batch 128 20.0 us in pairs, 20.5
+// without; 55296 -> 30 x 100 at 256 539 and 656 us; 1568 -> 100 x 300 at 1024 487 and 632.)
 // Roles in a CTA (672 threads, one CTA per SM, tiles walked persistently):
 //   warps 0-11   epilogue: accumulator, old trace (by TMA, the whole tile's blocks one tile ahead), arithmetic; new traces
 //                and weights leave by TMA

@@ -747,3 +747,36 @@ def test_long_batches_of_few_outputs_vs_oracle(port_kernels, tag, dtype, kind, B
             assert not dev.weights[np.repeat(ref.wmask == 0, Mc, axis=1)].any()
         for name in ("weights", "bias", "Ci", "Cj", "Cij"):
             setattr(dev, name, getattr(ref, name))
+
+
+@pytest.mark.parametrize("B", [1, 4, 5, 8, 9, 16, 17])
+@pytest.mark.parametrize("N,H,Mc", [(131, 3, 11), (33, 1, 33), (1025, 37, 9), (66, 1, 301), (5003, 5, 31), (7, 90, 33)])
+def test_train_steps_of_few_samples_of_odd_rows_vs_oracle(port_kernels, N, H, Mc, B):
+    """A float32 train step of up to 16 samples on rows that no 16-byte copy can address: every number of samples a kernel is
+    built for, rows and columns that fill their warps and that do not, four to thirty-two rows a warp, inputs that never
+    fire (no weights there), masks with one and many hypercolumns to a row."""
+    import streambrain_b200 as B200
+    hp = dict(khalf=-100.0, pmin=0.05, taubdt=0.02, density=0.5)
+    init = (0.5, 1 / Mc, 0.5 / Mc)
+    np.random.seed(5)
+    dev = B200.StructuralPlasticityLayer(N, H, Mc, 0.1, hp["khalf"], hp["pmin"], hp["taubdt"], hp["density"], 16, init, dtype=np.float32)
+    ref = oracle.OracleLayer(port_kernels, "plastic", N, H, Mc, 0.1, init, np.float32, **hp)
+    ref.wmask = dev.wmask
+    Ci = dev.Ci
+    Ci[N // 2:N // 2 + 3] = 1e-12   # below the threshold, and stays there
+    dev.Ci = Ci
+    for name in ("weights", "bias", "Ci", "Cj", "Cij"):
+        setattr(ref, name, getattr(dev, name))
+    rs = np.random.RandomState(B + N)
+    tol = TOL[np.dtype(np.float32)]
+    for step in range(2):
+        x = rs.rand(B, N).astype(np.float32)
+        x[:, N // 2:N // 2 + 3] = 0
+        y = rs.dirichlet(np.ones(Mc), size=(B, H)).reshape(B, H * Mc).astype(np.float32)
+        for layer in (ref, dev):
+            layer.train_step(x, y, None)
+        for name in ("Ci", "Cj", "Cij", "bias"):
+            assert rel_inf(getattr(dev, name), getattr(ref, name)) < tol, (name, step)
+        assert weight_err(dev.weights, ref.weights) < 10 * tol, step
+        assert not dev.weights[np.repeat(ref.wmask == 0, Mc, axis=1)].any()
+        assert not dev.weights[N // 2:N // 2 + 3].any()
