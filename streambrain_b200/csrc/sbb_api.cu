@@ -141,6 +141,15 @@ struct Scratch {
     cap = n;
     return SBB_OK;
   }
+  // For a workspace the caller can do without: false where the device has no room for it, or where it would have to grow
+  // while `st` is being captured (an allocation would end the capture).
+  bool room(size_t n, cudaStream_t st) {
+    if (n <= cap) return true;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const bool grown = cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone && reserve(n) == SBB_OK;
+    if (!grown) (void)cudaGetLastError();   // answered here: no later launch may find it
+    return grown;
+  }
   void release() {
     if (d) cudaFree(d);
     d = nullptr;
@@ -334,8 +343,8 @@ int layer_finish(sbb_layer *L, long h, cudaStream_t st) {
   return layer_mask<T>(L, h, st);
 }
 
-// Traces, weights and (bias.kbi != null) the bias of `N` input rows.  `L` (may be null) times the contraction; `vectors`
-// holds the reciprocals of Ci and Cj where the kernels take them.
+// Traces, weights and (bias.kbi != null) the bias of `N` input rows.  `L` times the contraction and keeps the products of a
+// batch's parts; `vectors` holds the reciprocals of Ci and Cj where the kernels take them.
 template <typename T>
 int train_rows(sbb_layer *L, const T *x, const T *y, long B, long N, long M, long H, T *Ci, T *Cj, T *Cij, T *W,
                const uint8_t *wmask, const sbb::TraceParams<T> &p, const sbb::BiasParams<T> &bias, Scratch &vectors,
@@ -347,12 +356,14 @@ int train_rows(sbb_layer *L, const T *x, const T *y, long B, long N, long M, lon
     rci = static_cast<T *>(vectors.d);
     rcj = rci + (N + 3) / 4 * 4;
   }
+  // All memory is there before the first launch: a step that moved the vectors and then gave up could not be repeated.  Without
+  // room for the products of the parts the fused kernel, which needs none, takes the whole batch.
+  int splits = N == 0 ? 1 : tc ? sbb::trace_splits_tc(B, N, M) : sbb::trace_splits<T>(B, N, M);
+  if (splits > 1 && !L->split_partial.room((size_t)splits * (size_t)(N * M) * sizeof(T), st)) splits = 1;
   SBB_CUDA(sbb::launch_column_vectors<T>(sbb::ColumnVectors<T>{x, N, Ci, rci}, sbb::ColumnVectors<T>{y, M, Cj, rcj}, B, p, bias, st));
   if (N == 0) return SBB_OK;
   PhaseTimer timer(L, SBB_PHASE_TRACE, st);
-  const int splits = L == nullptr ? 1 : tc ? sbb::trace_splits_tc(B, N, M) : sbb::trace_splits<T>(B, N, M);
   if (splits > 1) {
-    SBB_TRY(L->split_partial.reserve((size_t)splits * (size_t)(N * M) * sizeof(T)));
     T *const partial = static_cast<T *>(L->split_partial.d);
     if (tc) {
       if constexpr (std::is_same<T, float>::value) SBB_CUDA(sbb::launch_split_product_tc(x, y, B, N, M, splits, partial, st));

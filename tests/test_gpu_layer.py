@@ -780,3 +780,92 @@ def test_train_steps_of_few_samples_of_odd_rows_vs_oracle(port_kernels, N, H, Mc
         assert weight_err(dev.weights, ref.weights) < 10 * tol, step
         assert not dev.weights[np.repeat(ref.wmask == 0, Mc, axis=1)].any()
         assert not dev.weights[N // 2:N // 2 + 3].any()
+
+
+def _twins(kind, N, H, Mc, dtype):
+    """Two layers of the same state, and a long batch's inputs and outputs on the device."""
+    import torch
+    import streambrain_b200 as B200
+    init = (0.5, 1 / Mc, 0.5 / Mc)
+    twins = []
+    for _ in range(2):
+        np.random.seed(5)
+        twins.append(B200.DenseLayer(N, H, Mc, 0.1, init, dtype=dtype) if kind == "dense" else
+                     B200.StructuralPlasticityLayer(N, H, Mc, 0.1, -100.0, 0.05, 0.02, 0.5, 16, init, dtype=dtype))
+    t = torch.float32 if dtype is np.float32 else torch.float64
+
+    def batch(B, seed):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        x = torch.rand((B, N), generator=g, device="cuda", dtype=t)
+        y = torch.softmax(torch.rand((B, H, Mc), generator=g, device="cuda", dtype=t), dim=2).reshape(B, H * Mc)
+        return x, y
+    return twins, batch
+
+
+def _assert_same_step(a, b, dtype):
+    tol = TOL[np.dtype(dtype)]
+    for name in ("Ci", "Cj", "bias"):   # (not of the contraction: the same launch in both)
+        assert np.array_equal(getattr(a, name), getattr(b, name)), name
+    assert rel_inf(a.Cij, b.Cij) < tol
+    assert weight_err(a.weights, b.weights) < 10 * tol
+
+
+@pytest.mark.parametrize("tag,dtype,B,N,M", [("f32", np.float32, 782, 915, 2782), ("f64", np.float64, 1088, 1752, 1030),
+                                             ("f32", np.float32, 8196, 1268, 928)])
+def test_long_batch_without_room_for_the_products_of_its_parts(tag, dtype, B, N, M):
+    """The parts of a long batch want some 50 MB; on a device with less than that left the step is done in one piece, the
+    layer is as it would have been, and the steps after it know nothing of the failed allocation."""
+    import torch
+    from streambrain_b200._lib import lib
+    (roomy, tight), batch = _twins("plastic", N, 1, M, dtype)
+    x0, y0 = batch(16, 0)
+    x, y = batch(B, 1)
+    for layer in (roomy, tight):   # (what the kernels' code takes of the device is there before it is filled)
+        layer.train_step(x0, y0, None)
+    launches = lib.sbb_kernel_launches()
+    roomy.train_step(x, y, None)
+    split = lib.sbb_kernel_launches() - launches
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    hogs, size = [], torch.cuda.mem_get_info()[0]
+    while size >= 16 << 20:
+        try:
+            hogs.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+        except torch.OutOfMemoryError:
+            size //= 2
+    try:
+        launches = lib.sbb_kernel_launches()
+        tight.train_step(x, y, None)
+        whole = lib.sbb_kernel_launches() - launches
+        torch.cuda.synchronize()
+    finally:
+        hogs.clear()
+        torch.cuda.empty_cache()
+    assert whole == 2 and split >= whole   # (vectors, and the trace update in one launch)
+    _assert_same_step(tight, roomy, dtype)
+    for layer in (roomy, tight):
+        layer.train_step(x, y, None)
+    torch.cuda.synchronize()
+    _assert_same_step(tight, roomy, dtype)
+
+
+@pytest.mark.parametrize("tag,dtype", DTYPES)
+@pytest.mark.parametrize("kind,B,N,H,Mc", [("plastic", 1500, 88, 2, 66), ("plastic", 2049, 65, 3, 13), ("dense", 1024, 300, 1, 40)])
+def test_first_long_batch_of_a_layer_inside_a_capture(tag, dtype, kind, B, N, H, Mc):
+    """A captured step may not allocate: without the workspace of a split batch it is recorded in one piece."""
+    import torch
+    (eager, captured), batch = _twins(kind, N, H, Mc, dtype)
+    x, y = batch(B, 1)
+    step = (lambda layer: layer.train_step(x, y)) if kind == "dense" else (lambda layer: layer.train_step(x, y, None))
+    before = captured.Cij
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step(captured)
+    assert np.array_equal(captured.Cij, before)
+    for _ in range(2):
+        step(eager)
+        graph.replay()
+        torch.cuda.synchronize()
+        _assert_same_step(captured, eager, dtype)
+    del graph
