@@ -29,6 +29,7 @@ int fail(int code, const char *fmt, ...) {
 }
 
 int cuda_fail(cudaError_t e, const char *what) {
+  (void)cudaGetLastError();   // reported here: the launch that asks next may not find it and fail for it
   return fail(SBB_ERR_CUDA, "%s: %s (%s)", what, cudaGetErrorName(e), cudaGetErrorString(e));
 }
 

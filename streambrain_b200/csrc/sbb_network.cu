@@ -39,8 +39,10 @@ int net_fail(int code, const char *fmt, ...) {
 #define NET_CUDA(call)                                                                       \
   do {                                                                                       \
     cudaError_t e__ = (call);                                                                \
-    if (e__ != cudaSuccess)                                                                  \
+    if (e__ != cudaSuccess) {                                                                \
+      (void)cudaGetLastError();   /* reported here: no later launch may find it */           \
       return net_fail(SBB_ERR_CUDA, "%s: %s (%s)", #call, cudaGetErrorName(e__), cudaGetErrorString(e__)); \
+    }                                                                                        \
   } while (0)
 
 #define NET_TRY(call)               \
@@ -295,6 +297,7 @@ int sbb_network_create(int dtype, sbb_network **out) {
   cudaError_t e = cudaGetDevice(&net->device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&net->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
+    (void)cudaGetLastError();
     delete net;
     return net_fail(SBB_ERR_CUDA, "network_create: %s", cudaGetErrorString(e));
   }

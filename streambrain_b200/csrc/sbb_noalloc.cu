@@ -60,6 +60,7 @@ int scratch_for_current_device(void **out) {
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess || dev < 0 || dev >= kMaxDevices) {
+    (void)cudaGetLastError();
     snprintf(g_noalloc_error, sizeof(g_noalloc_error), "update_mask_noalloc: cannot identify the current device (%s)",
              cudaGetErrorString(e));
     return SBB_ERR_CUDA;
@@ -69,6 +70,7 @@ int scratch_for_current_device(void **out) {
     void *p = nullptr;
     e = cudaGetSymbolAddress(&p, g_mask_scratch);  // resolved with `dev` current, kept for later calls
     if (e != cudaSuccess || p == nullptr) {
+      (void)cudaGetLastError();
       snprintf(g_noalloc_error, sizeof(g_noalloc_error),
                "update_mask_noalloc: cudaGetSymbolAddress failed on device %d (%s)", dev, cudaGetErrorString(e));
       return SBB_ERR_CUDA;

@@ -869,3 +869,24 @@ def test_first_long_batch_of_a_layer_inside_a_capture(tag, dtype, kind, B, N, H,
         torch.cuda.synchronize()
         _assert_same_step(captured, eager, dtype)
     del graph
+
+
+@pytest.mark.parametrize("tag,dtype", DTYPES)
+def test_an_allocation_that_fails_is_reported_once(B200, tag, dtype):
+    """A layer larger than any device is refused; the next call on another layer does not fail for it half way."""
+    from streambrain_b200 import _lib
+    np.random.seed(0)
+    layer = B200.DenseLayer(60, 1, 40, 0.1, (0.5, 0.025, 0.0125), dtype=dtype)
+    x, y = np.random.rand(7, 60).astype(dtype), np.eye(40, dtype=dtype)[:7]
+    desc = _lib.LayerDesc(_lib.dtype_code(dtype), _lib.DENSE, 1 << 28, 1, 1 << 20, 0.1, 0.0, 0.0, 0.0, 0)
+    handle = ctypes.c_void_p()
+    assert _lib.lib.sbb_layer_create(ctypes.byref(desc), ctypes.byref(handle)) == 2
+    assert b"emory" in _lib.lib.sbb_last_error() and not handle.value
+    before = layer.Ci
+    layer.train_step(x, y)
+    assert not np.array_equal(layer.Ci, before)
+    net = B200.Network(dtype)
+    net.add_layer(layer)
+    assert _lib.lib.sbb_layer_create(ctypes.byref(desc), ctypes.byref(handle)) == 2
+    net.fit(x, y, 7, [(0, 1)])
+    assert np.isfinite(layer.weights).all()
