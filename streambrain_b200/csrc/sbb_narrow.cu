@@ -359,10 +359,20 @@ cudaError_t forward_mp(const T *x, const T *W, const T *bias, T *out, long B, lo
 // once per block of samples: with very many samples that is more L2 traffic than the tiled kernels cause.
 bool narrow_layer(long N, long M) { return M <= 32 && N < (1l << 30); }
 bool narrow_forward(long B, long N, long M, size_t elem) {
-  // float64: its weights are read 8 bytes at a time, rows apart; the tiles of the FP64 tensor-core kernel read them once.
-  // 1000 inputs, 10 units: 7.0 us here and 9.1 in tiles up to batch 128, 9.5 and 9.3 at 512, 48 and 24 at 4096; 16 units: 12.4
-  // and 9.1, 148 and 24; 300 inputs, 16 units 24.4 and 9.1; 20000 inputs, 10 units 28 and 19.
-  if (elem == 8) return narrow_layer(N, M) && M <= 10 && N <= 8192 && B <= 256;
+  // float64: a block of one sample reads all weights 8 bytes at a time, rows apart, and the cost grows with samples x inputs; the
+  // tiles of the FP64 tensor-core kernel read them once but wait for more inputs one after the other.  Where the line lies
+  // depends on the row's length: a unit costs twice as much in rows of 64 bytes (8 units) as in those of 72 to 88, in rows of 128
+  // (16 units) four times.  Measured, us, here and in tiles.  7 units: 20000 inputs at batch 8 6 and 22, at 256 29 and 34; 30001 at 256 43 and 44.  8
+  // units: 8192 at 64 12.9 and 15.5, 3000 at 180 16.4 and 10.5, 8192 at 256 38 and 15.  10 units: 20000 at 8 9.1 and 20.4, 8192 at 128
+  // 16.4 and 15.4, at 256 22.9 and 15.6.  11 units: 20000 at 32 15.5 and 23.3, 3000 at 256 13.0 and 12.2.  12 to 15 units: 1000 at
+  // 128 6.4 to 7.3 and 7.7 to 8.5, 8192 at 64 14.4 to 16.4 and 15.5 to 17.1, 3000 at 128 11.5 to 13.2 and 10.8 to 11.8.  16 units:
+  // 1000 at 64 12.2 and 7.7.  Up to four samples the other way is the kernel for few samples: 5000 -> 7 4.5 here and 6.5 there, 5000
+  // -> 11 5.7 and 9.1, 1000 -> 11 5.4 and 4.6, 1000 -> 15 6.4 and 5.6, 20000 -> 10 9.0 and 8.1.
+  if (elem == 8) {
+    if (!narrow_layer(N, M) || M > 15 || B > 256) return false;
+    if (B <= kFewSamples) return M <= 7 ? N <= 32768 : M <= 11 && N <= 8192;
+    return B * N <= (M <= 7 ? 1l << 23 : M == 8 ? 1l << 19 : M <= 10 ? 1l << 20 : M == 11 ? 5l << 17 : B <= 64 ? 1l << 19 : 1l << 17);
+  }
   const long r = narrow_samples(M, elem);
   return narrow_layer(N, M) && ((B + r - 1) / r) * N * M <= (1l << 28);
 }

@@ -593,6 +593,35 @@ def test_layers_of_few_units_vs_oracle(port_kernels, tag, dtype, kind, B, N, H, 
             setattr(dev, name, getattr(ref, name))
 
 
+def _forward_and_launches(port_kernels, dtype, B, N, H, Mc):
+    """A dense layer's forward pass within the tolerance of the oracle's in float64; returns the kernels it launched."""
+    import streambrain_b200 as B200
+    from streambrain_b200._lib import lib
+    rs = np.random.RandomState(B + N + Mc)
+    init = (0.5, 1 / Mc, 0.5 / Mc)
+    dev = B200.DenseLayer(N, H, Mc, 0.1, init, dtype=dtype)
+    ref = oracle.OracleLayer(port_kernels, "dense", N, H, Mc, 0.1, init, np.float64)
+    weights, bias = (rs.randn(N, H * Mc) / np.sqrt(N)).astype(dtype), (0.1 * rs.randn(H * Mc)).astype(dtype)
+    x = rs.rand(B, N).astype(dtype)
+    for layer in (dev, ref):
+        layer.weights, layer.bias = weights.astype(layer.dtype), bias.astype(layer.dtype)
+    launches = lib.sbb_kernel_launches()
+    got = dev.compute_activation(x)
+    launches = lib.sbb_kernel_launches() - launches
+    assert rel_inf(got, ref.compute_activation(x.astype(np.float64))) < TOL[np.dtype(dtype)]
+    return launches
+
+
+@pytest.mark.parametrize("B,N,H,Mc,one_launch", [
+    (8, 20000, 1, 10, True), (256, 32768, 1, 7, True), (257, 600, 1, 7, False), (64, 8192, 1, 8, True), (65, 8192, 1, 8, False),
+    (128, 8192, 2, 5, True), (129, 8192, 2, 5, False), (131, 5000, 1, 11, True), (132, 5000, 1, 11, False), (8, 9001, 3, 5, True),
+    (64, 8192, 7, 2, True), (64, 8193, 7, 2, False), (65, 2016, 1, 13, True), (65, 2017, 1, 13, False), (8, 640, 2, 8, False)])
+def test_float64_forward_of_few_units_on_both_sides_of_its_rule(port_kernels, B, N, H, Mc, one_launch):
+    """One launch where the kernel for layers of few units is the faster one, a product in tiles and a softmax elsewhere."""
+    launches = _forward_and_launches(port_kernels, np.float64, B, N, H, Mc)
+    assert (launches == 1) == one_launch, launches
+
+
 @pytest.mark.parametrize("B,N,H,Mc,scale", [(1, 128, 3, 12, 1.0), (16, 256, 2, 128, 1.0), (255, 260, 4, 65, 1.0),
                                             (256, 516, 33, 8, 1.0), (257, 252, 7, 36, 1e-5), (300, 600, 1, 260, 300.0),
                                             (2049, 132, 3, 88, 1.0), (40, 140, 80, 4, 1.0), (530, 257, 3, 40, 1.0)])
