@@ -266,13 +266,22 @@ struct PhaseTimer {
 // float32 layer that learns from its own activations a difference in the last digit of an activation reaches the weights
 // of all its inputs alike and adds up over them in the next forward pass, by a factor of some N taupdt / 10, and taupdt grows
 // with the root of the batch.  Where that is large those keep their order (4096 -> 32 at batch 512 moved 6e-5 in two steps), and
-// where the forward pass is the slower one: its reads of the weights take M lines of memory for each of M units.  (Two launches
-// a step instead of four: 206 -> 9 units at batch 44 27 -> 17 us, 72 -> 16 at 41 33 -> 18, 1024 -> 24 at 58 42 -> 27; but 1211 -> 30
-// at 400 44 -> 40, 3333 -> 32 at 57 42 -> 113.)
+// where the tiles are the faster ones.  Measured at 16 to 4096 inputs, 2 to 32 units, 8 to 5000 samples, us a step, here in two
+// launches and there in four: up to 8 units here (512 -> 8 at 400 13 and 20); up to 16 too (206 -> 9 at 44 8 and 14), but not
+// where a warp has a sample and its inputs for itself and those are many (512 -> 9 at 593 22 and 16, 400 -> 9 at 400 13.8 and 16.1);
+// more units up to 200 samples (206 -> 32 at 128 14 and 16, 1024 -> 24 at 44 13 and 19), then only against the tensor-core
+// kernels, which such a step waits 6 us longer for than for the others (300 -> 28 at 296 19 and 27; 300 -> 31 at 296 19 and 15), or with
+// few inputs and a long batch (64 -> 31 at 2048 19 and 21, at 400 16 and 13).  32 units are rows of 128 bytes, which a warp reads one by
+// one: 206 -> 32 at 400 42 and 18.
 template <typename T>
 bool narrow(const sbb_layer *L, long B) {
   if (std::is_same<T, double>::value || L->desc.kind == SBB_LAYER_DENSE) return true;
-  return L->N <= 4096 && L->M <= 32 && L->N * L->N * B <= (1l << 28) && L->M * L->M * (L->N / 256 + 1) <= 3000;
+  const long N = L->N, M = L->M;
+  if (N > 4096 || M > 32 || N * N * B > (1l << 28) || M * M * (N / 256 + 1) > 3000) return false;
+  if (M <= 8 || B <= 200) return true;
+  const bool tc = g_path == SBB_PATH_TENSOR && N % 4 == 0 && M % 4 == 0;
+  if (N > 64 && sbb::narrow_alone(B, N)) return (M <= 16 && N * M <= 4096) || (tc && (M < 16 || (M < 32 && N <= 128)));
+  return M <= 16 || (tc && M < 32) || (N <= 64 && B >= 1024);
 }
 
 template <typename T>

@@ -68,6 +68,7 @@ cudaError_t launch_column_vectors(const ColumnVectors<T> &x, const ColumnVectors
                                   BiasParams<T> bias, cudaStream_t st);
 bool narrow_layer(long N, long M);
 bool narrow_forward(long B, long N, long M, size_t elem);
+bool narrow_alone(long B, long N);   // the forward pass gives a sample to one warp instead of a block
 template <typename T>
 cudaError_t launch_narrow_forward(const T *x, const T *W, const T *bias, T *out, long B, long N, long M, long Mc,
                                   cudaStream_t st);

@@ -335,10 +335,10 @@ cudaError_t forward_mp(const T *x, const T *W, const T *bias, T *out, long B, lo
   const long per = (B + 295) / 296;
   unsigned ranks = B <= 18 ? 8 : B <= 37 ? 4 : B <= 74 ? 2 : 1;   // (one sample a block then, on SMs of their own)
   while (ranks > 1 && N < 512 * (long)ranks) ranks /= 2;
-  const bool alone = N <= 64 || (N <= 512 && per > 1);   // (500 -> 31 at batch 128, a step: 37 us alone, 25 shared)
+  const bool alone = narrow_alone(B, N);
 #define SBB_NARROW_FWD(R)                                                                                              \
   do {                                                                                                                 \
-    if (alone) /* not enough inputs to share among the warps of a block, or samples enough without */                  \
+    if (alone)                                                                                                         \
       launch_next(narrow_forward_kernel<T, MP, R, 1>, (unsigned)((B + 8 * R - 1) / (8 * R)), 256, 0, st, x, W, bias, out, B, (int)N, (int)M, (int)Mc); \
     else if (ranks > 1)                                                                                                \
       launch_clusters(narrow_forward_kernel<T, MP, R, 8>, dim3((unsigned)((B + R - 1) / R), ranks), dim3(1, ranks, 1), 256, 0, st, x, W, bias, out, B, (int)N, (int)M, (int)Mc); \
@@ -358,6 +358,9 @@ cudaError_t forward_mp(const T *x, const T *W, const T *bias, T *out, long B, lo
 // Up to 32 units; beyond that the tiles of the contraction kernels are full enough.  The forward pass reads all weights
 // once per block of samples: with very many samples that is more L2 traffic than the tiled kernels cause.
 bool narrow_layer(long N, long M) { return M <= 32 && N < (1l << 30); }
+// Not enough inputs to share among the warps of a block, or samples enough without (500 -> 31 at batch 128, a step: 37 us alone,
+// 25 shared).
+bool narrow_alone(long B, long N) { return N <= 64 || (N <= 512 && B > 296); }
 bool narrow_forward(long B, long N, long M, size_t elem) {
   // float64: a block of one sample reads all weights 8 bytes at a time, rows apart, and the cost grows with samples x inputs; the
   // tiles of the FP64 tensor-core kernel read them once but wait for more inputs one after the other.  Where the line lies

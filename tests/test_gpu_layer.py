@@ -622,6 +622,40 @@ def test_float64_forward_of_few_units_on_both_sides_of_its_rule(port_kernels, B,
     assert (launches == 1) == one_launch, launches
 
 
+@pytest.mark.parametrize("B,N,H,Mc,general,tensor", [
+    (400, 206, 1, 32, False, False), (297, 512, 2, 12, False, False), (400, 128, 3, 8, False, True), (593, 512, 3, 3, False, False),
+    (593, 448, 3, 3, True, True), (400, 512, 1, 12, False, True), (200, 300, 1, 31, True, True), (201, 300, 1, 31, False, False),
+    (201, 300, 4, 7, False, True), (1024, 64, 1, 32, True, True), (1023, 64, 8, 4, False, False), (1023, 64, 7, 4, False, True),
+    (2000, 300, 4, 2, True, True), (80, 1535, 3, 7, True, True), (80, 1792, 3, 7, False, False)])
+def test_float32_steps_of_few_units_on_both_sides_of_their_rule(port_kernels, contraction_path, B, N, H, Mc, general, tensor):
+    """A float32 layer that learns from its own activations: two launches a step where the kernels for layers of few units
+    are the faster ones, which depends on what the other way is; the same step either way."""
+    import streambrain_b200 as B200
+    from streambrain_b200._lib import lib
+    hp = dict(khalf=-100.0, pmin=0.05, taubdt=0.02, density=0.5)
+    init = (0.5, 1 / Mc, 0.5 / Mc)
+    np.random.seed(5)
+    dev = B200.StructuralPlasticityLayer(N, H, Mc, 0.02, hp["khalf"], hp["pmin"], hp["taubdt"], hp["density"], 16, init, dtype=np.float32)
+    ref = oracle.OracleLayer(port_kernels, "plastic", N, H, Mc, 0.02, init, np.float32, **hp)
+    ref.wmask = dev.wmask
+    rs = np.random.RandomState(B + N)
+    dev.weights = (0.05 * rs.randn(N, H * Mc)).astype(np.float32)
+    for name in ("weights", "bias"):
+        setattr(ref, name, getattr(dev, name))
+    x = rs.rand(B, N).astype(np.float32)
+    tol = TOL[np.dtype(np.float32)]
+    launches = lib.sbb_kernel_launches()
+    y = dev.compute_activation(x)
+    dev.train_step(x, y, None)
+    launches = lib.sbb_kernel_launches() - launches
+    assert (launches == 2) == (tensor if contraction_path == "tensor" else general), launches
+    assert rel_inf(y, ref.compute_activation(x)) < 10 * tol
+    ref.train_step(x, y, None)
+    for name in ("Ci", "Cj", "Cij", "bias"):
+        assert rel_inf(getattr(dev, name), getattr(ref, name)) < tol, name
+    assert weight_err(dev.weights, ref.weights) < 10 * tol
+
+
 @pytest.mark.parametrize("B,N,H,Mc,scale", [(1, 128, 3, 12, 1.0), (16, 256, 2, 128, 1.0), (255, 260, 4, 65, 1.0),
                                             (256, 516, 33, 8, 1.0), (257, 252, 7, 36, 1e-5), (300, 600, 1, 260, 300.0),
                                             (2049, 132, 3, 88, 1.0), (40, 140, 80, 4, 1.0), (530, 257, 3, 40, 1.0)])
