@@ -325,8 +325,9 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Samples a thread can keep sums for: 64 registers of them.
-constexpr int narrow_samples(long M, size_t elem) { return (M <= 8 ? 8 : (M <= 16 ? 4 : 2)) / (elem == 8 ? 2 : 1); }
+// Samples a thread keeps sums for: 64 registers of them in float32; one in float64 (narrow_forward admits no batch that would
+// share its reads of the weights).
+constexpr int narrow_samples(long M, size_t elem) { return elem == 8 ? 1 : M <= 8 ? 8 : M <= 16 ? 4 : 2; }
 
 template <typename T, int MP>
 cudaError_t forward_mp(const T *x, const T *W, const T *bias, T *out, long B, long N, long M, long Mc, cudaStream_t st) {
@@ -376,7 +377,7 @@ bool narrow_forward(long B, long N, long M, size_t elem) {
     if (B <= kFewSamples) return M <= 7 ? N <= 32768 : M <= 11 && N <= 8192;
     return B * N <= (M <= 7 ? 1l << 23 : M == 8 ? 1l << 19 : M <= 10 ? 1l << 20 : M == 11 ? 5l << 17 : B <= 64 ? 1l << 19 : 1l << 17);
   }
-  const long r = narrow_samples(M, elem);
+  const long r = narrow_samples(M, 4);
   return narrow_layer(N, M) && ((B + r - 1) / r) * N * M <= (1l << 28);
 }
 
@@ -384,8 +385,12 @@ template <typename T>
 cudaError_t launch_narrow_forward(const T *x, const T *W, const T *bias, T *out, long B, long N, long M, long Mc,
                                   cudaStream_t st) {
   if (M <= 8) return forward_mp<T, 8>(x, W, bias, out, B, N, M, Mc, st);
-  if (M <= 16) return forward_mp<T, 16>(x, W, bias, out, B, N, M, Mc, st);
-  return forward_mp<T, 32>(x, W, bias, out, B, N, M, Mc, st);
+  if constexpr (sizeof(T) == 8) {
+    return M <= 16 ? forward_mp<T, 16>(x, W, bias, out, B, N, M, Mc, st) : cudaErrorNotSupported;
+  } else {
+    if (M <= 16) return forward_mp<T, 16>(x, W, bias, out, B, N, M, Mc, st);
+    return forward_mp<T, 32>(x, W, bias, out, B, N, M, Mc, st);
+  }
 }
 template cudaError_t launch_narrow_forward<float>(const float *, const float *, const float *, float *, long, long, long, long,
                                                   cudaStream_t);
