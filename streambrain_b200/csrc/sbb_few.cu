@@ -192,7 +192,7 @@ bool few_plan(const void *W, long B, long N, long H, long Mc, FewPlan &p) {
   p.chunks = (int)((H + hcs - 1) / hcs);
   // two blocks per SM, at least sixteen inputs per thread
   const long groups = kFewThreads / p.lanes;
-  long ranges = (296 + p.chunks - 1) / p.chunks;
+  long ranges = (2 * sm_count() + p.chunks - 1) / p.chunks;
   const long most_ranges = (N + 16 * groups - 1) / (16 * groups);
   if (ranges > most_ranges) ranges = most_ranges;
   if (ranges > 64) ranges = 64;

@@ -677,7 +677,6 @@ static TracePairs to_pairs(const TraceEpilogue<double> &e) {
   return t;
 }
 
-static int sm_count();
 
 constexpr size_t kMostSmem = 232448;   // of one block; an SM has 1 KB more, and every block takes 1 KB besides its own
 
@@ -823,17 +822,16 @@ static cudaError_t launch_contraction(const T *A, long lda, const T *Bm, long ld
 // ----------------------------------------------------------------------------
 // Forward product (split over k so that small batches still fill the GPU).
 // ----------------------------------------------------------------------------
-static int g_sm_count = 0;
-static int sm_count() {
-  if (g_sm_count == 0) {
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0)
-      g_sm_count = n;
-    else
-      g_sm_count = 148;
+int sm_count() {
+  static std::atomic<int> known{0};
+  int n = known.load(std::memory_order_relaxed);
+  if (n == 0) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+      n = 148;
+    known.store(n, std::memory_order_relaxed);
   }
-  return g_sm_count;
+  return n;
 }
 
 // k-splits of the forward product.  float32: output tiles of 128 x 128 until two CTAs per SM are busy, at least eight slabs

@@ -21,6 +21,7 @@ template <typename T>
 TraceParams<T> make_trace_params(double taupdt, double cthr, long batch);
 
 unsigned long long kernel_launches();
+int sm_count();   // of the first device the process asks for (148 where there is none)
 
 // Number of K-splits the forward product uses for a [B,N]x[N,M] problem and the
 // number of REALs of scratch (splits*B*M) it needs.

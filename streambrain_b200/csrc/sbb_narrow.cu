@@ -333,8 +333,8 @@ template <typename T, int MP>
 cudaError_t forward_mp(const T *x, const T *W, const T *bias, T *out, long B, long N, long M, long Mc, cudaStream_t st) {
   constexpr int RMAX = narrow_samples(MP, sizeof(T));
   // few samples: one per block (or warp), so that all SMs take part; more of them share each read of the weights
-  const long per = (B + 295) / 296;
-  unsigned ranks = B <= 18 ? 8 : B <= 37 ? 4 : B <= 74 ? 2 : 1;   // (one sample a block then, on SMs of their own)
+  const long sms = sm_count(), per = (B + 2 * sms - 1) / (2 * sms);
+  unsigned ranks = B * 8 <= sms ? 8 : B * 4 <= sms ? 4 : B * 2 <= sms ? 2 : 1;   // (one sample a block then, on SMs of their own)
   while (ranks > 1 && N < 512 * (long)ranks) ranks /= 2;
   const bool alone = narrow_alone(B, N);
 #define SBB_NARROW_FWD(R)                                                                                              \
@@ -361,7 +361,7 @@ cudaError_t forward_mp(const T *x, const T *W, const T *bias, T *out, long B, lo
 bool narrow_layer(long N, long M) { return M <= 32 && N < (1l << 30); }
 // Not enough inputs to share among the warps of a block, or samples enough without (500 -> 31 at batch 128, a step: 37 us alone,
 // 25 shared).
-bool narrow_alone(long B, long N) { return N <= 64 || (N <= 512 && B > 296); }
+bool narrow_alone(long B, long N) { return N <= 64 || (N <= 512 && B > 2 * sm_count()); }
 bool narrow_forward(long B, long N, long M, size_t elem) {
   // float64: a block of one sample reads all weights 8 bytes at a time, rows apart, and the cost grows with samples x inputs; the
   // tiles of the FP64 tensor-core kernel read them once but wait for more inputs one after the other.  Where the line lies
@@ -404,7 +404,8 @@ cudaError_t launch_narrow_train(const T *x, const T *y, long B, long N, long M, 
   // Clusters where they find SMs of their own and every block a stage of samples: 664 inputs, float64, batch 5453 89 -> 29 us,
   // 300 inputs, float32, batch 1024 14.3 -> 6.8; without that room they lose (3000 inputs at batch 1024 21 -> 46 in eights).
   const long stages = (B + 127) / 128;
-  const int cl = blocks * 8 <= 148 && stages >= 8 ? 8 : blocks * 4 <= 148 && stages >= 4 ? 4 : blocks * 2 <= 148 && stages >= 4 ? 2 : 1;
+  const long sms = sm_count();
+  const int cl = blocks * 8 <= sms && stages >= 8 ? 8 : blocks * 4 <= sms && stages >= 4 ? 4 : blocks * 2 <= sms && stages >= 4 ? 2 : 1;
 #define SBB_NARROW_TRAIN(MP)                                                                                            \
   do {                                                                                                                  \
     if (cl == 8)                                                                                                        \
