@@ -136,6 +136,32 @@ def test_softmax_at_the_edges_of_its_slots(k, tag, dtype, Mc):
 
 
 @pytest.mark.parametrize("tag,dtype", DTYPES)
+@pytest.mark.parametrize("rows", [1, 67])
+@pytest.mark.parametrize("Mc", [1, 2, 3, 4, 5, 8, 9, 15, 16])
+def test_softmax_of_small_groups_with_special_values(k, tag, dtype, Mc, rows):
+    """A lane per unit, several groups to a warp: zeros, infinities and NaNs in one group stay out of its neighbours, and every
+    group is the same to the bit as by the kernel for groups of any size."""
+    rs = np.random.RandomState(Mc)
+    H = 11
+    a = (rs.randn(rows * H, Mc) * 3).astype(dtype)
+    a[1] = 0
+    a[2, ::2], a[2, 1::2] = 0, -0.0
+    a[3, -1] = np.inf
+    a[4, 0] = np.nan
+    a[5] = -np.inf
+    a[6, :-1] = -np.inf
+    a[7] = 1e30
+    a[8, Mc // 2] = -np.nan
+    a[9, 1:] = -np.inf
+    wide = np.full((rows * H, 544), -np.inf, dtype=dtype)
+    wide[:, :Mc] = a
+    got = k.softmax_minicolumns(a.reshape(rows, H * Mc).copy(), H, Mc).reshape(rows * H, Mc)
+    want = k.softmax_minicolumns(wide, 1, 544)[:, :Mc]
+    assert np.array_equal(got, want, equal_nan=True)
+    assert np.isfinite(got[[0, 1, 2, 7, 10]]).all() and np.isnan(got[[4, 5, 8]]).all()
+
+
+@pytest.mark.parametrize("tag,dtype", DTYPES)
 @pytest.mark.parametrize("B,N,H,Mc", SHAPES)
 def test_trace_update_vs_oracle(k, port_kernels, tag, dtype, B, N, H, Mc):
     rs = np.random.RandomState(B * 11 + N)

@@ -622,6 +622,17 @@ def test_float64_forward_of_few_units_on_both_sides_of_its_rule(port_kernels, B,
     assert (launches == 1) == one_launch, launches
 
 
+@pytest.mark.parametrize("tag,dtype", DTYPES)
+@pytest.mark.parametrize("B,N,H,Mc", [(1, 4096, 1, 10), (18, 4097, 2, 5), (5, 8191, 1, 7), (19, 4100, 1, 3), (18, 2048, 1, 8),
+                                      (37, 2049, 3, 3), (18, 1024, 1, 9), (38, 1024, 1, 10), (74, 1027, 5, 2), (74, 9001, 1, 7),
+                                      (75, 5000, 1, 9), (18, 1023, 1, 10), (17, 5000, 1, 32), (36, 2050, 2, 16), (40, 1025, 4, 5)])
+def test_forward_of_few_units_in_clusters(port_kernels, tag, dtype, B, N, H, Mc):
+    """Eight, four or two blocks share the inputs of a sample, whole and ragged parts; one block where samples or inputs are
+    one too many or too few."""
+    launches = _forward_and_launches(port_kernels, dtype, B, N, H, Mc)
+    assert launches == 1 or (tag == "f64" and H * Mc > 11), launches
+
+
 @pytest.mark.parametrize("B,N,H,Mc,general,tensor", [
     (400, 206, 1, 32, False, False), (297, 512, 2, 12, False, False), (400, 128, 3, 8, False, True), (593, 512, 3, 3, False, False),
     (593, 448, 3, 3, True, True), (400, 512, 1, 12, False, True), (200, 300, 1, 31, True, True), (201, 300, 1, 31, False, False),
