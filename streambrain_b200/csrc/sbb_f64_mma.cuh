@@ -141,7 +141,7 @@ __device__ __forceinline__ double log_positive(double x) {
 // k-split z covers [z*kper, min(K, (z+1)*kper)), kper a multiple of BK.  The epilogue receives the thread's
 // accumulators: ep.tile(acc, m, n, z) with acc[mi][ni][e] = output element (m + 8*mi, n + 8*ni + e), n even;
 // ep.prefetch(m, n, lane) is called before the main loop with the first element of the warp's 32 x 32 block.  Epilogue::LATE:
-// the kernel before this one in the stream does not write what the main loop reads.
+// the kernel before this one in the stream does not write what the main loop and ep.prefetch read (A, B, the old traces).
 template <bool A_KMAJOR, int BM, bool DEEP, int V, class Epilogue>
 __global__ void __launch_bounds__(Cfg<BM>::THREADS, Cfg<BM, DEEP>::CTAS_PER_SM)
     contraction_kernel(const double *__restrict__ A, long lda, const double *__restrict__ Bm, long ldb, long Mdim,

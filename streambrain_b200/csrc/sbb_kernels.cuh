@@ -88,7 +88,9 @@ cudaError_t launch_few_forward(const T *x, const T *W, const T *bias, T *out, lo
 // Fused trace step for rows [row_begin,row_end) of Cij: acc = x^T y over the batch,
 // Cij = EMA(Cij, acc), w = log-ratio(Cij, Ci, Cj) with rows/columns below cthr and
 // masked connections (wmask may be null) set to zero.  Ci, Cj hold the NEW values; rci, rcj (float64 only) their
-// reciprocals, 0 below the threshold.
+// reciprocals, 0 below the threshold.  A kernel directly ahead of it on `st` may write Ci, Cj, their reciprocals and the mask but
+// none of x, y and Cij, which the float64 kernel reads before that kernel has ended (sbb_launch.cuh); a copy ahead of it, or any
+// older work, may write all of them.
 template <typename T>
 cudaError_t launch_trace_update_fused(const T *x, const T *y, long B, long N, long M, long H, long Mc, const T *Ci,
                                       const T *Cj, const T *rci, const T *rcj, T *Cij, T *w, const uint8_t *wmask,

@@ -7,6 +7,10 @@ namespace sbb {
 // First statement of a kernel that launch_next starts, ahead of every access to global memory: waits until the kernels
 // before it in the stream have ended and what they wrote is visible, then lets the next kernel's blocks take the places that
 // this kernel's leave.  Every kernel of a chain waits, so each has all its predecessors behind it.
+// Two kernels wait later, only ahead of what the kernel directly before them in the stream writes: the trace updates of
+// sbb_tc_trace.cu and sbb_f64_mma.cuh, whose products and old traces do not depend on the column vectors formed there.
+// All that is older has ended before their blocks may start, because the kernel before let them start only after its own
+// wait.  Their launchers' declarations say what that kernel may not write.
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -28,6 +28,8 @@ cudaError_t launch_forward_product_tc(const float *x, const float *w, float *par
 
 // Fused trace step: Cij = moving average of x^T y / B, w = log(Cij / (Ci Cj)) under the mask (null: none), from the
 // reciprocals of the new Ci and Cj (0 where the trace is below the threshold).  x: N columns of rows `ldx` apart.
+// A kernel directly ahead of it on `st` may write the reciprocals and the mask but none of x, y and Cij, which are read before
+// that kernel has ended (sbb_launch.cuh); a copy ahead of it, or any older work, may write all of them.
 cudaError_t launch_trace_update_tc(const float *x, long ldx, const float *y, long B, long N, long M, long H, const float *rci,
                                    const float *rcj, float *Cij, float *w, const uint8_t *wmask, TraceParams<float> p,
                                    cudaStream_t st);
