@@ -4,11 +4,14 @@
 #include <chrono>
 #include <condition_variable>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <exception>
 #include <mutex>
 #include <thread>
 #include <vector>
+
+#include <sched.h>
 
 #ifdef __SSE2__
 #include <emmintrin.h>
@@ -17,7 +20,8 @@
 namespace sbb {
 
 // One job at a time, cut into pieces that the caller and the workers claim one by one: whoever is late, for a worker still
-// waking up, finds nothing left.  Workers spin for a while after a job (a copy is a series of jobs) before they sleep.
+// waking up, finds nothing left.  Workers spin for 200 us after a job (a copy is a series of jobs) before they sleep.  Up to 11
+// of them, and no more than the process's share of three quarters of the machine's hardware threads leaves beside the caller.
 class CopyThreads {
  public:
   static CopyThreads &get() {
@@ -75,8 +79,19 @@ class CopyThreads {
 #endif
     std::memcpy(dst, src, bytes);
   }
+  // Hardware threads this process may count on: those it is bound to, and an even part of the machine's where a launcher says
+  // that it started several processes here (eight of them with eleven spinning threads each would take the cores from one another).
+  static unsigned share() {
+    unsigned n = std::thread::hardware_concurrency();
+    const char *e = std::getenv("LOCAL_WORLD_SIZE");
+    const long processes = e != nullptr ? std::strtol(e, nullptr, 10) : 1;
+    if (processes > 1) n = (unsigned)(n / processes);
+    cpu_set_t bound;
+    if (sched_getaffinity(0, sizeof(bound), &bound) == 0 && (unsigned)CPU_COUNT(&bound) < n) n = (unsigned)CPU_COUNT(&bound);
+    return n;
+  }
   CopyThreads() {
-    unsigned n = std::thread::hardware_concurrency() / 4 * 3;
+    unsigned n = share() / 4 * 3;
     if (n > 12) n = 12;
     try {   // (a process may be out of threads or memory: the callers then copy with those there are, or by themselves)
       for (unsigned k = 1; k < n; ++k) workers_.emplace_back([this] { work(); });

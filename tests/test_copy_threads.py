@@ -16,10 +16,13 @@ PROGRAM = r"""
 #include <pthread.h>
 #include "sbb_copy_threads.h"
 
+static std::atomic<int> asked{0};
+
 // The system's limit on threads, in place of the real call: the first THREADS_ALLOWED succeed.
 extern "C" int pthread_create(pthread_t *t, const pthread_attr_t *a, void *(*f)(void *), void *arg) {
   static std::atomic<int> left{std::getenv("THREADS_ALLOWED") ? std::atoi(std::getenv("THREADS_ALLOWED")) : 1 << 20};
   if (left.fetch_sub(1) <= 0) return EAGAIN;
+  asked.fetch_add(1);
   typedef int (*Create)(pthread_t *, const pthread_attr_t *, void *(*)(void *), void *);
   static const Create real = reinterpret_cast<Create>(dlsym(RTLD_NEXT, "pthread_create"));
   return real(t, a, f, arg);
@@ -42,7 +45,7 @@ static bool copies(unsigned seed) {
 }
 int main(int argc, char **) {
   if (!copies(1)) return 1;   // (the first copy starts the threads)
-  if (argc > 1) return 0;
+  if (argc > 1) return std::printf("%d", asked.load()) < 0;
   std::atomic<int> bad{0};
   std::vector<std::thread> callers;
   for (unsigned k = 0; k < 4; ++k) callers.emplace_back([&bad, k] { bad += !copies(k + 2); });
@@ -74,3 +77,24 @@ def test_copies_from_several_callers(program):
 def test_copies_without_the_threads_it_asked_for(program, allowed):
     run = subprocess.run([program, "one caller"], capture_output=True, text=True, timeout=120, env=dict(os.environ, THREADS_ALLOWED=str(allowed)))
     assert run.returncode == 0, run.stdout + run.stderr
+
+
+def test_processes_of_one_machine_share_its_threads(program):
+    """With the number of processes that a launcher started here, each takes its part of the threads, down to none."""
+    def workers(env):
+        run = subprocess.run([program, "one caller"], capture_output=True, text=True, timeout=120, env=env)
+        assert run.returncode == 0, run.stdout + run.stderr
+        return int(run.stdout)
+    env = {k: v for k, v in os.environ.items() if k != "LOCAL_WORLD_SIZE"}
+    alone = workers(env)
+    cores = os.cpu_count()
+    assert alone <= 11 and alone == max(0, min(12, min(cores, len(os.sched_getaffinity(0))) // 4 * 3) - 1)
+    assert workers(dict(env, LOCAL_WORLD_SIZE="1")) == alone
+    for processes in (2, 8):
+        part = workers(dict(env, LOCAL_WORLD_SIZE=str(processes)))
+        assert part <= alone and processes * (part + 1) <= max(processes, cores)
+    assert workers(dict(env, LOCAL_WORLD_SIZE=str(cores))) == 0
+    one = sorted(os.sched_getaffinity(0))[:1]
+    run = subprocess.run(["taskset", "-c", str(one[0]), program, "one caller"], capture_output=True, text=True, timeout=120, env=env) \
+        if shutil.which("taskset") else None
+    assert run is None or (run.returncode == 0 and int(run.stdout) == 0)
