@@ -8,6 +8,7 @@
 
 #include <cstdarg>
 #include <cstdlib>
+#include <new>
 #include <type_traits>
 #include <vector>
 #include <cstdio>
@@ -133,14 +134,34 @@ long host_rows(long N, size_t row_bytes, const void *Cij, const void *weights) {
 struct Scratch {
   void *d = nullptr;
   size_t cap = 0;
+  bool recorded = false;   // work that uses `d` is part of a captured graph, which may run at any time
+  struct Retired {
+    void *d;
+    Retired *next;
+  };
+  Retired *retired = nullptr;   // recorded buffers that a larger one has replaced
   int reserve(size_t n) {
     if (n <= cap) return SBB_OK;
-    if (d) SBB_CUDA(cudaFree(d));
+    if (d && recorded) {
+      Retired *const r = new (std::nothrow) Retired{d, retired};
+      if (r == nullptr) return fail(SBB_ERR_CUDA, "out of host memory");
+      retired = r;
+    } else if (d) {
+      SBB_CUDA(cudaFree(d));
+    }
     d = nullptr;
     cap = 0;
+    recorded = false;
     SBB_CUDA(cudaMalloc(&d, n));
     cap = n;
     return SBB_OK;
+  }
+  // To be called where work that uses the buffer is queued on `st`.
+  void used_on(cudaStream_t st) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (recorded || d == nullptr) return;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) (void)cudaGetLastError();
+    recorded = capture != cudaStreamCaptureStatusNone;
   }
   // For a workspace the caller can do without: false where the device has no room for it, or where it would have to grow
   // while `st` is being captured (an allocation would end the capture).
@@ -155,6 +176,13 @@ struct Scratch {
     if (d) cudaFree(d);
     d = nullptr;
     cap = 0;
+    recorded = false;
+    while (retired) {
+      Retired *const r = retired;
+      retired = r->next;
+      cudaFree(r->d);
+      delete r;
+    }
   }
 };
 
@@ -296,6 +324,7 @@ int layer_forward(sbb_layer *L, const T *x, long B, T *y, cudaStream_t st) {
   size_t few = 0;
   if (sbb::few_samples<T>(W, B, L->N, L->H, L->Mc, &few)) {
     SBB_TRY(L->fwd_partial.reserve(few * sizeof(T)));
+    L->fwd_partial.used_on(st);
     PhaseTimer timer(L, SBB_PHASE_FORWARD, st);
     SBB_CUDA(sbb::launch_few_forward<T>(x, W, static_cast<const T *>(L->state[SBB_STATE_BIAS]), y, B, L->N, L->H, L->Mc,
                                         static_cast<T *>(L->fwd_partial.d), static_cast<int *>(L->ticket.d) + 1, st));
@@ -309,6 +338,7 @@ int layer_forward(sbb_layer *L, const T *x, long B, T *y, cudaStream_t st) {
   T *partial = y;
   if (splits > 1) {
     SBB_TRY(L->fwd_partial.reserve((size_t)splits * B * L->M * sizeof(T)));
+    L->fwd_partial.used_on(st);
     partial = static_cast<T *>(L->fwd_partial.d);
   }
   PhaseTimer timer(L, SBB_PHASE_FORWARD, st);
@@ -374,6 +404,7 @@ int train_rows(sbb_layer *L, const T *x, const T *y, long B, long N, long M, lon
   if (N == 0) return SBB_OK;
   PhaseTimer timer(L, SBB_PHASE_TRACE, st);
   if (splits > 1) {
+    L->split_partial.used_on(st);
     T *const partial = static_cast<T *>(L->split_partial.d);
     if (tc) {
       if constexpr (std::is_same<T, float>::value) SBB_CUDA(sbb::launch_split_product_tc(x, y, B, N, M, splits, partial, st));
@@ -421,6 +452,7 @@ int layer_dp_local(sbb_layer *L, const T *x, const T *y, long B, T *delta, long 
     // the first row block of a step also forms the column sums and, for the tensor path, the operands' low parts,
     // which the later row blocks of the same step (same x, y, B) re-use
     SBB_TRY(reserve_lo<T>(L->lo, B, L->N, L->M, L->dp_fast, &lo));
+    L->lo.used_on(st);
     SBB_CUDA(sbb::launch_colsum<T>(x, B, L->N, delta, st, lo_as<T>(lo.x)));
     SBB_CUDA(sbb::launch_colsum<T>(y, B, L->M, delta + L->N, st, lo_as<T>(lo.y)));
     L->lo_batch = lo.x ? B : 0;
@@ -1350,6 +1382,7 @@ int shard_forward(sbb_layer *L, long B, T *support, cudaStream_t st) {
   T *partial = support;
   if (splits > 1) {
     SBB_TRY(L->fwd_partial.reserve((size_t)splits * Bg * M * sizeof(T)));
+    L->fwd_partial.used_on(st);
     partial = static_cast<T *>(L->fwd_partial.d);
   }
   PhaseTimer timer(L, SBB_PHASE_FORWARD, st);
@@ -1369,6 +1402,7 @@ int shard_activate(sbb_layer *L, long B, const T *support, T *y_local, cudaStrea
   auto &S = L->shard;
   const long Bg = B * S.world, M = L->M;
   SBB_TRY(S.yg.reserve((size_t)Bg * M * sizeof(T)));
+  S.yg.used_on(st);
   T *yg = static_cast<T *>(S.yg.d);
   SBB_CUDA(sbb::launch_reduce_bias_softmax<T>(support, 1, static_cast<const T *>(L->state[SBB_STATE_BIAS]), yg, Bg, L->H,
                                               L->Mc, 1, st));

@@ -964,3 +964,39 @@ def test_an_allocation_that_fails_is_reported_once(B200, tag, dtype):
     assert _lib.lib.sbb_layer_create(ctypes.byref(desc), ctypes.byref(handle)) == 2
     net.fit(x, y, 7, [(0, 1)])
     assert np.isfinite(layer.weights).all()
+
+
+@pytest.mark.parametrize("tag,dtype", DTYPES)
+@pytest.mark.parametrize("kind,B,N,H,Mc", [("plastic", 1500, 88, 2, 66), ("plastic", 2049, 65, 3, 13), ("plastic", 40, 700, 3, 100)])
+def test_captured_step_after_a_larger_batch(tag, dtype, kind, B, N, H, Mc):
+    """The workspaces that a captured step uses outlive their replacement by larger ones: the graph runs as before after the
+    layer has taken a batch of four times the size, and other memory is left alone."""
+    import torch
+    (eager, captured), batch = _twins(kind, N, H, Mc, dtype)
+    x, y = batch(B, 1)
+    large, large_y = batch(4 * B + 1, 2)
+
+    def step(layer):
+        a = layer.compute_activation(x)
+        layer.train_step(x, y, None)
+        return a
+    for layer in (eager, captured):
+        step(layer)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = step(captured)
+    for layer in (eager, captured):
+        layer.compute_activation(large)
+        layer.train_step(large, large_y, None)
+    torch.cuda.synchronize()
+    bystanders = [torch.full((n,), 7, dtype=torch.uint8, device="cuda") for n in (1 << 21, 1 << 22, 1 << 23) for _ in range(4)]
+    for _ in range(2):
+        want = step(eager)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+        _assert_same_step(captured, eager, dtype)
+        assert np.array_equal(captured.Cij, eager.Cij)
+    assert all(bool((b == 7).all()) for b in bystanders)
+    del graph
