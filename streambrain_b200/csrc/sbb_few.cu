@@ -47,7 +47,9 @@ __global__ void __launch_bounds__(kFewThreads)
   const bool active = g < groups && c < width;
   if constexpr (STREAM) {
     constexpr int U = 8;
-    constexpr int KT = sizeof(T) * R <= 16 ? 1024 : 512;   // inputs in shared memory at a time
+    // inputs in shared memory at a time; each fill begins with the first group of threads again, so a range of several fills that
+    // `groups` does not divide is summed in another order than from registers
+    constexpr int KT = sizeof(T) * R <= 16 ? 1024 : 512;
     __shared__ T s_x[R][KT];
     for (int t0 = k0; t0 < k1; t0 += KT) {
       const int t1 = min(k1, t0 + KT);
